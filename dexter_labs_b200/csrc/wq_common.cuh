@@ -73,6 +73,16 @@ __device__ __forceinline__ uint32_t dup_hi(uint32_t w) { return prmt(w, w, 0x323
 __device__ __forceinline__ float bf16lo_f32(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16hi_f32(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
 
+// Value 0..15 of logical row k, column n of an int4 weight in either layout.
+__device__ __forceinline__ uint32_t fetch_q4(const uint8_t* __restrict__ qw, int N, int half, int k, int n,
+                                             int relaid) {
+  const int plane = k < half ? 0 : 1;
+  const int r = k - plane * half;  // packed row
+  if (!relaid) return (qw[static_cast<long long>(r) * N + n] >> (4 * plane)) & 0xFu;
+  const uint32_t word = reinterpret_cast<const uint32_t*>(qw)[(static_cast<long long>(r & ~1) + plane) * (N >> 2) + (n >> 2)];
+  return (word >> (16 * (r & 1) + 4 * (n & 3))) & 0xFu;
+}
+
 __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
   uint32_t v;
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");

@@ -1066,43 +1066,6 @@ __global__ void wq_relayout_w4_kernel(const uint32_t* __restrict__ in, uint32_t*
   }
 }
 
-// Value 0..15 of logical row k, column n of an int4 weight in either layout.
-__device__ __forceinline__ uint32_t fetch_q4(const uint8_t* __restrict__ qw, int N, int half, int k, int n,
-                                             int relaid) {
-  const int plane = k < half ? 0 : 1;
-  const int r = k - plane * half;  // packed row
-  if (!relaid) return (qw[static_cast<long long>(r) * N + n] >> (4 * plane)) & 0xFu;
-  const uint32_t word = reinterpret_cast<const uint32_t*>(qw)[(static_cast<long long>(r & ~1) + plane) * (N >> 2) + (n >> 2)];
-  return (word >> (16 * (r & 1) + 4 * (n & 3))) & 0xFu;
-}
-
-// --------------------------------------------- dense dequantised weight dump
-// W[k,n] bf16 with the same bit-pattern arithmetic as the tensor-core kernel;
-// used to check the dequantisation bit for bit against the reference.
-template <int BITS>
-__global__ void wq_dequant_kernel(const uint8_t* __restrict__ qw, const __nv_bfloat16* __restrict__ scales,
-                                  const __nv_bfloat16* __restrict__ zeros, __nv_bfloat16* __restrict__ out,
-                                  int N, int K, int group, int relaid) {
-  const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const long long total = static_cast<long long>(K) * N;
-  if (idx >= total) return;
-  const int k = static_cast<int>(idx / N);
-  const int n = static_cast<int>(idx % N);
-  const int gi = k / group;
-  const uint32_t sbits = __bfloat16_as_ushort(scales[static_cast<long long>(gi) * N + n]);
-  if (BITS == 4) {
-    const uint32_t byte = fetch_q4(qw, N, K / 2, k, n, relaid);
-    const uint32_t z = zeros ? __bfloat16_as_ushort(zeros[static_cast<long long>(gi) * N + n]) : 0x4308u;
-    const uint32_t r = deq4(byte, z | (z << 16), sbits | (sbits << 16));
-    out[idx] = __ushort_as_bfloat16(static_cast<unsigned short>(r & 0xFFFFu));
-  } else {
-    const uint32_t byte = qw[idx];
-    const float cz = 8388608.0f + (zeros ? __bfloat162float(zeros[static_cast<long long>(gi) * N + n]) : 128.0f);
-    const float v = deq8(byte, 0, cz, __uint_as_float(sbits << 16));
-    out[idx] = __ushort_as_bfloat16(static_cast<unsigned short>(cvt_bf16x2(0.0f, v) & 0xFFFFu));
-  }
-}
-
 // ------------------------------------------------------ any-shape CUDA path
 // Plain CUDA-core kernel for shapes the tensor-core kernel does not take (N not
 // a multiple of 16, groups that are not a multiple of 64 rows, K/2 not a multiple
@@ -1808,36 +1771,6 @@ size_t dxb_fused_reduce_bytes(int world, int64_t capacity_elems) {
 void dxb_set_wait_limit_ms(int ms) {
   const long long tries = static_cast<long long>(ms < 1 ? 1 : ms) * 4000;
   dx::g_wait_tries.store(static_cast<unsigned>(tries > 4000000000ll ? 4000000000ll : tries));
-}
-
-int dxb_dequantize_ex(const void* qweight, const void* scales, const void* zeros, void* w_out, int N,
-                      int K, int group_size, int bits, int weight_layout, void* cuda_stream) {
-  using namespace dx;
-  if (bits != 4 && bits != 8) return DXB_ERR_BITS;
-  if (!qweight || !scales || !w_out) return DXB_ERR_NULL;
-  if (N <= 0 || K <= 0 || group_size <= 0 || K % group_size || (bits == 4 && K % 2))
-    return DXB_ERR_SHAPE;
-  if (weight_layout != DXB_LAYOUT_DEXTER && (weight_layout != DXB_LAYOUT_B200 || bits != 4 || K % 4 || N % 4))
-    return DXB_ERR_UNSUPPORTED;
-  cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
-  const long long total = static_cast<long long>(K) * N;
-  const int block = 256;
-  const unsigned grid = static_cast<unsigned>((total + block - 1) / block);
-  if (bits == 4)
-    wq_dequant_kernel<4><<<grid, block, 0, stream>>>(
-        static_cast<const uint8_t*>(qweight), static_cast<const __nv_bfloat16*>(scales),
-        static_cast<const __nv_bfloat16*>(zeros), static_cast<__nv_bfloat16*>(w_out), N, K, group_size,
-        weight_layout == DXB_LAYOUT_B200);
-  else
-    wq_dequant_kernel<8><<<grid, block, 0, stream>>>(
-        static_cast<const uint8_t*>(qweight), static_cast<const __nv_bfloat16*>(scales),
-        static_cast<const __nv_bfloat16*>(zeros), static_cast<__nv_bfloat16*>(w_out), N, K, group_size, 0);
-  return cudaGetLastError() == cudaSuccess ? DXB_OK : DXB_ERR_CUDA;
-}
-
-int dxb_dequantize(const void* qweight, const void* scales, const void* zeros, void* w_out, int N,
-                   int K, int group_size, int bits, void* cuda_stream) {
-  return dxb_dequantize_ex(qweight, scales, zeros, w_out, N, K, group_size, bits, DXB_LAYOUT_DEXTER, cuda_stream);
 }
 
 int dxb_uses_tensor_cores(int M, int N, int K, int group_size, int bits) {

@@ -1,0 +1,41 @@
+"""Packing and unpacking kernels against the tensor expressions they stand for."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def d(b200_lib):
+    import dexter_labs_b200
+
+    return dexter_labs_b200
+
+
+# (K, N, bits, group): whole spans, spans cut at the end, output widths around the tile of 128 and
+# off every alignment, one scale per channel, groups that no span covers
+SHAPES = [(256, 128, 4, 128), (512, 131, 4, 128), (384, 40, 4, 64), (192, 9, 4, 32), (640, 1, 4, 160),
+          (3072, 260, 4, 3072), (256, 1000, 8, 128), (384, 127, 8, 64), (96, 33, 8, 32), (1040, 200, 8, 1040),
+          (14336, 72, 8, 14336)]
+
+
+@pytest.mark.parametrize("symmetric", [True, False])
+@pytest.mark.parametrize("k,n,bits,group,layout", [s + ("dexter",) for s in SHAPES] + [
+    (256, 128, 4, 128, "b200"), (512, 132, 4, 64, "b200"), (192, 12, 4, 96, "b200"), (20, 7, 4, 5, "dexter"),
+    (9, 5, 8, 3, "dexter")])
+def test_dequantize_matches_the_oracle(k, n, bits, group, layout, symmetric, d, oracle):
+    gen = torch.Generator().manual_seed(k + n)
+    rows = k // 2 if bits == 4 else k
+    q = torch.randint(0, 256, (rows, n), generator=gen, dtype=torch.uint8)
+    s = (torch.rand(k // group, n, generator=gen) * 0.1).to(torch.bfloat16)
+    z = None
+    if not symmetric:
+        z = (torch.randint(0, 2 ** bits, s.shape, generator=gen) + (128 if bits == 4 else 0)).to(torch.bfloat16)
+    want = oracle.torch_dequantize(q, s, z, group, bits)
+    qg = q.cuda()
+    if layout == "b200":
+        qg = d.ops.relayout_w4(qg)
+    got = d.dequantize(qg, s.cuda(), None if z is None else z.cuda(), group, bits) if layout == "dexter" else \
+        d.ops.dequantize(qg, s.cuda(), None if z is None else z.cuda(), group, bits, layout=layout)
+    assert np.array_equal(got.cpu().view(torch.int16).numpy(), want.view(torch.int16).numpy())
