@@ -60,6 +60,9 @@ SIGNATURES = {
     "dxb_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
     "dxb_dequantize": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                c_void_p]),
+    "dxb_quantize_scratch_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
+    "dxb_quantize": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
+                             c_int, c_void_p]),
     "dxb_uses_tensor_cores": (c_int, [c_int, c_int, c_int, c_int, c_int]),
     "dxb_read_status": (c_int, [c_void_p, c_void_p]),
     "dxb_strerror": (c_char_p, [c_int]),

@@ -162,9 +162,359 @@ static int launch_dequant(const void* qweight, const void* scales, const void* z
   return cudaGetLastError() == cudaSuccess ? DXB_OK : DXB_ERR_CUDA;
 }
 
+// -------------------------------------------------------------------- quantise
+// Packs a dense bf16 weight [N, K] (nn.Linear style): per group of `group` consecutive k and per
+// output n an fp32 scale (and zero point), codes round(w / scale + shift) clamped to the grid, the
+// codes transposed to [K, N] (int8) or [K/2, N] (int4, row i low and row i + K/2 high nibble).
+//
+// 2 bytes read and bits/8 written per weight, once each; bound by instruction issue (int4 14336 x 3072:
+// 43 us with about 20 instructions per weight, 931 us as element-wise passes; the copy alone would
+// take 17 us).  One CTA packs 128 outputs x
+// two spans of 128 k (for int4 the two spans share their packed rows: k and k + K/2).  A half warp
+// reads one output's span with one 16-byte load per lane (256 B runs), finds the group's extremes
+// by shuffles in packed bf16, codes its 8 values in registers, and four outputs make the 32-bit
+// words of the transposed tile, which goes through shared memory (swizzled: no bank conflicts) to
+// leave as whole 128-byte rows.
+//
+// Arithmetic, in the order of the framework's tensor expressions on this device (so the bytes
+// are those of that chain of element-wise passes): all fp32; division by a constant is
+// multiplication by its rounded reciprocal, division by the scale is an exact division; rounding
+// to nearest even.  The codes get there without dividing: a product with the reciprocal of
+// the scale is within 2e-4 of the quotient's own rounded sum while that is at most 512, so only values that
+// close to a rounding boundary (4 in 10 000, or far outside the grid) take the division.
+struct QuantGrid {
+  float levels, inv_levels, mid;
+  bool symmetric;
+};
+template <int BITS>
+__device__ __forceinline__ QuantGrid quant_grid(bool symmetric) {
+  constexpr float levels = BITS == 4 ? 15.0f : 255.0f;
+  return QuantGrid{levels, 1.0f / levels, BITS == 4 ? 8.0f : 128.0f, symmetric};
+}
+// A clamp that lets NaN through, as the tensor library's does.
+__device__ __forceinline__ float clamp_nan(float v, float lo, float hi) {
+  return v != v ? v : fminf(fmaxf(v, lo), hi);
+}
+// Scale and shift of a group from its extremes (symmetric: hi = largest magnitude).
+__device__ __forceinline__ void quant_scale(const QuantGrid& g, float lo, float hi, float& scale, float& shift) {
+  if (g.symmetric) {
+    const float peak = hi != hi ? hi : fmaxf(hi, 1e-8f);
+    scale = __fmul_rn(__fmul_rn(2.0f, peak), g.inv_levels);
+    shift = g.mid;
+  } else {
+    const float s = __fmul_rn(__fsub_rn(hi, lo), g.inv_levels);
+    scale = s != s ? s : fmaxf(s, 1e-8f);
+    shift = clamp_nan(rintf(__fdiv_rn(-lo, scale)), 0.0f, g.levels);
+  }
+}
+// Packed-bf16 max / min that let NaN through.
+__device__ __forceinline__ uint32_t max2_nan(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("max.NaN.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+__device__ __forceinline__ uint32_t min2_nan(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("min.NaN.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+__device__ __forceinline__ float max_halves(uint32_t v) {
+  return __uint_as_float(max2_nan(v, prmt(v, v, 0x1032u)) << 16);
+}
+__device__ __forceinline__ float min_halves(uint32_t v) {
+  return __uint_as_float(min2_nan(v, prmt(v, v, 0x1032u)) << 16);
+}
+
+__device__ __forceinline__ float rcp_approx(float v) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
+// One value's code by exact division.
+__device__ __forceinline__ uint32_t quant_code(const QuantGrid& g, float w, float scale, float shift) {
+  const float r = rintf(__fadd_rn(__fdiv_rn(w, scale), shift));
+  return static_cast<uint32_t>(static_cast<uint8_t>(clamp_nan(r, 0.0f, g.levels)));
+}
+// Codes of a lane's 8 values, eight bytes in k order.  Rounding is an addition of 1.5 * 2^23, whose sum
+// carries the integer in its low bits: no conversion instructions, which run at a quarter of the rate.
+// `inside`: every value's exact sum lies on the grid or within half a step of it, so that no code
+// needs clamping unless it is as close to a rounding boundary as sends it to the exact path.
+__device__ __forceinline__ uint2 quant_code8(const QuantGrid& g, const uint32_t (&x)[4], float scale, float inv,
+                                             float shift, bool inside) {
+  constexpr float kMagic = 12582912.0f, kFar = 0.4998f;
+  float far = 0.0f;  // largest distance from a whole number
+  uint32_t c[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float t = __fmaf_rn((j & 1) ? bf16hi_f32(x[j >> 1]) : bf16lo_f32(x[j >> 1]), inv, shift);
+    const float m = __fadd_rn(t, kMagic);
+    c[j] = __float_as_uint(m);
+    far = fmaxf(far, fabsf(__fsub_rn(t, __fsub_rn(m, kMagic))));
+  }
+  if (!inside || far > kFar) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float w = (j & 1) ? bf16hi_f32(x[j >> 1]) : bf16lo_f32(x[j >> 1]);
+      const float t = __fmaf_rn(w, inv, shift);
+      if (!inside || fabsf(__fsub_rn(t, __fsub_rn(__fadd_rn(t, kMagic), kMagic))) > kFar)
+        c[j] = quant_code(g, w, scale, shift);
+    }
+  }
+  return make_uint2(prmt(prmt(c[0], c[1], 0x0040u), prmt(c[2], c[3], 0x0040u), 0x5410u),
+                    prmt(prmt(c[4], c[5], 0x0040u), prmt(c[6], c[7], 0x0040u), 0x5410u));
+}
+__device__ __forceinline__ bool quant_inside(const QuantGrid& g, float lo, float hi, float inv, float shift) {
+  return __fmaf_rn(lo, inv, shift) >= -0.501f && __fmaf_rn(hi, inv, shift) <= g.levels + 0.501f;  // false for NaN
+}
+// The zero point as it is stored: int4 kernels build 128 + q, so their zero points carry the 128.
+template <int BITS>
+__device__ __forceinline__ __nv_bfloat16 stored_zero(float shift) {
+  return __float2bfloat16_rn(BITS == 4 ? __fadd_rn(shift, 128.0f) : shift);
+}
+// Extremes of groups that no span covers (one scale per output channel, or odd group sizes):
+// one warp per (output, group) reads the group's run of k; scale and shift go to fp32 scratch for
+// the coding pass and to the packed weight.
+template <int BITS>
+__global__ void __launch_bounds__(256, 4)
+wq_quant_stats_kernel(const __nv_bfloat16* __restrict__ w, float* __restrict__ scale32, float* __restrict__ shift32,
+                      __nv_bfloat16* __restrict__ scales, __nv_bfloat16* __restrict__ zeros, int N, int K, int group,
+                      int symmetric) {
+  const QuantGrid g = quant_grid<BITS>(symmetric != 0);
+  const int lane = threadIdx.x & 31;
+  const int groups = K / group;
+  const long long job = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  if (job >= static_cast<long long>(N) * groups) return;
+  const int n = static_cast<int>(job / groups), gi = static_cast<int>(job - static_cast<long long>(n) * groups);
+  const uint4* src = reinterpret_cast<const uint4*>(w + static_cast<long long>(n) * K + static_cast<long long>(gi) * group);
+  uint32_t hi = 0xFF80FF80u, lo = 0x7F807F80u;  // -inf, +inf
+#pragma unroll 4
+  for (int i = lane; i < (group >> 3); i += 32) {
+    const uint4 v = __ldg(src + i);
+    const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (symmetric) {
+        hi = max2_nan(hi, x[j] & 0x7FFF7FFFu);
+      } else {
+        hi = max2_nan(hi, x[j]);
+        lo = min2_nan(lo, x[j]);
+      }
+    }
+  }
+#pragma unroll
+  for (int d = 16; d >= 1; d >>= 1) {
+    hi = max2_nan(hi, __shfl_xor_sync(0xffffffffu, hi, d));
+    if (!symmetric) lo = min2_nan(lo, __shfl_xor_sync(0xffffffffu, lo, d));
+  }
+  if (lane == 0) {
+    float scale, shift;
+    quant_scale(g, min_halves(lo), max_halves(hi), scale, shift);
+    const long long o = static_cast<long long>(gi) * N + n;
+    scale32[o] = scale;
+    shift32[o] = shift;
+    scales[o] = __float2bfloat16_rn(scale);
+    if (zeros != nullptr) zeros[o] = stored_zero<BITS>(shift);
+  }
+}
+
+// LPG: lanes per group (group = 8 * LPG: 32, 64 or 128, extremes found here), or 0: scales and
+// shifts come from the pass above.
+template <int BITS, int LPG>
+__global__ void __launch_bounds__(256, 4)
+wq_quant_pack_kernel(const __nv_bfloat16* __restrict__ w, const float* __restrict__ scale32,
+                     const float* __restrict__ shift32, uint8_t* __restrict__ q, __nv_bfloat16* __restrict__ scales,
+                     __nv_bfloat16* __restrict__ zeros, int N, int K, int group, int symmetric) {
+  constexpr int kPlanes = BITS == 4 ? 1 : 2;  // spans that have packed rows of their own
+  __shared__ uint32_t tile[kPlanes][128][32];  // [span][row][word of 4 outputs], words rotated by row / 8
+  const QuantGrid g = quant_grid<BITS>(symmetric != 0);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int half = lane >> 4, l = lane & 15;
+  const int rows = BITS == 4 ? K >> 1 : K;      // packed rows
+  const int row0 = blockIdx.x * (BITS == 4 ? 128 : 256);  // spans first: neighbouring CTAs read on in the same rows
+  const int n0 = blockIdx.y * 128;
+  // this lane's 8 consecutive k
+  const int k = (BITS == 4 ? half * rows + row0 : row0 + half * 128) + 8 * l;
+  const bool k_ok = BITS == 4 ? row0 + 8 * l < rows : k < rows;
+  const int gi = k_ok ? k / group : 0;
+#pragma unroll 1
+  for (int quad = warp; quad < 32; quad += 8) {
+    uint4 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int n = n0 + 4 * quad + i;
+      v[i] = k_ok && n < N ? __ldcs(reinterpret_cast<const uint4*>(w + static_cast<long long>(n) * K + k))
+                           : make_uint4(0u, 0u, 0u, 0u);
+    }
+    uint2 code[4];  // [output] its 8 codes
+    if (LPG > 0) {
+      // Extremes of the four outputs' groups: the first two butterfly steps halve the number of
+      // outputs a lane carries, so it ends with those of ONE group (output `own`), computes that
+      // group's scale and shift once, and hands them to the other lanes of the group.
+      uint32_t hi[4], lo[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t x[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+        if (symmetric) {
+          hi[i] = max2_nan(max2_nan(x[0] & 0x7FFF7FFFu, x[1] & 0x7FFF7FFFu), max2_nan(x[2] & 0x7FFF7FFFu, x[3] & 0x7FFF7FFFu));
+        } else {
+          hi[i] = max2_nan(max2_nan(x[0], x[1]), max2_nan(x[2], x[3]));
+          lo[i] = min2_nan(min2_nan(x[0], x[1]), min2_nan(x[2], x[3]));
+        }
+      }
+      constexpr int D1 = LPG > 0 ? LPG / 2 : 1, D2 = LPG > 0 ? LPG / 4 : 1;
+      const bool up1 = (l & D1) != 0, up2 = (l & D2) != 0;
+      const int own = (up1 ? 2 : 0) + (up2 ? 1 : 0);
+      uint32_t h2[2], l2[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        h2[i] = max2_nan(up1 ? hi[2 + i] : hi[i], __shfl_xor_sync(0xffffffffu, up1 ? hi[i] : hi[2 + i], D1));
+        if (!symmetric) l2[i] = min2_nan(up1 ? lo[2 + i] : lo[i], __shfl_xor_sync(0xffffffffu, up1 ? lo[i] : lo[2 + i], D1));
+      }
+      uint32_t h1 = max2_nan(up2 ? h2[1] : h2[0], __shfl_xor_sync(0xffffffffu, up2 ? h2[0] : h2[1], D2)), l1 = 0u;
+      if (!symmetric) l1 = min2_nan(up2 ? l2[1] : l2[0], __shfl_xor_sync(0xffffffffu, up2 ? l2[0] : l2[1], D2));
+#pragma unroll
+      for (int d = LPG / 8; d >= 1; d >>= 1) {
+        h1 = max2_nan(h1, __shfl_xor_sync(0xffffffffu, h1, d));
+        if (!symmetric) l1 = min2_nan(l1, __shfl_xor_sync(0xffffffffu, l1, d));
+      }
+      const float hi_f = max_halves(h1), lo_f = symmetric ? -hi_f : min_halves(l1);
+      float scale, shift;
+      quant_scale(g, lo_f, hi_f, scale, shift);
+      const float inv = rcp_approx(scale);
+      const int inside = quant_inside(g, lo_f, hi_f, inv, shift) ? 1 : 0;
+      const int n_own = n0 + 4 * quad + own;
+      if ((l & (D2 - 1)) == 0 && k_ok && n_own < N) {
+        const long long o = static_cast<long long>(gi) * N + n_own;
+        scales[o] = __float2bfloat16_rn(scale);
+        if (zeros != nullptr) zeros[o] = stored_zero<BITS>(shift);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int from = (i >> 1) * D1 + (i & 1) * D2;  // a lane of this group that owns output i
+        const uint32_t x[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+        const float sc = __shfl_sync(0xffffffffu, scale, from, LPG > 0 ? LPG : 32);
+        const float iv = __shfl_sync(0xffffffffu, inv, from, LPG > 0 ? LPG : 32);
+        const float sh = __shfl_sync(0xffffffffu, shift, from, LPG > 0 ? LPG : 32);
+        const bool in = __shfl_sync(0xffffffffu, inside, from, LPG > 0 ? LPG : 32) != 0;
+        code[i] = quant_code8(g, x, sc, iv, sh, in);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int n = n0 + 4 * quad + i;
+        const uint32_t x[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+        const long long o = static_cast<long long>(gi) * N + (n < N ? n : 0);
+        const float scale = __ldg(scale32 + o), shift = __ldg(shift32 + o), inv = rcp_approx(scale);
+        const float hi = max_halves(max2_nan(max2_nan(x[0], x[1]), max2_nan(x[2], x[3])));
+        const float lo = min_halves(min2_nan(min2_nan(x[0], x[1]), min2_nan(x[2], x[3])));
+        code[i] = quant_code8(g, x, scale, inv, shift, quant_inside(g, lo, hi, inv, shift));
+      }
+    }
+    // 4 x 8 bytes -> the words of 8 rows (four outputs each)
+    uint32_t word[8];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t a = h ? code[0].y : code[0].x, b = h ? code[1].y : code[1].x;
+      const uint32_t c = h ? code[2].y : code[2].x, e = h ? code[3].y : code[3].x;
+      const uint32_t ab0 = prmt(a, b, 0x5140u), ab1 = prmt(a, b, 0x7362u);
+      const uint32_t ce0 = prmt(c, e, 0x5140u), ce1 = prmt(c, e, 0x7362u);
+      word[4 * h] = prmt(ab0, ce0, 0x5410u);
+      word[4 * h + 1] = prmt(ab0, ce0, 0x7632u);
+      word[4 * h + 2] = prmt(ab1, ce1, 0x5410u);
+      word[4 * h + 3] = prmt(ab1, ce1, 0x7632u);
+    }
+    if (BITS == 4) {
+      // The half warps hold the low and the high nibbles of the same rows: each takes the even or
+      // the odd rows of the pair.
+#pragma unroll
+      for (int j = 0; j < 8; j += 2) {
+        const uint32_t mine = half ? word[j + 1] : word[j];
+        const uint32_t other = __shfl_xor_sync(0xffffffffu, half ? word[j] : word[j + 1], 16);
+        const uint32_t packed = half ? (other | (mine << 4)) : (mine | (other << 4));
+        tile[0][8 * l + j + half][(quad + l + 16 * half) & 31] = packed;
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) tile[kPlanes - 1 ? half : 0][8 * l + j][(quad + l + 16 * half) & 31] = word[j];
+    }
+  }
+  __syncthreads();
+  const bool words = N % 4 == 0 && (reinterpret_cast<uintptr_t>(q) & 3) == 0;
+#pragma unroll 4
+  for (int i = warp; i < kPlanes * 128; i += 8) {
+    const int r = i & 127, pl = i >> 7;
+    const int row = row0 + i;
+    if (row >= rows) break;
+    const int rot = (r >> 3) + 16 * (BITS == 4 ? (r & 1) : pl);
+    const uint32_t v = tile[pl][r][(lane + rot) & 31];
+    const int n = n0 + 4 * lane;
+    uint8_t* dst = q + static_cast<long long>(row) * N + n;
+    if (words) {
+      if (n < N) *reinterpret_cast<uint32_t*>(dst) = v;
+    } else {
+      // rows that start on odd bytes: consecutive lanes store consecutive bytes
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const int col = 32 * b + lane;
+        const uint32_t wv = __shfl_sync(0xffffffffu, v, 8 * b + (lane >> 2));
+        if (n0 + col < N) q[static_cast<long long>(row) * N + n0 + col] = static_cast<uint8_t>(wv >> (8 * (lane & 3)));
+      }
+    }
+  }
+}
+
+template <int BITS>
+static int launch_quantize(const void* weight, void* qweight, void* scales, void* zeros, void* scratch, int N, int K,
+                           int group, int symmetric, cudaStream_t stream) {
+  const __nv_bfloat16* w = static_cast<const __nv_bfloat16*>(weight);
+  uint8_t* q = static_cast<uint8_t*>(qweight);
+  __nv_bfloat16* s = static_cast<__nv_bfloat16*>(scales);
+  __nv_bfloat16* z = static_cast<__nv_bfloat16*>(zeros);
+  const int rows = BITS == 4 ? K / 2 : K;
+  const int span = BITS == 4 ? 128 : 256;
+  const dim3 grid((rows + span - 1) / span, (N + 127) / 128);
+  if (grid.y > 65535) return DXB_ERR_UNSUPPORTED;
+  if (dxb_quantize_scratch_bytes(N, K, group, BITS) == 0) {
+    auto kernel = group == 128 ? wq_quant_pack_kernel<BITS, 16>
+                  : group == 64 ? wq_quant_pack_kernel<BITS, 8> : wq_quant_pack_kernel<BITS, 4>;
+    kernel<<<grid, 256, 0, stream>>>(w, nullptr, nullptr, q, s, z, N, K, group, symmetric);
+  } else {
+    const long long cells = static_cast<long long>(K / group) * N;
+    float* scale32 = static_cast<float*>(scratch);
+    wq_quant_stats_kernel<BITS><<<static_cast<unsigned>((cells + 7) / 8), 256, 0, stream>>>(
+        w, scale32, scale32 + cells, s, z, N, K, group, symmetric);
+    wq_quant_pack_kernel<BITS, 0><<<grid, 256, 0, stream>>>(w, scale32, scale32 + cells, q, s, z, N, K, group, symmetric);
+  }
+  return cudaGetLastError() == cudaSuccess ? DXB_OK : DXB_ERR_CUDA;
+}
+
 }  // namespace dx
 
 extern "C" {
+
+// Groups of 32, 64 or 128 that the spans of the packing kernel cover whole (for int4 both
+// halves of K in spans of 128) are done in one pass and need no scratch.
+size_t dxb_quantize_scratch_bytes(int N, int K, int group_size, int bits) {
+  if (N <= 0 || K <= 0 || group_size <= 0) return 0;
+  const int rows = bits == 4 ? K / 2 : K;
+  if ((group_size == 32 || group_size == 64 || group_size == 128) && rows % group_size == 0) return 0;
+  return static_cast<size_t>(K / group_size) * N * 2 * sizeof(float);
+}
+
+int dxb_quantize(const void* weight, void* qweight, void* scales, void* zeros, void* scratch, int N, int K,
+                 int group_size, int bits, int symmetric, void* cuda_stream) {
+  using namespace dx;
+  if (bits != 4 && bits != 8) return DXB_ERR_BITS;
+  if (!weight || !qweight || !scales || (!symmetric && !zeros)) return DXB_ERR_NULL;
+  if (N <= 0 || K <= 0 || group_size <= 0 || K % group_size) return DXB_ERR_SHAPE;
+  // lanes take 8 consecutive k of one group with one aligned load
+  if (K % (bits == 4 ? 16 : 8) || group_size % 8 || reinterpret_cast<uintptr_t>(weight) % 16) return DXB_ERR_UNSUPPORTED;
+  if (dxb_quantize_scratch_bytes(N, K, group_size, bits) && !scratch) return DXB_ERR_WORKSPACE;
+  cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
+  void* z = symmetric ? nullptr : zeros;
+  return bits == 4 ? launch_quantize<4>(weight, qweight, scales, z, scratch, N, K, group_size, symmetric ? 1 : 0, stream)
+                   : launch_quantize<8>(weight, qweight, scales, z, scratch, N, K, group_size, symmetric ? 1 : 0, stream);
+}
 
 int dxb_dequantize_ex(const void* qweight, const void* scales, const void* zeros, void* w_out, int N,
                       int K, int group_size, int bits, int weight_layout, void* cuda_stream) {

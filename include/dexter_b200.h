@@ -218,6 +218,18 @@ int dxb_dequantize(const void* qweight, const void* scales, const void* zeros, v
 int dxb_dequantize_ex(const void* qweight, const void* scales, const void* zeros, void* w_out, int N,
                       int K, int group_size, int bits, int weight_layout, void* cuda_stream);
 
+/*
+ * Packs a dense bf16 weight [N, K] (row-major, 16-byte aligned) into the layout above: qweight
+ * [K/2, N] or [K, N], scales and (symmetric == 0) zeros [K/group_size, N] bf16.  Counterpart of
+ * the reference's offline quantiser (python/dexter/quant.py:75-133), for weights already on the
+ * GPU.  K a multiple of 16 (int8: 8) and group_size of 8, else DXB_ERR_UNSUPPORTED.  `scratch`:
+ * dxb_quantize_scratch_bytes of fp32 scales and zero points between two passes; 0 bytes where the
+ * groups are small enough for one pass.
+ */
+size_t dxb_quantize_scratch_bytes(int N, int K, int group_size, int bits);
+int dxb_quantize(const void* weight, void* qweight, void* scales, void* zeros, void* scratch, int N, int K,
+                 int group_size, int bits, int symmetric, void* cuda_stream);
+
 /* 1 when dxb_wq_gemm runs this shape on the tcgen05 kernel, 0 when it takes the
  * plain CUDA-core kernel (the counterpart of the reference's `accepts` shape
  * predicate, python/dexter/registry.py:58-60). */

@@ -21,6 +21,23 @@ SHAPES = [(256, 128, 4, 128), (512, 131, 4, 128), (384, 40, 4, 64), (192, 9, 4, 
 
 
 @pytest.mark.parametrize("symmetric", [True, False])
+@pytest.mark.parametrize("k,n,bits,group", SHAPES)
+def test_quantize_gives_the_bytes_of_the_tensor_expressions(k, n, bits, group, symmetric, d):
+    torch.manual_seed(k + n)
+    w = (torch.randn(n, k, device="cuda") * 0.02).to(torch.bfloat16)
+    w[0, :group] = 0                      # a group without extent
+    w[-1, group // 2:] += 1.0             # a group far from zero
+    got = d.quantize(w, bits=bits, group_size=group, symmetric=symmetric)
+    # a weight that carries a gradient keeps the element-wise tensor expressions
+    want = d.quantize(w.clone().requires_grad_(), bits=bits, group_size=group, symmetric=symmetric)
+    assert torch.equal(got.qweight, want.qweight)
+    assert torch.equal(got.scales, want.scales.detach())
+    assert (got.zeros is None) == symmetric
+    if not symmetric:
+        assert torch.equal(got.zeros, want.zeros.detach())
+
+
+@pytest.mark.parametrize("symmetric", [True, False])
 @pytest.mark.parametrize("k,n,bits,group,layout", [s + ("dexter",) for s in SHAPES] + [
     (256, 128, 4, 128, "b200"), (512, 132, 4, 64, "b200"), (192, 12, 4, 96, "b200"), (20, 7, 4, 5, "dexter"),
     (9, 5, 8, 3, "dexter")])
