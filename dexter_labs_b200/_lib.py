@@ -101,5 +101,18 @@ def load_fast():
     return _dxb_fast.gemm
 
 
+def load_call(relaid: dict):
+    """The native eager call (``_dxb_call``) bound to this library and to the cache of repacked
+    weights, or None when it has not been built (ops.py then makes every call itself)."""
+    lib = load()
+    try:
+        from . import _dxb_call
+    except ImportError:
+        return None
+    _dxb_call.bind(ctypes.cast(lib.dxb_wq_gemm_ex, c_void_p).value,
+                   ctypes.cast(lib.dxb_workspace_bytes_ex, c_void_p).value, relaid)
+    return _dxb_call
+
+
 def strerror(code: int) -> str:
     return load().dxb_strerror(code).decode()

@@ -7,6 +7,7 @@ library on import -- is not imported first) or :func:`build` runs nvcc on
 """
 from __future__ import annotations
 
+import importlib.util
 import os
 import shutil
 import subprocess
@@ -21,6 +22,9 @@ LIB_PATH = PKG_DIR / "libdexter_b200.so"
 # compiled CPython binding of the hot call (csrc/fastcall.c); plain C, no CUDA
 FAST_SOURCE = PKG_DIR / "csrc" / "fastcall.c"
 FAST_PATH = PKG_DIR / ("_dxb_fast" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
+# the whole eager call, tensors to launch (csrc/torch_call.cpp); C++ against torch's own headers
+CALL_SOURCE = PKG_DIR / "csrc" / "torch_call.cpp"
+CALL_PATH = PKG_DIR / ("_dxb_call" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -66,10 +70,32 @@ def build_fast(force: bool = False) -> Path:
     return FAST_PATH
 
 
+def build_call(force: bool = False) -> Path:
+    """Compile the native eager call (host C++ only; it launches through the library)."""
+    newest = max(src.stat().st_mtime for src in (CALL_SOURCE, HEADERS[-1]))
+    if not force and CALL_PATH.exists() and CALL_PATH.stat().st_mtime >= newest:
+        return CALL_PATH
+    # found, not imported: as a script this file has its own folder (with a platform.py) first in sys.path
+    torch_dir = Path(importlib.util.find_spec("torch").origin).resolve().parent
+    cmd = [os.environ.get("CXX") or shutil.which("g++") or "c++", "-O2", "-std=c++17", "-shared", "-fPIC",
+           "-I", sysconfig.get_paths()["include"]]
+    for path in (torch_dir / "include", torch_dir / "include" / "torch" / "csrc" / "api" / "include",
+                 Path(_nvcc()).resolve().parent.parent / "include"):
+        cmd += ["-isystem", str(path)]
+    cmd += [str(CALL_SOURCE), "-o", str(CALL_PATH), "-L", str(torch_dir / "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu",
+            "-ltorch_python"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode:
+        sys.stderr.write(proc.stdout + proc.stderr)
+        raise RuntimeError(f"C++ compiler failed ({proc.returncode}): {' '.join(cmd)}")
+    return CALL_PATH
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
-    """Compile the library (and the CPython binding of its hot call) if missing or older
-    than the sources."""
+    """Compile the library (and the bindings of its hot call) if missing or older than the
+    sources."""
     build_fast(force)
+    build_call(force)
     if not force and not is_stale():
         return LIB_PATH
     cmd = [_nvcc(), *NVCC_FLAGS]

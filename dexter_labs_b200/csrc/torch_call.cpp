@@ -1,0 +1,186 @@
+// _dxb_call: one whole eager call of the registered kernels, from tensors to a launched kernel.
+//
+// A GEMM of this package lasts 5 to 15 us, and a call made of Python statements (attribute
+// reads, data_ptr(), dictionary look-ups, torch.empty) costs about as much host time as that, so
+// chains of small calls were bound by the host: 13.4 us per call against 5.5 us of GPU time at one
+// token.  call() does the same steps natively.  It serves the plain case only -- tensors of the right
+// types, contiguous, on the current device, weight already repacked, workspace already there -- and
+// returns None for everything else, errors included, which ops.py then handles as before.
+//
+//   bind(gemm_ex, workspace_bytes_ex, relaid)  addresses in the loaded library, the cache of repacked weights
+//   set_workspace(device, stream, ptr, bytes)  what ops.py holds for that stream (0 bytes: nothing)
+//   call(bits, x, qweight, scales, zeros, bias, group_size, max_ctas, layout, epilogue, pinned) -> Tensor | None
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <cstdlib>
+#include <unordered_map>
+
+#include "../../include/dexter_b200.h"
+
+namespace {
+
+using GemmEx = decltype(&dxb_wq_gemm_ex);
+using WorkspaceBytes = decltype(&dxb_workspace_bytes_ex);
+
+GemmEx g_gemm = nullptr;
+WorkspaceBytes g_workspace_bytes = nullptr;
+PyObject* g_relaid = nullptr;  // id(qweight) -> (weak reference, version, repacked copy or None), owned by ops.py
+
+struct Mix {
+  size_t operator()(const std::pair<uint64_t, uint64_t>& k) const {
+    return static_cast<size_t>((k.first ^ (k.second * 0x9E3779B97F4A7C15ull)) * 0xFF51AFD7ED558CCDull);
+  }
+};
+// All state below is only touched with the interpreter lock held.
+std::unordered_map<std::pair<uint64_t, uint64_t>, std::pair<void*, size_t>, Mix> g_workspaces;  // (device, stream)
+std::unordered_map<std::pair<uint64_t, uint64_t>, size_t, Mix> g_need;                          // (shape words)
+
+PyObject* bind(PyObject*, PyObject* args) {
+  unsigned long long gemm = 0, bytes = 0;
+  PyObject* relaid = nullptr;
+  if (!PyArg_ParseTuple(args, "KKO!", &gemm, &bytes, &PyDict_Type, &relaid)) return nullptr;
+  g_gemm = reinterpret_cast<GemmEx>(static_cast<uintptr_t>(gemm));
+  g_workspace_bytes = reinterpret_cast<WorkspaceBytes>(static_cast<uintptr_t>(bytes));
+  Py_INCREF(relaid);
+  Py_XSETREF(g_relaid, relaid);
+  Py_RETURN_NONE;
+}
+
+PyObject* set_workspace(PyObject*, PyObject* args) {
+  int device = 0;
+  unsigned long long stream = 0, ptr = 0, bytes = 0;
+  if (!PyArg_ParseTuple(args, "iKKK", &device, &stream, &ptr, &bytes)) return nullptr;
+  g_workspaces[{static_cast<uint64_t>(device), stream}] = {reinterpret_cast<void*>(static_cast<uintptr_t>(ptr)),
+                                                           static_cast<size_t>(bytes)};
+  Py_RETURN_NONE;
+}
+
+// A plain torch.Tensor or Parameter (no subclass that might want to see the call itself).
+const at::Tensor* plain_tensor(PyObject* o) {
+  return THPVariable_CheckExact(o) ? &THPVariable_Unpack(o) : nullptr;
+}
+
+// Looks an int4 weight up in the cache of repacked copies: false when ops.py has not seen it yet (or
+// it has changed since); else `copy` is its repacked copy, or nullptr where its shape takes none.
+bool repacked(PyObject* obj, const at::Tensor& q, const at::Tensor** copy) {
+  *copy = nullptr;
+  PyObject* key = PyLong_FromVoidPtr(obj);
+  if (!key) { PyErr_Clear(); return false; }
+  PyObject* hit = PyDict_GetItemWithError(g_relaid, key);  // borrowed
+  Py_DECREF(key);
+  if (!hit || !PyTuple_CheckExact(hit) || PyTuple_GET_SIZE(hit) < 3) { PyErr_Clear(); return false; }
+  if (PyWeakref_GetObject(PyTuple_GET_ITEM(hit, 0)) != obj) return false;
+  if (q.is_inference() || PyLong_AsUnsignedLong(PyTuple_GET_ITEM(hit, 1)) != q._version()) { PyErr_Clear(); return false; }
+  PyObject* item = PyTuple_GET_ITEM(hit, 2);
+  if (item == Py_None) return true;
+  if (!THPVariable_CheckExact(item)) return false;
+  *copy = &THPVariable_Unpack(item);
+  return true;
+}
+
+PyObject* call(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  if (n_args != 11) {
+    PyErr_SetString(PyExc_TypeError, "_dxb_call.call takes exactly 11 arguments");
+    return nullptr;
+  }
+  if (!g_gemm) Py_RETURN_NONE;
+  const long bits = PyLong_AsLong(a[0]), group = PyLong_AsLong(a[6]), max_ctas = PyLong_AsLong(a[7]);
+  const long layout = PyLong_AsLong(a[8]), epilogue = PyLong_AsLong(a[9]);
+  if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
+  // A caller that came through the registry honours its DEXTER_KERNEL pin, which is parsed there.
+  if (a[10] == Py_True && std::getenv("DEXTER_KERNEL") != nullptr) Py_RETURN_NONE;
+  const at::Tensor *x = plain_tensor(a[1]), *q = plain_tensor(a[2]), *s = plain_tensor(a[3]);
+  const at::Tensor *z = a[4] == Py_None ? nullptr : plain_tensor(a[4]);
+  const at::Tensor *b = a[5] == Py_None ? nullptr : plain_tensor(a[5]);
+  if (!x || !q || !s || (a[4] != Py_None && !z) || (a[5] != Py_None && !b)) Py_RETURN_NONE;
+  if (!x->is_cuda() || x->scalar_type() != at::kBFloat16 || s->scalar_type() != at::kBFloat16 ||
+      q->scalar_type() != at::kByte || q->dim() != 2 || s->dim() != 2 || (z && z->scalar_type() != at::kBFloat16) ||
+      (b && b->scalar_type() != at::kBFloat16))
+    Py_RETURN_NONE;
+  const auto dev = x->device();
+  if (dev.index() != c10::cuda::current_device() || q->device() != dev || s->device() != dev ||
+      (z && z->device() != dev) || (b && b->device() != dev))
+    Py_RETURN_NONE;
+  if (!q->is_contiguous() || !s->is_contiguous() || (z && !z->is_contiguous()) || (b && !b->is_contiguous()))
+    Py_RETURN_NONE;
+  const int64_t n = q->size(1), k = bits == 4 ? 2 * q->size(0) : q->size(0);
+  const int64_t dims = x->dim();
+  if (dims < 1 || x->size(dims - 1) != k || k <= 0) Py_RETURN_NONE;
+  int64_t m, ldx;
+  if (dims == 2) {
+    m = x->size(0);
+    ldx = x->stride(0);
+    if (x->stride(1) != 1 || ldx % 8) Py_RETURN_NONE;
+  } else {
+    if (!x->is_contiguous() || k % 8) Py_RETURN_NONE;
+    m = x->numel() / k;
+    ldx = k;
+  }
+  const void* xp = x->const_data_ptr();
+  if (m <= 0 || reinterpret_cast<uintptr_t>(xp) % 16 || m > INT32_MAX || n > INT32_MAX || k > INT32_MAX) Py_RETURN_NONE;
+
+  dxb_gemm_opts opts = {};
+  opts.weight_layout = static_cast<int>(layout);
+  opts.epilogue = static_cast<int>(epilogue);
+  opts.max_ctas = static_cast<int>(max_ctas);
+  if (layout == DXB_LAYOUT_DEXTER && bits == 4) {
+    const at::Tensor* copy;
+    if (!repacked(a[2], *q, &copy)) Py_RETURN_NONE;
+    if (copy) {
+      q = copy;
+      opts.weight_layout = DXB_LAYOUT_B200;
+    }
+  }
+
+  const auto stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+  const auto ws = g_workspaces.find({static_cast<uint64_t>(dev.index()), reinterpret_cast<uint64_t>(stream)});
+  if (ws == g_workspaces.end()) Py_RETURN_NONE;
+  const std::pair<uint64_t, uint64_t> shape{(static_cast<uint64_t>(m) << 32) | static_cast<uint64_t>(n),
+                                            (static_cast<uint64_t>(k) << 32) | (static_cast<uint64_t>(max_ctas & 0xFFFFFF) << 8) |
+                                                static_cast<uint64_t>(bits)};
+  auto need = g_need.find(shape);
+  if (need == g_need.end()) {
+    if (g_need.size() > 4096) g_need.clear();
+    need = g_need.emplace(shape, g_workspace_bytes(static_cast<int>(m), static_cast<int>(n), static_cast<int>(k),
+                                                   static_cast<int>(bits), static_cast<int>(max_ctas))).first;
+  }
+  if (ws->second.second < need->second) Py_RETURN_NONE;
+
+  try {
+    at::Tensor out;
+    if (dims == 2) {
+      out = at::empty({m, n}, x->options());
+    } else {
+      auto sizes = x->sizes().vec();
+      sizes.back() = n;
+      out = at::empty(sizes, x->options());
+    }
+    const int rc = g_gemm(static_cast<int>(bits), xp, ldx, q->const_data_ptr(), s->const_data_ptr(),
+                          z ? z->const_data_ptr() : nullptr, b ? b->const_data_ptr() : nullptr, out.mutable_data_ptr(), n,
+                          static_cast<int>(m), static_cast<int>(n), static_cast<int>(k), static_cast<int>(group),
+                          ws->second.first, ws->second.second, &opts, stream);
+    if (rc != DXB_OK) Py_RETURN_NONE;  // the general path reports it
+    return THPVariable_Wrap(std::move(out));
+  } catch (const std::exception&) {
+    Py_RETURN_NONE;  // out of memory and the like: the general path raises it
+  }
+}
+
+PyMethodDef methods[] = {
+    {"bind", bind, METH_VARARGS, "bind(gemm_ex, workspace_bytes_ex, relaid)"},
+    {"set_workspace", set_workspace, METH_VARARGS, "set_workspace(device, stream, ptr, bytes)"},
+    {"call", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(call)), METH_FASTCALL,
+     "one eager GEMM, or None where the general path has to take it"},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_dxb_call", "native eager call", -1, methods,
+                          nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__dxb_call() { return PyModule_Create(&module_def); }

@@ -20,7 +20,7 @@ import torch
 
 from . import _lib
 from .platform import ArchVersion, Capability
-from .registry import Priority, register, select
+from .registry import Priority, leading, register, select
 
 __all__ = ["w4a16", "w8a16", "w4a16_gelu", "w8a16_gelu", "linear", "dequantize", "accepts", "KERNEL_NAMES",
            "register_with", "last_status", "PeerAllReduce",
@@ -71,6 +71,11 @@ def _run(bits: int, x: torch.Tensor, qweight: torch.Tensor, scales: torch.Tensor
          zeros: Optional[torch.Tensor], bias: Optional[torch.Tensor], group_size: int,
          max_ctas: int = 0, *, layout: str = "dexter", epilogue: Optional[str] = None,
          reduce: Optional["FusedReduce"] = None) -> torch.Tensor:
+    if _CALL is not None and reduce is None:
+        out = _CALL(bits, x, qweight, scales, zeros, bias, group_size, max_ctas, _LAYOUTS[layout],
+                    _EPILOGUES[epilogue], False)
+        if out is not None:
+            return out
     if not x.is_cuda:
         raise RuntimeError("the B200 backend needs CUDA tensors; there is no CPU path")
     if x.dtype != torch.bfloat16 or scales.dtype != torch.bfloat16:
@@ -126,6 +131,8 @@ def _run(bits: int, x: torch.Tensor, qweight: torch.Tensor, scales: torch.Tensor
     if ws is None or ws[2] < need:
         t = _workspace(x.device, stream, need)
         ws = _ws_fast[(dev, stream)] = (t, t.data_ptr(), t.numel())
+        if _NATIVE is not None:
+            _NATIVE.set_workspace(dev, stream, ws[1], ws[2])
     if reduce is None and _FAST is not None:
         # compiled binding: same entry point, arguments as plain integers (0 = NULL)
         rc = _FAST(bits, x2.data_ptr(), x2.stride(0), qweight.data_ptr(), scales.data_ptr(),
@@ -165,9 +172,14 @@ def _run(bits: int, x: torch.Tensor, qweight: torch.Tensor, scales: torch.Tensor
 _CHECK = bool(os.environ.get("DEXTER_B200_CHECK"))
 
 # ------------------------------------------------------------ load-time re-layout (int4)
-# id(qweight) -> (weak reference to it, its version counter, the repacked copy)
-_relaid: Dict[int, Tuple[object, int, torch.Tensor]] = {}
+# id(qweight) -> (weak reference to it, its version counter, the repacked copy or None)
+_relaid: Dict[int, Tuple[object, int, Optional[torch.Tensor]]] = {}
 _AUTO_RELAYOUT = os.environ.get("DEXTER_B200_RELAYOUT", "1") != "0"
+
+# The plain eager call in native code (csrc/torch_call.cpp).  It answers None whenever anything about
+# the call is out of the ordinary, errors included: _run below then takes it.
+_NATIVE = None if os.environ.get("DEXTER_B200_FASTCALL", "1") == "0" else _lib.load_call(_relaid)
+_CALL = None if _NATIVE is None or _CHECK else _NATIVE.call
 
 
 def relayout_w4(qweight: torch.Tensor, *, inverse: bool = False,
@@ -210,15 +222,15 @@ def prepared_w4(qweight: torch.Tensor, m: int, n: int, k_dim: int,
     key = id(qweight)
     hit = _relaid.get(key)
     if hit is not None and hit[0]() is qweight and hit[1] == qweight._version:
-        return hit[2], False
-    if (qweight.shape[0] % 2 or n % 4 or qweight.data_ptr() % 16
-            or not _LIB.dxb_uses_tensor_cores(m, n, k_dim, group_size, 4)
-            or torch.cuda.is_current_stream_capturing()):
+        return None if hit[2] is None else (hit[2], False)
+    takes_none = (qweight.shape[0] % 2 or n % 4 or qweight.data_ptr() % 16
+                  or not _LIB.dxb_uses_tensor_cores(m, n, k_dim, group_size, 4))
+    if not takes_none and torch.cuda.is_current_stream_capturing():
         return None
-    relaid = relayout_w4(qweight)
-    _relaid[key] = (weakref.ref(qweight, lambda _r, key=key: _relaid.pop(key, None)),
+    relaid = None if takes_none else relayout_w4(qweight)
+    _relaid[key] = (weakref.ref(qweight, lambda _r, key=key, table=_relaid: table.pop(key, None)),
                     qweight._version, relaid)
-    return relaid, True
+    return None if relaid is None else (relaid, True)
 
 
 def last_status(device: Optional[torch.device] = None) -> int:
@@ -419,8 +431,14 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
         raise NotImplementedError("dense gemm is not part of the B200 weight-only backend")
     if bits not in (4, 8):
         raise ValueError(f"weight-only quantisation supports 4 or 8 bits, got {bits}")
-    mode = f"w{bits}a16"
-    return select("gemm", mode, x, weight, scales)(x, weight, scales, zeros, bias, group_size)
+    key = _KEYS[bits]
+    if _CALL is not None and not torch.compiler.is_compiling() and leading(key) is _SPECS[bits]:
+        # this package's kernel is the one select() tries first: take the call there if it is a
+        # plain one (its checks include those of `accepts`) and no pin is set
+        out = _CALL(bits, x, weight, scales, zeros, bias, group_size, 0, 0, 0, True)
+        if out is not None:
+            return out
+    return select("gemm", key[5:], x, weight, scales)(x, weight, scales, zeros, bias, group_size)
 
 
 _CAPABILITY = dict(vendors=frozenset({"nvidia"}), features=frozenset({"matrix:bf16"}))
@@ -429,6 +447,9 @@ register("gemm", "w4a16", name=KERNEL_NAMES["w4a16"], priority=Priority.SPECIALI
          capability=Capability(min_arch=ArchVersion(10, 0), **_CAPABILITY), accepts=accepts)(w4a16)
 register("gemm", "w8a16", name=KERNEL_NAMES["w8a16"], priority=Priority.SPECIALISED,
          capability=Capability(min_arch=ArchVersion(10, 0), **_CAPABILITY), accepts=accepts)(w8a16)
+
+_KEYS = {4: "gemm/w4a16", 8: "gemm/w8a16"}
+_SPECS = {4: w4a16.dexter_spec, 8: w8a16.dexter_spec}
 
 
 def register_with(dexter_registry, dexter_platform) -> None:

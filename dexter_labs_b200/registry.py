@@ -51,6 +51,8 @@ class KernelSpec:
 
 
 _REGISTRY: Dict[str, List[KernelSpec]] = {}
+# key -> (platform, first viable kernel): capability checks are made once per platform, not per call
+_leading: Dict[str, tuple] = {}
 
 
 def register(family: str, mode: str, *, name: str, capability: Optional[Capability] = None,
@@ -64,6 +66,7 @@ def register(family: str, mode: str, *, name: str, capability: Optional[Capabili
         if name in (s.name for s in bucket):
             raise ValueError(f"duplicate kernel {spec.key}:{name}")
         bucket.append(spec)
+        _leading.clear()
         bucket.sort(key=lambda s: -int(s.priority))  # stable: ties keep registration order
         fn.dexter_spec = spec
         return fn
@@ -75,6 +78,17 @@ def candidates(family: str, mode: str,
                platform: Optional[PlatformInfo] = None) -> Iterator[KernelSpec]:
     platform = platform or current_platform()
     return (s for s in _REGISTRY.get(f"{family}/{mode}", []) if s.capability.satisfied_by(platform))
+
+
+def leading(key: str) -> Optional[KernelSpec]:
+    """The highest-priority viable kernel of ``key``: what :func:`select` tries first when no
+    pin is set."""
+    platform = current_platform()
+    hit = _leading.get(key)
+    if hit is None or hit[0] is not platform:
+        family, _, mode = key.partition("/")
+        hit = _leading[key] = (platform, next(candidates(family, mode, platform), None))
+    return hit[1]
 
 
 def _pin_for(key: str) -> Optional[str]:

@@ -1,0 +1,81 @@
+"""The native eager call: taken for plain calls, declined for everything else, same results."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def d(b200_lib):
+    import dexter_labs_b200
+
+    return dexter_labs_b200
+
+
+def weight(d, n=144, k=256, bits=4, group=128):
+    torch.manual_seed(n + k)
+    w = (torch.randn(n, k, device="cuda") * 0.02).to(torch.bfloat16)
+    return d.quantize(w, bits=bits, group_size=group, bias=torch.randn(n, device="cuda").to(torch.bfloat16))
+
+
+def native(d, x, q, **over):
+    a = dict(x=x, w=q.qweight, s=q.scales, z=q.zeros, b=q.bias) | over
+    return d.ops._CALL(q.bits, a["x"], a["w"], a["s"], a["z"], a["b"], q.group_size, 0, 0, 0, False)
+
+
+@pytest.mark.parametrize("bits,n", [(4, 144), (4, 141), (8, 144)])  # 141: a width that is never repacked
+def test_native_call_equals_the_general_path(bits, n, d, monkeypatch):
+    q = weight(d, n=n, bits=bits)
+    x = torch.randn(2, 3, 256, device="cuda").to(torch.bfloat16)
+    y = d.linear(x, q.qweight, q.bias, scales=q.scales, zeros=q.zeros, group_size=128, bits=bits)
+    got = native(d, x, q)  # workspace and repacked copy exist by now
+    assert got is not None and got.shape == (2, 3, n)
+    monkeypatch.setattr(d.ops, "_CALL", None)
+    want = d.linear(x, q.qweight, q.bias, scales=q.scales, zeros=q.zeros, group_size=128, bits=bits)
+    assert torch.equal(got, want) and torch.equal(y, want)
+
+
+def test_native_call_declines_what_is_not_plain(d):
+    q = weight(d)
+    x = torch.randn(6, 256, device="cuda").to(torch.bfloat16)
+    d.w4a16(x, q.qweight, q.scales, q.zeros, q.bias, 128)
+    assert native(d, x, q) is not None
+    wide = torch.randn(6, 512, device="cuda").to(torch.bfloat16)
+    assert native(d, wide[:, :256], q) is not None                    # a row stride is plain
+    assert native(d, x.t().contiguous().t(), q) is None               # inner stride
+    assert native(d, wide[:, 4:260], q) is None                       # alignment
+    assert native(d, x[:, :128].contiguous(), q) is None              # K mismatch
+    assert native(d, x[:0], q) is None
+    assert native(d, x.float(), q) is None
+    assert native(d, x.cpu(), q) is None
+    assert native(d, x, q, s=q.scales.t().contiguous().t()) is None
+    assert native(d, x, q, w=q.qweight.clone()) is None               # never seen: no repacked copy yet
+    before = d.w4a16(x, q.qweight, q.scales, q.zeros, q.bias, 128)
+    q.qweight.zero_()                                                 # modified in place: the copy is stale
+    assert native(d, x, q) is None
+    assert not torch.equal(d.w4a16(x, q.qweight, q.scales, q.zeros, q.bias, 128), before)
+
+
+def test_pin_and_platform_still_rule_the_call(d, monkeypatch):
+    from dexter_labs_b200 import platform, registry
+
+    q = weight(d)
+    x = torch.randn(6, 256, device="cuda").to(torch.bfloat16)
+
+    def linear():
+        return d.linear(x, q.qweight, q.bias, scales=q.scales, zeros=q.zeros, group_size=128, bits=4)
+
+    linear()
+    monkeypatch.setenv("DEXTER_KERNEL", "gemm/w4a16:no_such_kernel")
+    with pytest.raises(LookupError):
+        linear()
+    monkeypatch.delenv("DEXTER_KERNEL")
+    linear()
+    try:
+        platform.override_platform(platform._cpu_platform())
+        with pytest.raises(LookupError):
+            linear()
+    finally:
+        platform.override_platform(None)
+    linear()
+    assert registry.leading("gemm/w4a16") is d.ops._SPECS[4]
