@@ -159,6 +159,11 @@ __device__ __forceinline__ float4 ld_smem_f4(uint32_t addr) {
 }
 // Hardware barrier over every thread of the cluster; release/acquire at cluster scope,
 // so shared-memory writes made before it are visible to peer CTAs after it.
+// Its two halves: arrive without ordering memory (only "this CTA has started"), and wait.
+__device__ __forceinline__ void cluster_arrive_relaxed() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // Rank of this CTA in its cluster and index of the cluster in the grid (x), read from the
 // special registers: no division by the cluster size.
 __device__ __forceinline__ uint32_t cluster_cta_rank() {

@@ -68,6 +68,17 @@ __device__ __forceinline__ float deq8(uint32_t word, uint32_t byte_sel, float cz
   const float f = __uint_as_float(prmt(word, 0x4B000000u, 0x7650u + byte_sel));
   return (f - cz) * scale;
 }
+// Two bytes (bits 0..7 and 16..23 of `w`; the other bits are ignored) -> two bf16 weights.  q - 128 has
+// eight significant bits, so it is exact in bf16: the low seven bits of q OR-ed into 0x4300 give 128 +
+// (q & 127), and the eighth flips the 256 (0x4380) to subtract into a 128.  `zero2` = zero point - 128,
+// subtracted exactly as well (differences of bytes fit eight significant bits); the multiply is the only
+// rounding, as with deq8.
+__device__ __forceinline__ uint32_t deq8x2(uint32_t w, uint32_t zero2, uint32_t scale2, bool has_zero) {
+  const uint32_t v = (w & 0x007F007Fu) | 0x43004300u;
+  uint32_t d = sub_bf16x2(v, (w & 0x00800080u) ^ 0x43804380u);
+  if (has_zero) d = sub_bf16x2(d, zero2);
+  return mul_bf16x2(d, scale2);
+}
 __device__ __forceinline__ uint32_t dup_lo(uint32_t w) { return prmt(w, w, 0x1010u); }
 __device__ __forceinline__ uint32_t dup_hi(uint32_t w) { return prmt(w, w, 0x3232u); }
 __device__ __forceinline__ float bf16lo_f32(uint32_t w) { return __uint_as_float(w << 16); }
@@ -81,6 +92,14 @@ __device__ __forceinline__ uint32_t fetch_q4(const uint8_t* __restrict__ qw, int
   if (!relaid) return (qw[static_cast<long long>(r) * N + n] >> (4 * plane)) & 0xFu;
   const uint32_t word = reinterpret_cast<const uint32_t*>(qw)[(static_cast<long long>(r & ~1) + plane) * (N >> 2) + (n >> 2)];
   return (word >> (16 * (r & 1) + 4 * (n & 3))) & 0xFu;
+}
+
+// tanh-GELU of a value that has already been rounded to bf16, as the reference applies it
+// between the FFN linears (torch gelu(approximate="tanh") on the bf16 output of the up
+// projection, python/dexter/models/dreamzero/model.py:279-285): evaluated in fp32, rounded once.
+__device__ __forceinline__ float gelu_tanh(float v) {
+  const float inner = 0.7978845608028654f * (v + 0.044715f * v * v * v);
+  return 0.5f * v * (1.0f + tanhf(inner));
 }
 
 __device__ __forceinline__ uint32_t lds32(uint32_t addr) {

@@ -33,6 +33,7 @@
 // thread-block cluster per tile that splits K and adds through distributed shared memory.
 // More than 128 tokens: every (token block of 128, column tile) pair is a tile, one launch.
 #include "wq_common.cuh"
+#include "wq_small.cuh"
 
 namespace dx {
 #ifdef DXB_TRACE
@@ -169,14 +170,6 @@ struct WqParams {
   int debug;           // -DDXB_TRACE builds only: parts of the pipeline to leave out (timing experiments)
 };
 
-
-// tanh-GELU of a value that has already been rounded to bf16, as the reference applies it
-// between the FFN linears (torch gelu(approximate="tanh") on the bf16 output of the up
-// projection, python/dexter/models/dreamzero/model.py:279-285): evaluated in fp32, rounded once.
-__device__ __forceinline__ float gelu_tanh(float v) {
-  const float inner = 0.7978845608028654f * (v + 0.044715f * v * v * v);
-  return 0.5f * v * (1.0f + tanhf(inner));
-}
 
 // Four fp32 sums of one token row -> four bf16 outputs, in the reference's order of
 // roundings: round the matmul to bf16, add the bias in bf16 arithmetic (second rounding),
@@ -1504,6 +1497,124 @@ static int launch_tc(const void* x, long long ldx, const void* qw, const void* s
   return cudaGetLastError() == cudaSuccess ? DXB_OK : DXB_ERR_CUDA;
 }
 
+// ------------------------------------------------------------- few tokens, odd shapes
+// Shapes wq_gemm_small takes: whole steps of 32 packed rows with one scale row per plane each, and
+// activations it can load 16 bytes at a time.
+static bool small_supported(const void* x, long long ldx, int K, int group, int bits) {
+  const int rows = bits == 4 ? K / 2 : K;
+  return rows % 32 == 0 && group % 32 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && ldx % 8 == 0;
+}
+
+struct SmallKernel {
+  void (*fn)(const SmallParams);
+  int warp_bytes;  // one warp's ring
+};
+template <int KIND, bool RAGGED, int CPW>
+static SmallKernel pick_small(int mt) {
+  using S1 = SmallStage<KIND, RAGGED, CPW, 1>;
+  using S2 = SmallStage<KIND, RAGGED, CPW, 2>;
+  return mt == 1 ? SmallKernel{wq_gemm_small<KIND, RAGGED, CPW, 1>, S1::kBytes * S1::kStages}
+                 : SmallKernel{wq_gemm_small<KIND, RAGGED, CPW, 2>, S2::kBytes * S2::kStages};
+}
+
+// Lets the kernel use more than 48 KB of shared memory; once per kernel, device and thread.
+static bool small_smem_ready(void (*fn)(const SmallParams)) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  static thread_local std::unordered_map<size_t, bool> done;
+  const size_t key = reinterpret_cast<size_t>(fn) * 64 + static_cast<size_t>(dev);
+  if (done.find(key) != done.end()) return true;
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) return false;
+  done[key] = true;
+  return true;
+}
+
+static int launch_small(int bits, const void* x, long long ldx, const void* qw, const void* scales, const void* zeros,
+                        const void* bias, void* out, long long ldo, int M, int N, int K, int group, const Opts& opts,
+                        cudaStream_t stream) {
+  const int sms = device_info().sms;
+  const int budget = (opts.max_ctas > 0 && opts.max_ctas < sms) ? opts.max_ctas : sms;
+  SmallParams p{};
+  p.x = static_cast<const __nv_bfloat16*>(x);
+  p.qw = static_cast<const uint8_t*>(qw);
+  p.scales = static_cast<const __nv_bfloat16*>(scales);
+  p.zeros = static_cast<const __nv_bfloat16*>(zeros);
+  p.bias = static_cast<const __nv_bfloat16*>(bias);
+  p.out = static_cast<__nv_bfloat16*>(out);
+  p.ldx = ldx; p.ldo = ldo;
+  p.M = M; p.N = N; p.K = K; p.group = group;
+  p.rows = bits == 4 ? K / 2 : K;
+  p.steps = p.rows / 32;
+  p.epilogue = opts.epilogue;
+  const int mt = M <= 8 ? 1 : 2;
+  const int blocks = (M + 8 * mt - 1) / (8 * mt);
+  // Tiles of 32 columns.  Up to one per SM: sixteen warps each, and clusters that split K while SMs
+  // are left over and every warp keeps at least two steps.  More: eight warps, two CTAs per SM.
+  // (All of this fixes the order of the sums, so it must not depend on the weight's layout.)
+  const long long tiles32 = static_cast<long long>((N + 31) / 32) * blocks;
+  int warps = 8, cluster = 1;
+  if (tiles32 <= budget) {
+    warps = 16;
+    while (cluster < 8 && tiles32 * cluster * 2 <= budget && p.steps >= 64 * cluster) cluster *= 2;
+  }
+  p.cluster = cluster;
+  {
+    const int g32 = group / 32;
+    p.group_shift = -1;
+    for (int b = 0; b < 20; ++b)
+      if ((1 << b) == g32) p.group_shift = b;
+  }
+  // Whole 16-byte chunks of packed rows and scale rows, or the variant for rows on any byte.
+  const uintptr_t p16 = reinterpret_cast<uintptr_t>(qw) | reinterpret_cast<uintptr_t>(scales) | reinterpret_cast<uintptr_t>(zeros);
+  const bool ragged = N % 16 != 0 || p16 % 16 != 0;
+  if (ragged && (opts.relaid || p16 % 4 != 0)) return DXB_ERR_UNSUPPORTED;
+  const int kind = bits == 8 ? kSmallW8 : opts.relaid ? kSmallW4Relaid : kSmallW4;
+  // More tiles than two per SM: twice the width, so that they all still run at once.
+  const bool wide = tiles32 > 2 * budget && !ragged && kind != kSmallW4;
+  SmallKernel k;
+  if (ragged) k = kind == kSmallW8 ? pick_small<kSmallW8, true, 1>(mt) : pick_small<kSmallW4, true, 1>(mt);
+  else if (wide) k = kind == kSmallW8 ? pick_small<kSmallW8, false, 2>(mt) : pick_small<kSmallW4Relaid, false, 2>(mt);
+  else k = kind == kSmallW8 ? pick_small<kSmallW8, false, 1>(mt)
+         : kind == kSmallW4 ? pick_small<kSmallW4, false, 1>(mt) : pick_small<kSmallW4Relaid, false, 1>(mt);
+  const int bn = wide ? 64 : 32;
+  p.tiles_n = (N + bn - 1) / bn;
+  if (static_cast<long long>(p.tiles_n) * blocks > (1 << 30)) return DXB_ERR_SHAPE;
+  p.tiles = p.tiles_n * blocks;
+  // A caller's cap limits the CTAs, which then walk several tiles; without one every tile has its own.
+  int grid = p.tiles;
+  if (budget < sms && grid > budget * (16 / warps)) grid = budget * (16 / warps);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid) * cluster);
+  cfg.blockDim = dim3(32 * warps);
+  p.ring_bytes = warps * k.warp_bytes;
+  const int red_bytes = (warps * 8 * mt * (bn + 1) * 4 + 15) / 16 * 16;
+  if (p.ring_bytes < red_bytes) p.ring_bytes = red_bytes;
+  cfg.dynamicSmemBytes = static_cast<size_t>(p.ring_bytes) + static_cast<size_t>(cluster - 1) * 8 * mt * bn * 4;
+  if (!small_smem_ready(k.fn)) return DXB_ERR_CUDA;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int nattr = 0;
+  if (cluster > 1) {
+    attr[nattr].id = cudaLaunchAttributeClusterDimension;
+    attr[nattr].val.clusterDim.x = cluster;
+    attr[nattr].val.clusterDim.y = 1;
+    attr[nattr].val.clusterDim.z = 1;
+    ++nattr;
+  }
+  if (pdl_enabled() && !opts.serialize) {
+    attr[nattr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[nattr].val.programmaticStreamSerializationAllowed = 1;
+    ++nattr;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = nattr;
+  if (cudaLaunchKernelEx(&cfg, k.fn, p) != cudaSuccess) {
+    cudaGetLastError();
+    return DXB_ERR_CUDA;
+  }
+  return DXB_OK;
+}
+
 template <int BITS>
 static int launch_simt(const void* x, long long ldx, const void* qw, const void* scales,
                        const void* zeros, const void* bias, void* out, long long ldo, int M, int N,
@@ -1568,6 +1679,16 @@ static int read_opts(const dxb_gemm_opts* o, int bits, int M, int N, int K, Opts
   return DXB_OK;
 }
 
+// Few tokens and a weight that is read in little more than the fixed cost of a launch: there the kernel
+// without set-up is ahead; with more to convert the tcgen05 pipeline is.  (One token: int4 512 x
+// 1024 2.1 against 2.8 us, 3072 x 3072 4.6 against 5.5, 3072 x 14336 10.7 against 10.5; int8 512 x 1024
+// 2.3 against 2.9, 3072 x 3072 6.7 against 6.3.)
+static bool small_is_faster(int M, int N, int K, int bits) {
+  static const int forced = [] { const char* e = getenv("DEXTER_B200_SMALL_TOKENS"); return e ? atoi(e) : -1; }();
+  if (forced >= 0) return M <= forced;
+  return M <= 8 && static_cast<long long>(N) * K <= (bits == 4 ? 10ll << 20 : 5ll << 20);
+}
+
 static int gemm_dispatch(int bits, const void* x, int64_t ldx, const void* qweight, const void* scales,
                          const void* zeros, const void* bias, void* out, int64_t ldo, int M, int N, int K,
                          int group_size, void* workspace, size_t workspace_bytes, const Opts& opts,
@@ -1588,6 +1709,12 @@ static int gemm_dispatch(int bits, const void* x, int64_t ldx, const void* qweig
   // The sum over ranks lives in the tensor-core kernel's epilogue only.
   if (opts.peer.world > 1 && !(aligned && gemm_tc_supported(M, N, K, group_size, bits)))
     return DXB_ERR_UNSUPPORTED;
+  // Few tokens, and whatever the tensor-core pipeline cannot take.
+  const bool tc = aligned && gemm_tc_supported(M <= 128 ? M : 128, N, K, group_size, bits);
+  if (opts.peer.world <= 1 && (!tc || small_is_faster(M, N, K, bits)) && small_supported(x, ldx, K, group_size, bits)) {
+    const int rc = launch_small(bits, x, ldx, qweight, scales, zeros, bias, out, ldo, M, N, K, group_size, opts, stream);
+    if (rc != DXB_ERR_UNSUPPORTED) return rc;
+  }
   // More than 128 tokens: one launch over all token blocks when the workspace holds the
   // partial sums of that plan (dxb_workspace_bytes asks for it); a smaller workspace still
   // works, block by block.

@@ -1,0 +1,70 @@
+"""The kernel for few tokens and odd shapes, against the oracle at the edges of its tiles and steps."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-2
+
+
+@pytest.fixture(scope="module")
+def d(b200_lib):
+    import dexter_labs_b200
+
+    return dexter_labs_b200
+
+
+def problem(d, m, k, n, bits, group, symmetric, seed):
+    torch.manual_seed(seed)
+    x = torch.randn(m, k, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(n, k, device="cuda") * 0.02).to(torch.bfloat16)
+    return x, d.quantize(w, bits=bits, group_size=group, symmetric=symmetric,
+                         bias=torch.randn(n, device="cuda").to(torch.bfloat16))
+
+
+def err(got, want):
+    got, want = got.double(), want.double()
+    return (got - want).abs().max().item() / max(want.abs().max().item(), 1e-6)
+
+
+@pytest.mark.parametrize("m,k,n,bits,group,why", [
+    (1, 64, 1, 4, 32, "one step, one column"),
+    (1, 3072, 3072, 4, 128, "96 tiles: sixteen warps, no cluster"),
+    (8, 3072, 9216, 4, 128, "288 tiles: eight warps"),
+    (9, 3072, 14336, 4, 128, "448 tiles: twice the width, second token tile"),
+    (16, 14336, 1536, 4, 128, "48 tiles, long K: clusters"),
+    (3, 14336, 96, 4, 128, "3 tiles: clusters of 8"),
+    (5, 1984, 264, 8, 32, "steps that do not divide by the warps"),
+    (16, 3072, 14344, 8, 3072, "last wide tile cut, one group per channel"),
+    (7, 6144, 100, 8, 128, "four columns past a tile, clusters"),
+    (2, 512, 200, 4, 64, "width no multiple of 16"),
+    (50, 1536, 1000, 4, 32, "several token blocks of groups of 32"),
+    (17, 1024, 131, 4, 32, "odd width: byte-wise loads"),
+    (128, 256, 33, 8, 32, "odd width, int8, eight token blocks"),
+    (130, 320, 77, 8, 64, "more than 128 tokens"),
+])
+@pytest.mark.parametrize("symmetric", [True, False])
+def test_small_kernel_matches_the_oracle(m, k, n, bits, group, why, symmetric, d, oracle):
+    x, q, = problem(d, m, k, n, bits, group, symmetric, seed=m + n)
+    fn = d.w4a16 if bits == 4 else d.w8a16
+    y = fn(x, q.qweight, q.scales, q.zeros, q.bias, group)
+    want = oracle.torch_wq_gemm(x, q.qweight, q.scales, q.zeros, q.bias, group, bits)
+    assert err(y, want) < TOL, why
+    again = fn(x, q.qweight, q.scales, q.zeros, q.bias, group, max_ctas=5)
+    assert err(again, want) < TOL, why + " (capped grid: CTAs walk several tiles)"
+    assert torch.equal(fn(x, q.qweight, q.scales, q.zeros, q.bias, group), y), "not deterministic: " + why
+    gelu = (d.ops.w4a16_gelu if bits == 4 else d.ops.w8a16_gelu)(x, q.qweight, q.scales, q.zeros, q.bias, group)
+    assert torch.equal(gelu, torch.nn.functional.gelu(y.float(), approximate="tanh").to(torch.bfloat16)) or \
+        err(gelu, torch.nn.functional.gelu(want.float(), approximate="tanh")) < TOL
+
+
+@pytest.mark.parametrize("bits,symmetric", [(4, True), (4, False), (8, True), (8, False)])
+def test_single_nonzero_activation_reads_back_the_exact_weight(bits, symmetric, d, oracle):
+    # x = one-hot: the output row IS a dequantised weight row, so layout and arithmetic are checked bit for bit
+    k, n = 256, 40
+    _, q = problem(d, 1, k, n, bits, 64, symmetric, seed=bits)
+    want = oracle.torch_dequantize(q.qweight, q.scales, q.zeros, 64, bits)
+    fn = d.w4a16 if bits == 4 else d.w8a16
+    for k0 in range(0, k, 16):
+        x = torch.zeros(16, k, device="cuda", dtype=torch.bfloat16)
+        x[torch.arange(16), k0 + torch.arange(16)] = 1
+        assert torch.equal(fn(x, q.qweight, q.scales, q.zeros, None, 64), want[k0:k0 + 16])
