@@ -53,12 +53,20 @@ __device__ __forceinline__ uint32_t cvt_bf16x2(float hi, float lo) {
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
   return d;
 }
+// (w & mask) | bits in ONE instruction.  Written as a C expression, its two constants become immediates of two instructions (a three-input LOP3 takes one immediate only), which makes the
+// conversion, bound by the integer pipe, 20 % slower: 405 against 325 cycles per 128 x 128 int4 weights
+// with sixteen warps at it.
+__device__ __forceinline__ uint32_t and_or(uint32_t w, uint32_t mask, uint32_t bits) {
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(w), "r"(mask), "r"(bits));
+  return d;
+}
 // Two nibbles (bits 0..3 and 16..19 of `w`) -> two bf16 weights.  OR-ing a nibble
 // into the mantissa of 0x4300 gives 128 + q exactly; `zero2` holds 128 + zero
 // point in both halves (0x4308 = 136.0 for the symmetric midpoint 8), so the
 // subtract is exact and the multiply is the only rounding.
 __device__ __forceinline__ uint32_t deq4(uint32_t w, uint32_t zero2, uint32_t scale2) {
-  const uint32_t v = (w & 0x000F000Fu) | 0x43004300u;
+  const uint32_t v = and_or(w, 0x000F000Fu, 0x43004300u);
   return mul_bf16x2(sub_bf16x2(v, zero2), scale2);
 }
 // One byte -> fp32 by bit pattern: 0x4B0000qq = 8388608 + q.  `cz` = 8388608 +
@@ -68,17 +76,25 @@ __device__ __forceinline__ float deq8(uint32_t word, uint32_t byte_sel, float cz
   const float f = __uint_as_float(prmt(word, 0x4B000000u, 0x7650u + byte_sel));
   return (f - cz) * scale;
 }
-// Two bytes (bits 0..7 and 16..23 of `w`; the other bits are ignored) -> two bf16 weights.  q - 128 has
-// eight significant bits, so it is exact in bf16: the low seven bits of q OR-ed into 0x4300 give 128 +
-// (q & 127), and the eighth flips the 256 (0x4380) to subtract into a 128.  `zero2` = zero point - 128,
-// subtracted exactly as well (differences of bytes fit eight significant bits); the multiply is the only
-// rounding, as with deq8.
-__device__ __forceinline__ uint32_t deq8x2(uint32_t w, uint32_t zero2, uint32_t scale2, bool has_zero) {
-  const uint32_t v = (w & 0x007F007Fu) | 0x43004300u;
-  uint32_t d = sub_bf16x2(v, (w & 0x00800080u) ^ 0x43804380u);
-  if (has_zero) d = sub_bf16x2(d, zero2);
-  return mul_bf16x2(d, scale2);
+// Bytes in GEMMs: 0x4300qq00 = 128 + q / 256 in fp32, so that ONE fused multiply-add with 256 * scale and
+// -(128 + zero / 256) * 256 * scale gives (q - zero) * scale: the constant has 16 + 8 significant bits and the
+// result 17, so all of it is exact in fp32 and the later cvt.rn to bf16 is the only rounding, as with
+// deq8.  Five instructions per two weights (two byte permutes, two multiply-adds, one conversion),
+// zero points included.
+__device__ __forceinline__ float deq8_fma(uint32_t word, uint32_t byte_sel, float scale256, float offset) {
+  return __fmaf_rn(__uint_as_float(prmt(word, 0x43000000u, 0x7504u + (byte_sel << 4))), scale256, offset);
 }
+// The two constants of a column from its bf16 scale and zero point (as fp32).
+__device__ __forceinline__ void deq8_constants(float scale, float zero, float& scale256, float& offset) {
+  scale256 = scale * 256.0f;
+  offset = -__fmaf_rn(zero, 1.0f / 256.0f, 128.0f) * scale256;
+}
+// Byte `b` of two words (consecutive k of one column) -> a bf16 pair.
+__device__ __forceinline__ uint32_t deq8_pair(uint32_t w0, uint32_t w1, uint32_t b, uint32_t scale256, uint32_t offset) {
+  return cvt_bf16x2(deq8_fma(w1, b, __uint_as_float(scale256), __uint_as_float(offset)),
+                    deq8_fma(w0, b, __uint_as_float(scale256), __uint_as_float(offset)));
+}
+
 __device__ __forceinline__ uint32_t dup_lo(uint32_t w) { return prmt(w, w, 0x1010u); }
 __device__ __forceinline__ uint32_t dup_hi(uint32_t w) { return prmt(w, w, 0x3232u); }
 __device__ __forceinline__ float bf16lo_f32(uint32_t w) { return __uint_as_float(w << 16); }

@@ -37,10 +37,8 @@
 
 namespace dx {
 #ifdef DXB_TRACE
-#define DX_DEBUG(bit) (p.debug & (bit))
 #define DX_TRACE(role, i) do { if (p.trace && (i) < 32) p.trace[(static_cast<long long>(blockIdx.x) * 8 + (role)) * 32 + (i)] = clock64() - t_start; } while (0)
 #else
-#define DX_DEBUG(bit) false
 #define DX_TRACE(role, i) do { } while (0)
 #endif
 
@@ -154,6 +152,8 @@ struct WqParams {
   int max_slots;       // partial slots reserved per tile
   int nacc;            // accumulator buffers in TMEM (2 when NU <= 128)
   int group_shift;     // log2(group / 64) when that is a power of two, else -1
+  int sz_step;         // scale rows a dequant team moves on per unit inside a tile, in 4 x bf16; -1: no
+                       // constant (the group does not divide the teams' stride)
   int cluster;         // CTAs per tile (thread-block cluster along x); 1 = no cluster
   int recv_off;        // cluster mode: byte offset of the receive buffers in shared memory
   int recv_alias;      // cluster mode: the receive buffers lie over the (then idle) rings, so
@@ -167,7 +167,6 @@ struct WqParams {
                          // size, or tiles by the grid size (see the kernel's range arithmetic)
   PeerFuse peer;       // peer.world > 1: the sum over ranks is part of this launch (see below)
   long long* trace;    // only used when built with -DDXB_TRACE
-  int debug;           // -DDXB_TRACE builds only: parts of the pipeline to leave out (timing experiments)
 };
 
 
@@ -273,12 +272,8 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   auto w_issue = [&]() {
     if (elect_one()) {
       const uint32_t fw = bar0 + 8 * (kBarFullW + w_s);
-      if (DX_DEBUG(2) && w_u >= u_begin + SW) {
-        mbar_arrive(fw);  // experiment: reuse what the stage already holds
-      } else {
-        mbar_expect_tx(fw, W_STAGE);
-        tma_load_2d(w_ring + w_s * W_STAGE, &tm_q, fw, (MULTI ? w_ntile : w_tile) * kTileN, w_ku * UNIT_ROWS);
-      }
+      mbar_expect_tx(fw, W_STAGE);
+      tma_load_2d(w_ring + w_s * W_STAGE, &tm_q, fw, (MULTI ? w_ntile : w_tile) * kTileN, w_ku * UNIT_ROWS);
     }
     __syncwarp();
     w_u += 2;
@@ -594,109 +589,98 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     // Activations may be the output of the previous kernel in the stream.
     pdl_wait();
     if (lane == 0) DX_TRACE(5, 3);  // the previous kernel of the stream is complete
-    {
-      int ku = ku_begin, t = 0;
+    // One elected thread runs the whole loop, unrolled over the ring's stages (see the MMA issuer).
+    if (elect_one()) {
+      int ku = ku_begin;
       int ntile = MULTI ? tile_begin % p.tiles_n : 0;
       int row0 = MULTI ? (tile_begin / p.tiles_n) * 128 : 0;  // first token row of the token block
-      uint32_t ph = 0;
-      int issued = 0;
+      uint32_t ph = 1;
+      int u = u_begin;
       bool ok = true;
       const uint32_t x_bytes = p.x_stage_bytes;
-      for (int u = u_begin; u < u_end; ++u) {
-        ok = __all_sync(0xffffffffu, mbar_wait(bar0 + 8 * (kBarFree + t), ph ^ 1u, abortp));
-        if (!ok) break;
-        if (elect_one()) {
-          const uint32_t rb = bar0 + 8 * (kBarReady + t);
-          if (DX_DEBUG(1) && u >= u_begin + kAStages) {
-            mbar_arrive(rb);  // experiment: reuse what the slot already holds
-          } else {
-          mbar_expect_tx(rb, x_bytes);
-          if (BITS == 4) {
-            tma_load_3d(x_ring + t * p.x_stage_bytes, &tm_x, rb, ku * 64, row0, 0);
-          } else {  // two k-blocks of 64, one per plane
-            tma_load_2d(x_ring + t * p.x_stage_bytes, &tm_x, rb, ku * 128, row0);
-            tma_load_2d(x_ring + t * p.x_stage_bytes + (x_bytes >> 1), &tm_x, rb, ku * 128 + 64, row0);
-          }
+      while (u < u_end && ok) {
+#pragma unroll
+        for (int t = 0; t < kAStages; ++t) {
+          if (u < u_end && ok) {
+            ok = mbar_wait(bar0 + 8 * (kBarFree + t), ph, abortp);
+            if (ok) {
+              const uint32_t rb = bar0 + 8 * (kBarReady + t);
+              const uint32_t dst = x_ring + t * p.x_stage_bytes;
+              mbar_expect_tx(rb, x_bytes);
+              if (BITS == 4) {
+                tma_load_3d(dst, &tm_x, rb, ku * 64, row0, 0);
+              } else {  // two k-blocks of 64, one per plane
+                tma_load_2d(dst, &tm_x, rb, ku * 128, row0);
+                tma_load_2d(dst + (x_bytes >> 1), &tm_x, rb, ku * 128 + 64, row0);
+              }
+              ++u;
+              if (++ku == U) {
+                ku = 0;
+                if (MULTI && ++ntile == p.tiles_n) { ntile = 0; row0 += 128; }
+              }
+            }
           }
         }
-        __syncwarp();
-        ++issued;
-        if (++t == kAStages) { t = 0; ph ^= 1u; }
-        if (++ku == U) {
-          ku = 0;
-          if (MULTI && ++ntile == p.tiles_n) { ntile = 0; row0 += 128; }
-        }
+        ph ^= 1u;
       }
-      if (!ok && lane == 0) {
+      if (!ok) {
         // Leaving early: give copies already issued time to land before the CTA exits.
         const long long t0 = clock64();
         while (clock64() - t0 < 2000000) {}
       }
-      (void)issued;
     }
     __syncwarp();
   } else if (warp == 1) {
     // ======================================================= MMA issuer ====
-    // Warp-uniform loop as well: descriptors, TMEM addresses and barrier addresses
-    // live in uniform registers; one elected lane issues the MMAs and commits.
-    {
+    // One elected thread runs the whole loop, unrolled over the four slots so that every operand of a
+    // slot is a constant away from its base.  This warp shares its scheduler with four dequant
+    // warps that keep it about 80 % busy, so each of its instructions waits for a turn: as a
+    // warp-uniform loop with a slot counter a unit's 8 products and its wait took 840 cycles beside
+    // them, twice what the tensor pipe needs for 96 tokens; in this form they take 460.
+    if (elect_one()) {
       const uint32_t idesc = idesc_bf16_f32(kTileN, p.NU);
       const uint64_t xdesc0 = smem_desc_kmajor_sw128(x_ring);
       const uint32_t x_stage16 = static_cast<uint32_t>(p.x_stage_bytes) >> 4;
       const uint32_t plane16 = static_cast<uint32_t>(p.NU * 128) >> 4;
-      int t = 0, b = 0;
-      uint32_t ph = 0, accph = 0;
-      uint64_t xd = xdesc0;
-      uint32_t a_tmem = tmem0 + kACol0;
-      bool ok = true;
-      int u = u_begin, ku0 = ku_begin, done = 0;
-      const bool leader = elect_one();  // the one lane that issues; fixed for the whole loop
-      while (u < u_end && ok) {
-        const int left = u_end - u;
-        const int nun = left < (U - ku0) ? left : (U - ku0);
-        ok = __all_sync(0xffffffffu, mbar_wait(bar0 + 8 * (kBarAccEmpty + b), accph ^ 1u, abortp));
-        if (!ok) break;
-        const uint32_t d_tmem = tmem0 + b * p.NU;
-        uint32_t accumulate = 0;
-        for (int i = 0; i < nun; ++i) {
-          if (!mbar_wait(bar0 + 8 * (kBarReady + t), ph, abortp)) { ok = false; break; }
-          tc_fence_after();
-          if (lane == 0 && done == 0) DX_TRACE(5, 4);  // first unit ready (weights in TMEM, activations in smem)
-          if (leader && DX_DEBUG(32)) {
-            // experiment: the two planes accumulate into different accumulators, alternating
-            const uint32_t d2 = tmem0 + (b ^ 1) * p.NU;
+      const uint32_t a_tmem0 = tmem0 + kACol0;
+      int b = 0;
+      uint32_t ph = 0, accph = 1, accumulate = 0;
+      int left = u_end - u_begin;                        // units of this CTA still to do
+      int seg = left < U - ku_begin ? left : U - ku_begin;  // of them in the current tile
+      uint32_t d_tmem = tmem0;
+      bool ok = left > 0 && mbar_wait(bar0 + 8 * kBarAccEmpty, accph, abortp);
+      while (left > 0 && ok) {
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-              mma_ts(d_tmem, a_tmem + kk * 8, xd + kk * 2, idesc, kk == 0 ? accumulate : 1u);
-              mma_ts(d2, a_tmem + 32 + kk * 8, xd + plane16 + kk * 2, idesc, kk == 0 ? accumulate : 1u);
-            }
-            tc_commit(bar0 + 8 * (kBarFree + t));
-          } else if (leader && !DX_DEBUG(8)) {
-            mma_ts(d_tmem, a_tmem, xd, idesc, accumulate);
+        for (int t = 0; t < kAStages; ++t) {
+          if (left > 0 && ok) {
+            ok = mbar_wait(bar0 + 8 * (kBarReady + t), ph, abortp);
+            if (ok) {
+              tc_fence_after();
+              const uint64_t xd = xdesc0 + t * x_stage16;
+              const uint32_t a_tmem = a_tmem0 + t * A_STAGE_COLS;
+              mma_ts(d_tmem, a_tmem, xd, idesc, accumulate);
 #pragma unroll
-            for (int kk = 1; kk < 4; ++kk) mma_ts(d_tmem, a_tmem + kk * 8, xd + kk * 2, idesc, 1u);
-            if (PLANES == 2) {
+              for (int kk = 1; kk < 4; ++kk) mma_ts(d_tmem, a_tmem + kk * 8, xd + kk * 2, idesc, 1u);
 #pragma unroll
               for (int kk = 0; kk < 4; ++kk)
                 mma_ts(d_tmem, a_tmem + 32 + kk * 8, xd + plane16 + kk * 2, idesc, 1u);
+              tc_commit(bar0 + 8 * (kBarFree + t));
+              accumulate = 1;
+              --left;
+              if (--seg == 0) {
+                tc_commit(bar0 + 8 * (kBarAccFull + b));
+                if (++b == 2) { b = 0; accph ^= 1u; }
+                if (left > 0) {
+                  seg = left < U ? left : U;
+                  accumulate = 0;
+                  d_tmem = tmem0 + b * p.NU;
+                  ok = mbar_wait(bar0 + 8 * (kBarAccEmpty + b), accph, abortp);
+                }
+              }
             }
-            tc_commit(bar0 + 8 * (kBarFree + t));
-          } else if (leader) {
-            tc_commit(bar0 + 8 * (kBarFree + t));
           }
-          accumulate = 1;
-          if (lane == 0) DX_TRACE(3, done);
-          ++done;
-          xd += x_stage16;
-          a_tmem += A_STAGE_COLS;
-          if (++t == kAStages) { t = 0; ph ^= 1u; xd = xdesc0; a_tmem = tmem0 + kACol0; }
         }
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        if (leader) tc_commit(bar0 + 8 * (kBarAccFull + b));
-        u += nun;
-        ku0 = 0;
-        if (++b == 2) { b = 0; accph ^= 1u; }
+        ph ^= 1u;
       }
     }
     __syncwarp();
@@ -744,50 +728,46 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     const int n_local = 32 * q + 4 * g;
     const int group_units = p.group / 64;   // quantisation group in planes of 64 k
     const int half_units = p.half_k / 64;    // int4: planes between the low and the high nibbles
-    const uint2* sc_ptr = reinterpret_cast<const uint2*>(p.scales);
-    const uint2* zr_ptr = reinterpret_cast<const uint2*>(p.zeros);
     const uint32_t a_tmem = tmem0 + kACol0 + team * A_STAGE_COLS;
     const uint32_t a_full_bar = bar0 + 8 * (kBarReady + team);
     const uint32_t a_empty_bar = bar0 + 8 * (kBarFree + team);
 
-    // cursor of this team's current unit
-    int u = u_begin + team;
+    // What a unit costs here beyond its conversion counts: the sixteen warps keep the schedulers
+    // about 80 % busy, and ten instructions more per unit made a launch 9 % longer.
+    int left = (u_end - u_begin - team + kAStages - 1) / kAStages;  // units of this team still to do
     int tile = tile_begin, ku = ku_begin + team;
     while (ku >= U) { ku -= U; ++tile; }
-    int ntile = MULTI ? tile % p.tiles_n : 0;  // column tile of `tile`, kept in step without divisions
     int s = team;  // SW is a multiple of the team count: stages j, j+4, ... belong to team j
     uint32_t ph = 0;
     uint32_t aph = 0;
     bool ok = true;
     // Scales / zero points come straight from global memory (they are tiny and stay in
-    // L2), fetched one team-unit ahead so the load latency is never waited for.
-    uint2 sc[PLANES], zr[PLANES], sc_nx[PLANES], zr_nx[PLANES];
-    const int n4_stride = p.N >> 2;  // uint2 (4 x bf16) elements per scale row
-    auto load_sz = [&](int tile_, int ntile_, int ku_, uint2 (&s_out)[PLANES], uint2 (&z_out)[PLANES]) {
-      const int n = ntile_ * kTileN + n_local;
-      const bool in = n < p.N && tile_ < p.tiles;
+    // L2), fetched one team-unit ahead so the load latency is never waited for.  Inside a tile their
+    // row moves on by the same amount from unit to unit (p.sz_step) unless the group is no
+    // divisor of the teams' stride.
+    uint2 sc[PLANES], zr[PLANES];
+    int sz[PLANES];  // offset of the current rows, in 4 x bf16
+    const int n4_stride = p.N >> 2;
+    auto seek_sz = [&]() {  // rows of unit (tile, ku); columns beyond N (last tile) re-read the last ones
+      int n4 = ((MULTI ? tile % p.tiles_n : tile) * kTileN + n_local) >> 2;
+      n4 = n4 < n4_stride ? n4 : n4_stride - 1;
 #pragma unroll
       for (int pl = 0; pl < PLANES; ++pl) {
-        const int kunit = BITS == 4 ? ku_ + pl * half_units : 2 * ku_ + pl;  // plane of 64 k
-        const int grp = p.group_shift >= 0 ? (kunit >> p.group_shift) : (kunit / group_units);
-        const int idx = grp * n4_stride + (n >> 2);
-        s_out[pl] = in ? __ldg(sc_ptr + idx) : make_uint2(0u, 0u);
-        if (HAS_ZERO) z_out[pl] = in ? __ldg(zr_ptr + idx) : make_uint2(0u, 0u);
+        const int kunit = BITS == 4 ? ku + pl * half_units : 2 * ku + pl;  // plane of 64 k
+        sz[pl] = (p.group_shift >= 0 ? (kunit >> p.group_shift) : (kunit / group_units)) * n4_stride + n4;
       }
     };
-    if (u < u_end) load_sz(tile, MULTI ? ntile : tile, ku, sc_nx, zr_nx);
-    while (u < u_end) {
+    auto load_sz = [&]() {
 #pragma unroll
-      for (int pl = 0; pl < PLANES; ++pl) { sc[pl] = sc_nx[pl]; if (HAS_ZERO) zr[pl] = zr_nx[pl]; }
-      {
-        int ku_n = ku + kAStages, tile_n = tile;
-        int ntile_n = ntile;
-        while (ku_n >= U) { ku_n -= U; ++tile_n; if (MULTI && ++ntile_n == p.tiles_n) ntile_n = 0; }
-        if (u + kAStages < u_end) load_sz(tile_n, MULTI ? ntile_n : tile_n, ku_n, sc_nx, zr_nx);
+      for (int pl = 0; pl < PLANES; ++pl) {
+        sc[pl] = __ldg(reinterpret_cast<const uint2*>(p.scales) + sz[pl]);
+        if (HAS_ZERO) zr[pl] = __ldg(reinterpret_cast<const uint2*>(p.zeros) + sz[pl]);
       }
+    };
+    if (left > 0) { seek_sz(); load_sz(); }
+    while (left > 0) {
       ok = mbar_wait(bar0 + 8 * (kBarFullW + s), ph, abortp);
       if (!ok) break;
-      if (q == 0 && lane == 0) DX_TRACE(4, (u - u_begin));
       const uint32_t wsrc = w_ring + s * W_STAGE;
       uint32_t w0[8], w1[8];
 #pragma unroll
@@ -799,56 +779,80 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         __syncwarp();  // every lane has its words in registers
         if (lane == 0) mbar_arrive(bar0 + 8 * (kBarEmptyW + s));
       }
+      // This unit's scales and zero points as the conversion wants them (int4: in both halves of a
+      // word; int8: the constants of deq8_fma); then the next unit's rows.
+      uint32_t s2[PLANES][4], z2[PLANES][4];
+#pragma unroll
+      for (int pl = 0; pl < PLANES; ++pl) {
+        if (BITS == 4) {
+          s2[pl][0] = dup_lo(sc[pl].x); s2[pl][1] = dup_hi(sc[pl].x);
+          s2[pl][2] = dup_lo(sc[pl].y); s2[pl][3] = dup_hi(sc[pl].y);
+          if (HAS_ZERO) {
+            z2[pl][0] = dup_lo(zr[pl].x); z2[pl][1] = dup_hi(zr[pl].x);
+            z2[pl][2] = dup_lo(zr[pl].y); z2[pl][3] = dup_hi(zr[pl].y);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) z2[pl][i] = 0x43084308u;  // 128 + 8
+          }
+        } else {
+          const float sf[4] = {bf16lo_f32(sc[pl].x), bf16hi_f32(sc[pl].x), bf16lo_f32(sc[pl].y), bf16hi_f32(sc[pl].y)};
+          float zf[4] = {128.0f, 128.0f, 128.0f, 128.0f};
+          if (HAS_ZERO) {
+            zf[0] = bf16lo_f32(zr[pl].x); zf[1] = bf16hi_f32(zr[pl].x);
+            zf[2] = bf16lo_f32(zr[pl].y); zf[3] = bf16hi_f32(zr[pl].y);
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            float s256, off;
+            deq8_constants(sf[i], zf[i], s256, off);
+            s2[pl][i] = __float_as_uint(s256);
+            z2[pl][i] = __float_as_uint(off);
+          }
+        }
+      }
+      if (--left > 0) {
+        ku += kAStages;
+        if (ku >= U || p.sz_step < 0) {
+          while (ku >= U) { ku -= U; ++tile; }
+          seek_sz();
+        } else {
+#pragma unroll
+          for (int pl = 0; pl < PLANES; ++pl) sz[pl] += p.sz_step;
+        }
+        load_sz();
+      }
       ok = mbar_wait(a_empty_bar, aph ^ 1u, abortp);
       if (!ok) break;
-      if (q == 0 && lane == 0) DX_TRACE(6, (u - u_begin));
       tc_fence_after();
       if (BITS == 4) {
 #pragma unroll
         for (int pl = 0; pl < 2; ++pl) {
-          const uint32_t s2[4] = {dup_lo(sc[pl].x), dup_hi(sc[pl].x), dup_lo(sc[pl].y),
-                                  dup_hi(sc[pl].y)};
-          uint32_t z2[4];
-          if (HAS_ZERO) {
-            z2[0] = dup_lo(zr[pl].x); z2[1] = dup_hi(zr[pl].x);
-            z2[2] = dup_lo(zr[pl].y); z2[3] = dup_hi(zr[pl].y);
-          } else {
-            z2[0] = z2[1] = z2[2] = z2[3] = 0x43084308u;  // 128 + 8
-          }
 #pragma unroll
           for (int rh = 0; rh < 2; ++rh) {
             uint32_t ra[8], rb[8];
 #pragma unroll
             for (int sl = 0; sl < 4; ++sl) {
-              if (DX_DEBUG(4)) {
-                ra[2 * sl] = w0[4 * rh + sl]; ra[2 * sl + 1] = w1[4 * rh + sl];
-                rb[2 * sl] = w0[4 * rh + sl]; rb[2 * sl + 1] = w1[4 * rh + sl];
-              } else if (RELAID) {
+              if (RELAID) {
                 // The word of the even row holds the low-nibble plane, the word of the odd
                 // row the high-nibble plane: nibble b is byte column b of the even row,
                 // nibble 4 + b the same column of the odd row, so masking with 0x000F000F
                 // after a shift by 4b yields the k-pair of column b directly.
                 const uint32_t W = pl == 0 ? w0[4 * rh + sl] : w1[4 * rh + sl];
-                ra[2 * sl + 0] = deq4(W, z2[0], s2[0]);
-                ra[2 * sl + 1] = deq4(W >> 4, z2[1], s2[1]);
-                rb[2 * sl + 0] = deq4(W >> 8, z2[2], s2[2]);
-                rb[2 * sl + 1] = deq4(W >> 12, z2[3], s2[3]);
+                ra[2 * sl + 0] = deq4(W, z2[pl][0], s2[pl][0]);
+                ra[2 * sl + 1] = deq4(W >> 4, z2[pl][1], s2[pl][1]);
+                rb[2 * sl + 0] = deq4(W >> 8, z2[pl][2], s2[pl][2]);
+                rb[2 * sl + 1] = deq4(W >> 12, z2[pl][3], s2[pl][3]);
               } else {
                 const uint32_t P = prmt(w0[4 * rh + sl], w1[4 * rh + sl], 0x5410u) >> (4 * pl);
                 const uint32_t Q = prmt(w0[4 * rh + sl], w1[4 * rh + sl], 0x7632u) >> (4 * pl);
-                ra[2 * sl + 0] = deq4(P, z2[0], s2[0]);
-                ra[2 * sl + 1] = deq4(P >> 8, z2[1], s2[1]);
-                rb[2 * sl + 0] = deq4(Q, z2[2], s2[2]);
-                rb[2 * sl + 1] = deq4(Q >> 8, z2[3], s2[3]);
+                ra[2 * sl + 0] = deq4(P, z2[pl][0], s2[pl][0]);
+                ra[2 * sl + 1] = deq4(P >> 8, z2[pl][1], s2[pl][1]);
+                rb[2 * sl + 0] = deq4(Q, z2[pl][2], s2[pl][2]);
+                rb[2 * sl + 1] = deq4(Q >> 8, z2[pl][3], s2[pl][3]);
               }
             }
-            if (!DX_DEBUG(16)) {
-              tmem_st_16x128b_x4(tmem_addr(a_tmem + pl * 32 + 16 * rh, lane_base, 0), ra);
-              tmem_st_16x128b_x4(tmem_addr(a_tmem + pl * 32 + 16 * rh, lane_base + 16, 0), rb);
-            } else {
-              asm volatile("" ::"r"(ra[0] ^ ra[1] ^ ra[2] ^ ra[3] ^ ra[4] ^ ra[5] ^ ra[6] ^ ra[7] ^ rb[0] ^ rb[1] ^ rb[2] ^
-                                    rb[3] ^ rb[4] ^ rb[5] ^ rb[6] ^ rb[7]));  // keep the conversion alive
-            }
+            tmem_st_16x128b_x4(tmem_addr(a_tmem + pl * 32 + 16 * rh, lane_base, 0), ra);
+            tmem_st_16x128b_x4(tmem_addr(a_tmem + pl * 32 + 16 * rh, lane_base + 16, 0), rb);
           }
         }
       } else {
@@ -864,25 +868,16 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
             __syncwarp();
             if (lane == 0) mbar_arrive(bar0 + 8 * (kBarEmptyW + s));
           }
-          const float sf[4] = {bf16lo_f32(sc[pl].x), bf16hi_f32(sc[pl].x), bf16lo_f32(sc[pl].y),
-                               bf16hi_f32(sc[pl].y)};
-          float cz[4];
-          if (HAS_ZERO) {
-            cz[0] = 8388608.0f + bf16lo_f32(zr[pl].x); cz[1] = 8388608.0f + bf16hi_f32(zr[pl].x);
-            cz[2] = 8388608.0f + bf16lo_f32(zr[pl].y); cz[3] = 8388608.0f + bf16hi_f32(zr[pl].y);
-          } else {
-            cz[0] = cz[1] = cz[2] = cz[3] = 8388608.0f + 128.0f;
-          }
 #pragma unroll
           for (int rh = 0; rh < 2; ++rh) {
             uint32_t ra[8], rb[8];
 #pragma unroll
             for (int sl = 0; sl < 4; ++sl) {
               const uint32_t x0 = w0[4 * rh + sl], x1 = w1[4 * rh + sl];
-              ra[2 * sl + 0] = cvt_bf16x2(deq8(x1, 0, cz[0], sf[0]), deq8(x0, 0, cz[0], sf[0]));
-              ra[2 * sl + 1] = cvt_bf16x2(deq8(x1, 1, cz[1], sf[1]), deq8(x0, 1, cz[1], sf[1]));
-              rb[2 * sl + 0] = cvt_bf16x2(deq8(x1, 2, cz[2], sf[2]), deq8(x0, 2, cz[2], sf[2]));
-              rb[2 * sl + 1] = cvt_bf16x2(deq8(x1, 3, cz[3], sf[3]), deq8(x0, 3, cz[3], sf[3]));
+              ra[2 * sl + 0] = deq8_pair(x0, x1, 0, s2[pl][0], z2[pl][0]);
+              ra[2 * sl + 1] = deq8_pair(x0, x1, 1, s2[pl][1], z2[pl][1]);
+              rb[2 * sl + 0] = deq8_pair(x0, x1, 2, s2[pl][2], z2[pl][2]);
+              rb[2 * sl + 1] = deq8_pair(x0, x1, 3, s2[pl][3], z2[pl][3]);
             }
             tmem_st_16x128b_x4(tmem_addr(a_tmem + pl * 32 + 16 * rh, lane_base, 0), ra);
             tmem_st_16x128b_x4(tmem_addr(a_tmem + pl * 32 + 16 * rh, lane_base + 16, 0), rb);
@@ -893,13 +888,9 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(a_full_bar);
-      if (q == 0 && lane == 0) DX_TRACE(2, (u - u_begin));
       aph ^= 1u;
       s += kAStages;
       if (s >= SW) { s -= SW; ph ^= 1u; }
-      ku += kAStages;
-      while (ku >= U) { ku -= U; ++tile; if (MULTI && ++ntile == p.tiles_n) ntile = 0; }
-      u += kAStages;
     }
   }
 
@@ -1446,12 +1437,11 @@ static int launch_tc(const void* x, long long ldx, const void* qw, const void* s
     int sh = -1;
     for (int b = 0; b < 20; ++b) if ((1 << b) == gu) sh = b;
     p.group_shift = sh;
+    // Planes of 64 k from one of a team's units to its next, in quantisation groups.
+    const int stride = kAStages * (BITS == 4 ? 1 : 2);
+    p.sz_step = group == K ? 0 : stride % gu == 0 ? stride / gu * (N / 4) : -1;
   }
   p.trace = g_trace;
-  {
-    static const int dbg = [] { const char* e = getenv("DXB_DEBUG"); return e ? atoi(e) : 0; }();
-    p.debug = dbg;
-  }
   p.epilogue = opts.epilogue;
   p.tile_ranges = (cluster == 1 && pl.whole) ? 1 : 0;
   p.peer = opts.peer;

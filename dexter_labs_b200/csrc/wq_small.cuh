@@ -273,14 +273,18 @@ __global__ void __launch_bounds__(CPW == 1 ? 512 : 256, CPW == 1 ? 1 : 2) wq_gem
           for (int th = 0; th < 2; ++th) {  // 16 columns: 4g + 2 th and the next, of word wd
             const int t = 2 * wd + th;
             const uint32_t sp = th ? sv.y : sv.x;
-            const uint32_t s0 = dup_lo(sp), s1 = dup_hi(sp);
-            uint32_t z0, z1;
-            if (has_zero) {
-              const uint32_t zp = th ? zv.y : zv.x;
-              z0 = dup_lo(zp); z1 = dup_hi(zp);
-              if (!W4) { z0 = sub_bf16x2(z0, 0x43004300u); z1 = sub_bf16x2(z1, 0x43004300u); }
+            const uint32_t zp = th ? zv.y : zv.x;
+            uint32_t s0, s1, z0, z1;
+            if (W4) {
+              s0 = dup_lo(sp); s1 = dup_hi(sp);
+              z0 = has_zero ? dup_lo(zp) : 0x43084308u;
+              z1 = has_zero ? dup_hi(zp) : 0x43084308u;
             } else {
-              z0 = z1 = W4 ? 0x43084308u : 0u;
+              float f, o;
+              deq8_constants(bf16lo_f32(sp), has_zero ? bf16lo_f32(zp) : 128.0f, f, o);
+              s0 = __float_as_uint(f); z0 = __float_as_uint(o);
+              deq8_constants(bf16hi_f32(sp), has_zero ? bf16hi_f32(zp) : 128.0f, f, o);
+              s1 = __float_as_uint(f); z1 = __float_as_uint(o);
             }
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -298,8 +302,8 @@ __global__ void __launch_bounds__(CPW == 1 ? 512 : 256, CPW == 1 ? 1 : 2) wq_gem
                   a[2 * j] = deq4(P, z0, s0);
                   a[2 * j + 1] = deq4(P >> 8, z1, s1);
                 } else {
-                  a[2 * j] = deq8x2(prmt(we, wo, th ? 0x0602u : 0x0400u), z0, s0, has_zero);
-                  a[2 * j + 1] = deq8x2(prmt(we, wo, th ? 0x0703u : 0x0501u), z1, s1, has_zero);
+                  a[2 * j] = deq8_pair(we, wo, 2 * th, s0, z0);
+                  a[2 * j + 1] = deq8_pair(we, wo, 2 * th + 1, s1, z1);
                 }
               }
 #pragma unroll
