@@ -196,11 +196,9 @@ __device__ __forceinline__ uint2 finish_row4(float f0, float f1, float f2, float
 // common launches execute, which keeps their code a third of the general instance's: these
 // launches last 8-15 us, and a kernel whose code is larger than the instruction cache pays for
 // fetching it again in every launch (measured: 12.6 against 13.5 us on the headline shape).
-//   kModeGeneral  every epilogue (activation, sum over ranks), tiles shared between CTAs
-//                 through global partial sums, clusters
-//   kModeWhole    whole tiles per CTA, plain epilogue (optional bias), no cluster
-//   kModeCluster  one tile per cluster (K split, sum through distributed shared memory),
-//                 plain epilogue
+//   kModeGeneral  the sum over ranks, tiles shared between CTAs through global partial sums, clusters
+//   kModeWhole    whole tiles per CTA, no cluster
+//   kModeCluster  one tile per cluster (K split, sum through distributed shared memory)
 enum : int { kModeGeneral = 0, kModeWhole = 1, kModeCluster = 2 };
 
 template <int BITS, bool HAS_ZERO, bool MULTI, bool RELAID, int MODE>
@@ -387,7 +385,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     // Sum over ranks fused into this launch (one token block only): finished rows go to
     // every rank's receive buffer instead of `out`; fused_finish then completes the tile.
     const bool fused = !kLean && p.peer.world > 1;
-    const bool plain = kLean || (!fused && p.epilogue == DXB_EPILOGUE_NONE);
+    const bool plain = !fused && p.epilogue == DXB_EPILOGUE_NONE;
     const unsigned parity =
         fused ? (__ldcg(reinterpret_cast<const unsigned*>(p.peer.region[p.peer.rank])) & 1u) : 0u;
     auto fused_finish = [&]() -> bool {
@@ -939,7 +937,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     pdl_wait();
     if (threadIdx.x == 0) DX_TRACE(7, 4);  // previous kernel complete
     const bool fused = !kLean && p.peer.world > 1;
-    const int epi = kLean ? static_cast<int>(DXB_EPILOGUE_NONE) : p.epilogue;
+    const int epi = p.epilogue;
     const unsigned parity =
         fused ? (__ldcg(reinterpret_cast<const unsigned*>(p.peer.region[p.peer.rank])) & 1u) : 0u;
     if (n < p.N) {
@@ -1330,8 +1328,8 @@ static int launch_tc(const void* x, long long ldx, const void* qw, const void* s
   }
   const bool multi = plp->tiles > plp->tiles_n;
   const bool relaid = BITS == 4 && opts.relaid;
-  // The lean instances serve the plain epilogue; which of the two follows from the plan below.
-  const bool lean = opts.epilogue == DXB_EPILOGUE_NONE && opts.peer.world <= 1;
+  // The lean instances serve every launch without a sum over ranks; which of the two follows from the plan below.
+  const bool lean = opts.peer.world <= 1;
   auto kernel = pick_kernel<BITS, HAS_ZERO>(multi, relaid, lean ? kModeCluster : kModeGeneral);
 
   // Few tiles: split each tile's K range over a thread-block cluster (<= 8 CTAs) that
