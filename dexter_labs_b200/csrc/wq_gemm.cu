@@ -352,9 +352,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   // epilogue warps (one per TMEM lane quadrant).  Accumulator lane 32q + 8b + g holds weight
   // column 32q + 4g + b (see the dequant mapping), so the 16x128b load shape hands thread
   // (g, c) the four consecutive columns 4g..4g+3 of token 4*rep + c: one 8-byte store each.
-  // Returns false when a bounded wait ran out.  (Letting the then idle dequant warps share
-  // the last segment's columns was measured: it shortens a whole tile's epilogue by 0.3 us
-  // but its register cost slows the cluster-split launches by more.)
+  // Returns false when a bounded wait ran out.
   // Bias of this thread's four columns of a tile (fetched before waiting for the accumulator,
   // so that its latency is not added to the tail of the tile).
   auto load_bias4 = [&](int tile, float (&bias4)[4]) {
@@ -367,8 +365,10 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       bias4[2] = bf16lo_f32(bb.y); bias4[3] = bf16hi_f32(bb.y);
     }
   };
-  auto epilogue_segment = [&](int tile, int ku0, int nun, int b, const float (&bias4)[4]) -> bool {
-    constexpr int wk = 0, nwk = 1, nthr = kEpilogueThreads;  // the four epilogue warps, all columns
+  // `wk` of `nwk`: which 16-token chunks of the accumulator the calling warp takes.
+  auto epilogue_segment = [&](int tile, int ku0, int nun, int b, const float (&bias4)[4], const int wk,
+                              const int nwk) -> bool {
+    constexpr int nthr = kEpilogueThreads;  // (the sum over ranks and shared tiles: the four epilogue warps)
     const int wtid = (warp - 4) * 32 + lane;
     const int q = warp & 3;
     const int c = lane & 3;
@@ -452,7 +452,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0 && wk == 0) mbar_arrive(bar0 + 8 * (kBarAccEmpty + b));
+      if (lane == 0 && nwk == 1) mbar_arrive(bar0 + 8 * (kBarAccEmpty + b));
       if (fused && !fused_finish()) return false;
     } else if (clustered) {
       // Cluster mode: CTA r of the cluster finishes token rows [r*rows_per, (r+1)*rows_per)
@@ -697,7 +697,8 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       if (!mbar_wait(bar0 + 8 * (kBarAccFull + b), accph, abortp)) break;
       if (etid == 0) DX_TRACE(0, tile - tile_begin);
       tc_fence_after();
-      if (!epilogue_segment(tile, ku0, nun, b, bias4)) break;
+      if (MODE == kModeWhole && u + nun == u_end) break;  // the last tile is everybody's, see below
+      if (!epilogue_segment(tile, ku0, nun, b, bias4, 0, 1)) break;
       if (etid == 0) DX_TRACE(1, tile - tile_begin);
       u += nun;
       ku0 = 0;
@@ -895,6 +896,20 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   tc_fence_before();
   __syncthreads();
   if (threadIdx.x == 0) DX_TRACE(7, 1);  // every role is through its loop
+  if (MODE == kModeWhole && !abort_flag) {
+    // The CTA's last tile: its accumulator is complete (the epilogue warps have waited for it) and
+    // every other warp is idle, so all 24 finish it, six per TMEM lane quadrant with a 16-token chunk
+    // each, instead of four walking six chunks.
+    const int tiles = cut_end - cut_begin;
+    const int tile = cut_end - 1;
+    float bias4[4];
+    load_bias4(tile, bias4);
+    pdl_wait();
+    tc_fence_after();
+    epilogue_segment(tile, 0, U, (tiles - 1) & 1, bias4, warp >> 2, kThreads / 128);
+    tc_fence_before();
+    __syncthreads();  // before the accumulator's TMEM is given back
+  }
   if (clustered) {
     // The cluster's tile: token block and column tile.
     const int tblock = MULTI ? ctile / p.tiles_n : 0;
