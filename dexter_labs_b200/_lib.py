@@ -101,17 +101,25 @@ def load_fast():
     return _dxb_fast.gemm
 
 
-def load_call(relaid: dict):
-    """The native eager call (``_dxb_call``) bound to this library and to the cache of repacked
-    weights, or None when it has not been built (ops.py then makes every call itself)."""
-    lib = load()
-    try:
-        from . import _dxb_call
-    except ImportError:
-        return None
-    _dxb_call.bind(ctypes.cast(lib.dxb_wq_gemm_ex, c_void_p).value,
-                   ctypes.cast(lib.dxb_workspace_bytes_ex, c_void_p).value, relaid)
-    return _dxb_call
+_relaid: dict = {}  # repacked int4 weights; kept and explained in ops.py
+_call_module = None
+
+
+def load_call():
+    """The native eager calls (``_dxb_call``) bound to this library and to the cache of repacked
+    weights, or None when they have not been built (the callers then do everything themselves)."""
+    global _call_module
+    if _call_module is None:
+        lib = load()
+        try:
+            from . import _dxb_call
+        except ImportError:
+            return None
+        entries = (lib.dxb_wq_gemm_ex, lib.dxb_workspace_bytes_ex, lib.dxb_quantize, lib.dxb_quantize_scratch_bytes,
+                   lib.dxb_dequantize_ex)
+        _dxb_call.bind(*(ctypes.cast(fn, c_void_p).value for fn in entries), _relaid)
+        _call_module = _dxb_call
+    return _call_module
 
 
 def strerror(code: int) -> str:

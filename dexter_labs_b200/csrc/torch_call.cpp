@@ -1,4 +1,5 @@
-// _dxb_call: one whole eager call of the registered kernels, from tensors to a launched kernel.
+// _dxb_call: whole eager calls, from tensors to a launched kernel: the registered GEMM kernels, and the
+// two ends of a weight's life (packing and unpacking).
 //
 // A GEMM of this package lasts 5 to 15 us, and a call made of Python statements (attribute
 // reads, data_ptr(), dictionary look-ups, torch.empty) costs about as much host time as that, so
@@ -7,9 +8,12 @@
 // types, contiguous, on the current device, weight already repacked, workspace already there -- and
 // returns None for everything else, errors included, which ops.py then handles as before.
 //
-//   bind(gemm_ex, workspace_bytes_ex, relaid)  addresses in the loaded library, the cache of repacked weights
+//   bind(gemm_ex, workspace_bytes_ex, quantize, quantize_scratch_bytes, dequantize_ex, relaid)
+//                                              addresses in the loaded library, the cache of repacked weights
 //   set_workspace(device, stream, ptr, bytes)  what ops.py holds for that stream (0 bytes: nothing)
 //   call(bits, x, qweight, scales, zeros, bias, group_size, max_ctas, layout, epilogue, pinned) -> Tensor | None
+//   quantize(weight, bits, group_size, symmetric) -> (qweight, scales, zeros | None) | None
+//   dequantize(qweight, scales, zeros, group_size, bits, layout) -> Tensor | None
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -27,9 +31,15 @@ namespace {
 
 using GemmEx = decltype(&dxb_wq_gemm_ex);
 using WorkspaceBytes = decltype(&dxb_workspace_bytes_ex);
+using Quantize = decltype(&dxb_quantize);
+using ScratchBytes = decltype(&dxb_quantize_scratch_bytes);
+using Dequantize = decltype(&dxb_dequantize_ex);
 
 GemmEx g_gemm = nullptr;
 WorkspaceBytes g_workspace_bytes = nullptr;
+Quantize g_quantize = nullptr;
+ScratchBytes g_scratch_bytes = nullptr;
+Dequantize g_dequantize = nullptr;
 PyObject* g_relaid = nullptr;  // id(qweight) -> (weak reference, version, repacked copy or None), owned by ops.py
 
 struct Mix {
@@ -41,12 +51,19 @@ struct Mix {
 std::unordered_map<std::pair<uint64_t, uint64_t>, std::pair<void*, size_t>, Mix> g_workspaces;  // (device, stream)
 std::unordered_map<std::pair<uint64_t, uint64_t>, size_t, Mix> g_need;                          // (shape words)
 
+template <class F>
+F at_address(unsigned long long v) { return reinterpret_cast<F>(static_cast<uintptr_t>(v)); }
+
 PyObject* bind(PyObject*, PyObject* args) {
-  unsigned long long gemm = 0, bytes = 0;
+  unsigned long long gemm = 0, bytes = 0, quantize = 0, scratch = 0, dequantize = 0;
   PyObject* relaid = nullptr;
-  if (!PyArg_ParseTuple(args, "KKO!", &gemm, &bytes, &PyDict_Type, &relaid)) return nullptr;
-  g_gemm = reinterpret_cast<GemmEx>(static_cast<uintptr_t>(gemm));
-  g_workspace_bytes = reinterpret_cast<WorkspaceBytes>(static_cast<uintptr_t>(bytes));
+  if (!PyArg_ParseTuple(args, "KKKKKO!", &gemm, &bytes, &quantize, &scratch, &dequantize, &PyDict_Type, &relaid))
+    return nullptr;
+  g_gemm = at_address<GemmEx>(gemm);
+  g_workspace_bytes = at_address<WorkspaceBytes>(bytes);
+  g_quantize = at_address<Quantize>(quantize);
+  g_scratch_bytes = at_address<ScratchBytes>(scratch);
+  g_dequantize = at_address<Dequantize>(dequantize);
   Py_INCREF(relaid);
   Py_XSETREF(g_relaid, relaid);
   Py_RETURN_NONE;
@@ -172,11 +189,79 @@ PyObject* call(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   }
 }
 
+PyObject* quantize(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  if (n_args != 4) {
+    PyErr_SetString(PyExc_TypeError, "_dxb_call.quantize takes exactly 4 arguments");
+    return nullptr;
+  }
+  const at::Tensor* w = plain_tensor(a[0]);
+  const long bits = PyLong_AsLong(a[1]), group = PyLong_AsLong(a[2]);
+  if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
+  const bool symmetric = a[3] == Py_True;
+  if (!g_quantize || !w || (bits != 4 && bits != 8) || !w->is_cuda() || w->scalar_type() != at::kBFloat16 || w->dim() != 2 ||
+      !w->is_contiguous() || w->device().index() != c10::cuda::current_device())
+    Py_RETURN_NONE;
+  const int64_t n = w->size(0), k = w->size(1);
+  if (n <= 0 || k <= 0 || group <= 0 || k % group || n > INT32_MAX || k > INT32_MAX) Py_RETURN_NONE;
+  try {
+    const auto bytes = w->options().dtype(at::kByte);
+    at::Tensor q = at::empty({bits == 4 ? k / 2 : k, n}, bytes), s = at::empty({k / group, n}, w->options()), z, scratch;
+    if (!symmetric) z = at::empty({k / group, n}, w->options());
+    const size_t need = g_scratch_bytes(static_cast<int>(n), static_cast<int>(k), static_cast<int>(group), static_cast<int>(bits));
+    if (need) scratch = at::empty({static_cast<int64_t>(need)}, bytes);
+    const auto stream = c10::cuda::getCurrentCUDAStream(w->device().index()).stream();
+    const int rc = g_quantize(w->const_data_ptr(), q.mutable_data_ptr(), s.mutable_data_ptr(),
+                              symmetric ? nullptr : z.mutable_data_ptr(), need ? scratch.mutable_data_ptr() : nullptr,
+                              static_cast<int>(n), static_cast<int>(k), static_cast<int>(group), static_cast<int>(bits),
+                              symmetric ? 1 : 0, stream);
+    if (rc != DXB_OK) Py_RETURN_NONE;  // shapes the kernel does not take
+    PyObject* zeros = Py_NewRef(Py_None);
+    if (!symmetric) Py_SETREF(zeros, THPVariable_Wrap(std::move(z)));
+    return Py_BuildValue("(NNN)", THPVariable_Wrap(std::move(q)), THPVariable_Wrap(std::move(s)), zeros);
+  } catch (const std::exception&) {
+    Py_RETURN_NONE;
+  }
+}
+
+PyObject* dequantize(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  if (n_args != 6) {
+    PyErr_SetString(PyExc_TypeError, "_dxb_call.dequantize takes exactly 6 arguments");
+    return nullptr;
+  }
+  const at::Tensor *q = plain_tensor(a[0]), *s = plain_tensor(a[1]);
+  const at::Tensor* z = a[2] == Py_None ? nullptr : plain_tensor(a[2]);
+  const long group = PyLong_AsLong(a[3]), bits = PyLong_AsLong(a[4]), layout = PyLong_AsLong(a[5]);
+  if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
+  if (!g_dequantize || !q || !s || (a[2] != Py_None && !z) || !q->is_cuda() || q->scalar_type() != at::kByte || q->dim() != 2 ||
+      !q->is_contiguous() || s->scalar_type() != at::kBFloat16 || !s->is_contiguous() ||
+      (z && (z->scalar_type() != at::kBFloat16 || !z->is_contiguous())))
+    Py_RETURN_NONE;
+  const auto dev = q->device();
+  if (dev.index() != c10::cuda::current_device() || s->device() != dev || (z && z->device() != dev)) Py_RETURN_NONE;
+  const int64_t n = q->size(1), k = q->size(0) * (bits == 4 ? 2 : 1);
+  if (n <= 0 || k <= 0 || n > INT32_MAX || k > INT32_MAX || group > INT32_MAX) Py_RETURN_NONE;
+  try {
+    at::Tensor out = at::empty({k, n}, s->options());
+    const auto stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+    const int rc = g_dequantize(q->const_data_ptr(), s->const_data_ptr(), z ? z->const_data_ptr() : nullptr,
+                                out.mutable_data_ptr(), static_cast<int>(n), static_cast<int>(k), static_cast<int>(group),
+                                static_cast<int>(bits), static_cast<int>(layout), stream);
+    if (rc != DXB_OK) Py_RETURN_NONE;  // the general path reports it
+    return THPVariable_Wrap(std::move(out));
+  } catch (const std::exception&) {
+    Py_RETURN_NONE;
+  }
+}
+
+PyCFunction fastcall(PyObject* (*f)(PyObject*, PyObject* const*, Py_ssize_t)) {
+  return reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f));
+}
 PyMethodDef methods[] = {
-    {"bind", bind, METH_VARARGS, "bind(gemm_ex, workspace_bytes_ex, relaid)"},
+    {"bind", bind, METH_VARARGS, "bind(addresses in the library..., relaid)"},
     {"set_workspace", set_workspace, METH_VARARGS, "set_workspace(device, stream, ptr, bytes)"},
-    {"call", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(call)), METH_FASTCALL,
-     "one eager GEMM, or None where the general path has to take it"},
+    {"call", fastcall(call), METH_FASTCALL, "one eager GEMM, or None where the general path has to take it"},
+    {"quantize", fastcall(quantize), METH_FASTCALL, "a weight packed, or None where the general path has to do it"},
+    {"dequantize", fastcall(dequantize), METH_FASTCALL, "the dense weight, or None where the general path has to make it"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_dxb_call", "native eager call", -1, methods,
                           nullptr, nullptr, nullptr, nullptr};

@@ -173,12 +173,12 @@ _CHECK = bool(os.environ.get("DEXTER_B200_CHECK"))
 
 # ------------------------------------------------------------ load-time re-layout (int4)
 # id(qweight) -> (weak reference to it, its version counter, the repacked copy or None)
-_relaid: Dict[int, Tuple[object, int, Optional[torch.Tensor]]] = {}
+_relaid: Dict[int, Tuple[object, int, Optional[torch.Tensor]]] = _lib._relaid
 _AUTO_RELAYOUT = os.environ.get("DEXTER_B200_RELAYOUT", "1") != "0"
 
 # The plain eager call in native code (csrc/torch_call.cpp).  It answers None whenever anything about
 # the call is out of the ordinary, errors included: _run below then takes it.
-_NATIVE = None if os.environ.get("DEXTER_B200_FASTCALL", "1") == "0" else _lib.load_call(_relaid)
+_NATIVE = None if os.environ.get("DEXTER_B200_FASTCALL", "1") == "0" else _lib.load_call()
 _CALL = None if _NATIVE is None or _CHECK else _NATIVE.call
 
 
@@ -403,6 +403,10 @@ def dequantize(qweight: torch.Tensor, scales: torch.Tensor, zeros: Optional[torc
     """
     if bits not in (4, 8):
         raise ValueError(f"weight-only quantisation supports 4 or 8 bits, got {bits}")
+    if _NATIVE is not None:
+        out = _NATIVE.dequantize(qweight, scales, zeros, group_size, bits, _LAYOUTS[layout])
+        if out is not None:
+            return out
     if not qweight.is_cuda:
         raise RuntimeError("the B200 backend needs CUDA tensors; there is no CPU path")
     k_dim = qweight.shape[0] * (2 if bits == 4 else 1)

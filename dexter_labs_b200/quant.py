@@ -72,6 +72,11 @@ def _quantize_cuda(weight: torch.Tensor, bits: int, group_size: int, bias: Optio
     bytes as that chain gives on the GPU, which takes about fifteen fp32 passes over the weight."""
     from . import _lib
 
+    native = _lib.load_call()
+    if native is not None:
+        packed = native.quantize(weight, bits, group_size, bool(symmetric))
+        if packed is not None:
+            return QuantizedWeight(*packed, bias, group_size, bits, (weight.shape[1], weight.shape[0]))
     lib = _lib.load()
     n_out, k_in = weight.shape
     weight = weight.contiguous()
