@@ -73,65 +73,65 @@ wq_dequant_kernel(const uint8_t* __restrict__ qw, const __nv_bfloat16* __restric
   }
 }
 
-// Any shape (output widths that are no multiple of 8, odd groups): a thread takes 8 consecutive
-// packed bytes in memory order, whatever rows they fall in, so loads and stores stay wide where the
-// row length would misalign them; scales are looked up per element (they hit L1).
+// Any shape (output widths that are no multiple of 8, odd groups).  Rows start on any byte there, so lanes
+// take single columns: consecutive lanes on consecutive bytes and bf16s, four columns 32 apart per
+// lane, scales kept in registers from row to row.  (Eight consecutive columns per thread with scales
+// looked up per weight: 72 us for int4 3072 x 14335.)
+constexpr int kDequantRows = 16;  // packed rows per warp
 template <int BITS>
-__global__ void __launch_bounds__(128)
-wq_dequant_flat_kernel(const uint8_t* __restrict__ qw, const __nv_bfloat16* __restrict__ scales,
+__global__ void __launch_bounds__(256)
+wq_dequant_cols_kernel(const uint8_t* __restrict__ qw, const __nv_bfloat16* __restrict__ scales,
                        const __nv_bfloat16* __restrict__ zeros, __nv_bfloat16* __restrict__ out, int N, int K,
                        int group, int relaid) {
-  const int rows = BITS == 4 ? K >> 1 : K;
-  const long long total = static_cast<long long>(rows) * N;
-  const long long f = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) << 3;
-  if (f >= total) return;
-  const int cnt = total - f < 8 ? static_cast<int>(total - f) : 8;
-  const int r_first = static_cast<int>(f / N), n_first = static_cast<int>(f - static_cast<long long>(r_first) * N);
-  const bool wide = cnt == 8 && (reinterpret_cast<uintptr_t>(qw) & 7) == 0;
-  uint32_t raw[2] = {0u, 0u};
-  if (BITS == 8 || !relaid) {
-    if (wide) {
-      const uint2 v = __ldcs(reinterpret_cast<const uint2*>(qw + f));
-      raw[0] = v.x; raw[1] = v.y;
-    } else {
-      for (int j = 0; j < cnt; ++j) raw[j >> 2] |= static_cast<uint32_t>(qw[f + j]) << (8 * (j & 3));
-    }
-  }
   constexpr int PLANES = BITS == 4 ? 2 : 1;
+  const int rows = BITS == 4 ? K >> 1 : K;
+  const int r0 = (blockIdx.y * 8 + (threadIdx.x >> 5)) * kDequantRows;
+  const int r1 = r0 + kDequantRows < rows ? r0 + kDequantRows : rows;
+  const int n = blockIdx.x * 128 + (threadIdx.x & 31);
+  if (r0 >= rows) return;
+  uint32_t s[PLANES][4], z[PLANES][4];
+  float cz[4];
+  int left[PLANES];  // rows until the plane's next group
+  auto load = [&](int pl, int gi) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (n + 32 * j >= N) continue;
+      const long long so = static_cast<long long>(gi) * N + n + 32 * j;
+      s[pl][j] = __bfloat16_as_ushort(scales[so]);
+      if (BITS == 4) z[pl][j] = zeros ? __bfloat16_as_ushort(zeros[so]) : 0x4308u;
+      else cz[j] = 8388608.0f + (zeros ? __bfloat162float(zeros[so]) : 128.0f);
+    }
+  };
 #pragma unroll
   for (int pl = 0; pl < PLANES; ++pl) {
-    uint32_t v[4] = {0u, 0u, 0u, 0u};
-    int r = r_first, n = n_first, gi = (r + pl * rows) / group;
-    int left = group - ((r + pl * rows) - gi * group);  // rows until the next group
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (j < cnt) {
-        const long long so = static_cast<long long>(gi) * N + n;
-        const uint32_t sb = __bfloat16_as_ushort(scales[so]);
-        uint32_t o;
-        if (BITS == 4) {
-          const uint32_t zb = zeros ? __bfloat16_as_ushort(zeros[so]) : 0x4308u;
-          const uint32_t q = relaid ? fetch_q4(qw, N, rows, r + pl * rows, n, 1)
-                                    : (raw[j >> 2] >> (8 * (j & 3) + 4 * pl)) & 0xFu;
-          o = deq4(q, zb, sb) & 0xFFFFu;
-        } else {
-          const float cz = 8388608.0f + (zeros ? __bfloat162float(zeros[so]) : 128.0f);
-          o = cvt_bf16x2(0.0f, deq8(raw[j >> 2], j & 3, cz, __uint_as_float(sb << 16))) & 0xFFFFu;
-        }
-        v[j >> 1] |= o << (16 * (j & 1));
-        if (++n == N) {
-          n = 0;
-          ++r;
-          if (--left == 0) { left = group; ++gi; }
-        }
+    for (int j = 0; j < 4; ++j) s[pl][j] = z[pl][j] = 0u;
+    const int k = r0 + pl * rows, gi = k / group;
+    left[pl] = group - (k - gi * group);
+    load(pl, gi);
+  }
+#pragma unroll 4
+  for (int r = r0; r < r1; ++r) {
+    uint32_t q[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      q[j] = n + 32 * j >= N ? 0u
+             : BITS == 4 && relaid ? fetch_q4(qw, N, rows, r, n + 32 * j, 1) | (fetch_q4(qw, N, rows, r + rows, n + 32 * j, 1) << 4)
+                                   : qw[static_cast<long long>(r) * N + n + 32 * j];
+#pragma unroll
+    for (int pl = 0; pl < PLANES; ++pl) {
+      if (left[pl]-- == 0) {
+        load(pl, (r + pl * rows) / group);
+        left[pl] = group - 1;
       }
-    }
-    __nv_bfloat16* dst = out + static_cast<long long>(pl) * total + f;
-    if (cnt == 8 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-      __stcs(reinterpret_cast<uint4*>(dst), make_uint4(v[0], v[1], v[2], v[3]));
-    } else {
-      for (int j = 0; j < cnt; ++j)
-        dst[j] = __ushort_as_bfloat16(static_cast<unsigned short>((v[j >> 1] >> (16 * (j & 1))) & 0xFFFFu));
+      __nv_bfloat16* dst = out + (static_cast<long long>(r) + static_cast<long long>(pl) * rows) * N + n;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (n + 32 * j >= N) continue;
+        const uint32_t v = BITS == 4 ? deq4(q[j] >> (4 * pl), z[pl][j], s[pl][j])
+                                     : cvt_bf16x2(0.0f, deq8(q[j], 0, cz[j], __uint_as_float(s[pl][j] << 16)));
+        dst[32 * j] = __ushort_as_bfloat16(static_cast<unsigned short>(v & 0xFFFFu));
+      }
     }
   }
 }
@@ -155,9 +155,9 @@ static int launch_dequant(const void* qweight, const void* scales, const void* z
     else
       wq_dequant_kernel<BITS, false><<<grid, 128, 0, stream>>>(q, s, z, o, N, K, group);
   } else {
-    const long long total = static_cast<long long>(rows) * N;
-    const unsigned grid = static_cast<unsigned>((total + 1023) / 1024);
-    wq_dequant_flat_kernel<BITS><<<grid, 128, 0, stream>>>(q, s, z, o, N, K, group, relaid);
+    const dim3 grid((N + 127) / 128, (rows + 8 * kDequantRows - 1) / (8 * kDequantRows));
+    if (grid.y > 65535) return DXB_ERR_SHAPE;
+    wq_dequant_cols_kernel<BITS><<<grid, 256, 0, stream>>>(q, s, z, o, N, K, group, relaid);
   }
   return cudaGetLastError() == cudaSuccess ? DXB_OK : DXB_ERR_CUDA;
 }
