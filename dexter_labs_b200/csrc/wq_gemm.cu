@@ -142,7 +142,8 @@ struct WqParams {
   int units_per_tile;  // packed rows / 64
   int tiles;           // ceil(N / 128) x token blocks: tile t is token block t / tiles_n,
                        // weight columns 128 * (t % tiles_n)
-  int tiles_n;         // ceil(N / 128)
+  int tiles_n;         // ceil(N / 128); CTA pairs: ceil(N / 256)
+  int block;           // tokens per token block: 128; CTA pairs: at most 256
   int total_units;
   int half_k;          // int4: K/2 (first activation column of the high-nibble plane)
   int stages;          // activation (X) ring depth
@@ -150,7 +151,7 @@ struct WqParams {
                        // stage is only ever used by one dequant team, in order
   int x_stage_bytes;   // planes * NU * 128
   int max_slots;       // partial slots reserved per tile
-  int nacc;            // accumulator buffers in TMEM (2 when NU <= 128)
+  int nacc;            // accumulator buffers in TMEM: 2; CTA pairs with more than 128 tokens per block: 1
   int group_shift;     // log2(group / 64) when that is a power of two, else -1
   int sz_step;         // scale rows a dequant team moves on per unit inside a tile, in 4 x bf16; -1: no
                        // constant (the group does not divide the teams' stride)
@@ -199,7 +200,10 @@ __device__ __forceinline__ uint2 finish_row4(float f0, float f1, float f2, float
 //   kModeGeneral  the sum over ranks, tiles shared between CTAs through global partial sums, clusters
 //   kModeWhole    whole tiles per CTA, no cluster
 //   kModeCluster  one tile per cluster (K split, sum through distributed shared memory)
-enum : int { kModeGeneral = 0, kModeWhole = 1, kModeCluster = 2 };
+//   kModePair     whole tiles of 256 columns per CTA PAIR (cta_group::2): each CTA converts 128 columns and
+//                 loads half the tokens, one MMA multiplies both, so a converted weight serves up to
+//                 256 tokens and an activation is read once per 256 columns
+enum : int { kModeGeneral = 0, kModeWhole = 1, kModeCluster = 2, kModePair = 3 };
 
 template <int BITS, bool HAS_ZERO, bool MULTI, bool RELAID, int MODE>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -239,16 +243,19 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   const int G = static_cast<int>(gridDim.x);
   const int U = p.units_per_tile;
   constexpr bool kLean = MODE != kModeGeneral;
-  const int C = MODE == kModeWhole ? 1 : p.cluster;  // kModeCluster is only launched with C > 1
+  constexpr bool PAIR = MODE == kModePair;
+  constexpr bool WHOLE = MODE == kModeWhole || PAIR;
+  const int NACC = PAIR ? p.nacc : 2;
+  const int C = WHOLE ? 1 : p.cluster;  // kModeCluster is only launched with C > 1
   const bool clustered = MODE == kModeCluster || (MODE == kModeGeneral && C > 1);
-  const bool tile_ranges = MODE == kModeWhole || (MODE == kModeGeneral && p.tile_ranges);
+  const bool tile_ranges = WHOLE || (MODE == kModeGeneral && p.tile_ranges);
   // Ranges without a division on the way to the first weight load (a 64-bit division is a few
   // hundred cycles at the head of every launch): `range_q`, `range_r` are quotient and remainder
   // of what is being cut (a cluster's units by its size, or the tiles by the grid), so part i
   // starts at i * q + min(i, r).  Only unit ranges that cut tiles still divide.
-  const int crank = clustered ? static_cast<int>(cluster_cta_rank()) : 0;
+  const int crank = clustered || PAIR ? static_cast<int>(cluster_cta_rank()) : 0;
   const int ctile = clustered ? static_cast<int>(cluster_id_x()) : 0;
-  const int part = clustered ? crank : static_cast<int>(blockIdx.x);
+  const int part = clustered ? crank : PAIR ? static_cast<int>(cluster_id_x()) : static_cast<int>(blockIdx.x);
   const int cut_begin = part * p.range_q + (part < p.range_r ? part : p.range_r);
   const int cut_end = cut_begin + p.range_q + (part < p.range_r ? 1 : 0);
   const bool unit_ranges = MODE == kModeGeneral && !clustered && !tile_ranges;
@@ -258,6 +265,8 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                     : !unit_ranges ? cut_end * U : static_cast<int>(range_begin(blockIdx.x + 1, TU, G));
   const int tile_begin = clustered ? ctile : !unit_ranges ? cut_begin : u_begin / U;
   const int ku_begin = clustered ? cut_begin : !unit_ranges ? 0 : u_begin - tile_begin * U;
+  // This CTA's 128 columns of a tile.
+  auto column_of = [&](int ntile) { return (PAIR ? 2 * ntile + crank : ntile) * kTileN; };
 
   // Packed-weight producers (warps 0 and 3, alternate units): cursor of the next unit to load.
   // (Issuing the first loads before the CTA-wide set-up barrier, with the producers only
@@ -271,7 +280,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     if (elect_one()) {
       const uint32_t fw = bar0 + 8 * (kBarFullW + w_s);
       mbar_expect_tx(fw, W_STAGE);
-      tma_load_2d(w_ring + w_s * W_STAGE, &tm_q, fw, (MULTI ? w_ntile : w_tile) * kTileN, w_ku * UNIT_ROWS);
+      tma_load_2d(w_ring + w_s * W_STAGE, &tm_q, fw, column_of(MULTI ? w_ntile : w_tile), w_ku * UNIT_ROWS);
     }
     __syncwarp();
     w_u += 2;
@@ -292,7 +301,10 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       mbar_init(bar0 + 8 * (kBarFullW + wp + 2 * lane), bar_count(kBarFullW + wp + 2 * lane));
       mbar_init(bar0 + 8 * (kBarEmptyW + wp + 2 * lane), bar_count(kBarEmptyW + wp + 2 * lane));
     } else if (warp == 3 && kBarReady + lane - 8 < kNumBars) {
-      mbar_init(bar0 + 8 * (kBarReady + lane - 8), bar_count(kBarReady + lane - 8));
+      const int i = kBarReady + lane - 8;
+      // a pair's accumulators are drained by both CTAs' epilogue warps
+      const uint32_t twice = PAIR && i >= kBarAccEmpty && i < kBarPeer ? 2u : 1u;
+      mbar_init(bar0 + 8 * i, twice * bar_count(i));
     }
     if (lane == 0) {
       abort_flag = 0;
@@ -310,11 +322,17 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   } else if (warp == 2 && lane == 0) {
     tma_prefetch_desc(&tm_x);
   } else if (warp == 1) {
-    tmem_alloc(smem_u32(&tmem_base_s), 512);
-    tmem_relinquish();
+    if (PAIR) {
+      tmem_alloc_pair(smem_u32(&tmem_base_s), 512);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(smem_u32(&tmem_base_s), 512);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync_all();  // the other CTA's barriers exist, its TMEM is allocated
   tc_fence_after();
   const uint32_t tmem0 = tmem_base_s;
   if (threadIdx.x == 0) DX_TRACE(5, 1);  // set-up barrier passed
@@ -357,7 +375,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   // so that its latency is not added to the tail of the tile).
   auto load_bias4 = [&](int tile, float (&bias4)[4]) {
     const int ntile = MULTI ? tile % p.tiles_n : tile;
-    const int n = ntile * kTileN + 32 * (warp & 3) + 4 * (lane >> 2);
+    const int n = column_of(ntile) + 32 * (warp & 3) + 4 * (lane >> 2);
     bias4[0] = bias4[1] = bias4[2] = bias4[3] = 0.f;
     if (p.bias != nullptr && n < p.N) {
       const uint2 bb = __ldg(reinterpret_cast<const uint2*>(p.bias + n));
@@ -375,12 +393,12 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     const int g = lane >> 2;
     const int n_local = 32 * q + 4 * g;
     const bool has_bias = p.bias != nullptr;
-    const bool whole = MODE == kModeWhole || (MODE == kModeGeneral && nun == U);
+    const bool whole = WHOLE || (MODE == kModeGeneral && nun == U);
     const int tblock = MULTI ? tile / p.tiles_n : 0;  // token block of this tile
     const int ntile = tile - tblock * p.tiles_n;      // its 128 weight columns
-    const int row0 = tblock * 128;
-    const int m_rows = MULTI ? ((p.M - row0) < 128 ? (p.M - row0) : 128) : p.M;  // token rows in this block
-    const int n = ntile * kTileN + n_local;
+    const int row0 = tblock * p.block;
+    const int m_rows = MULTI ? ((p.M - row0) < p.block ? (p.M - row0) : p.block) : p.M;  // token rows in this block
+    const int n = column_of(ntile) + n_local;
     const bool n_ok = n < p.N;
     // Sum over ranks fused into this launch (one token block only): finished rows go to
     // every rank's receive buffer instead of `out`; fused_finish then completes the tile.
@@ -452,7 +470,10 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0 && nwk == 1) mbar_arrive(bar0 + 8 * (kBarAccEmpty + b));
+      if (lane == 0 && nwk == 1) {
+        if (PAIR) mbar_arrive_remote(bar0 + 8 * (kBarAccEmpty + b), 0);  // the leader issues for both
+        else mbar_arrive(bar0 + 8 * (kBarAccEmpty + b));
+      }
       if (fused && !fused_finish()) return false;
     } else if (clustered) {
       // Cluster mode: CTA r of the cluster finishes token rows [r*rows_per, (r+1)*rows_per)
@@ -591,7 +612,8 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     if (elect_one()) {
       int ku = ku_begin;
       int ntile = MULTI ? tile_begin % p.tiles_n : 0;
-      int row0 = MULTI ? (tile_begin / p.tiles_n) * 128 : 0;  // first token row of the token block
+      // first token row of the token block (a pair's CTAs load half of it each)
+      int row0 = MULTI ? (tile_begin / p.tiles_n) * p.block + (PAIR ? crank * (p.NU >> 1) : 0) : 0;
       uint32_t ph = 1;
       int u = u_begin;
       bool ok = true;
@@ -614,7 +636,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
               ++u;
               if (++ku == U) {
                 ku = 0;
-                if (MULTI && ++ntile == p.tiles_n) { ntile = 0; row0 += 128; }
+                if (MULTI && ++ntile == p.tiles_n) { ntile = 0; row0 += p.block; }
               }
             }
           }
@@ -635,39 +657,70 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     // warps that keep it about 80 % busy, so each of its instructions waits for a turn: as a
     // warp-uniform loop with a slot counter a unit's 8 products and its wait took 840 cycles beside
     // them, twice what the tensor pipe needs for 96 tokens; in this form they take 460.
-    if (elect_one()) {
-      const uint32_t idesc = idesc_bf16_f32(kTileN, p.NU);
+    if (PAIR && crank == 1) {
+      // The other CTA issues the MMAs: tell it about every unit that is ready here.
+      if (elect_one()) {
+        uint32_t ph = 0;
+        int left = u_end - u_begin;
+        bool ok = true;
+        while (left > 0 && ok) {
+#pragma unroll
+          for (int t = 0; t < kAStages; ++t) {
+            if (left > 0 && ok) {
+              ok = mbar_wait(bar0 + 8 * (kBarReady + t), ph, abortp);
+              if (ok) {
+                tc_fence_after();
+                tc_fence_before();
+                mbar_arrive_remote(bar0 + 8 * (kBarPeer + t), 0);
+                --left;
+              }
+            }
+          }
+          ph ^= 1u;
+        }
+      }
+    } else if (elect_one()) {
+      const uint32_t idesc = idesc_bf16_f32(PAIR ? 2 * kTileN : kTileN, p.NU);
       const uint64_t xdesc0 = smem_desc_kmajor_sw128(x_ring);
       const uint32_t x_stage16 = static_cast<uint32_t>(p.x_stage_bytes) >> 4;
-      const uint32_t plane16 = static_cast<uint32_t>(p.NU * 128) >> 4;
+      const uint32_t plane16 = static_cast<uint32_t>(p.x_stage_bytes >> 1) >> 4;
       const uint32_t a_tmem0 = tmem0 + kACol0;
       int b = 0;
       uint32_t ph = 0, accph = 1, accumulate = 0;
       int left = u_end - u_begin;                        // units of this CTA still to do
       int seg = left < U - ku_begin ? left : U - ku_begin;  // of them in the current tile
       uint32_t d_tmem = tmem0;
+      auto mma = [](uint32_t d, uint32_t a, uint64_t b, uint32_t id, uint32_t acc) {
+        if (PAIR) mma_ts_pair(d, a, b, id, acc);
+        else mma_ts(d, a, b, id, acc);
+      };
+      auto commit = [](uint32_t bar) {
+        if (PAIR) tc_commit_pair(bar);
+        else tc_commit(bar);
+      };
       bool ok = left > 0 && mbar_wait(bar0 + 8 * kBarAccEmpty, accph, abortp);
       while (left > 0 && ok) {
 #pragma unroll
         for (int t = 0; t < kAStages; ++t) {
           if (left > 0 && ok) {
-            ok = mbar_wait(bar0 + 8 * (kBarReady + t), ph, abortp);
+            ok = mbar_wait(bar0 + 8 * (kBarReady + t), ph, abortp) &&
+                 (!PAIR || mbar_wait(bar0 + 8 * (kBarPeer + t), ph, abortp));
             if (ok) {
               tc_fence_after();
               const uint64_t xd = xdesc0 + t * x_stage16;
               const uint32_t a_tmem = a_tmem0 + t * A_STAGE_COLS;
-              mma_ts(d_tmem, a_tmem, xd, idesc, accumulate);
+              mma(d_tmem, a_tmem, xd, idesc, accumulate);
 #pragma unroll
-              for (int kk = 1; kk < 4; ++kk) mma_ts(d_tmem, a_tmem + kk * 8, xd + kk * 2, idesc, 1u);
+              for (int kk = 1; kk < 4; ++kk) mma(d_tmem, a_tmem + kk * 8, xd + kk * 2, idesc, 1u);
 #pragma unroll
               for (int kk = 0; kk < 4; ++kk)
-                mma_ts(d_tmem, a_tmem + 32 + kk * 8, xd + plane16 + kk * 2, idesc, 1u);
-              tc_commit(bar0 + 8 * (kBarFree + t));
+                mma(d_tmem, a_tmem + 32 + kk * 8, xd + plane16 + kk * 2, idesc, 1u);
+              commit(bar0 + 8 * (kBarFree + t));
               accumulate = 1;
               --left;
               if (--seg == 0) {
-                tc_commit(bar0 + 8 * (kBarAccFull + b));
-                if (++b == 2) { b = 0; accph ^= 1u; }
+                commit(bar0 + 8 * (kBarAccFull + b));
+                if (++b == NACC) { b = 0; accph ^= 1u; }
                 if (left > 0) {
                   seg = left < U ? left : U;
                   accumulate = 0;
@@ -697,13 +750,13 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       if (!mbar_wait(bar0 + 8 * (kBarAccFull + b), accph, abortp)) break;
       if (etid == 0) DX_TRACE(0, tile - tile_begin);
       tc_fence_after();
-      if (MODE == kModeWhole && u + nun == u_end) break;  // the last tile is everybody's, see below
+      if (WHOLE && u + nun == u_end) break;  // the last tile is everybody's, see below
       if (!epilogue_segment(tile, ku0, nun, b, bias4, 0, 1)) break;
       if (etid == 0) DX_TRACE(1, tile - tile_begin);
       u += nun;
       ku0 = 0;
       ++tile;
-      if (++b == 2) { b = 0; accph ^= 1u; }
+      if (++b == NACC) { b = 0; accph ^= 1u; }
     }
   } else if (warp >= 8) {
     // ========================================================== dequant ====
@@ -748,7 +801,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     int sz[PLANES];  // offset of the current rows, in 4 x bf16
     const int n4_stride = p.N >> 2;
     auto seek_sz = [&]() {  // rows of unit (tile, ku); columns beyond N (last tile) re-read the last ones
-      int n4 = ((MULTI ? tile % p.tiles_n : tile) * kTileN + n_local) >> 2;
+      int n4 = (column_of(MULTI ? tile % p.tiles_n : tile) + n_local) >> 2;
       n4 = n4 < n4_stride ? n4 : n4_stride - 1;
 #pragma unroll
       for (int pl = 0; pl < PLANES; ++pl) {
@@ -896,7 +949,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   tc_fence_before();
   __syncthreads();
   if (threadIdx.x == 0) DX_TRACE(7, 1);  // every role is through its loop
-  if (MODE == kModeWhole && !abort_flag) {
+  if (WHOLE && !abort_flag) {
     // The CTA's last tile: its accumulator is complete (the epilogue warps have waited for it) and
     // every other warp is idle, so all 24 finish it, six per TMEM lane quadrant with a 16-token chunk
     // each, instead of four walking six chunks.
@@ -906,7 +959,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     load_bias4(tile, bias4);
     pdl_wait();
     tc_fence_after();
-    epilogue_segment(tile, 0, U, (tiles - 1) & 1, bias4, warp >> 2, kThreads / 128);
+    epilogue_segment(tile, 0, U, NACC == 2 ? (tiles - 1) & 1 : 0, bias4, warp >> 2, kThreads / 128);
     tc_fence_before();
     __syncthreads();  // before the accumulator's TMEM is given back
   }
@@ -914,8 +967,8 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     // The cluster's tile: token block and column tile.
     const int tblock = MULTI ? ctile / p.tiles_n : 0;
     const int ntile = ctile - tblock * p.tiles_n;
-    const int row0 = tblock * 128;
-    const int m_rows = MULTI ? ((p.M - row0) < 128 ? (p.M - row0) : 128) : p.M;
+    const int row0 = tblock * p.block;
+    const int m_rows = MULTI ? ((p.M - row0) < p.block ? (p.M - row0) : p.block) : p.M;
     const int m_lo = crank * p.rows_per;
     const int m_hi = (m_lo + p.rows_per) < m_rows ? (m_lo + p.rows_per) : m_rows;
     const uint32_t recv0 = smem0 + static_cast<uint32_t>(p.recv_off);
@@ -1023,7 +1076,12 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     }
   }
   if (threadIdx.x == 0) DX_TRACE(7, 0);
-  if (warp == 1) tmem_dealloc(tmem0, 512);
+  // Neither CTA of a pair may leave while the other can still signal it or use its memory.
+  if (PAIR) cluster_sync_all();
+  if (warp == 1) {
+    if (PAIR) tmem_dealloc_pair(tmem0, 512);
+    else tmem_dealloc(tmem0, 512);
+  }
   if (threadIdx.x == 0 && abort_flag) {
     pdl_wait();
     atomicExch(p.status, DXB_ERR_KERNEL_TIMEOUT);
@@ -1136,7 +1194,7 @@ struct Opts {
 
 struct Plan {
   int NU, planes, rows, unit_rows, w_stage_bytes, units_per_tile, tiles, tiles_n, total_units, stages,
-      w_stages, x_stage_bytes, ctas,
+      w_stages, x_stage_bytes, x_rows, ctas, block,
       max_slots, nacc, recv_bytes, recv_off, recv_alias, whole;
   size_t smem_bytes;
 };
@@ -1169,7 +1227,9 @@ static Plan make_plan_uncached(int M, int N, int K, int bits, int sms, int max_c
   pl.tiles_n = (N + kTileN - 1) / kTileN;
   pl.tiles = pl.tiles_n * blocks;
   pl.total_units = pl.units_per_tile * pl.tiles;
-  pl.x_stage_bytes = pl.planes * pl.NU * 128;
+  pl.block = 128;
+  pl.x_rows = pl.NU;
+  pl.x_stage_bytes = pl.planes * pl.x_rows * 128;
   // Shared memory: four activation stages (one per unit slot, like the TMEM ring) and
   // as deep a ring of packed-weight stages as still fits: those come from HBM and
   // need the most bytes in flight.  The depth is a multiple of four so that every
@@ -1225,6 +1285,34 @@ static Plan make_plan_uncached(int M, int N, int K, int bits, int sms, int max_c
     if (c1 - c0 + 1 > max_slots) max_slots = c1 - c0 + 1;
   }
   pl.max_slots = max_slots;
+  return pl;
+}
+
+// Plan for CTA pairs over `pairs` clusters of two, tokens in `blocks` equal blocks of at most 256.
+static Plan make_pair_plan(int M, int N, int K, int bits, int pairs, int blocks) {
+  Plan pl{};
+  if (blocks < (M + 255) / 256) blocks = (M + 255) / 256;  // more tokens than an MMA takes are not encodable
+  pl.block = ((M + blocks - 1) / blocks + 31) / 32 * 32;  // a pair MMA takes its N in steps of 32
+  pl.NU = pl.block;
+  pl.planes = 2;
+  pl.rows = bits == 4 ? K / 2 : K;
+  pl.unit_rows = bits == 4 ? 64 : 128;
+  pl.w_stage_bytes = pl.unit_rows * kTileN;
+  pl.units_per_tile = pl.rows / pl.unit_rows;
+  pl.tiles_n = (N + 2 * kTileN - 1) / (2 * kTileN);
+  pl.tiles = pl.tiles_n * ((M + pl.block - 1) / pl.block);
+  pl.total_units = pl.units_per_tile * pl.tiles;
+  pl.x_rows = pl.NU / 2;
+  pl.x_stage_bytes = pl.planes * pl.x_rows * 128;
+  pl.stages = kAStages;
+  int w_stages = (kSmemBudget - kAStages * pl.x_stage_bytes) / pl.w_stage_bytes / kAStages * kAStages;
+  pl.w_stages = w_stages > kMaxWStages ? kMaxWStages : w_stages;
+  pl.smem_bytes = static_cast<size_t>(pl.w_stages) * pl.w_stage_bytes + pl.stages * pl.x_stage_bytes + 1024;
+  const int rounds = (pl.tiles + pairs - 1) / pairs;
+  pl.ctas = (pl.tiles + rounds - 1) / rounds;  // pairs
+  pl.whole = 1;
+  pl.nacc = pl.NU <= 128 ? 2 : 1;
+  pl.max_slots = 1;
   return pl;
 }
 
@@ -1301,6 +1389,7 @@ static TcKernel pick_mode(int mode) {
   switch (mode) {
     case kModeWhole: return wq_gemm_tc<BITS, HAS_ZERO, MULTI, RELAID, kModeWhole>;
     case kModeCluster: return wq_gemm_tc<BITS, HAS_ZERO, MULTI, RELAID, kModeCluster>;
+    case kModePair: return wq_gemm_tc<BITS, HAS_ZERO, true, RELAID, kModePair>;
     default: return wq_gemm_tc<BITS, HAS_ZERO, MULTI, RELAID, kModeGeneral>;
   }
 }
@@ -1312,6 +1401,67 @@ static TcKernel pick_kernel(bool multi, bool relaid, int mode) {
   return multi ? pick_mode<BITS, HAS_ZERO, true, false>(mode) : pick_mode<BITS, HAS_ZERO, false, false>(mode);
 }
 
+// CTA pairs that are resident at once, within a budget of CTAs.
+static int resident_pairs(const void* kernel, int budget) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  static thread_local std::unordered_map<size_t, int> cache;
+  const size_t key = reinterpret_cast<size_t>(kernel) * 64 + static_cast<size_t>(dev);
+  auto it = cache.find(key);
+  if (it == cache.end()) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kSmemBudget + 1024;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+    it = cache.emplace(key, n).first;
+  }
+  return it->second < budget / 2 ? it->second : budget / 2;
+}
+
+// Token blocks for CTA pairs, or 0 where the other plans are the better ones: the shortest of the
+// times below, all fitted to measurements on shapes between 160 x 3072 x 3072 and 913 x 13824 x 5120.
+// What they trade: a pair's unit takes as long as the MMA of its tokens (0.56 us at 256, 0.31 at
+// 128), converted once for all of them, but its accumulator of more than 128 tokens is not
+// double-buffered, so every further tile shows its epilogue; single CTAs convert a unit per 128
+// tokens (0.36 us int4, 0.42 int8); few tiles are split over clusters instead, at 7.5 us for the
+// exchange.  Which wins turns mostly on how full the last round of tiles is.
+static int choose_pair_blocks(const Plan& pl, int M, int N, int K, int bits, int pairs, int budget) {
+  static const int forced = [] { const char* e = getenv("DEXTER_B200_PAIR"); return e ? atoi(e) : -1; }();
+  const int least = (M + 255) / 256;  // a block has at most 256 tokens
+  if (pairs < 1) return 0;
+  if (forced >= 0) return forced == 0 ? 0 : forced < least ? least : forced;
+  const double U = pl.units_per_tile, unit = bits == 4 ? 0.36 : 0.42;
+  double best;
+  if (pl.recv_bytes > 0 && pl.tiles * 2 <= budget && pl.units_per_tile >= 2) {
+    int c = budget / pl.tiles;
+    c = c > 8 ? 8 : c > pl.units_per_tile ? pl.units_per_tile : c;
+    best = 7.5 + (U / c) * unit;
+  } else {
+    const int rounds = (pl.tiles + budget - 1) / budget;
+    best = 2.5 + rounds * (U * unit + (bits == 4 ? 0.7 : 1.2));
+  }
+  int blocks = 0;
+  for (int nb = least; nb <= least + 7; ++nb) {
+    const Plan pp = make_pair_plan(M, N, K, bits, pairs, nb);
+    const int rounds = (pp.tiles + pairs - 1) / pairs;
+    double u = 0.02 + 0.0022 * pp.NU;
+    const double least_unit = bits == 4 ? 0.30 : 0.46;
+    if (u < least_unit) u = least_unit;
+    const double t = 1.15 * (4.2 + rounds * U * u + (rounds - 1) * (pp.nacc == 1 ? 0.006 * pp.NU : 0.5));
+    if (t < best) { best = t; blocks = nb; }
+  }
+  return blocks;
+}
+
 template <int BITS, bool HAS_ZERO>
 static int launch_tc(const void* x, long long ldx, const void* qw, const void* scales,
                      const void* zeros, const void* bias, void* out, long long ldo, int M, int N,
@@ -1321,6 +1471,7 @@ static int launch_tc(const void* x, long long ldx, const void* qw, const void* s
   const int max_ctas = opts.max_ctas;
   Plan plan = make_plan(M, N, K, BITS, di.sms, max_ctas);
   const Plan* plp = &plan;
+  const bool multi = plp->tiles > plp->tiles_n;
   if (plp->w_stages < kAStages) return DXB_ERR_UNSUPPORTED;
   // Status word and counters are always needed; the partial sums only if the launch ends up
   // splitting tiles through global scratch (checked below, once the cluster size is known).
@@ -1337,11 +1488,10 @@ static int launch_tc(const void* x, long long ldx, const void* qw, const void* s
     };
     for (int multi = 0; multi < 2; ++multi)
       for (int relaid = 0; relaid < (BITS == 4 ? 2 : 1); ++relaid)
-        for (int mode = 0; mode < 3; ++mode) set(pick_kernel<BITS, HAS_ZERO>(multi, relaid, mode));
+        for (int mode = 0; mode < 4; ++mode) set(pick_kernel<BITS, HAS_ZERO>(multi, relaid, mode));
     if (!ok) return DXB_ERR_CUDA;
     attr_dev = dev;
   }
-  const bool multi = plp->tiles > plp->tiles_n;
   const bool relaid = BITS == 4 && opts.relaid;
   // The lean instances serve every launch without a sum over ranks; which of the two follows from the plan below.
   const bool lean = opts.peer.world <= 1;
@@ -1351,8 +1501,25 @@ static int launch_tc(const void* x, long long ldx, const void* qw, const void* s
   // reduces through distributed shared memory.  The cluster size is the largest one for
   // which all clusters are resident at once; the answer is cached per configuration.
   int cluster = 1;
+  int pair_blocks = 0;  // > 0: CTA pairs, this many token blocks
   const int budget = (max_ctas > 0 && max_ctas < di.sms) ? max_ctas : di.sms;
-  if (plp->recv_bytes > 0 && plp->tiles * 2 <= budget && plp->units_per_tile >= 2) {
+  if (multi && lean) {
+    const int pairs = resident_pairs(reinterpret_cast<const void*>(pick_kernel<BITS, HAS_ZERO>(true, relaid, kModePair)), budget);
+    static thread_local std::unordered_map<size_t, int> chosen;
+    const size_t key = ((static_cast<size_t>(M) * 1000003u + static_cast<size_t>(N)) * 1000003u + static_cast<size_t>(K)) * 512u +
+                       static_cast<size_t>(budget);
+    auto it = chosen.find(key);
+    if (it == chosen.end()) {
+      if (chosen.size() > 4096) chosen.clear();
+      it = chosen.emplace(key, choose_pair_blocks(*plp, M, N, K, BITS, pairs, budget)).first;
+    }
+    pair_blocks = it->second;
+    if (pair_blocks > 0) {
+      plan = make_pair_plan(M, N, K, BITS, pairs, pair_blocks);
+      kernel = pick_kernel<BITS, HAS_ZERO>(true, relaid, kModePair);
+    }
+  }
+  if (pair_blocks == 0 && plp->recv_bytes > 0 && plp->tiles * 2 <= budget && plp->units_per_tile >= 2) {
     static thread_local std::unordered_map<long long, int> cache;
     const long long key = (static_cast<long long>(dev) << 48) ^ (static_cast<long long>(plp->tiles) << 28) ^
                           (static_cast<long long>(plp->units_per_tile) << 8) ^ static_cast<long long>(plp->NU >> 4) ^
@@ -1388,7 +1555,7 @@ static int launch_tc(const void* x, long long ldx, const void* qw, const void* s
       cache[key] = cluster;
     }
   }
-  if (cluster == 1) {
+  if (cluster == 1 && pair_blocks == 0) {
     const size_t need = kStatusBytes + counters_bytes(plp->tiles) +
                         static_cast<size_t>(plp->tiles) * plp->max_slots * plp->NU * kTileN * sizeof(float);
     if (workspace_bytes < need) {
@@ -1398,7 +1565,7 @@ static int launch_tc(const void* x, long long ldx, const void* qw, const void* s
     }
   }
   const Plan& pl = *plp;
-  if (cluster == 1)
+  if (cluster == 1 && pair_blocks == 0)
     kernel = pick_kernel<BITS, HAS_ZERO>(multi, relaid, lean && pl.whole ? kModeWhole : kModeGeneral);
 
   const CUtensorMap* tq = cached_map(MapKey{qw, N, pl.rows, 0, BITS}, [&](CUtensorMap* m) {
@@ -1407,18 +1574,18 @@ static int launch_tc(const void* x, long long ldx, const void* qw, const void* s
     const uint32_t box[2] = {kTileN, static_cast<uint32_t>(pl.unit_rows)};
     return make_map(m, qw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
   });
-  const CUtensorMap* tx = cached_map(MapKey{x, ldx, (static_cast<long long>(M) << 32) | K, pl.NU, 16 + BITS},
+  const CUtensorMap* tx = cached_map(MapKey{x, ldx, (static_cast<long long>(M) << 32) | K, pl.x_rows, 16 + BITS},
                                      [&](CUtensorMap* m) {
     if (BITS == 4) {
       // X seen as [plane][token][k within the plane]: one box brings both k-slices of a unit.
       const uint64_t dims[3] = {static_cast<uint64_t>(K / 2), static_cast<uint64_t>(M), 2};
       const uint64_t strides[2] = {static_cast<uint64_t>(ldx) * 2, static_cast<uint64_t>(K / 2) * 2};
-      const uint32_t box[3] = {64, static_cast<uint32_t>(pl.NU), 2};
+      const uint32_t box[3] = {64, static_cast<uint32_t>(pl.x_rows), 2};
       return make_map(m, x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
     }
     const uint64_t dims[2] = {static_cast<uint64_t>(K), static_cast<uint64_t>(M)};
     const uint64_t strides[1] = {static_cast<uint64_t>(ldx) * 2};
-    const uint32_t box[2] = {64, static_cast<uint32_t>(pl.NU)};
+    const uint32_t box[2] = {64, static_cast<uint32_t>(pl.x_rows)};
     return make_map(m, x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
   });
   if (!tq || !tx) return DXB_ERR_TENSORMAP;
@@ -1438,6 +1605,7 @@ static int launch_tc(const void* x, long long ldx, const void* qw, const void* s
   p.units_per_tile = pl.units_per_tile;
   p.tiles = pl.tiles;
   p.tiles_n = pl.tiles_n;
+  p.block = pl.block;
   p.total_units = pl.total_units;
   p.half_k = BITS == 4 ? K / 2 : 0;
   p.stages = pl.stages;
@@ -1471,15 +1639,15 @@ static int launch_tc(const void* x, long long ldx, const void* qw, const void* s
   p.rows_inv = (65536 + p.rows_per - 1) / p.rows_per;
 
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(cluster > 1 ? pl.tiles * cluster : pl.ctas);
+  cfg.gridDim = dim3(pair_blocks > 0 ? 2 * pl.ctas : cluster > 1 ? pl.tiles * cluster : pl.ctas);
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = pl.smem_bytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   int nattr = 0;
-  if (cluster > 1) {
+  if (cluster > 1 || pair_blocks > 0) {
     attr[nattr].id = cudaLaunchAttributeClusterDimension;
-    attr[nattr].val.clusterDim.x = cluster;
+    attr[nattr].val.clusterDim.x = pair_blocks > 0 ? 2 : cluster;
     attr[nattr].val.clusterDim.y = 1;
     attr[nattr].val.clusterDim.z = 1;
     ++nattr;
