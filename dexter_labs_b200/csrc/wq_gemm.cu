@@ -618,20 +618,29 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       int u = u_begin;
       bool ok = true;
       const uint32_t x_bytes = p.x_stage_bytes;
+      // Four stages go with the four slots; with three (int8) the unit three ago has to be done.
+      constexpr bool kMayBeThree = BITS == 8 && !MULTI;
+      const bool three = kMayBeThree && p.stages == 3;
+      uint32_t dst = x_ring;
       while (u < u_end && ok) {
 #pragma unroll
         for (int t = 0; t < kAStages; ++t) {
           if (u < u_end && ok) {
-            ok = mbar_wait(bar0 + 8 * (kBarFree + t), ph, abortp);
+            ok = three ? mbar_wait(bar0 + 8 * (kBarFree + (t + 1) % kAStages), t < 3 ? ph : ph ^ 1u, abortp)
+                       : mbar_wait(bar0 + 8 * (kBarFree + t), ph, abortp);
             if (ok) {
               const uint32_t rb = bar0 + 8 * (kBarReady + t);
-              const uint32_t dst = x_ring + t * p.x_stage_bytes;
+              if (!kMayBeThree) dst = x_ring + t * p.x_stage_bytes;
               mbar_expect_tx(rb, x_bytes);
               if (BITS == 4) {
                 tma_load_3d(dst, &tm_x, rb, ku * 64, row0, 0);
               } else {  // two k-blocks of 64, one per plane
                 tma_load_2d(dst, &tm_x, rb, ku * 128, row0);
                 tma_load_2d(dst + (x_bytes >> 1), &tm_x, rb, ku * 128 + 64, row0);
+                if (kMayBeThree) {
+                  dst += x_bytes;
+                  if (dst == x_ring + p.stages * x_bytes) dst = x_ring;
+                }
               }
               ++u;
               if (++ku == U) {
@@ -686,6 +695,9 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       const uint32_t plane16 = static_cast<uint32_t>(p.x_stage_bytes >> 1) >> 4;
       const uint32_t a_tmem0 = tmem0 + kACol0;
       int b = 0;
+      uint64_t xd = xdesc0;
+      uint32_t x_lo = static_cast<uint32_t>(xdesc0);  // its address half, where the stages are counted
+      const uint32_t x_lo_end = x_lo + p.stages * x_stage16;
       uint32_t ph = 0, accph = 1, accumulate = 0;
       int left = u_end - u_begin;                        // units of this CTA still to do
       int seg = left < U - ku_begin ? left : U - ku_begin;  // of them in the current tile
@@ -707,7 +719,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                  (!PAIR || mbar_wait(bar0 + 8 * (kBarPeer + t), ph, abortp));
             if (ok) {
               tc_fence_after();
-              const uint64_t xd = xdesc0 + t * x_stage16;
+              if (BITS == 4 || MULTI) xd = xdesc0 + t * x_stage16;
               const uint32_t a_tmem = a_tmem0 + t * A_STAGE_COLS;
               mma(d_tmem, a_tmem, xd, idesc, accumulate);
 #pragma unroll
@@ -717,6 +729,11 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                 mma(d_tmem, a_tmem + 32 + kk * 8, xd + plane16 + kk * 2, idesc, 1u);
               commit(bar0 + 8 * (kBarFree + t));
               accumulate = 1;
+              if (BITS == 8 && !MULTI) {
+                x_lo += x_stage16;
+                if (x_lo == x_lo_end) x_lo = static_cast<uint32_t>(xdesc0);
+                xd = (xdesc0 & 0xFFFFFFFF00000000ull) | x_lo;
+              }
               --left;
               if (--seg == 0) {
                 commit(bar0 + 8 * (kBarAccFull + b));
@@ -1212,6 +1229,15 @@ static int fixup_units(int NU) {
   return NU > 96 ? 32 : 20;
 }
 
+// int8 units are 16 KB: with four weight stages a team has one, and waits for HBM in every unit.  Three
+// activation stages instead of four make room for eight with 65 to 112 tokens (83 tokens 3072 x 14336
+// 15.1 -> 13.7 us); elsewhere four fit anyway or the stage costs more than it brings (913 tokens: 66.8 ->
+// 72.3 us; with two stages everything is slower).
+static int activation_stages(int bits, int blocks, int x_stage_bytes, int reserved) {
+  auto w_stages = [&](int x) { return (kSmemBudget - reserved - x * x_stage_bytes) / (128 * kTileN); };
+  return bits == 8 && blocks == 1 && w_stages(4) < 2 * kAStages && w_stages(3) >= 2 * kAStages ? 3 : kAStages;
+}
+
 static Plan make_plan_uncached(int M, int N, int K, int bits, int sms, int max_ctas, bool allow_split) {
   Plan pl{};
   // More than 128 tokens: token blocks of 128, each (block, column tile) pair is a tile of
@@ -1230,22 +1256,28 @@ static Plan make_plan_uncached(int M, int N, int K, int bits, int sms, int max_c
   pl.block = 128;
   pl.x_rows = pl.NU;
   pl.x_stage_bytes = pl.planes * pl.x_rows * 128;
-  // Shared memory: four activation stages (one per unit slot, like the TMEM ring) and
+  // Shared memory: four activation stages (one per unit slot, like the TMEM ring; int8: see above) and
   // as deep a ring of packed-weight stages as still fits: those come from HBM and
   // need the most bytes in flight.  The depth is a multiple of four so that every
   // stage is only ever used by one dequant team, in order.
-  pl.stages = kAStages;
   // Launches that may split tiles over a cluster keep room for its receive buffers
   // (at most NU + 8 token rows of 128 fp32) behind the two rings.
   const int budget_ctas = (max_ctas > 0 && max_ctas < sms) ? max_ctas : sms;
   pl.recv_bytes = (pl.tiles * 2 <= budget_ctas && pl.units_per_tile >= 2) ? (pl.NU + 8) * kTileN * 4 : 0;
-  int w_stages = (kSmemBudget - pl.recv_bytes - kAStages * pl.x_stage_bytes) / pl.w_stage_bytes;
+  pl.stages = activation_stages(bits, blocks, pl.x_stage_bytes, pl.recv_bytes);
+  int w_stages = (kSmemBudget - pl.recv_bytes - pl.stages * pl.x_stage_bytes) / pl.w_stage_bytes;
   pl.recv_alias = 0;
-  if (pl.recv_bytes > 0 && (w_stages / kAStages) * kAStages * pl.w_stage_bytes < 2 * kAStages * kWStage) {
+  // Units a cluster's CTA gets (the launcher may end up with a smaller cluster and more).
+  const int share = pl.recv_bytes > 0 ? budget_ctas / pl.tiles : 1;
+  const int cluster_units = pl.units_per_tile / (share > 8 ? 8 : share < 1 ? 1 : share);
+  if (pl.recv_bytes > 0 && ((w_stages / kAStages) * kAStages * pl.w_stage_bytes < 2 * kAStages * kWStage ||
+                            (w_stages < 2 * kAStages && bits == 8 && cluster_units >= 12))) {
     // Not enough room for a useful weight ring next to the receive buffers (more than 96
-    // tokens): let them lie over the rings instead.  The partial rows are then sent after
-    // a cluster barrier at the end of the main loop, when the rings are idle.
-    w_stages = (kSmemBudget - kAStages * pl.x_stage_bytes) / pl.w_stage_bytes;
+    // tokens; long shares of int8, which want eight stages of 16 KB): let them lie over the rings
+    // instead.  The partial rows are then sent after a cluster barrier at the end of the main loop,
+    // when the rings are idle.
+    pl.stages = activation_stages(bits, blocks, pl.x_stage_bytes, 0);
+    w_stages = (kSmemBudget - pl.stages * pl.x_stage_bytes) / pl.w_stage_bytes;
     pl.recv_alias = 1;
   }
   w_stages = (w_stages / kAStages) * kAStages;
@@ -1305,7 +1337,7 @@ static Plan make_pair_plan(int M, int N, int K, int bits, int pairs, int blocks)
   pl.x_rows = pl.NU / 2;
   pl.x_stage_bytes = pl.planes * pl.x_rows * 128;
   pl.stages = kAStages;
-  int w_stages = (kSmemBudget - kAStages * pl.x_stage_bytes) / pl.w_stage_bytes / kAStages * kAStages;
+  int w_stages = (kSmemBudget - pl.stages * pl.x_stage_bytes) / pl.w_stage_bytes / kAStages * kAStages;
   pl.w_stages = w_stages > kMaxWStages ? kMaxWStages : w_stages;
   pl.smem_bytes = static_cast<size_t>(pl.w_stages) * pl.w_stage_bytes + pl.stages * pl.x_stage_bytes + 1024;
   const int rounds = (pl.tiles + pairs - 1) / pairs;
@@ -1851,13 +1883,19 @@ static int read_opts(const dxb_gemm_opts* o, int bits, int M, int N, int K, Opts
 }
 
 // Few tokens and a weight that is read in little more than the fixed cost of a launch: there the kernel
-// without set-up is ahead; with more to convert the tcgen05 pipeline is.  (One token: int4 512 x
-// 1024 2.1 against 2.8 us, 3072 x 3072 4.6 against 5.5, 3072 x 14336 10.7 against 10.5; int8 512 x 1024
-// 2.3 against 2.9, 3072 x 3072 6.7 against 6.3.)
+// without set-up is ahead; with more to convert (once per 16 tokens, there) the tcgen05 pipeline is.
+// The lines lie where the two crossed, us small / tcgen05: int4 1 token 3072 x 9216 6.9 / 7.8, 8 tokens 7.9 /
+// 7.9, 16 tokens 3072 x 3072 5.4 / 5.9, 32 tokens 2048 x 2048 4.5 / 4.9, 64 tokens 1024 x 1024 3.4 / 4.7; int8
+// 8 tokens 3072 x 3072 6.5 / 6.7, 16 tokens 2048 x 2048 5.1 / 5.1, 64 tokens 1024 x 1024 4.0 / 4.9, 128 tokens 5.6 /
+// 7.0 (from 97 tokens on the pipeline's split launches cost two more us).
 static bool small_is_faster(int M, int N, int K, int bits) {
   static const int forced = [] { const char* e = getenv("DEXTER_B200_SMALL_TOKENS"); return e ? atoi(e) : -1; }();
   if (forced >= 0) return M <= forced;
-  return M <= 8 && static_cast<long long>(N) * K <= (bits == 4 ? 10ll << 20 : 5ll << 20);
+  const long long weights = static_cast<long long>(N) * K, mega = 1 << 20;
+  if (M <= 8) return weights <= (bits == 8 ? 10 : M <= 4 ? 30 : 16) * mega;
+  const long long converted = weights * ((M + 15) / 16);
+  if (bits == 4) return converted <= (M <= 16 ? 10 : M <= 96 ? 8 : M <= 128 ? 16 : 5) * mega;
+  return converted <= (M <= 16 ? 4 : M <= 96 ? 5 : M <= 128 ? 9 : 5) * mega;
 }
 
 static int gemm_dispatch(int bits, const void* x, int64_t ldx, const void* qweight, const void* scales,
