@@ -69,6 +69,23 @@ __device__ __forceinline__ uint32_t deq4(uint32_t w, uint32_t zero2, uint32_t sc
   const uint32_t v = and_or(w, 0x000F000Fu, 0x43004300u);
   return mul_bf16x2(sub_bf16x2(v, zero2), scale2);
 }
+// The same for nibbles at bits 4..7 and 20..23, without shifting them down: as bf16 such a pattern is at most
+// in the first normal binade, whose step is that of the subnormals, so its value is 16 q * 2^-133 for
+// all sixteen q.  One exact multiply-add makes (q - zero) / 4 of it (times 2^127, plus `zero4` =
+// -zero / 4), `scale4` = 4 * scale puts the factor back, and its multiply is the only rounding.  Two of
+// four shifts of a word of nibbles go: with them the conversion, bound by the integer pipe, loses 32 of
+// 400 instructions per 128 x 128 weights.
+__device__ __forceinline__ uint32_t deq4_mid(uint32_t w, uint32_t zero4, uint32_t scale4) {
+  uint32_t d;
+  asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(w & 0x00F000F0u), "r"(0x7F007F00u), "r"(zero4));
+  return mul_bf16x2(d, scale4);
+}
+__device__ __forceinline__ uint32_t mid_scale(uint32_t scale2) { return mul_bf16x2(scale2, 0x40804080u); }
+__device__ __forceinline__ uint32_t mid_zero(uint32_t zero2) {  // from 128 + zero
+  uint32_t d;
+  asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(zero2), "r"(0xBE80BE80u), "r"(0x42004200u));
+  return d;
+}
 // One byte -> fp32 by bit pattern: 0x4B0000qq = 8388608 + q.  `cz` = 8388608 +
 // zero point; subtract and multiply are both exact in fp32 (8-bit x 8-bit
 // significands), so the later cvt.rn to bf16 is the only rounding.

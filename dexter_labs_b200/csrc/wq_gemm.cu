@@ -863,6 +863,13 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
 #pragma unroll
             for (int i = 0; i < 4; ++i) z2[pl][i] = 0x43084308u;  // 128 + 8
           }
+          if (RELAID) {  // columns 1 and 3 of a word are converted where they stand, see deq4_mid
+#pragma unroll
+            for (int i = 1; i < 4; i += 2) {
+              s2[pl][i] = mid_scale(s2[pl][i]);
+              z2[pl][i] = HAS_ZERO ? mid_zero(z2[pl][i]) : 0xC000C000u;  // -8 / 4
+            }
+          }
         } else {
           const float sf[4] = {bf16lo_f32(sc[pl].x), bf16hi_f32(sc[pl].x), bf16lo_f32(sc[pl].y), bf16hi_f32(sc[pl].y)};
           float zf[4] = {128.0f, 128.0f, 128.0f, 128.0f};
@@ -905,12 +912,12 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                 // The word of the even row holds the low-nibble plane, the word of the odd
                 // row the high-nibble plane: nibble b is byte column b of the even row,
                 // nibble 4 + b the same column of the odd row, so masking with 0x000F000F
-                // after a shift by 4b yields the k-pair of column b directly.
+                // after a shift by 4b (0x00F000F0 after 4b - 4) yields the k-pair of column b.
                 const uint32_t W = pl == 0 ? w0[4 * rh + sl] : w1[4 * rh + sl];
                 ra[2 * sl + 0] = deq4(W, z2[pl][0], s2[pl][0]);
-                ra[2 * sl + 1] = deq4(W >> 4, z2[pl][1], s2[pl][1]);
+                ra[2 * sl + 1] = deq4_mid(W, z2[pl][1], s2[pl][1]);
                 rb[2 * sl + 0] = deq4(W >> 8, z2[pl][2], s2[pl][2]);
-                rb[2 * sl + 1] = deq4(W >> 12, z2[pl][3], s2[pl][3]);
+                rb[2 * sl + 1] = deq4_mid(W >> 8, z2[pl][3], s2[pl][3]);
               } else {
                 const uint32_t P = prmt(w0[4 * rh + sl], w1[4 * rh + sl], 0x5410u) >> (4 * pl);
                 const uint32_t Q = prmt(w0[4 * rh + sl], w1[4 * rh + sl], 0x7632u) >> (4 * pl);

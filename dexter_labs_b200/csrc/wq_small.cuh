@@ -279,6 +279,10 @@ __global__ void __launch_bounds__(CPW == 1 ? 512 : 256, CPW == 1 ? 1 : 2) wq_gem
               s0 = dup_lo(sp); s1 = dup_hi(sp);
               z0 = has_zero ? dup_lo(zp) : 0x43084308u;
               z1 = has_zero ? dup_hi(zp) : 0x43084308u;
+              if (KIND == kSmallW4Relaid) {  // odd columns of a word are converted where they stand
+                s1 = mid_scale(s1);
+                z1 = has_zero ? mid_zero(z1) : 0xC000C000u;
+              }
             } else {
               float f, o;
               deq8_constants(bf16lo_f32(sp), has_zero ? bf16lo_f32(zp) : 128.0f, f, o);
@@ -296,7 +300,7 @@ __global__ void __launch_bounds__(CPW == 1 ? 512 : 256, CPW == 1 ? 1 : 2) wq_gem
                 if (KIND == kSmallW4Relaid) {
                   const uint32_t W = (pl == 0 ? we : wo) >> (8 * th);
                   a[2 * j] = deq4(W, z0, s0);
-                  a[2 * j + 1] = deq4(W >> 4, z1, s1);
+                  a[2 * j + 1] = deq4_mid(W, z1, s1);
                 } else if (KIND == kSmallW4) {
                   const uint32_t P = prmt(we, wo, th ? 0x7632u : 0x5410u) >> (4 * pl);
                   a[2 * j] = deq4(P, z0, s0);
