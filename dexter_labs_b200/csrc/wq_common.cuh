@@ -86,6 +86,26 @@ __device__ __forceinline__ uint32_t mid_zero(uint32_t zero2) {  // from 128 + ze
   asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(zero2), "r"(0xBE80BE80u), "r"(0x42004200u));
   return d;
 }
+// Symmetric grid (zero point 8): ONE multiply-add per two weights.  With the nibbles read as above (16 q or
+// q times 2^-133), q * scale - 8 * scale is exact up to the final rounding -- 8 * scale is a bf16, which
+// zero * scale in general is not -- so (q - 8) * scale needs no subtraction of its own.  2^133 * scale would
+// overflow, so the weights come out divided by 2^16, and so do the products and their fp32 sums, bit for
+// bit; whoever reads an accumulator multiplies by kSymAcc (exact).  Good for |scale| < 2^11 and
+// products above 2^-110.
+constexpr float kSymAcc = 65536.0f;
+__device__ __forceinline__ uint32_t sym4_low(uint32_t w, uint32_t scale, uint32_t offset) {  // bits 0..3, 16..19
+  uint32_t d;
+  asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(w & 0x000F000Fu), "r"(scale), "r"(offset));
+  return d;
+}
+__device__ __forceinline__ uint32_t sym4_mid(uint32_t w, uint32_t scale, uint32_t offset) {  // bits 4..7, 20..23
+  uint32_t d;
+  asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(w & 0x00F000F0u), "r"(scale), "r"(offset));
+  return d;
+}
+__device__ __forceinline__ uint32_t sym4_scale_low(uint32_t s2) { return mul_bf16x2(s2, 0x7A007A00u); }  // 2^(133-16)
+__device__ __forceinline__ uint32_t sym4_scale_mid(uint32_t s2) { return mul_bf16x2(s2, 0x78007800u); }  // 2^(129-16)
+__device__ __forceinline__ uint32_t sym4_offset(uint32_t s2) { return mul_bf16x2(s2, 0xB900B900u); }     // -8 * 2^-16
 // One byte -> fp32 by bit pattern: 0x4B0000qq = 8388608 + q.  `cz` = 8388608 +
 // zero point; subtract and multiply are both exact in fp32 (8-bit x 8-bit
 // significands), so the later cvt.rn to bf16 is the only rounding.

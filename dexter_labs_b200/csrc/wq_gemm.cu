@@ -242,6 +242,8 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   const int TU = p.total_units;
   const int G = static_cast<int>(gridDim.x);
   const int U = p.units_per_tile;
+  constexpr bool SYM4 = BITS == 4 && !HAS_ZERO;  // weights and sums are scaled by 2^-16, see sym4_low
+  constexpr float ACC = SYM4 ? kSymAcc : 1.0f;
   constexpr bool kLean = MODE != kModeGeneral;
   constexpr bool PAIR = MODE == kModePair;
   constexpr bool WHOLE = MODE == kModeWhole || PAIR;
@@ -445,8 +447,8 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         for (int rep = 0; rep < 4; ++rep) {
           const int m = c0 + 4 * rep + c;
           if (n_ok && m < m_rows) {
-            const float f0 = __uint_as_float(ra[2 * rep]), f1 = __uint_as_float(ra[2 * rep + 1]);
-            const float f2 = __uint_as_float(rb[2 * rep]), f3 = __uint_as_float(rb[2 * rep + 1]);
+            const float f0 = ACC * __uint_as_float(ra[2 * rep]), f1 = ACC * __uint_as_float(ra[2 * rep + 1]);
+            const float f2 = ACC * __uint_as_float(rb[2 * rep]), f3 = ACC * __uint_as_float(rb[2 * rep + 1]);
             uint2* dst = reinterpret_cast<uint2*>(p.out + static_cast<long long>(row0 + m) * p.ldo + n);
             if (plain) {  // the common case, kept free of the optional epilogues' code
               uint2 pk;
@@ -560,8 +562,10 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
           for (int rep = 0; rep < 4; ++rep) {
             const int m = c0 + 4 * rep + c;
             if (n_ok && m < m_rows) {
-              const float f0 = __uint_as_float(ra[2 * rep]) + v[rep].x, f1 = __uint_as_float(ra[2 * rep + 1]) + v[rep].y;
-              const float f2 = __uint_as_float(rb[2 * rep]) + v[rep].z, f3 = __uint_as_float(rb[2 * rep + 1]) + v[rep].w;
+              const float f0 = ACC * (__uint_as_float(ra[2 * rep]) + v[rep].x);
+              const float f1 = ACC * (__uint_as_float(ra[2 * rep + 1]) + v[rep].y);
+              const float f2 = ACC * (__uint_as_float(rb[2 * rep]) + v[rep].z);
+              const float f3 = ACC * (__uint_as_float(rb[2 * rep + 1]) + v[rep].w);
               if (fused)
                 fused_push4(p.peer, parity, static_cast<long long>(m) * p.N + n, f0, f1, f2, f3);
               else
@@ -860,14 +864,18 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
             z2[pl][0] = dup_lo(zr[pl].x); z2[pl][1] = dup_hi(zr[pl].x);
             z2[pl][2] = dup_lo(zr[pl].y); z2[pl][3] = dup_hi(zr[pl].y);
           } else {
+            // Repacked: columns 1 and 3 stand at bits 4..7; otherwise those of the high-nibble plane do.
 #pragma unroll
-            for (int i = 0; i < 4; ++i) z2[pl][i] = 0x43084308u;  // 128 + 8
+            for (int i = 0; i < 4; ++i) {
+              z2[pl][i] = sym4_offset(s2[pl][i]);
+              s2[pl][i] = (RELAID ? (i & 1) : pl) ? sym4_scale_mid(s2[pl][i]) : sym4_scale_low(s2[pl][i]);
+            }
           }
-          if (RELAID) {  // columns 1 and 3 of a word are converted where they stand, see deq4_mid
+          if (RELAID && HAS_ZERO) {  // columns 1 and 3 of a word are converted where they stand, see deq4_mid
 #pragma unroll
             for (int i = 1; i < 4; i += 2) {
               s2[pl][i] = mid_scale(s2[pl][i]);
-              z2[pl][i] = HAS_ZERO ? mid_zero(z2[pl][i]) : 0xC000C000u;  // -8 / 4
+              z2[pl][i] = mid_zero(z2[pl][i]);
             }
           }
         } else {
@@ -914,17 +922,34 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                 // nibble 4 + b the same column of the odd row, so masking with 0x000F000F
                 // after a shift by 4b (0x00F000F0 after 4b - 4) yields the k-pair of column b.
                 const uint32_t W = pl == 0 ? w0[4 * rh + sl] : w1[4 * rh + sl];
-                ra[2 * sl + 0] = deq4(W, z2[pl][0], s2[pl][0]);
-                ra[2 * sl + 1] = deq4_mid(W, z2[pl][1], s2[pl][1]);
-                rb[2 * sl + 0] = deq4(W >> 8, z2[pl][2], s2[pl][2]);
-                rb[2 * sl + 1] = deq4_mid(W >> 8, z2[pl][3], s2[pl][3]);
+                if (SYM4) {
+                  ra[2 * sl + 0] = sym4_low(W, s2[pl][0], z2[pl][0]);
+                  ra[2 * sl + 1] = sym4_mid(W, s2[pl][1], z2[pl][1]);
+                  rb[2 * sl + 0] = sym4_low(W >> 8, s2[pl][2], z2[pl][2]);
+                  rb[2 * sl + 1] = sym4_mid(W >> 8, s2[pl][3], z2[pl][3]);
+                } else {
+                  ra[2 * sl + 0] = deq4(W, z2[pl][0], s2[pl][0]);
+                  ra[2 * sl + 1] = deq4_mid(W, z2[pl][1], s2[pl][1]);
+                  rb[2 * sl + 0] = deq4(W >> 8, z2[pl][2], s2[pl][2]);
+                  rb[2 * sl + 1] = deq4_mid(W >> 8, z2[pl][3], s2[pl][3]);
+                }
               } else {
-                const uint32_t P = prmt(w0[4 * rh + sl], w1[4 * rh + sl], 0x5410u) >> (4 * pl);
-                const uint32_t Q = prmt(w0[4 * rh + sl], w1[4 * rh + sl], 0x7632u) >> (4 * pl);
-                ra[2 * sl + 0] = deq4(P, z2[pl][0], s2[pl][0]);
-                ra[2 * sl + 1] = deq4(P >> 8, z2[pl][1], s2[pl][1]);
-                rb[2 * sl + 0] = deq4(Q, z2[pl][2], s2[pl][2]);
-                rb[2 * sl + 1] = deq4(Q >> 8, z2[pl][3], s2[pl][3]);
+                const uint32_t P = prmt(w0[4 * rh + sl], w1[4 * rh + sl], 0x5410u);
+                const uint32_t Q = prmt(w0[4 * rh + sl], w1[4 * rh + sl], 0x7632u);
+                if (SYM4) {
+                  auto sym4 = [&](uint32_t w, int i) {
+                    return pl ? sym4_mid(w, s2[pl][i], z2[pl][i]) : sym4_low(w, s2[pl][i], z2[pl][i]);
+                  };
+                  ra[2 * sl + 0] = sym4(P, 0);
+                  ra[2 * sl + 1] = sym4(P >> 8, 1);
+                  rb[2 * sl + 0] = sym4(Q, 2);
+                  rb[2 * sl + 1] = sym4(Q >> 8, 3);
+                } else {
+                  ra[2 * sl + 0] = deq4(P >> (4 * pl), z2[pl][0], s2[pl][0]);
+                  ra[2 * sl + 1] = deq4(P >> (4 * pl + 8), z2[pl][1], s2[pl][1]);
+                  rb[2 * sl + 0] = deq4(Q >> (4 * pl), z2[pl][2], s2[pl][2]);
+                  rb[2 * sl + 1] = deq4(Q >> (4 * pl + 8), z2[pl][3], s2[pl][3]);
+                }
               }
             }
             tmem_st_16x128b_x4(tmem_addr(a_tmem + pl * 32 + 16 * rh, lane_base, 0), ra);
@@ -1045,6 +1070,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         for (int r = 0; r < 8; ++r) {  // rank order: the sum does not depend on timing
           acc.x += v[r].x; acc.y += v[r].y; acc.z += v[r].z; acc.w += v[r].w;
         }
+        acc.x *= ACC; acc.y *= ACC; acc.z *= ACC; acc.w *= ACC;
         if (fused)
           fused_push4(p.peer, parity, static_cast<long long>(m_lo + j) * p.N + n, acc.x, acc.y, acc.z, acc.w);
         else
@@ -1778,14 +1804,16 @@ static int launch_small(int bits, const void* x, long long ldx, const void* qw, 
   const uintptr_t p16 = reinterpret_cast<uintptr_t>(qw) | reinterpret_cast<uintptr_t>(scales) | reinterpret_cast<uintptr_t>(zeros);
   const bool ragged = N % 16 != 0 || p16 % 16 != 0;
   if (ragged && (opts.relaid || p16 % 4 != 0)) return DXB_ERR_UNSUPPORTED;
-  const int kind = bits == 8 ? kSmallW8 : opts.relaid ? kSmallW4Relaid : kSmallW4;
+  const int kind = bits == 8 ? kSmallW8 : !opts.relaid ? kSmallW4 : zeros ? kSmallW4Relaid : kSmallW4Sym;
   // More tiles than two per SM: twice the width, so that they all still run at once.
   const bool wide = tiles32 > 2 * budget && !ragged && kind != kSmallW4;
   SmallKernel k;
   if (ragged) k = kind == kSmallW8 ? pick_small<kSmallW8, true, 1>(mt) : pick_small<kSmallW4, true, 1>(mt);
-  else if (wide) k = kind == kSmallW8 ? pick_small<kSmallW8, false, 2>(mt) : pick_small<kSmallW4Relaid, false, 2>(mt);
+  else if (wide) k = kind == kSmallW8 ? pick_small<kSmallW8, false, 2>(mt)
+                    : kind == kSmallW4Sym ? pick_small<kSmallW4Sym, false, 2>(mt) : pick_small<kSmallW4Relaid, false, 2>(mt);
   else k = kind == kSmallW8 ? pick_small<kSmallW8, false, 1>(mt)
-         : kind == kSmallW4 ? pick_small<kSmallW4, false, 1>(mt) : pick_small<kSmallW4Relaid, false, 1>(mt);
+         : kind == kSmallW4 ? pick_small<kSmallW4, false, 1>(mt)
+         : kind == kSmallW4Sym ? pick_small<kSmallW4Sym, false, 1>(mt) : pick_small<kSmallW4Relaid, false, 1>(mt);
   const int bn = wide ? 64 : 32;
   p.tiles_n = (N + bn - 1) / bn;
   if (static_cast<long long>(p.tiles_n) * blocks > (1 << 30)) return DXB_ERR_SHAPE;

@@ -42,7 +42,8 @@ struct SmallParams {
   int ring_bytes;   // all warps' rings (the sums lie over them afterwards)
 };
 
-enum : int { kSmallW4 = 0, kSmallW4Relaid = 1, kSmallW8 = 2 };
+// kSmallW4Sym: repacked and on the symmetric grid (no zero points), whose sums come divided by kSymAcc.
+enum : int { kSmallW4 = 0, kSmallW4Relaid = 1, kSmallW8 = 2, kSmallW4Sym = 3 };
 
 __device__ __forceinline__ void mma_m16n8k16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                              uint32_t b0, uint32_t b1) {
@@ -100,7 +101,7 @@ __global__ void __launch_bounds__(CPW == 1 ? 512 : 256, CPW == 1 ? 1 : 2) wq_gem
   const int c = lane & 3, g = lane >> 2;
   const int crank = p.cluster > 1 ? static_cast<int>(cluster_cta_rank()) : 0;
   const int stride = warps * p.cluster;  // steps between two of this warp
-  const bool has_zero = p.zeros != nullptr;
+  const bool has_zero = KIND != kSmallW4Sym && p.zeros != nullptr;
   const uint32_t ring = smem_u32(small_smem) + warp * STAGES * St::kBytes;
   pdl_launch_dependents();
   if (p.cluster > 1) cluster_arrive_relaxed();  // "this CTA runs", before anyone writes to its shared memory
@@ -279,7 +280,10 @@ __global__ void __launch_bounds__(CPW == 1 ? 512 : 256, CPW == 1 ? 1 : 2) wq_gem
               s0 = dup_lo(sp); s1 = dup_hi(sp);
               z0 = has_zero ? dup_lo(zp) : 0x43084308u;
               z1 = has_zero ? dup_hi(zp) : 0x43084308u;
-              if (KIND == kSmallW4Relaid) {  // odd columns of a word are converted where they stand
+              if (KIND == kSmallW4Sym) {
+                z0 = sym4_offset(s0); z1 = sym4_offset(s1);
+                s0 = sym4_scale_low(s0); s1 = sym4_scale_mid(s1);
+              } else if (KIND == kSmallW4Relaid) {  // odd columns of a word are converted where they stand
                 s1 = mid_scale(s1);
                 z1 = has_zero ? mid_zero(z1) : 0xC000C000u;
               }
@@ -297,7 +301,11 @@ __global__ void __launch_bounds__(CPW == 1 ? 512 : 256, CPW == 1 ? 1 : 2) wq_gem
               for (int j = 0; j < 2; ++j) {
                 const int pr = 2 * h + j;  // pair of rows 2 pr, 2 pr + 1
                 const uint32_t we = w[(2 * pr) * CPW + wd], wo = w[(2 * pr + 1) * CPW + wd];
-                if (KIND == kSmallW4Relaid) {
+                if (KIND == kSmallW4Sym) {
+                  const uint32_t W = (pl == 0 ? we : wo) >> (8 * th);
+                  a[2 * j] = sym4_low(W, s0, z0);
+                  a[2 * j + 1] = sym4_mid(W, s1, z1);
+                } else if (KIND == kSmallW4Relaid) {
                   const uint32_t W = (pl == 0 ? we : wo) >> (8 * th);
                   a[2 * j] = deq4(W, z0, s0);
                   a[2 * j + 1] = deq4_mid(W, z1, s1);
@@ -355,6 +363,7 @@ __global__ void __launch_bounds__(CPW == 1 ? 512 : 256, CPW == 1 ? 1 : 2) wq_gem
         if (n0 + col < p.N) {
           float v = red[m * kRedRow + col];
           for (int k = 1; k < p.cluster; ++k) v += recv[(k - 1) * TOK * BN + i];
+          if (KIND == kSmallW4Sym) v *= kSymAcc;
           __nv_bfloat16 o = __float2bfloat16_rn(v);
           if (p.bias != nullptr) o = __float2bfloat16_rn(__bfloat162float(o) + __bfloat162float(p.bias[n0 + col]));
           if (p.epilogue == DXB_EPILOGUE_GELU_TANH) o = __float2bfloat16_rn(gelu_tanh(__bfloat162float(o)));
