@@ -72,7 +72,8 @@ __device__ __forceinline__ uint32_t deq4(uint32_t w, uint32_t zero2, uint32_t sc
 // The same for nibbles at bits 4..7 and 20..23, without shifting them down: as bf16 such a pattern is at most
 // in the first normal binade, whose step is that of the subnormals, so its value is 16 q * 2^-133 for
 // all sixteen q.  One exact multiply-add makes (q - zero) / 4 of it (times 2^127, plus `zero4` =
-// -zero / 4), `scale4` = 4 * scale puts the factor back, and its multiply is the only rounding.  Two of
+// -zero / 4), `scale4` = 4 * scale (for scales below 2^126) puts the factor back, and its multiply is
+// the only rounding.  Two of
 // four shifts of a word of nibbles go: with them the conversion, bound by the integer pipe, loses 32 of
 // 400 instructions per 128 x 128 weights.
 __device__ __forceinline__ uint32_t deq4_mid(uint32_t w, uint32_t zero4, uint32_t scale4) {
@@ -89,10 +90,17 @@ __device__ __forceinline__ uint32_t mid_zero(uint32_t zero2) {  // from 128 + ze
 // Symmetric grid (zero point 8): ONE multiply-add per two weights.  With the nibbles read as above (16 q or
 // q times 2^-133), q * scale - 8 * scale is exact up to the final rounding -- 8 * scale is a bf16, which
 // zero * scale in general is not -- so (q - 8) * scale needs no subtraction of its own.  2^133 * scale would
-// overflow, so the weights come out divided by 2^16, and so do the products and their fp32 sums, bit for
-// bit; whoever reads an accumulator multiplies by kSymAcc (exact).  Good for |scale| < 2^11 and
-// products above 2^-110.
-constexpr float kSymAcc = 65536.0f;
+// overflow, so the weights come out divided by 64, and so do the products and their fp32 sums, bit for
+// bit; whoever reads an accumulator multiplies by kSymAcc (exact down to 2^-120).  2^127 * scale still
+// overflows for |scale| >= 2, where sym4_any converts the long way (never with a model's weights, so the
+// check is one OR of exponents per unit: sym4_large).  Measured against deq4 / deq4_mid: 83 tokens 3072 x 14336
+// 10.9 -> 10.65 us, 14336 x 3072 12.4 -> 11.85, 16 tokens 9.25 -> 9.0; the check costs 0.25 us of it.
+constexpr float kSymAcc = 64.0f;
+__device__ __forceinline__ bool sym4_large(uint32_t scales) { return (scales & 0x40004000u) != 0; }
+// `offset`: sym4_offset of the scale, from which the scale comes back exactly.
+__device__ __forceinline__ uint32_t sym4_any(uint32_t w, uint32_t offset) {  // bits 0..3, 16..19
+  return mul_bf16x2(deq4(w, 0x43084308u, mul_bf16x2(offset, 0xC100C100u)), 0x3C803C80u);
+}
 __device__ __forceinline__ uint32_t sym4_low(uint32_t w, uint32_t scale, uint32_t offset) {  // bits 0..3, 16..19
   uint32_t d;
   asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(w & 0x000F000Fu), "r"(scale), "r"(offset));
@@ -103,9 +111,9 @@ __device__ __forceinline__ uint32_t sym4_mid(uint32_t w, uint32_t scale, uint32_
   asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(w & 0x00F000F0u), "r"(scale), "r"(offset));
   return d;
 }
-__device__ __forceinline__ uint32_t sym4_scale_low(uint32_t s2) { return mul_bf16x2(s2, 0x7A007A00u); }  // 2^(133-16)
-__device__ __forceinline__ uint32_t sym4_scale_mid(uint32_t s2) { return mul_bf16x2(s2, 0x78007800u); }  // 2^(129-16)
-__device__ __forceinline__ uint32_t sym4_offset(uint32_t s2) { return mul_bf16x2(s2, 0xB900B900u); }     // -8 * 2^-16
+__device__ __forceinline__ uint32_t sym4_scale_low(uint32_t s2) { return mul_bf16x2(s2, 0x7F007F00u); }  // 2^(133-6)
+__device__ __forceinline__ uint32_t sym4_scale_mid(uint32_t s2) { return mul_bf16x2(s2, 0x7D007D00u); }  // 2^(129-6)
+__device__ __forceinline__ uint32_t sym4_offset(uint32_t s2) { return mul_bf16x2(s2, 0xBE00BE00u); }     // -8 * 2^-6
 // One byte -> fp32 by bit pattern: 0x4B0000qq = 8388608 + q.  `cz` = 8388608 +
 // zero point; subtract and multiply are both exact in fp32 (8-bit x 8-bit
 // significands), so the later cvt.rn to bf16 is the only rounding.

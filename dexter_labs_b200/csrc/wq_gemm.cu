@@ -18,9 +18,8 @@
 //   warp 2       TMA producer: the matching activation k-slices (both nibble planes
 //                in one 3-D box for int4).
 //   warps 8-23   four dequant teams of four warps, one unit each in flight:
-//                ld.shared of packed words, nibble -> bf16 by bit pattern (OR into
-//                0x4300 = 128.0, exact subtract, one multiply; no int->float convert),
-//                k-pairs formed with two byte permutes, written straight into TMEM with
+//                ld.shared of packed words, values -> bf16 by bit pattern (deq4, sym4_low,
+//                deq8_fma; no int->float convert), written straight into TMEM with
 //                tcgen05.st.16x128b (the dequantised tile never touches shared memory);
 //                scales and zero points come from global memory one unit ahead.
 //   warp 1       one lane issues tcgen05.mma (A = weights from TMEM, B = activations
@@ -28,10 +27,12 @@
 //   warps 4-7    epilogue: tcgen05.ld, bias, bf16 stores; or fp32 partial sums.
 // How the (tile, unit) space is handed to CTAs is chosen per launch (make_plan,
 // launch_tc): whole tiles per CTA; equal contiguous unit ranges (stream-K), where a tile
-// shared by several CTAs is finished by whichever CTA arrives last (no CTA ever waits for
-// another one), summing the partials in a fixed order; or, for few tiles, one
+// shared by several CTAs is finished by the one that holds its first units, which adds the
+// others' partial sums in a fixed order; or, for few tiles, one
 // thread-block cluster per tile that splits K and adds through distributed shared memory.
-// More than 128 tokens: every (token block of 128, column tile) pair is a tile, one launch.
+// More than 128 tokens: every (token block, column tile) pair is a tile, one launch; on single CTAs
+// (blocks of 128 tokens) or on CTA pairs (256 columns x up to 256 tokens).
+// Few tokens on small weights, and shapes off these tiles, take wq_gemm_small (wq_small.cuh) instead.
 #include "wq_common.cuh"
 #include "wq_small.cuh"
 
@@ -242,7 +243,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   const int TU = p.total_units;
   const int G = static_cast<int>(gridDim.x);
   const int U = p.units_per_tile;
-  constexpr bool SYM4 = BITS == 4 && !HAS_ZERO;  // weights and sums are scaled by 2^-16, see sym4_low
+  constexpr bool SYM4 = BITS == 4 && !HAS_ZERO;  // weights and sums are divided by kSymAcc, see sym4_low
   constexpr float ACC = SYM4 ? kSymAcc : 1.0f;
   constexpr bool kLean = MODE != kModeGeneral;
   constexpr bool PAIR = MODE == kModePair;
@@ -855,6 +856,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       // This unit's scales and zero points as the conversion wants them (int4: in both halves of a
       // word; int8: the constants of deq8_fma); then the next unit's rows.
       uint32_t s2[PLANES][4], z2[PLANES][4];
+      const bool large = SYM4 && __any_sync(0xffffffffu, sym4_large(sc[0].x | sc[0].y | sc[1].x | sc[1].y));
 #pragma unroll
       for (int pl = 0; pl < PLANES; ++pl) {
         if (BITS == 4) {
@@ -908,7 +910,35 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       ok = mbar_wait(a_empty_bar, aph ^ 1u, abortp);
       if (!ok) break;
       tc_fence_after();
-      if (BITS == 4) {
+      if (large) {
+        // The same with scales of 2 and more, see sym4_any; a body of its own, so that the usual one is
+        // scheduled as if this did not exist (a branch in front of each store made launches 6 % longer).
+#pragma unroll
+        for (int pl = 0; pl < 2; ++pl) {
+#pragma unroll
+          for (int rh = 0; rh < 2; ++rh) {
+            uint32_t ra[8], rb[8];
+#pragma unroll
+            for (int sl = 0; sl < 4; ++sl) {
+              uint32_t v[4];  // the four columns' pairs at bits 0..3 and 16..19
+              if (RELAID) {
+                const uint32_t W = pl == 0 ? w0[4 * rh + sl] : w1[4 * rh + sl];
+                v[0] = W; v[1] = W >> 4; v[2] = W >> 8; v[3] = W >> 12;
+              } else {
+                v[0] = prmt(w0[4 * rh + sl], w1[4 * rh + sl], 0x5410u) >> (4 * pl);
+                v[2] = prmt(w0[4 * rh + sl], w1[4 * rh + sl], 0x7632u) >> (4 * pl);
+                v[1] = v[0] >> 8; v[3] = v[2] >> 8;
+              }
+              ra[2 * sl + 0] = sym4_any(v[0], z2[pl][0]);
+              ra[2 * sl + 1] = sym4_any(v[1], z2[pl][1]);
+              rb[2 * sl + 0] = sym4_any(v[2], z2[pl][2]);
+              rb[2 * sl + 1] = sym4_any(v[3], z2[pl][3]);
+            }
+            tmem_st_16x128b_x4(tmem_addr(a_tmem + pl * 32 + 16 * rh, lane_base, 0), ra);
+            tmem_st_16x128b_x4(tmem_addr(a_tmem + pl * 32 + 16 * rh, lane_base + 16, 0), rb);
+          }
+        }
+      } else if (BITS == 4) {
 #pragma unroll
         for (int pl = 0; pl < 2; ++pl) {
 #pragma unroll

@@ -19,6 +19,8 @@
 // h-th m16n8k16 product.  Columns are the products' m, tokens their n.  Few tiles and long K: a
 // cluster shares a tile's steps and adds through distributed shared memory.
 #pragma once
+#include <type_traits>
+
 #include "wq_common.cuh"
 
 namespace dx {
@@ -250,81 +252,98 @@ __global__ void __launch_bounds__(CPW == 1 ? 512 : 256, CPW == 1 ? 1 : 2) wq_gem
           w[2 * r + CPW - 1] = v.y;
         }
       }
+      // Scales (and zero points) of this lane's columns, two bf16 per word.
+      auto row4 = [&](int pl, int rs, const __nv_bfloat16* base, int wd) -> uint2 {
+        const uint32_t a = st + St::kS + rs * St::kScaleRow;
+        if (!RAGGED) return lds64(a + (4 * CPW * g + 4 * wd) * 2);
+        const uint32_t off = static_cast<uint32_t>(
+            (reinterpret_cast<uintptr_t>(base) +
+             2 * (static_cast<uintptr_t>((first + i * stride + pl * p.steps) / (p.group >> 5)) * p.N + n0)) & 3);
+        const uint32_t b = a + off + 8 * g;
+        return make_uint2(lds16(b) | (lds16(b + 2) << 16), lds16(b + 4) | (lds16(b + 6) << 16));
+      };
+      uint2 scale[PLANES][CPW];
+      uint32_t any = 0;
 #pragma unroll
-      for (int pl = 0; pl < PLANES; ++pl) {
-        uint4 xv[MT];
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) xv[mt] = lds128(st + St::kX + (pl * TOK + 8 * mt + g) * 64 + 16 * c);
-        // Scales (and zero points) of this lane's columns, two bf16 per word.
-        auto row4 = [&](int rs, const __nv_bfloat16* base, int wd) -> uint2 {
-          const uint32_t a = st + St::kS + rs * St::kScaleRow;
-          if (!RAGGED) return lds64(a + (4 * CPW * g + 4 * wd) * 2);
-          const uint32_t off = static_cast<uint32_t>(
-              (reinterpret_cast<uintptr_t>(base) +
-               2 * (static_cast<uintptr_t>((first + i * stride + pl * p.steps) / (p.group >> 5)) * p.N + n0)) & 3);
-          const uint32_t b = a + off + 8 * g;
-          return make_uint2(lds16(b) | (lds16(b + 2) << 16), lds16(b + 4) | (lds16(b + 6) << 16));
-        };
+      for (int pl = 0; pl < PLANES; ++pl)
 #pragma unroll
         for (int wd = 0; wd < CPW; ++wd) {
-          const uint2 sv = row4(pl, p.scales, wd);
-          uint2 zv = make_uint2(0u, 0u);
-          if (has_zero) zv = row4(PLANES + pl, p.zeros, wd);
+          scale[pl][wd] = row4(pl, pl, p.scales, wd);
+          any |= scale[pl][wd].x | scale[pl][wd].y;
+        }
+      auto products = [&](auto way) {
+        constexpr bool LARGE = decltype(way)::value;
 #pragma unroll
-          for (int th = 0; th < 2; ++th) {  // 16 columns: 4g + 2 th and the next, of word wd
-            const int t = 2 * wd + th;
-            const uint32_t sp = th ? sv.y : sv.x;
-            const uint32_t zp = th ? zv.y : zv.x;
-            uint32_t s0, s1, z0, z1;
-            if (W4) {
-              s0 = dup_lo(sp); s1 = dup_hi(sp);
-              z0 = has_zero ? dup_lo(zp) : 0x43084308u;
-              z1 = has_zero ? dup_hi(zp) : 0x43084308u;
-              if (KIND == kSmallW4Sym) {
-                z0 = sym4_offset(s0); z1 = sym4_offset(s1);
-                s0 = sym4_scale_low(s0); s1 = sym4_scale_mid(s1);
-              } else if (KIND == kSmallW4Relaid) {  // odd columns of a word are converted where they stand
-                s1 = mid_scale(s1);
-                z1 = has_zero ? mid_zero(z1) : 0xC000C000u;
-              }
-            } else {
-              float f, o;
-              deq8_constants(bf16lo_f32(sp), has_zero ? bf16lo_f32(zp) : 128.0f, f, o);
-              s0 = __float_as_uint(f); z0 = __float_as_uint(o);
-              deq8_constants(bf16hi_f32(sp), has_zero ? bf16hi_f32(zp) : 128.0f, f, o);
-              s1 = __float_as_uint(f); z1 = __float_as_uint(o);
-            }
+        for (int pl = 0; pl < PLANES; ++pl) {
+          uint4 xv[MT];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              uint32_t a[4];
+          for (int mt = 0; mt < MT; ++mt) xv[mt] = lds128(st + St::kX + (pl * TOK + 8 * mt + g) * 64 + 16 * c);
 #pragma unroll
-              for (int j = 0; j < 2; ++j) {
-                const int pr = 2 * h + j;  // pair of rows 2 pr, 2 pr + 1
-                const uint32_t we = w[(2 * pr) * CPW + wd], wo = w[(2 * pr + 1) * CPW + wd];
+          for (int wd = 0; wd < CPW; ++wd) {
+            const uint2 sv = scale[pl][wd];
+            uint2 zv = make_uint2(0u, 0u);
+            if (has_zero) zv = row4(pl, PLANES + pl, p.zeros, wd);
+#pragma unroll
+            for (int th = 0; th < 2; ++th) {  // 16 columns: 4g + 2 th and the next, of word wd
+              const int t = 2 * wd + th;
+              const uint32_t sp = th ? sv.y : sv.x;
+              const uint32_t zp = th ? zv.y : zv.x;
+              uint32_t s0, s1, z0, z1;
+              if (W4) {
+                s0 = dup_lo(sp); s1 = dup_hi(sp);
+                z0 = has_zero ? dup_lo(zp) : 0x43084308u;
+                z1 = has_zero ? dup_hi(zp) : 0x43084308u;
                 if (KIND == kSmallW4Sym) {
-                  const uint32_t W = (pl == 0 ? we : wo) >> (8 * th);
-                  a[2 * j] = sym4_low(W, s0, z0);
-                  a[2 * j + 1] = sym4_mid(W, s1, z1);
-                } else if (KIND == kSmallW4Relaid) {
-                  const uint32_t W = (pl == 0 ? we : wo) >> (8 * th);
-                  a[2 * j] = deq4(W, z0, s0);
-                  a[2 * j + 1] = deq4_mid(W, z1, s1);
-                } else if (KIND == kSmallW4) {
-                  const uint32_t P = prmt(we, wo, th ? 0x7632u : 0x5410u) >> (4 * pl);
-                  a[2 * j] = deq4(P, z0, s0);
-                  a[2 * j + 1] = deq4(P >> 8, z1, s1);
-                } else {
-                  a[2 * j] = deq8_pair(we, wo, 2 * th, s0, z0);
-                  a[2 * j + 1] = deq8_pair(we, wo, 2 * th + 1, s1, z1);
+                  z0 = sym4_offset(s0); z1 = sym4_offset(s1);
+                  s0 = sym4_scale_low(s0); s1 = sym4_scale_mid(s1);
+                } else if (KIND == kSmallW4Relaid) {  // odd columns of a word are converted where they stand
+                  s1 = mid_scale(s1);
+                  z1 = has_zero ? mid_zero(z1) : 0xC000C000u;
                 }
+              } else {
+                float f, o;
+                deq8_constants(bf16lo_f32(sp), has_zero ? bf16lo_f32(zp) : 128.0f, f, o);
+                s0 = __float_as_uint(f); z0 = __float_as_uint(o);
+                deq8_constants(bf16hi_f32(sp), has_zero ? bf16hi_f32(zp) : 128.0f, f, o);
+                s1 = __float_as_uint(f); z1 = __float_as_uint(o);
               }
 #pragma unroll
-              for (int mt = 0; mt < MT; ++mt)
-                mma_m16n8k16(acc[t][mt], a[0], a[1], a[2], a[3], h ? xv[mt].z : xv[mt].x, h ? xv[mt].w : xv[mt].y);
+              for (int h = 0; h < 2; ++h) {
+                uint32_t a[4];
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                  const int pr = 2 * h + j;  // pair of rows 2 pr, 2 pr + 1
+                  const uint32_t we = w[(2 * pr) * CPW + wd], wo = w[(2 * pr + 1) * CPW + wd];
+                  if (KIND == kSmallW4Sym) {
+                    const uint32_t W = (pl == 0 ? we : wo) >> (8 * th);
+                    a[2 * j] = LARGE ? sym4_any(W, z0) : sym4_low(W, s0, z0);
+                    a[2 * j + 1] = LARGE ? sym4_any(W >> 4, z1) : sym4_mid(W, s1, z1);
+                  } else if (KIND == kSmallW4Relaid) {
+                    const uint32_t W = (pl == 0 ? we : wo) >> (8 * th);
+                    a[2 * j] = deq4(W, z0, s0);
+                    a[2 * j + 1] = deq4_mid(W, z1, s1);
+                  } else if (KIND == kSmallW4) {
+                    const uint32_t P = prmt(we, wo, th ? 0x7632u : 0x5410u) >> (4 * pl);
+                    a[2 * j] = deq4(P, z0, s0);
+                    a[2 * j + 1] = deq4(P >> 8, z1, s1);
+                  } else {
+                    a[2 * j] = deq8_pair(we, wo, 2 * th, s0, z0);
+                    a[2 * j + 1] = deq8_pair(we, wo, 2 * th + 1, s1, z1);
+                  }
+                }
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt)
+                  mma_m16n8k16(acc[t][mt], a[0], a[1], a[2], a[3], h ? xv[mt].z : xv[mt].x, h ? xv[mt].w : xv[mt].y);
+              }
             }
           }
         }
-      }
+      };
+      // (kSmallW4Sym only: see sym4_any)
+      if (KIND == kSmallW4Sym && __any_sync(0xffffffffu, sym4_large(any)))
+        products(std::integral_constant<bool, KIND == kSmallW4Sym>{});
+      else
+        products(std::false_type{});
       fill = st;
       st += St::kBytes;
       if (st == ring_end) st = ring;

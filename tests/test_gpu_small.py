@@ -68,3 +68,25 @@ def test_single_nonzero_activation_reads_back_the_exact_weight(bits, symmetric, 
         x = torch.zeros(16, k, device="cuda", dtype=torch.bfloat16)
         x[torch.arange(16), k0 + torch.arange(16)] = 1
         assert torch.equal(fn(x, q.qweight, q.scales, q.zeros, None, 64), want[k0:k0 + 16])
+
+
+@pytest.mark.parametrize("relaid", [True, False])
+@pytest.mark.parametrize("m,k,n", [(16, 256, 48), (128, 2048, 2048), (256, 4096, 14336)])
+def test_symmetric_int4_over_the_whole_range_of_scales(m, k, n, relaid, d, oracle, monkeypatch):
+    """Few-token kernel, single CTAs and CTA pairs; scales from 2^-60 to 2^100, mixed in every group row and
+    alone: one-hot activations read the exact weights back."""
+    if not relaid:
+        monkeypatch.setattr(d.ops, "_AUTO_RELAYOUT", False)
+        monkeypatch.setattr(d.ops, "_CALL", None)
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    q = torch.randint(0, 256, (k // 2, n), generator=gen, device="cuda", dtype=torch.uint8)
+    exponent = torch.randint(-60, 101, (k // 64, n), generator=gen, device="cuda")
+    exponent[:, : n // 2] = -9                                     # what models have
+    exponent[0, : n // 4] = torch.arange(n // 4, device="cuda") % 5 - 1  # around the line between the two ways
+    s = (torch.rand(exponent.shape, generator=gen, device="cuda") + 1) * torch.exp2(exponent.float())
+    s = s.to(torch.bfloat16)
+    want = oracle.torch_dequantize(q, s, None, 64, 4)
+    rows = torch.arange(m, device="cuda") * (k // m)
+    x = torch.zeros(m, k, device="cuda", dtype=torch.bfloat16)
+    x[torch.arange(m, device="cuda"), rows] = 1
+    assert torch.equal(d.w4a16(x, q, s, None, None, 64), want[rows])
