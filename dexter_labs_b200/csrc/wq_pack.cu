@@ -168,7 +168,7 @@ static int launch_dequant(const void* qweight, const void* scales, const void* z
 // codes transposed to [K, N] (int8) or [K/2, N] (int4, row i low and row i + K/2 high nibble).
 //
 // 2 bytes read and bits/8 written per weight, once each; bound by instruction issue (int4 14336 x 3072:
-// 43 us with about 20 instructions per weight, 931 us as element-wise passes; the copy alone would
+// 40 us with about 20 instructions per weight, 931 us as element-wise passes; the copy alone would
 // take 17 us).  One CTA packs 128 outputs x
 // two spans of 128 k (for int4 the two spans share their packed rows: k and k + K/2).  A half warp
 // reads one output's span with one 16-byte load per lane (256 B runs), finds the group's extremes
@@ -239,9 +239,11 @@ __device__ __forceinline__ uint32_t quant_code(const QuantGrid& g, float w, floa
 // carries the integer in its low bits: no conversion instructions, which run at a quarter of the rate.
 // `inside`: every value's exact sum lies on the grid or within half a step of it, so that no code
 // needs clamping unless it is as close to a rounding boundary as sends it to the exact path.
+// PEAKS: `inv` went through quant_peaks, so that a group's extremes are no such case.
+template <bool PEAKS>
 __device__ __forceinline__ uint2 quant_code8(const QuantGrid& g, const uint32_t (&x)[4], float scale, float inv,
                                              float shift, bool inside) {
-  constexpr float kMagic = 12582912.0f, kFar = 0.4998f;
+  constexpr float kMagic = 12582912.0f, kFar = PEAKS ? 0.49986f : 0.4998f;
   float far = 0.0f;  // largest distance from a whole number
   uint32_t c[8];
 #pragma unroll
@@ -260,8 +262,23 @@ __device__ __forceinline__ uint2 quant_code8(const QuantGrid& g, const uint32_t 
         c[j] = quant_code(g, w, scale, shift);
     }
   }
-  return make_uint2(prmt(prmt(c[0], c[1], 0x0040u), prmt(c[2], c[3], 0x0040u), 0x5410u),
-                    prmt(prmt(c[4], c[5], 0x0040u), prmt(c[6], c[7], 0x0040u), 0x5410u));
+  uint2 v = make_uint2(prmt(prmt(c[0], c[1], 0x0040u), prmt(c[2], c[3], 0x0040u), 0x5410u),
+                       prmt(prmt(c[4], c[5], 0x0040u), prmt(c[6], c[7], 0x0040u), 0x5410u));
+  if (PEAKS) {  // 16 -> 15
+    v.x -= (v.x >> 4) & 0x01010101u;
+    v.y -= (v.y >> 4) & 0x01010101u;
+  }
+  return v;
+}
+// On the symmetric int4 grid the largest magnitude of every group falls on a rounding boundary: +-7.5 + 8,
+// which sent a lane of every group to the division (53 us for 14336 x 3072, 41 so; 43 on the other grid).  The
+// negative one's code (0 or 1) is found once per group, exactly, and the reciprocal is moved by 2e-5 so
+// that both extremes land clearly on their codes' side (the positive one on 15 or 16, see above).
+// Their distance from the boundary is then 1.5e-4; sums near any OTHER boundary move by at most 6.5 / 7.5
+// of that, 1.3e-4, so 1.4e-4 tells the two apart (all errors of computation: 4e-6).  int8 has its
+// second boundary too close to the first for this (126.5 / 127.5).
+__device__ __forceinline__ float quant_peaks(const QuantGrid& g, float peak, float scale, float inv, float shift) {
+  return inv * (quant_code(g, -peak, scale, shift) == 0 ? 1.00002f : 0.99998f);
 }
 __device__ __forceinline__ bool quant_inside(const QuantGrid& g, float lo, float hi, float inv, float shift) {
   return __fmaf_rn(lo, inv, shift) >= -0.501f && __fmaf_rn(hi, inv, shift) <= g.levels + 0.501f;  // false for NaN
@@ -319,14 +336,14 @@ wq_quant_stats_kernel(const __nv_bfloat16* __restrict__ w, float* __restrict__ s
 
 // LPG: lanes per group (group = 8 * LPG: 32, 64 or 128, extremes found here), or 0: scales and
 // shifts come from the pass above.
-template <int BITS, int LPG>
+template <int BITS, int LPG, bool SYM>
 __global__ void __launch_bounds__(256, 4)
 wq_quant_pack_kernel(const __nv_bfloat16* __restrict__ w, const float* __restrict__ scale32,
                      const float* __restrict__ shift32, uint8_t* __restrict__ q, __nv_bfloat16* __restrict__ scales,
-                     __nv_bfloat16* __restrict__ zeros, int N, int K, int group, int symmetric) {
+                     __nv_bfloat16* __restrict__ zeros, int N, int K, int group) {
   constexpr int kPlanes = BITS == 4 ? 1 : 2;  // spans that have packed rows of their own
   __shared__ uint32_t tile[kPlanes][128][32];  // [span][row][word of 4 outputs], words rotated by row / 8
-  const QuantGrid g = quant_grid<BITS>(symmetric != 0);
+  const QuantGrid g = quant_grid<BITS>(SYM);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int half = lane >> 4, l = lane & 15;
   const int rows = BITS == 4 ? K >> 1 : K;      // packed rows
@@ -354,7 +371,7 @@ wq_quant_pack_kernel(const __nv_bfloat16* __restrict__ w, const float* __restric
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const uint32_t x[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
-        if (symmetric) {
+        if (SYM) {
           hi[i] = max2_nan(max2_nan(x[0] & 0x7FFF7FFFu, x[1] & 0x7FFF7FFFu), max2_nan(x[2] & 0x7FFF7FFFu, x[3] & 0x7FFF7FFFu));
         } else {
           hi[i] = max2_nan(max2_nan(x[0], x[1]), max2_nan(x[2], x[3]));
@@ -368,20 +385,22 @@ wq_quant_pack_kernel(const __nv_bfloat16* __restrict__ w, const float* __restric
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         h2[i] = max2_nan(up1 ? hi[2 + i] : hi[i], __shfl_xor_sync(0xffffffffu, up1 ? hi[i] : hi[2 + i], D1));
-        if (!symmetric) l2[i] = min2_nan(up1 ? lo[2 + i] : lo[i], __shfl_xor_sync(0xffffffffu, up1 ? lo[i] : lo[2 + i], D1));
+        if (!SYM) l2[i] = min2_nan(up1 ? lo[2 + i] : lo[i], __shfl_xor_sync(0xffffffffu, up1 ? lo[i] : lo[2 + i], D1));
       }
       uint32_t h1 = max2_nan(up2 ? h2[1] : h2[0], __shfl_xor_sync(0xffffffffu, up2 ? h2[0] : h2[1], D2)), l1 = 0u;
-      if (!symmetric) l1 = min2_nan(up2 ? l2[1] : l2[0], __shfl_xor_sync(0xffffffffu, up2 ? l2[0] : l2[1], D2));
+      if (!SYM) l1 = min2_nan(up2 ? l2[1] : l2[0], __shfl_xor_sync(0xffffffffu, up2 ? l2[0] : l2[1], D2));
 #pragma unroll
       for (int d = LPG / 8; d >= 1; d >>= 1) {
         h1 = max2_nan(h1, __shfl_xor_sync(0xffffffffu, h1, d));
-        if (!symmetric) l1 = min2_nan(l1, __shfl_xor_sync(0xffffffffu, l1, d));
+        if (!SYM) l1 = min2_nan(l1, __shfl_xor_sync(0xffffffffu, l1, d));
       }
-      const float hi_f = max_halves(h1), lo_f = symmetric ? -hi_f : min_halves(l1);
+      const float hi_f = max_halves(h1), lo_f = SYM ? -hi_f : min_halves(l1);
       float scale, shift;
       quant_scale(g, lo_f, hi_f, scale, shift);
-      const float inv = rcp_approx(scale);
+      float inv = rcp_approx(scale);
       const int inside = quant_inside(g, lo_f, hi_f, inv, shift) ? 1 : 0;
+      constexpr bool kPeaks = BITS == 4 && SYM;
+      if (kPeaks) inv = quant_peaks(g, hi_f, scale, inv, shift);
       const int n_own = n0 + 4 * quad + own;
       if ((l & (D2 - 1)) == 0 && k_ok && n_own < N) {
         const long long o = static_cast<long long>(gi) * N + n_own;
@@ -396,7 +415,7 @@ wq_quant_pack_kernel(const __nv_bfloat16* __restrict__ w, const float* __restric
         const float iv = __shfl_sync(0xffffffffu, inv, from, LPG > 0 ? LPG : 32);
         const float sh = __shfl_sync(0xffffffffu, shift, from, LPG > 0 ? LPG : 32);
         const bool in = __shfl_sync(0xffffffffu, inside, from, LPG > 0 ? LPG : 32) != 0;
-        code[i] = quant_code8(g, x, sc, iv, sh, in);
+        code[i] = quant_code8<kPeaks>(g, x, sc, iv, sh, in);
       }
     } else {
 #pragma unroll
@@ -407,7 +426,7 @@ wq_quant_pack_kernel(const __nv_bfloat16* __restrict__ w, const float* __restric
         const float scale = __ldg(scale32 + o), shift = __ldg(shift32 + o), inv = rcp_approx(scale);
         const float hi = max_halves(max2_nan(max2_nan(x[0], x[1]), max2_nan(x[2], x[3])));
         const float lo = min_halves(min2_nan(min2_nan(x[0], x[1]), min2_nan(x[2], x[3])));
-        code[i] = quant_code8(g, x, scale, inv, shift, quant_inside(g, lo, hi, inv, shift));
+        code[i] = quant_code8<false>(g, x, scale, inv, shift, quant_inside(g, lo, hi, inv, shift));
       }
     }
     // 4 x 8 bytes -> the words of 8 rows (four outputs each)
@@ -475,15 +494,16 @@ static int launch_quantize(const void* weight, void* qweight, void* scales, void
   const dim3 grid((rows + span - 1) / span, (N + 127) / 128);
   if (grid.y > 65535) return DXB_ERR_UNSUPPORTED;
   if (dxb_quantize_scratch_bytes(N, K, group, BITS) == 0) {
-    auto kernel = group == 128 ? wq_quant_pack_kernel<BITS, 16>
-                  : group == 64 ? wq_quant_pack_kernel<BITS, 8> : wq_quant_pack_kernel<BITS, 4>;
-    kernel<<<grid, 256, 0, stream>>>(w, nullptr, nullptr, q, s, z, N, K, group, symmetric);
+    auto kernel = group == 128 ? (symmetric ? wq_quant_pack_kernel<BITS, 16, true> : wq_quant_pack_kernel<BITS, 16, false>)
+                  : group == 64 ? (symmetric ? wq_quant_pack_kernel<BITS, 8, true> : wq_quant_pack_kernel<BITS, 8, false>)
+                                : (symmetric ? wq_quant_pack_kernel<BITS, 4, true> : wq_quant_pack_kernel<BITS, 4, false>);
+    kernel<<<grid, 256, 0, stream>>>(w, nullptr, nullptr, q, s, z, N, K, group);
   } else {
     const long long cells = static_cast<long long>(K / group) * N;
     float* scale32 = static_cast<float*>(scratch);
     wq_quant_stats_kernel<BITS><<<static_cast<unsigned>((cells + 7) / 8), 256, 0, stream>>>(
         w, scale32, scale32 + cells, s, z, N, K, group, symmetric);
-    wq_quant_pack_kernel<BITS, 0><<<grid, 256, 0, stream>>>(w, scale32, scale32 + cells, q, s, z, N, K, group, symmetric);
+    wq_quant_pack_kernel<BITS, 0, false><<<grid, 256, 0, stream>>>(w, scale32, scale32 + cells, q, s, z, N, K, group);
   }
   return cudaGetLastError() == cudaSuccess ? DXB_OK : DXB_ERR_CUDA;
 }

@@ -56,3 +56,21 @@ def test_dequantize_matches_the_oracle(k, n, bits, group, layout, symmetric, d, 
     got = d.dequantize(qg, s.cuda(), None if z is None else z.cuda(), group, bits) if layout == "dexter" else \
         d.ops.dequantize(qg, s.cuda(), None if z is None else z.cuda(), group, bits, layout=layout)
     assert np.array_equal(got.cpu().view(torch.int16).numpy(), want.view(torch.int16).numpy())
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("symmetric", [True, False])
+def test_quantize_of_values_on_rounding_boundaries(bits, symmetric, d):
+    # weights at (and one bf16 step beside) whole and half steps of their group's grid, extremes of either sign
+    gen = torch.Generator(device="cuda").manual_seed(bits)
+    n, k, steps = 512, 512, 2 ** bits - 1
+    peak = (torch.rand(n, k // 128, 1, generator=gen, device="cuda") + 1) * torch.exp2(
+        torch.randint(-40, 20, (n, k // 128, 1), generator=gen, device="cuda").float())
+    step = torch.randint(-steps, steps + 1, (n, k // 128, 128), generator=gen, device="cuda").float() / steps
+    step[..., 0] = torch.where(torch.rand(n, k // 128, generator=gen, device="cuda") < 0.5, 1.0, -1.0)
+    w = (peak * step).reshape(n, k).to(torch.bfloat16)
+    w = (w.view(torch.int16) + torch.randint(-1, 2, (n, k), generator=gen, device="cuda", dtype=torch.int16)).view(torch.bfloat16)
+    w[~torch.isfinite(w)] = 0
+    got = d.quantize(w, bits=bits, symmetric=symmetric)
+    want = d.quantize(w.clone().requires_grad_(), bits=bits, symmetric=symmetric)
+    assert torch.equal(got.qweight, want.qweight) and torch.equal(got.scales, want.scales.detach())
