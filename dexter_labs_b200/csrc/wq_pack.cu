@@ -168,7 +168,7 @@ static int launch_dequant(const void* qweight, const void* scales, const void* z
 // codes transposed to [K, N] (int8) or [K/2, N] (int4, row i low and row i + K/2 high nibble).
 //
 // 2 bytes read and bits/8 written per weight, once each; bound by instruction issue (int4 14336 x 3072:
-// 40 us with about 20 instructions per weight, 931 us as element-wise passes; the copy alone would
+// 39 us, 931 us as element-wise passes; the copy alone would
 // take 17 us).  One CTA packs 128 outputs x
 // two spans of 128 k (for int4 the two spans share their packed rows: k and k + K/2).  A half warp
 // reads one output's span with one 16-byte load per lane (256 B runs), finds the group's extremes
@@ -180,8 +180,8 @@ static int launch_dequant(const void* qweight, const void* scales, const void* z
 // are those of that chain of element-wise passes): all fp32; division by a constant is
 // multiplication by its rounded reciprocal, division by the scale is an exact division; rounding
 // to nearest even.  The codes get there without dividing: a product with the reciprocal of
-// the scale is within 2e-4 of the quotient's own rounded sum while that is at most 512, so only values that
-// close to a rounding boundary (4 in 10 000, or far outside the grid) take the division.
+// the scale is within 1.2e-5 (int8: 1.1e-4) of the quotient's own rounded sum, so only values closer than
+// that to a rounding boundary, and groups that the grid does not cover, take the division.
 struct QuantGrid {
   float levels, inv_levels, mid;
   bool symmetric;
@@ -235,53 +235,69 @@ __device__ __forceinline__ uint32_t quant_code(const QuantGrid& g, float w, floa
   const float r = rintf(__fadd_rn(__fdiv_rn(w, scale), shift));
   return static_cast<uint32_t>(static_cast<uint8_t>(clamp_nan(r, 0.0f, g.levels)));
 }
-// Codes of a lane's 8 values, eight bytes in k order.  Rounding is an addition of 1.5 * 2^23, whose sum
-// carries the integer in its low bits: no conversion instructions, which run at a quarter of the rate.
-// `inside`: every value's exact sum lies on the grid or within half a step of it, so that no code
-// needs clamping unless it is as close to a rounding boundary as sends it to the exact path.
+// Codes of a lane's 8 values, eight bytes in k order, from ONE multiply-add per value: with 192.5 (int8:
+// 768.5) added, the sum's mantissa is a fixed-point number whose bits 16.. are the rounded code (int8
+// after a shift by two) and whose low 16 bits say how far above a rounding boundary it lies.  The
+// constant carries a margin as well, so values within the margin of a boundary are those with less than
+// twice the margin there.  (Rounding by adding and subtracting 1.5 * 2^23 and taking the distance as a
+// difference took three instructions more per value: 40 us for int4 14336 x 3072, 39 so.)
+// `inside`: every value's sum lies on the grid or so little beside it that it is within the margin.
 // PEAKS: `inv` went through quant_peaks, so that a group's extremes are no such case.
-template <bool PEAKS>
+template <int BITS, bool PEAKS>
+struct QuantFixed {
+  static constexpr uint32_t kMargin = PEAKS ? 18 : BITS == 4 ? 2 : 16;  // in 2^-16
+  static constexpr float kBase = (BITS == 4 ? 192.5f : 768.5f) + kMargin / 65536.0f;  // exact, as is shift + kBase
+};
+__device__ __forceinline__ uint32_t min_u16x2(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("min.u16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+template <int BITS, bool PEAKS>
 __device__ __forceinline__ uint2 quant_code8(const QuantGrid& g, const uint32_t (&x)[4], float scale, float inv,
                                              float shift, bool inside) {
-  constexpr float kMagic = 12582912.0f, kFar = PEAKS ? 0.49986f : 0.4998f;
-  float far = 0.0f;  // largest distance from a whole number
-  uint32_t c[8];
+  constexpr uint32_t kNear = 2 * QuantFixed<BITS, PEAKS>::kMargin;
+  const float base = shift + QuantFixed<BITS, PEAKS>::kBase;
+  uint32_t u[8], nearest = 0xFFFFFFFFu;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    const float t = __fmaf_rn((j & 1) ? bf16hi_f32(x[j >> 1]) : bf16lo_f32(x[j >> 1]), inv, shift);
-    const float m = __fadd_rn(t, kMagic);
-    c[j] = __float_as_uint(m);
-    far = fmaxf(far, fabsf(__fsub_rn(t, __fsub_rn(m, kMagic))));
+    u[j] = __float_as_uint(__fmaf_rn((j & 1) ? bf16hi_f32(x[j >> 1]) : bf16lo_f32(x[j >> 1]), inv, base));
+    if (BITS == 8) u[j] <<= 2;
+    if (j & 1) nearest = min_u16x2(nearest, prmt(u[j - 1], u[j], 0x5410u));
   }
-  if (!inside || far > kFar) {
+  if (!inside || (nearest & 0xFFFFu) < kNear || (nearest >> 16) < kNear) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float w = (j & 1) ? bf16hi_f32(x[j >> 1]) : bf16lo_f32(x[j >> 1]);
-      const float t = __fmaf_rn(w, inv, shift);
-      if (!inside || fabsf(__fsub_rn(t, __fsub_rn(__fadd_rn(t, kMagic), kMagic))) > kFar)
-        c[j] = quant_code(g, w, scale, shift);
-    }
+    for (int j = 0; j < 8; ++j)
+      if (!inside || (u[j] & 0xFFFFu) < kNear)
+        u[j] = quant_code(g, (j & 1) ? bf16hi_f32(x[j >> 1]) : bf16lo_f32(x[j >> 1]), scale, shift) << 16;
   }
-  uint2 v = make_uint2(prmt(prmt(c[0], c[1], 0x0040u), prmt(c[2], c[3], 0x0040u), 0x5410u),
-                       prmt(prmt(c[4], c[5], 0x0040u), prmt(c[6], c[7], 0x0040u), 0x5410u));
-  if (PEAKS) {  // 16 -> 15
+  uint2 v = make_uint2(prmt(prmt(u[0], u[1], 0x0062u), prmt(u[2], u[3], 0x0062u), 0x5410u),
+                       prmt(prmt(u[4], u[5], 0x0062u), prmt(u[6], u[7], 0x0062u), 0x5410u));
+  if (PEAKS) {  // 16 -> 15 (bytes are 64 + code so far)
     v.x -= (v.x >> 4) & 0x01010101u;
     v.y -= (v.y >> 4) & 0x01010101u;
+  }
+  if (BITS == 4) {
+    v.x &= 0x0F0F0F0Fu;
+    v.y &= 0x0F0F0F0Fu;
   }
   return v;
 }
 // On the symmetric int4 grid the largest magnitude of every group falls on a rounding boundary: +-7.5 + 8,
 // which sent a lane of every group to the division (53 us for 14336 x 3072, 41 so; 43 on the other grid).  The
-// negative one's code (0 or 1) is found once per group, exactly, and the reciprocal is moved by 2e-5 so
+// negative one's code (0 or 1) is found once per group, exactly, and the reciprocal is moved by 4e-5 so
 // that both extremes land clearly on their codes' side (the positive one on 15 or 16, see above).
-// Their distance from the boundary is then 1.5e-4; sums near any OTHER boundary move by at most 6.5 / 7.5
-// of that, 1.3e-4, so 1.4e-4 tells the two apart (all errors of computation: 4e-6).  int8 has its
-// second boundary too close to the first for this (126.5 / 127.5).
+// Their distance from the boundary is then 3e-4; sums near any OTHER boundary move by at most 6.5 / 7.5
+// of that, 2.6e-4, so a margin of 18 * 2^-16 = 2.75e-4 tells the two apart (all errors of computation:
+// 1.2e-5).  int8 has its second boundary too close to the first for this (126.5 / 127.5).
 __device__ __forceinline__ float quant_peaks(const QuantGrid& g, float peak, float scale, float inv, float shift) {
-  return inv * (quant_code(g, -peak, scale, shift) == 0 ? 1.00002f : 0.99998f);
+  return inv * (quant_code(g, -peak, scale, shift) == 0 ? 1.00004f : 0.99996f);
 }
+// Sums of extremes that miss the grid by rounding errors only are within the margin of a boundary.
+template <int BITS>
 __device__ __forceinline__ bool quant_inside(const QuantGrid& g, float lo, float hi, float inv, float shift) {
-  return __fmaf_rn(lo, inv, shift) >= -0.501f && __fmaf_rn(hi, inv, shift) <= g.levels + 0.501f;  // false for NaN
+  constexpr float slack = BITS == 4 ? 1.5e-5f : 1.2e-4f;
+  return __fmaf_rn(lo, inv, shift) >= -0.5f - slack && __fmaf_rn(hi, inv, shift) <= g.levels + 0.5f + slack;  // false for NaN
 }
 // The zero point as it is stored: int4 kernels build 128 + q, so their zero points carry the 128.
 template <int BITS>
@@ -398,7 +414,7 @@ wq_quant_pack_kernel(const __nv_bfloat16* __restrict__ w, const float* __restric
       float scale, shift;
       quant_scale(g, lo_f, hi_f, scale, shift);
       float inv = rcp_approx(scale);
-      const int inside = quant_inside(g, lo_f, hi_f, inv, shift) ? 1 : 0;
+      const int inside = quant_inside<BITS>(g, lo_f, hi_f, inv, shift) ? 1 : 0;
       constexpr bool kPeaks = BITS == 4 && SYM;
       if (kPeaks) inv = quant_peaks(g, hi_f, scale, inv, shift);
       const int n_own = n0 + 4 * quad + own;
@@ -415,7 +431,7 @@ wq_quant_pack_kernel(const __nv_bfloat16* __restrict__ w, const float* __restric
         const float iv = __shfl_sync(0xffffffffu, inv, from, LPG > 0 ? LPG : 32);
         const float sh = __shfl_sync(0xffffffffu, shift, from, LPG > 0 ? LPG : 32);
         const bool in = __shfl_sync(0xffffffffu, inside, from, LPG > 0 ? LPG : 32) != 0;
-        code[i] = quant_code8<kPeaks>(g, x, sc, iv, sh, in);
+        code[i] = quant_code8<BITS, kPeaks>(g, x, sc, iv, sh, in);
       }
     } else {
 #pragma unroll
@@ -426,7 +442,7 @@ wq_quant_pack_kernel(const __nv_bfloat16* __restrict__ w, const float* __restric
         const float scale = __ldg(scale32 + o), shift = __ldg(shift32 + o), inv = rcp_approx(scale);
         const float hi = max_halves(max2_nan(max2_nan(x[0], x[1]), max2_nan(x[2], x[3])));
         const float lo = min_halves(min2_nan(min2_nan(x[0], x[1]), min2_nan(x[2], x[3])));
-        code[i] = quant_code8<false>(g, x, scale, inv, shift, quant_inside(g, lo, hi, inv, shift));
+        code[i] = quant_code8<BITS, false>(g, x, scale, inv, shift, quant_inside<BITS>(g, lo, hi, inv, shift));
       }
     }
     // 4 x 8 bytes -> the words of 8 rows (four outputs each)
