@@ -168,13 +168,13 @@ static int launch_dequant(const void* qweight, const void* scales, const void* z
 // codes transposed to [K, N] (int8) or [K/2, N] (int4, row i low and row i + K/2 high nibble).
 //
 // 2 bytes read and bits/8 written per weight, once each; bound by instruction issue (int4 14336 x 3072:
-// 39 us, 931 us as element-wise passes; the copy alone would
-// take 17 us).  One CTA packs 128 outputs x
+// 37 us, 931 us as element-wise passes; the copy alone would
+// take 17 us).  One CTA packs 64 outputs x
 // two spans of 128 k (for int4 the two spans share their packed rows: k and k + K/2).  A half warp
 // reads one output's span with one 16-byte load per lane (256 B runs), finds the group's extremes
 // by shuffles in packed bf16, codes its 8 values in registers, and four outputs make the 32-bit
 // words of the transposed tile, which goes through shared memory (swizzled: no bank conflicts) to
-// leave as whole 128-byte rows.
+// leave as 64-byte rows.
 //
 // Arithmetic, in the order of the framework's tensor expressions on this device (so the bytes
 // are those of that chain of element-wise passes): all fp32; division by a constant is
@@ -350,6 +350,9 @@ wq_quant_stats_kernel(const __nv_bfloat16* __restrict__ w, float* __restrict__ s
   }
 }
 
+// Outputs per CTA.  (128: a 14336 x 3072 weight is 2.3 rounds of CTAs on the chip and takes three.)
+constexpr int kQuantOuts = 64;
+
 // LPG: lanes per group (group = 8 * LPG: 32, 64 or 128, extremes found here), or 0: scales and
 // shifts come from the pass above.
 template <int BITS, int LPG, bool SYM>
@@ -358,19 +361,23 @@ wq_quant_pack_kernel(const __nv_bfloat16* __restrict__ w, const float* __restric
                      const float* __restrict__ shift32, uint8_t* __restrict__ q, __nv_bfloat16* __restrict__ scales,
                      __nv_bfloat16* __restrict__ zeros, int N, int K, int group) {
   constexpr int kPlanes = BITS == 4 ? 1 : 2;  // spans that have packed rows of their own
-  __shared__ uint32_t tile[kPlanes][128][32];  // [span][row][word of 4 outputs], words rotated by row / 8
+  // [span][row][word of 4 outputs], words rotated by row / 8; the second span half a bank row on
+  __shared__ uint32_t tile[kPlanes * (128 * 16 + 16)];
+  auto cell = [&](int pl, int row, int wd) -> uint32_t& {
+    return tile[pl * (128 * 16 + 16) + row * 16 + ((wd + (row >> 3)) & 15)];
+  };
   const QuantGrid g = quant_grid<BITS>(SYM);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int half = lane >> 4, l = lane & 15;
   const int rows = BITS == 4 ? K >> 1 : K;      // packed rows
   const int row0 = blockIdx.x * (BITS == 4 ? 128 : 256);  // spans first: neighbouring CTAs read on in the same rows
-  const int n0 = blockIdx.y * 128;
+  const int n0 = blockIdx.y * kQuantOuts;
   // this lane's 8 consecutive k
   const int k = (BITS == 4 ? half * rows + row0 : row0 + half * 128) + 8 * l;
   const bool k_ok = BITS == 4 ? row0 + 8 * l < rows : k < rows;
   const int gi = k_ok ? k / group : 0;
 #pragma unroll 1
-  for (int quad = warp; quad < 32; quad += 8) {
+  for (int quad = warp; quad < kQuantOuts / 4; quad += 8) {
     uint4 v[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -466,33 +473,31 @@ wq_quant_pack_kernel(const __nv_bfloat16* __restrict__ w, const float* __restric
         const uint32_t mine = half ? word[j + 1] : word[j];
         const uint32_t other = __shfl_xor_sync(0xffffffffu, half ? word[j] : word[j + 1], 16);
         const uint32_t packed = half ? (other | (mine << 4)) : (mine | (other << 4));
-        tile[0][8 * l + j + half][(quad + l + 16 * half) & 31] = packed;
+        cell(0, 8 * l + j + half, quad) = packed;
       }
     } else {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) tile[kPlanes - 1 ? half : 0][8 * l + j][(quad + l + 16 * half) & 31] = word[j];
+      for (int j = 0; j < 8; ++j) cell(kPlanes - 1 ? half : 0, 8 * l + j, quad) = word[j];
     }
   }
   __syncthreads();
   const bool words = N % 4 == 0 && (reinterpret_cast<uintptr_t>(q) & 3) == 0;
 #pragma unroll 4
-  for (int i = warp; i < kPlanes * 128; i += 8) {
-    const int r = i & 127, pl = i >> 7;
+  for (int i = 2 * warp + half; i < kPlanes * 128; i += 16) {  // a half warp per row
     const int row = row0 + i;
-    if (row >= rows) break;
-    const int rot = (r >> 3) + 16 * (BITS == 4 ? (r & 1) : pl);
-    const uint32_t v = tile[pl][r][(lane + rot) & 31];
-    const int n = n0 + 4 * lane;
+    const uint32_t v = cell(i >> 7, i & 127, l);
+    const int n = n0 + 4 * l;
     uint8_t* dst = q + static_cast<long long>(row) * N + n;
     if (words) {
-      if (n < N) *reinterpret_cast<uint32_t*>(dst) = v;
+      if (row < rows && n < N) *reinterpret_cast<uint32_t*>(dst) = v;
     } else {
       // rows that start on odd bytes: consecutive lanes store consecutive bytes
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
-        const int col = 32 * b + lane;
-        const uint32_t wv = __shfl_sync(0xffffffffu, v, 8 * b + (lane >> 2));
-        if (n0 + col < N) q[static_cast<long long>(row) * N + n0 + col] = static_cast<uint8_t>(wv >> (8 * (lane & 3)));
+        const int col = 16 * b + l;
+        const uint32_t wv = __shfl_sync(0xffffffffu, v, 4 * b + (l >> 2), 16);
+        if (row < rows && n0 + col < N)
+          q[static_cast<long long>(row) * N + n0 + col] = static_cast<uint8_t>(wv >> (8 * (l & 3)));
       }
     }
   }
@@ -507,7 +512,7 @@ static int launch_quantize(const void* weight, void* qweight, void* scales, void
   __nv_bfloat16* z = static_cast<__nv_bfloat16*>(zeros);
   const int rows = BITS == 4 ? K / 2 : K;
   const int span = BITS == 4 ? 128 : 256;
-  const dim3 grid((rows + span - 1) / span, (N + 127) / 128);
+  const dim3 grid((rows + span - 1) / span, (N + kQuantOuts - 1) / kQuantOuts);
   if (grid.y > 65535) return DXB_ERR_UNSUPPORTED;
   if (dxb_quantize_scratch_bytes(N, K, group, BITS) == 0) {
     auto kernel = group == 128 ? (symmetric ? wq_quant_pack_kernel<BITS, 16, true> : wq_quant_pack_kernel<BITS, 16, false>)
