@@ -156,6 +156,7 @@ struct WqParams {
   int group_shift;     // log2(group / 64) when that is a power of two, else -1
   int sz_step;         // scale rows a dequant team moves on per unit inside a tile, in 4 x bf16; -1: no
                        // constant (the group does not divide the teams' stride)
+  int split;           // CTA pairs per tile, each with a slice of its K units (kModeSplit; else 1)
   int cluster;         // CTAs per tile (thread-block cluster along x); 1 = no cluster
   int recv_off;        // cluster mode: byte offset of the receive buffers in shared memory
   int recv_alias;      // cluster mode: the receive buffers lie over the (then idle) rings, so
@@ -204,7 +205,9 @@ __device__ __forceinline__ uint2 finish_row4(float f0, float f1, float f2, float
 //   kModePair     whole tiles of 256 columns per CTA PAIR (cta_group::2): each CTA converts 128 columns and
 //                 loads half the tokens, one MMA multiplies both, so a converted weight serves up to
 //                 256 tokens and an activation is read once per 256 columns
-enum : int { kModeGeneral = 0, kModeWhole = 1, kModeCluster = 2, kModePair = 3 };
+//   kModeSplit    CTA pairs, several per tile: each takes a slice of K, the last one adds the sums (an instance
+//                 of its own: inside kModePair its code made those launches 2 % longer)
+enum : int { kModeGeneral = 0, kModeWhole = 1, kModeCluster = 2, kModePair = 3, kModeSplit = 4 };
 
 template <int BITS, bool HAS_ZERO, bool MULTI, bool RELAID, int MODE>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -246,7 +249,8 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   constexpr bool SYM4 = BITS == 4 && !HAS_ZERO;  // weights and sums are divided by kSymAcc, see sym4_low
   constexpr float ACC = SYM4 ? kSymAcc : 1.0f;
   constexpr bool kLean = MODE != kModeGeneral;
-  constexpr bool PAIR = MODE == kModePair;
+  constexpr bool ksplit = MODE == kModeSplit;
+  constexpr bool PAIR = MODE == kModePair || ksplit;
   constexpr bool WHOLE = MODE == kModeWhole || PAIR;
   const int NACC = PAIR ? p.nacc : 2;
   const int C = WHOLE ? 1 : p.cluster;  // kModeCluster is only launched with C > 1
@@ -257,17 +261,21 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   // of what is being cut (a cluster's units by its size, or the tiles by the grid), so part i
   // starts at i * q + min(i, r).  Only unit ranges that cut tiles still divide.
   const int crank = clustered || PAIR ? static_cast<int>(cluster_cta_rank()) : 0;
-  const int ctile = clustered ? static_cast<int>(cluster_id_x()) : 0;
-  const int part = clustered ? crank : PAIR ? static_cast<int>(cluster_id_x()) : static_cast<int>(blockIdx.x);
+  // Split pairs: the last slice's pairs, which wait for the others, are the last in the grid.
+  const int slice = ksplit ? static_cast<int>(cluster_id_x()) / p.tiles : 0;
+  const int ctile = clustered ? static_cast<int>(cluster_id_x())
+                    : ksplit ? static_cast<int>(cluster_id_x()) - slice * p.tiles : 0;
+  const int part = clustered ? crank : ksplit ? slice : PAIR ? static_cast<int>(cluster_id_x()) : static_cast<int>(blockIdx.x);
   const int cut_begin = part * p.range_q + (part < p.range_r ? part : p.range_r);
   const int cut_end = cut_begin + p.range_q + (part < p.range_r ? 1 : 0);
   const bool unit_ranges = MODE == kModeGeneral && !clustered && !tile_ranges;
-  const int u_begin = clustered ? ctile * U + cut_begin
+  const bool sliced = clustered || ksplit;  // a slice of one tile
+  const int u_begin = sliced ? ctile * U + cut_begin
                       : !unit_ranges ? cut_begin * U : static_cast<int>(range_begin(blockIdx.x, TU, G));
-  const int u_end = clustered ? ctile * U + cut_end
+  const int u_end = sliced ? ctile * U + cut_end
                     : !unit_ranges ? cut_end * U : static_cast<int>(range_begin(blockIdx.x + 1, TU, G));
-  const int tile_begin = clustered ? ctile : !unit_ranges ? cut_begin : u_begin / U;
-  const int ku_begin = clustered ? cut_begin : !unit_ranges ? 0 : u_begin - tile_begin * U;
+  const int tile_begin = sliced ? ctile : !unit_ranges ? cut_begin : u_begin / U;
+  const int ku_begin = sliced ? cut_begin : !unit_ranges ? 0 : u_begin - tile_begin * U;
   // This CTA's 128 columns of a tile.
   auto column_of = [&](int ntile) { return (PAIR ? 2 * ntile + crank : ntile) * kTileN; };
 
@@ -1028,7 +1036,65 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   tc_fence_before();
   __syncthreads();
   if (threadIdx.x == 0) DX_TRACE(7, 1);  // every role is through its loop
-  if (WHOLE && !abort_flag) {
+  if (ksplit && !abort_flag) {
+    // K split over pairs: all but the last slice park their fp32 sums in global scratch (each CTA its own
+    // 128 columns) and leave; the last slice's CTAs add them to their own in slice order.
+    const int slots = p.split - 1;
+    const int q = warp & 3, c = lane & 3, n_local = 32 * q + 4 * (lane >> 2);
+    const int tblock = ctile / p.tiles_n, ntile = ctile - tblock * p.tiles_n;
+    const int row0 = tblock * p.block;
+    const int m_rows = (p.M - row0) < p.block ? (p.M - row0) : p.block;
+    const int n = column_of(ntile) + n_local;
+    const long long slot_elems = static_cast<long long>(p.NU) * kTileN;
+    float* slot0 = p.partials + static_cast<long long>(2 * ctile + crank) * slots * slot_elems;
+    int* counter = p.counters + 2 * ctile + crank;
+    float bias4[4];
+    load_bias4(ctile, bias4);
+    pdl_wait();
+    tc_fence_after();
+    const bool last = slice == slots;
+    if (last) {
+      if (threadIdx.x == 0 && wait_flag_ge(counter, slots, abortp)) *counter = 0;  // ready for the next launch
+      __syncthreads();
+    }
+    const uint32_t d_tmem = tmem_addr(tmem0, 32 * q, 0);
+    for (int c0 = 16 * (warp >> 2); c0 < p.NU && !abort_flag; c0 += 16 * (kThreads / 128)) {
+      float4 v[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) v[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int sl = 0; last && sl < slots; ++sl) {
+        float4 t4[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const int m = c0 + 4 * r + c;
+          t4[r] = m < m_rows ? __ldcg(reinterpret_cast<const float4*>(slot0 + sl * slot_elems + m * kTileN + n_local))
+                             : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) { v[r].x += t4[r].x; v[r].y += t4[r].y; v[r].z += t4[r].z; v[r].w += t4[r].w; }
+      }
+      uint32_t ra[8], rb[8];
+      tmem_ld_16x128b_x4(d_tmem + c0, ra);
+      tmem_ld_16x128b_x4(d_tmem + (16u << 16) + c0, rb);
+      tc_wait_ld();
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int m = c0 + 4 * r + c;
+        if (m >= m_rows) continue;
+        const float f0 = __uint_as_float(ra[2 * r]) + v[r].x, f1 = __uint_as_float(ra[2 * r + 1]) + v[r].y;
+        const float f2 = __uint_as_float(rb[2 * r]) + v[r].z, f3 = __uint_as_float(rb[2 * r + 1]) + v[r].w;
+        if (!last)
+          __stcg(reinterpret_cast<float4*>(slot0 + slice * slot_elems + m * kTileN + n_local), make_float4(f0, f1, f2, f3));
+        else if (n < p.N)
+          *reinterpret_cast<uint2*>(p.out + static_cast<long long>(row0 + m) * p.ldo + n) =
+              finish_row4(ACC * f0, ACC * f1, ACC * f2, ACC * f3, bias4, p.bias != nullptr, p.epilogue);
+      }
+    }
+    tc_fence_before();
+    if (!last) __threadfence();
+    __syncthreads();  // every store of this CTA is out; before the accumulator's TMEM is given back
+    if (!last && threadIdx.x == 0) atomicAdd(counter, 1);
+  } else if (WHOLE && !abort_flag) {
     // The CTA's last tile: its accumulator is complete (the epilogue warps have waited for it) and
     // every other warp is idle, so all 24 finish it, six per TMEM lane quadrant with a 16-token chunk
     // each, instead of four walking six chunks.
@@ -1485,6 +1551,7 @@ static TcKernel pick_mode(int mode) {
     case kModeWhole: return wq_gemm_tc<BITS, HAS_ZERO, MULTI, RELAID, kModeWhole>;
     case kModeCluster: return wq_gemm_tc<BITS, HAS_ZERO, MULTI, RELAID, kModeCluster>;
     case kModePair: return wq_gemm_tc<BITS, HAS_ZERO, true, RELAID, kModePair>;
+    case kModeSplit: return wq_gemm_tc<BITS, HAS_ZERO, true, RELAID, kModeSplit>;
     default: return wq_gemm_tc<BITS, HAS_ZERO, MULTI, RELAID, kModeGeneral>;
   }
 }
@@ -1522,18 +1589,38 @@ static int resident_pairs(const void* kernel, int budget) {
   return it->second < budget / 2 ? it->second : budget / 2;
 }
 
-// Token blocks for CTA pairs, or 0 where the other plans are the better ones: the shortest of the
+// Scratch of a pair plan whose K is split: fp32 sums of all slices but one.
+static size_t pair_split_bytes(const Plan& pp, int split) {
+  return static_cast<size_t>(pp.tiles) * 2 * (split - 1) * pp.NU * kTileN * sizeof(float);
+}
+
+// What CTA pairs are to do: token blocks (0: the other plans are the better ones) and pairs per tile.
+constexpr int kMaxPairSplit = 8;
+struct PairChoice {
+  int blocks = 0, split = 1;
+};
+// The shortest of the
 // times below, all fitted to measurements on shapes between 160 x 3072 x 3072 and 913 x 13824 x 5120.
 // What they trade: a pair's unit takes as long as the MMA of its tokens (0.56 us at 256, 0.31 at
 // 128), converted once for all of them, but its accumulator of more than 128 tokens is not
 // double-buffered, so every further tile shows its epilogue; single CTAs convert a unit per 128
 // tokens (0.36 us int4, 0.42 int8); few tiles are split over clusters instead, at 7.5 us for the
 // exchange.  Which wins turns mostly on how full the last round of tiles is.
-static int choose_pair_blocks(const Plan& pl, int M, int N, int K, int bits, int pairs, int budget) {
+static PairChoice choose_pairs(const Plan& pl, int M, int N, int K, int bits, int pairs, int budget, bool may_split) {
   static const int forced = [] { const char* e = getenv("DEXTER_B200_PAIR"); return e ? atoi(e) : -1; }();
   const int least = (M + 255) / 256;  // a block has at most 256 tokens
-  if (pairs < 1) return 0;
-  if (forced >= 0) return forced == 0 ? 0 : forced < least ? least : forced;
+  PairChoice choice;
+  if (pairs < 1) return choice;
+  if (forced >= 0) {  // blocks + 1000 * split
+    choice.blocks = forced % 1000;
+    if (choice.blocks > 0 && choice.blocks < least) choice.blocks = least;
+    choice.split = may_split && forced >= 1000 ? forced / 1000 : 1;
+    if (choice.blocks > 0) {
+      const Plan pp = make_pair_plan(M, N, K, bits, pairs, choice.blocks);
+      if (choice.split > pp.units_per_tile || pp.tiles * choice.split > pairs) choice.split = 1;
+    }
+    return choice;
+  }
   const double U = pl.units_per_tile, unit = bits == 4 ? 0.36 : 0.42;
   double best;
   if (pl.recv_bytes > 0 && pl.tiles * 2 <= budget && pl.units_per_tile >= 2) {
@@ -1544,7 +1631,6 @@ static int choose_pair_blocks(const Plan& pl, int M, int N, int K, int bits, int
     const int rounds = (pl.tiles + budget - 1) / budget;
     best = 2.5 + rounds * (U * unit + (bits == 4 ? 0.7 : 1.2));
   }
-  int blocks = 0;
   for (int nb = least; nb <= least + 7; ++nb) {
     const Plan pp = make_pair_plan(M, N, K, bits, pairs, nb);
     const int rounds = (pp.tiles + pairs - 1) / pairs;
@@ -1552,9 +1638,15 @@ static int choose_pair_blocks(const Plan& pl, int M, int N, int K, int bits, int
     const double least_unit = bits == 4 ? 0.30 : 0.46;
     if (u < least_unit) u = least_unit;
     const double t = 1.15 * (4.2 + rounds * U * u + (rounds - 1) * (pp.nacc == 1 ? 0.006 * pp.NU : 0.5));
-    if (t < best) { best = t; blocks = nb; }
+    if (t < best) { best = t; choice.blocks = nb; choice.split = 1; }
+    // Few tiles: several pairs per tile, with a slice of K each.  Parking and adding the sums measured
+    // about 2.6 us per slice (512 tokens int8 14336 x 3072, 3 slices: 39.4 us, 48.8 without).
+    for (int s = 2; may_split && s <= kMaxPairSplit && pp.tiles * s <= pairs && s <= pp.units_per_tile / 4; ++s) {
+      const double ts = 1.15 * (4.2 + (U / s) * u + 0.8 + 2.6 * (s - 1));
+      if (ts < best) { best = ts; choice.blocks = nb; choice.split = s; }
+    }
   }
-  return blocks;
+  return choice;
 }
 
 template <int BITS, bool HAS_ZERO>
@@ -1583,7 +1675,7 @@ static int launch_tc(const void* x, long long ldx, const void* qw, const void* s
     };
     for (int multi = 0; multi < 2; ++multi)
       for (int relaid = 0; relaid < (BITS == 4 ? 2 : 1); ++relaid)
-        for (int mode = 0; mode < 4; ++mode) set(pick_kernel<BITS, HAS_ZERO>(multi, relaid, mode));
+        for (int mode = 0; mode < 5; ++mode) set(pick_kernel<BITS, HAS_ZERO>(multi, relaid, mode));
     if (!ok) return DXB_ERR_CUDA;
     attr_dev = dev;
   }
@@ -1597,21 +1689,32 @@ static int launch_tc(const void* x, long long ldx, const void* qw, const void* s
   // which all clusters are resident at once; the answer is cached per configuration.
   int cluster = 1;
   int pair_blocks = 0;  // > 0: CTA pairs, this many token blocks
+  int pair_split = 1;   // and this many pairs per tile
   const int budget = (max_ctas > 0 && max_ctas < di.sms) ? max_ctas : di.sms;
   if (multi && lean) {
     const int pairs = resident_pairs(reinterpret_cast<const void*>(pick_kernel<BITS, HAS_ZERO>(true, relaid, kModePair)), budget);
-    static thread_local std::unordered_map<size_t, int> chosen;
-    const size_t key = ((static_cast<size_t>(M) * 1000003u + static_cast<size_t>(N)) * 1000003u + static_cast<size_t>(K)) * 512u +
-                       static_cast<size_t>(budget);
-    auto it = chosen.find(key);
-    if (it == chosen.end()) {
-      if (chosen.size() > 4096) chosen.clear();
-      it = chosen.emplace(key, choose_pair_blocks(*plp, M, N, K, BITS, pairs, budget)).first;
+    static thread_local std::unordered_map<size_t, PairChoice> chosen;
+    const Plan base = *plp;
+    auto choose = [&](bool may_split) {
+      const size_t key = (((static_cast<size_t>(M) * 1000003u + static_cast<size_t>(N)) * 1000003u + static_cast<size_t>(K)) * 512u +
+                          static_cast<size_t>(budget)) * 2u + (may_split ? 1u : 0u);
+      auto it = chosen.find(key);
+      if (it == chosen.end()) {
+        if (chosen.size() > 4096) chosen.clear();
+        it = chosen.emplace(key, choose_pairs(base, M, N, K, BITS, pairs, budget, may_split)).first;
+      }
+      return it->second;
+    };
+    PairChoice choice = choose(true);
+    if (choice.split > 1) {  // only with room for the partial sums
+      const Plan pp = make_pair_plan(M, N, K, BITS, pairs, choice.blocks);
+      if (workspace_bytes < kStatusBytes + counters_bytes(0) + pair_split_bytes(pp, choice.split)) choice = choose(false);
     }
-    pair_blocks = it->second;
+    pair_blocks = choice.blocks;
+    pair_split = choice.split;
     if (pair_blocks > 0) {
       plan = make_pair_plan(M, N, K, BITS, pairs, pair_blocks);
-      kernel = pick_kernel<BITS, HAS_ZERO>(true, relaid, kModePair);
+      kernel = pick_kernel<BITS, HAS_ZERO>(true, relaid, pair_split > 1 ? kModeSplit : kModePair);
     }
   }
   if (pair_blocks == 0 && plp->recv_bytes > 0 && plp->tiles * 2 <= budget && plp->units_per_tile >= 2) {
@@ -1721,20 +1824,21 @@ static int launch_tc(const void* x, long long ldx, const void* qw, const void* s
   p.epilogue = opts.epilogue;
   p.tile_ranges = (cluster == 1 && pl.whole) ? 1 : 0;
   p.peer = opts.peer;
+  p.split = pair_blocks > 0 ? pair_split : 1;
   p.cluster = cluster;
   p.recv_off = pl.recv_off;
   p.recv_alias = cluster > 1 ? pl.recv_alias : 0;
   p.rows_per = ((M > 128 ? 128 : M) + cluster - 1) / cluster;  // token rows of one block per CTA
   {
-    const int what = cluster > 1 ? pl.units_per_tile : pl.tiles;
-    const int parts = cluster > 1 ? cluster : pl.ctas;
+    const int what = cluster > 1 || p.split > 1 ? pl.units_per_tile : pl.tiles;
+    const int parts = cluster > 1 ? cluster : p.split > 1 ? p.split : pl.ctas;
     p.range_q = what / parts;
     p.range_r = what % parts;
   }
   p.rows_inv = (65536 + p.rows_per - 1) / p.rows_per;
 
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(pair_blocks > 0 ? 2 * pl.ctas : cluster > 1 ? pl.tiles * cluster : pl.ctas);
+  cfg.gridDim = dim3(p.split > 1 ? 2 * pl.tiles * p.split : pair_blocks > 0 ? 2 * pl.ctas : cluster > 1 ? pl.tiles * cluster : pl.ctas);
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = pl.smem_bytes;
   cfg.stream = stream;
@@ -2142,7 +2246,16 @@ size_t dxb_workspace_bytes_ex(int M, int N, int K, int bits, int max_ctas) {
   if (block96 > one_block) one_block = block96;
   if (static_cast<long long>((N + kTileN - 1) / kTileN) * ((M + 127) / 128) > kMaxTiles)
     return one_block;
-  const size_t all_blocks = plan_workspace_bytes(M, N, K, bits, max_ctas);
+  size_t all_blocks = plan_workspace_bytes(M, N, K, bits, max_ctas);
+  // CTA pairs that split K park partial sums too; with less they do not split.
+  const int sms = device_info().sms > 0 ? device_info().sms : 148;
+  const int budget = (max_ctas > 0 && max_ctas < sms) ? max_ctas : sms;
+  const PairChoice choice = choose_pairs(make_plan(M, N, K, bits, sms, max_ctas), M, N, K, bits, budget / 2, budget, true);
+  if (choice.split > 1) {
+    const Plan pp = make_pair_plan(M, N, K, bits, budget / 2, choice.blocks);
+    const size_t split = kStatusBytes + counters_bytes(0) + pair_split_bytes(pp, choice.split);
+    if (split > all_blocks) all_blocks = split;
+  }
   return all_blocks > one_block ? all_blocks : one_block;
 }
 

@@ -23,6 +23,9 @@ def d(b200_lib):
     (913, 3072, 3072, 4, 128, True, "six blocks, one round"),
     (1000, 640, 10000, 4, 128, False, "many rounds with one accumulator, ragged last block and tile"),
     (2049, 256, 2048, 4, 128, True, "nine blocks"),
+    (512, 14336, 3072, 8, 14336, True, "three pairs per tile, a slice of K each"),
+    (400, 8192, 2064, 4, 128, False, "K split, last pair tile of 16 columns, ragged last block"),
+    (256, 14592, 2048, 8, 128, False, "K split unevenly"),
 ])
 def test_many_tokens(m, k, n, bits, group, symmetric, why, d, oracle):
     torch.manual_seed(m)
@@ -40,3 +43,35 @@ def test_many_tokens(m, k, n, bits, group, symmetric, why, d, oracle):
     ref = torch.nn.functional.gelu(want, approximate="tanh")
     assert (gelu.float() - ref).abs().max() / ref.abs().max() < TOL, why
     assert d.ops.last_status() == 0
+
+
+def test_split_pairs_replay_in_a_graph_and_run_without_room_for_the_sums(d, oracle, b200_lib):
+    import ctypes
+
+    torch.manual_seed(3)
+    m, k, n = 512, 14336, 3072
+    x = torch.randn(m, k, device="cuda").to(torch.bfloat16)
+    q = d.quantize((torch.randn(n, k, device="cuda") * 0.02).to(torch.bfloat16), bits=8, group_size=k, symmetric=True)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        want = d.w8a16(x, q.qweight, q.scales, None, None, k)
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            out = d.w8a16(x, q.qweight, q.scales, None, None, k)
+    for _ in range(3):  # the counters must reset themselves
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+    nbytes = b200_lib.dxb_workspace_bytes(128, n, k, 8)
+    ws = torch.zeros(nbytes, dtype=torch.uint8, device="cuda")
+    small = torch.empty_like(want)
+    rc = b200_lib.dxb_wq_gemm(8, ctypes.c_void_p(x.data_ptr()), k, ctypes.c_void_p(q.qweight.data_ptr()),
+                              ctypes.c_void_p(q.scales.data_ptr()), None, None, ctypes.c_void_p(small.data_ptr()), n, m, n, k, k,
+                              ctypes.c_void_p(ws.data_ptr()), nbytes, 0,
+                              ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    torch.cuda.synchronize()
+    assert (small.float() - want.float()).abs().max() / want.float().abs().max() < TOL
