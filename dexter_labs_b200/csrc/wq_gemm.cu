@@ -708,16 +708,16 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       const uint32_t plane16 = static_cast<uint32_t>(p.x_stage_bytes >> 1) >> 4;
       const uint32_t a_tmem0 = tmem0 + kACol0;
       int b = 0;
-      uint64_t xd = xdesc0;
-      uint32_t x_lo = static_cast<uint32_t>(xdesc0);  // its address half, where the stages are counted
+      const uint32_t x_lo0 = static_cast<uint32_t>(xdesc0), x_hi = static_cast<uint32_t>(xdesc0 >> 32);
+      uint32_t x_lo = x_lo0;  // the half that holds the address
       const uint32_t x_lo_end = x_lo + p.stages * x_stage16;
       uint32_t ph = 0, accph = 1, accumulate = 0;
       int left = u_end - u_begin;                        // units of this CTA still to do
       int seg = left < U - ku_begin ? left : U - ku_begin;  // of them in the current tile
       uint32_t d_tmem = tmem0;
-      auto mma = [](uint32_t d, uint32_t a, uint64_t b, uint32_t id, uint32_t acc) {
-        if (PAIR) mma_ts_pair(d, a, b, id, acc);
-        else mma_ts(d, a, b, id, acc);
+      auto mma = [x_hi](uint32_t d, uint32_t a, uint32_t b, uint32_t id, uint32_t acc) {
+        if (PAIR) mma_ts_pair(d, a, b, x_hi, id, acc);
+        else mma_ts(d, a, b, x_hi, id, acc);
       };
       auto commit = [](uint32_t bar) {
         if (PAIR) tc_commit_pair(bar);
@@ -732,20 +732,19 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                  (!PAIR || mbar_wait(bar0 + 8 * (kBarPeer + t), ph, abortp));
             if (ok) {
               tc_fence_after();
-              if (BITS == 4 || MULTI) xd = xdesc0 + t * x_stage16;
+              if (BITS == 4 || MULTI) x_lo = x_lo0 + t * x_stage16;
               const uint32_t a_tmem = a_tmem0 + t * A_STAGE_COLS;
-              mma(d_tmem, a_tmem, xd, idesc, accumulate);
+              mma(d_tmem, a_tmem, x_lo, idesc, accumulate);
 #pragma unroll
-              for (int kk = 1; kk < 4; ++kk) mma(d_tmem, a_tmem + kk * 8, xd + kk * 2, idesc, 1u);
+              for (int kk = 1; kk < 4; ++kk) mma(d_tmem, a_tmem + kk * 8, x_lo + kk * 2, idesc, 1u);
 #pragma unroll
               for (int kk = 0; kk < 4; ++kk)
-                mma(d_tmem, a_tmem + 32 + kk * 8, xd + plane16 + kk * 2, idesc, 1u);
+                mma(d_tmem, a_tmem + 32 + kk * 8, x_lo + plane16 + kk * 2, idesc, 1u);
               commit(bar0 + 8 * (kBarFree + t));
               accumulate = 1;
               if (BITS == 8 && !MULTI) {
                 x_lo += x_stage16;
-                if (x_lo == x_lo_end) x_lo = static_cast<uint32_t>(xdesc0);
-                xd = (xdesc0 & 0xFFFFFFFF00000000ull) | x_lo;
+                if (x_lo == x_lo_end) x_lo = x_lo0;
               }
               --left;
               if (--seg == 0) {
