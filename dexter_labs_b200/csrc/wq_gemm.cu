@@ -712,8 +712,9 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       uint32_t x_lo = x_lo0;  // the half that holds the address
       const uint32_t x_lo_end = x_lo + p.stages * x_stage16;
       uint32_t ph = 0, accph = 1, accumulate = 0;
-      int left = u_end - u_begin;                        // units of this CTA still to do
-      int seg = left < U - ku_begin ? left : U - ku_begin;  // of them in the current tile
+      int left = u_end - u_begin;                           // units of this CTA that are in no segment yet
+      int seg = left < U - ku_begin ? left : U - ku_begin;  // units still to do in the current tile
+      left -= seg;
       uint32_t d_tmem = tmem0;
       auto mma = [x_hi](uint32_t d, uint32_t a, uint32_t b, uint32_t id, uint32_t acc) {
         if (PAIR) mma_ts_pair(d, a, b, x_hi, id, acc);
@@ -723,11 +724,11 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         if (PAIR) tc_commit_pair(bar);
         else tc_commit(bar);
       };
-      bool ok = left > 0 && mbar_wait(bar0 + 8 * kBarAccEmpty, accph, abortp);
-      while (left > 0 && ok) {
+      bool ok = seg > 0 && mbar_wait(bar0 + 8 * kBarAccEmpty, accph, abortp);  // there is more to do
+      while (ok) {
 #pragma unroll
         for (int t = 0; t < kAStages; ++t) {
-          if (left > 0 && ok) {
+          if (ok) {
             ok = mbar_wait(bar0 + 8 * (kBarReady + t), ph, abortp) &&
                  (!PAIR || mbar_wait(bar0 + 8 * (kBarPeer + t), ph, abortp));
             if (ok) {
@@ -746,12 +747,13 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                 x_lo += x_stage16;
                 if (x_lo == x_lo_end) x_lo = x_lo0;
               }
-              --left;
               if (--seg == 0) {
                 commit(bar0 + 8 * (kBarAccFull + b));
                 if (++b == NACC) { b = 0; accph ^= 1u; }
-                if (left > 0) {
+                ok = left > 0;
+                if (ok) {
                   seg = left < U ? left : U;
+                  left -= seg;
                   accumulate = 0;
                   d_tmem = tmem0 + b * p.NU;
                   ok = mbar_wait(bar0 + 8 * (kBarAccEmpty + b), accph, abortp);
