@@ -1888,6 +1888,9 @@ static SmallKernel pick_small(int mt) {
                  : SmallKernel{wq_gemm_small<KIND, RAGGED, CPW, 2>, S2::kBytes * S2::kStages};
 }
 
+// Shared memory a CTA may have (227 KB).
+constexpr int kSmallSmem = 227 * 1024;
+
 // Lets the kernel use more than 48 KB of shared memory; once per kernel, device and thread.
 static bool small_smem_ready(void (*fn)(const SmallParams)) {
   int dev = 0;
@@ -1895,7 +1898,7 @@ static bool small_smem_ready(void (*fn)(const SmallParams)) {
   static thread_local std::unordered_map<size_t, bool> done;
   const size_t key = reinterpret_cast<size_t>(fn) * 64 + static_cast<size_t>(dev);
   if (done.find(key) != done.end()) return true;
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) return false;
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem) != cudaSuccess) return false;
   done[key] = true;
   return true;
 }
@@ -1921,14 +1924,13 @@ static int launch_small(int bits, const void* x, long long ldx, const void* qw, 
   const int blocks = (M + 8 * mt - 1) / (8 * mt);
   // Tiles of 32 columns.  Up to one per SM: sixteen warps each, and clusters that split K while SMs
   // are left over and every warp keeps at least two steps.  More: eight warps, two CTAs per SM.
-  // (All of this fixes the order of the sums, so it must not depend on the weight's layout.)
+  // (All of this fixes the order of the sums, so it must be the same for a weight and its repacked copy.)
   const long long tiles32 = static_cast<long long>((N + 31) / 32) * blocks;
   int warps = 8, cluster = 1;
   if (tiles32 <= budget) {
     warps = 16;
     while (cluster < 8 && tiles32 * cluster * 2 <= budget && p.steps >= 64 * cluster) cluster *= 2;
   }
-  p.cluster = cluster;
   {
     const int g32 = group / 32;
     p.group_shift = -1;
@@ -1953,16 +1955,21 @@ static int launch_small(int bits, const void* x, long long ldx, const void* qw, 
   p.tiles_n = (N + bn - 1) / bn;
   if (static_cast<long long>(p.tiles_n) * blocks > (1 << 30)) return DXB_ERR_SHAPE;
   p.tiles = p.tiles_n * blocks;
+  p.ring_bytes = warps * k.warp_bytes;
+  const int red_bytes = (warps * 8 * mt * (bn + 1) * 4 + 15) / 16 * 16;
+  if (p.ring_bytes < red_bytes) p.ring_bytes = red_bytes;
+  // A cluster's first CTA also has a receive slot for every other one.  Next to sixteen rings of ragged int4
+  // rows (222,208 B with more than 8 tokens) there is room for three of 2 KB, so clusters of four.
+  const int slot_bytes = 8 * mt * bn * 4;
+  while (cluster > 1 && p.ring_bytes + (cluster - 1) * slot_bytes > kSmallSmem) cluster /= 2;
+  p.cluster = cluster;
   // A caller's cap limits the CTAs, which then walk several tiles; without one every tile has its own.
   int grid = p.tiles;
   if (budget < sms && grid > budget * (16 / warps)) grid = budget * (16 / warps);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(grid) * cluster);
   cfg.blockDim = dim3(32 * warps);
-  p.ring_bytes = warps * k.warp_bytes;
-  const int red_bytes = (warps * 8 * mt * (bn + 1) * 4 + 15) / 16 * 16;
-  if (p.ring_bytes < red_bytes) p.ring_bytes = red_bytes;
-  cfg.dynamicSmemBytes = static_cast<size_t>(p.ring_bytes) + static_cast<size_t>(cluster - 1) * 8 * mt * bn * 4;
+  cfg.dynamicSmemBytes = static_cast<size_t>(p.ring_bytes) + static_cast<size_t>(cluster - 1) * slot_bytes;
   if (!small_smem_ready(k.fn)) return DXB_ERR_CUDA;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];

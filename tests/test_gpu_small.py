@@ -32,7 +32,13 @@ def err(got, want):
     (8, 3072, 9216, 4, 128, "288 tiles: eight warps"),
     (9, 3072, 14336, 4, 128, "448 tiles: twice the width, second token tile"),
     (16, 14336, 1536, 4, 128, "48 tiles, long K: clusters"),
-    (3, 14336, 96, 4, 128, "3 tiles: clusters of 8"),
+    (3, 14336, 96, 4, 128, "3 tiles, 224 steps of K: clusters of 4"),
+    (3, 16384, 96, 4, 128, "3 tiles, 256 steps: clusters of 8"),
+    (9, 16384, 192, 4, 128, "clusters of 8 beside the largest aligned rings"),
+    (16, 16384, 100, 4, 128, "clusters of 4: 8 do not fit beside the largest ragged rings"),
+    (64, 16384, 100, 4, 128, "the same with four token blocks"),
+    (9, 20480, 33, 4, 32, "the same, odd width"),
+    (16, 8192, 100, 8, 128, "clusters of 8, ragged int8"),
     (5, 1984, 264, 8, 32, "steps that do not divide by the warps"),
     (16, 3072, 14344, 8, 3072, "last wide tile cut, one group per channel"),
     (7, 6144, 100, 8, 128, "four columns past a tile, clusters"),
