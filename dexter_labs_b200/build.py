@@ -17,7 +17,7 @@ from pathlib import Path
 
 PKG_DIR = Path(__file__).resolve().parent
 SOURCES = [PKG_DIR / "csrc" / name for name in ("wq_gemm.cu", "wq_pack.cu", "peer_reduce.cu")]
-HEADERS = [*(PKG_DIR / "csrc" / name for name in ("sm100_ptx.cuh", "wq_common.cuh", "wq_small.cuh")),
+HEADERS = [*(PKG_DIR / "csrc" / name for name in ("sm100_ptx.cuh", "tile_counter.h", "wq_common.cuh", "wq_small.cuh")),
            PKG_DIR.parent / "include" / "dexter_b200.h"]
 LIB_PATH = PKG_DIR / "libdexter_b200.so"
 # compiled CPython binding of the hot call (csrc/fastcall.c); plain C, no CUDA

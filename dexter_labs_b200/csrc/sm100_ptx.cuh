@@ -7,6 +7,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "tile_counter.h"
+
 namespace dx {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -113,17 +115,22 @@ __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
   asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-// Bounded wait (one calling thread) until *p >= target.  Gives up after about a second
+// Bounded wait (one calling thread) until all sums of a tile are parked.  Gives up after about a second
 // or as soon as another role of the CTA has given up, setting the CTA's abort flag.
 constexpr uint32_t kFlagTries = 4000000u;
-__device__ __forceinline__ bool wait_flag_ge(const int* p, int target, volatile int* abort_flag) {
+__device__ __forceinline__ bool wait_tile_parked(const int* counter, int sharers, volatile int* abort_flag) {
   for (uint32_t tries = 0; tries < kFlagTries; ++tries) {
-    if (ld_acquire_gpu(p) >= target) return true;
+    if (tile_all_parked(static_cast<unsigned>(ld_acquire_gpu(counter)), sharers)) return true;
     if (*abort_flag) return false;
     __nanosleep(tries < 64 ? 32 : 256);
   }
   *abort_flag = 1;
   return false;
+}
+// One thread, after its CTA's sums are out (or once it has given up).
+__device__ __forceinline__ void tile_leave(int* counter, int sharers, bool parked) {
+  const unsigned before = atomicAdd(reinterpret_cast<unsigned*>(counter), tile_leave_add(parked));
+  if (tile_all_left(before, sharers)) *counter = 0;
 }
 
 // ------------------------------------------- programmatic dependent launch --

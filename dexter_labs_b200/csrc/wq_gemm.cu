@@ -227,6 +227,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   __shared__ __align__(8) uint64_t bars[kNumBars];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
+  __shared__ int left_tiles;  // unit ranges: 1 = left the shared tile it began in, 2 = the one it ended in
 #ifdef DXB_TRACE
   __shared__ long long t_start;
 #endif
@@ -319,6 +320,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     }
     if (lane == 0) {
       abort_flag = 0;
+      if (MODE == kModeGeneral) left_tiles = 0;
 #ifdef DXB_TRACE
       if (warp == 3) {
         t_start = t_entry;  // trace builds: every stamp counts from the thread's first instruction
@@ -529,13 +531,19 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         if (lane == 0 && wk == 0) mbar_arrive(bar0 + 8 * (kBarAccEmpty + b));
         __threadfence();
         named_bar_sync(1, nthr);
-        if (wtid == 0) atomicAdd(&p.counters[tile], 1);
+        if (wtid == 0) {
+          tile_leave(&p.counters[tile], c_last - c_first + 1, true);
+          left_tiles |= 1;
+        }
       } else {
         // finisher: wait (bounded) until every contributor has published
         const int ncontrib = c_last - c_first;
         if (wtid == 0) {
-          if (wait_flag_ge(&p.counters[tile], ncontrib, abortp))
+          if (wait_tile_parked(&p.counters[tile], ncontrib + 1, abortp))
             p.counters[tile] = 0;  // ready for the next launch / graph replay
+          else
+            tile_leave(&p.counters[tile], ncontrib + 1, false);
+          left_tiles |= 2;
         }
         named_bar_sync(1, nthr);
         if (*abortp) return false;
@@ -1035,9 +1043,14 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   }
 
   tc_fence_before();
-  __syncthreads();
+  const bool aborted = __syncthreads_or(abort_flag) != 0;  // one answer for all threads
   if (threadIdx.x == 0) DX_TRACE(7, 1);  // every role is through its loop
-  if (ksplit && !abort_flag) {
+  if (ksplit && aborted) {
+    if (threadIdx.x == 0) {
+      pdl_wait();
+      tile_leave(p.counters + 2 * ctile + crank, p.split, false);
+    }
+  } else if (ksplit) {
     // K split over pairs: all but the last slice park their fp32 sums in global scratch (each CTA its own
     // 128 columns) and leave; the last slice's CTAs add them to their own in slice order.
     const int slots = p.split - 1;
@@ -1055,7 +1068,10 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     tc_fence_after();
     const bool last = slice == slots;
     if (last) {
-      if (threadIdx.x == 0 && wait_flag_ge(counter, slots, abortp)) *counter = 0;  // ready for the next launch
+      if (threadIdx.x == 0) {
+        if (wait_tile_parked(counter, p.split, abortp)) *counter = 0;  // ready for the next launch
+        else tile_leave(counter, p.split, false);
+      }
       __syncthreads();
     }
     const uint32_t d_tmem = tmem_addr(tmem0, 32 * q, 0);
@@ -1094,8 +1110,8 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     tc_fence_before();
     if (!last) __threadfence();
     __syncthreads();  // every store of this CTA is out; before the accumulator's TMEM is given back
-    if (!last && threadIdx.x == 0) atomicAdd(counter, 1);
-  } else if (WHOLE && !abort_flag) {
+    if (!last && threadIdx.x == 0) tile_leave(counter, p.split, true);
+  } else if (WHOLE && !aborted) {
     // The CTA's last tile: its accumulator is complete (the epilogue warps have waited for it) and
     // every other warp is idle, so all 24 finish it, six per TMEM lane quadrant with a 16-token chunk
     // each, instead of four walking six chunks.
@@ -1231,6 +1247,17 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   }
   if (threadIdx.x == 0 && abort_flag) {
     pdl_wait();
+    if (unit_ranges && u_begin < u_end) {
+      // Shared tiles that this CTA has not got to: leave them, so that their counters end at zero.
+      const int t1 = (u_end - 1) / U;
+      auto leave = [&](int tile) {
+        const int sharers = owner_of(static_cast<long long>(tile) * U + U - 1, TU, G) -
+                            owner_of(static_cast<long long>(tile) * U, TU, G) + 1;
+        tile_leave(&p.counters[tile], sharers, false);
+      };
+      if (ku_begin > 0 && !(left_tiles & 1)) leave(tile_begin);
+      if (t1 * U >= u_begin && u_end < (t1 + 1) * U && !(left_tiles & 2)) leave(t1);
+    }
     atomicExch(p.status, DXB_ERR_KERNEL_TIMEOUT);
   }
 }

@@ -75,3 +75,36 @@ def test_split_pairs_replay_in_a_graph_and_run_without_room_for_the_sums(d, orac
     assert rc == 0
     torch.cuda.synchronize()
     assert (small.float() - want.float()).abs().max() / want.float().abs().max() < TOL
+
+
+@pytest.mark.parametrize("m,k,n,bits,max_ctas,counter,why", [
+    (512, 14336, 3072, 8, 0, 0, "K split over pairs"),
+    (83, 4096, 2688, 4, 20, 1, "unit ranges that cut tiles: CTA 0 holds tile 0 and the first units of tile 1"),
+])
+def test_a_wait_that_runs_out_leaves_the_counters_clean(m, k, n, bits, max_ctas, counter, why, d, b200_lib):
+    import ctypes
+
+    torch.manual_seed(5)
+    x = torch.randn(m, k, device="cuda").to(torch.bfloat16)
+    q = d.quantize((torch.randn(n, k, device="cuda") * 0.02).to(torch.bfloat16), bits=bits, group_size=128, symmetric=True)
+    nbytes = b200_lib.dxb_workspace_bytes_ex(m, n, k, bits, max_ctas)
+    ws = torch.zeros(nbytes, dtype=torch.uint8, device="cuda")
+    counters = ws[256:256 + 4 * 16384].view(torch.int32)
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def call():
+        y = torch.zeros(m, n, device="cuda", dtype=torch.bfloat16)
+        rc = b200_lib.dxb_wq_gemm(bits, ctypes.c_void_p(x.data_ptr()), k, ctypes.c_void_p(q.qweight.data_ptr()),
+                                  ctypes.c_void_p(q.scales.data_ptr()), None, None, ctypes.c_void_p(y.data_ptr()), n, m, n, k,
+                                  128, ctypes.c_void_p(ws.data_ptr()), nbytes, max_ctas, stream)
+        assert rc == 0
+        return y, b200_lib.dxb_read_status(ctypes.c_void_p(ws.data_ptr()), stream)
+
+    want, status = call()
+    assert status == 0 and not counters.any(), why
+    counters[counter] = 0x8000  # no number of parked sums reaches what the tile's finisher waits for
+    _, status = call()
+    assert status == -8 and not counters.any(), why
+    ws[:4] = 0
+    got, status = call()
+    assert status == 0 and torch.equal(got, want), why

@@ -292,3 +292,48 @@ def test_custom_op_is_declared_with_a_shape_function(b200_lib):
         assert y.shape == (2, 83, 512)
         with pytest.raises(Exception):
             torch.ops.dexter_b200.wq_gemm(x, q8, s, None, None, 128, 4)  # K = 6144 != 3072
+
+
+def test_tile_counter_ends_at_zero_whoever_gives_up(tmp_path):
+    """csrc/tile_counter.h in every order in which the CTAs of a shared tile can leave it: all but one park
+    or give up, the finisher (which needs all of them parked to finish) finishes or gives up."""
+    import subprocess
+
+    source = tmp_path / "orders.cpp"
+    source.write_text(r"""
+#include <algorithm>
+#include <cstdio>
+#include <vector>
+#include "tile_counter.h"
+int main() {
+  int seen = 0;
+  for (int n = 2; n <= 6; ++n)
+    for (int gives_up = 0; gives_up < 1 << n; ++gives_up) {  // bit n - 1: the finisher
+      std::vector<int> order(n);
+      for (int i = 0; i < n; ++i) order[i] = i;
+      do {
+        unsigned counter = 0;
+        auto leave = [&](bool parked) {
+          const unsigned before = counter;
+          counter += dx::tile_leave_add(parked);
+          if (dx::tile_all_left(before, n)) counter = 0;
+        };
+        bool possible = true;
+        for (int i : order) {
+          const bool up = gives_up >> i & 1;
+          if (i < n - 1) leave(!up);
+          else if (up) leave(false);
+          else if (dx::tile_all_parked(counter, n)) counter = 0;
+          else { possible = false; break; }  // it waits on
+        }
+        if (possible && counter) { std::printf("%d CTAs, %x: %x\n", n, gives_up, counter); return 1; }
+        seen += possible;
+      } while (std::next_permutation(order.begin(), order.end()));
+    }
+  std::printf("%d\n", seen);
+}
+""")
+    exe = tmp_path / "orders"
+    subprocess.run(["g++", "-std=c++17", "-I", str(ROOT / "dexter_labs_b200" / "csrc"), str(source), "-o", str(exe)], check=True)
+    out = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert out.returncode == 0 and int(out.stdout) > 1000, out.stdout
