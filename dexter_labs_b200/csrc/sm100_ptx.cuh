@@ -85,6 +85,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   *abort_flag = 1;
   return false;
 }
+// The same for all lanes of a warp, which get one answer: what follows a wait are warp-wide instructions
+// (tcgen05.ld / st, __syncwarp), and lanes that saw the abort flag while others saw the phase complete would
+// leave the rest of their warp waiting for them without a limit.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
 
 // --------------------------------------------------------------------- TMA --
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {

@@ -187,6 +187,18 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
+// The same barrier, telling every thread whether any of them says yes.
+__device__ __forceinline__ bool named_bar_any(int id, int nthreads, bool yes) {
+  uint32_t any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %3, 0;\n\tbar.red.or.pred q, %1, %2, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(any)
+      : "r"(id), "r"(nthreads), "r"(yes ? 1u : 0u)
+      : "memory");
+  return any != 0;
+}
 
 // First unit of CTA c and the CTA that owns unit u, for `total` units cut into
 // `ctas` contiguous ranges.
