@@ -255,11 +255,59 @@ __device__ __forceinline__ void mma_ts_pair(uint32_t d_tmem, uint32_t a_tmem, ui
       ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Arrive on the barrier at the same place in CTA `rank` of the cluster.  What it announces lies in TMEM or was
-// written by TMA and has been waited for, so no memory has to be made visible to the other CTA: a
-// release at cluster scope (and an acquire on the other side) cost about a thousand cycles per unit.
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t bar, uint32_t rank) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(dsmem_addr(bar, rank)) : "memory");
+// Across the pair, at cluster scope.  An arrival announces what its warp has read from or written to TMEM, which
+// tcgen05.wait and tcgen05.fence::before_thread_sync / after_thread_sync order around it, so it is relaxed: it
+// makes no shared or global memory visible.  (Activations do not pass through a thread: their copies complete
+// on the leader's barrier themselves, see tma_load_3d_pair.)  So are waits for a commit of the leader's; the
+// leader's own waits, which also stand for those copies, acquire.  (Arrivals that release as well: 913 x 13824 x
+// 5120 147 us instead of 98.)
+__device__ __forceinline__ void mbar_arrive_pair(uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+template <bool ACQUIRE>
+__device__ __forceinline__ bool mbar_try_wait_pair(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  if (ACQUIRE)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity), "r"(kWaitHintNs)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity), "r"(kWaitHintNs)
+        : "memory");
+  return ok != 0;
+}
+template <bool ACQUIRE>
+__device__ __forceinline__ bool mbar_wait_pair(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  for (uint32_t tries = 0; tries < kWaitTries; ++tries) {
+    if (mbar_try_wait_pair<ACQUIRE>(bar, parity)) return true;
+    if (*abort_flag) return false;
+  }
+  *abort_flag = 1;
+  return false;
+}
+// Loads into this CTA's shared memory that complete on a barrier of either CTA of the pair.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void* tmap, uint32_t cluster_bar, int x, int y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2"
+      " [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(cluster_bar), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const void* tmap, uint32_t cluster_bar, int x, int y, int z) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2"
+      " [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(cluster_bar), "r"(x), "r"(y), "r"(z)
+      : "memory");
 }
 
 // D[tmem] (+)= A[smem desc] * B[smem desc]; bf16 inputs, fp32 accumulate.

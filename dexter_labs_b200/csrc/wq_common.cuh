@@ -215,7 +215,7 @@ __host__ __device__ inline int owner_of(long long u, long long total, long long 
 // dequantised weights in TMEM (128 arrivals of one team); free[t]: the MMAs that
 // read slot t are done (one tcgen05.commit), so both may be overwritten.
 constexpr int kBarFullW = 0, kBarEmptyW = 16, kBarReady = 32, kBarFree = 36, kBarAccFull = 40,
-              kBarAccEmpty = 42, kBarPeer = 44, kNumBars = 48;
+              kBarAccEmpty = 42, kNumBars = 44;
 
 __device__ __forceinline__ uint32_t bar_count(int i) {
   if (i < kBarEmptyW) return 1;                    // full_w: producer's expect_tx
@@ -224,8 +224,7 @@ __device__ __forceinline__ uint32_t bar_count(int i) {
   if (i < kBarReady) return kTeamWarps;            // empty_w: the four warps of one team
   if (i < kBarFree) return kTeamWarps + 1;         // ready: team warps + activation producer
   if (i < kBarAccEmpty) return 1;                  // free, acc_full: one tcgen05.commit
-  if (i < kBarPeer) return kEpilogueThreads / 32;  // acc_empty: the four epilogue warps (CTA pairs: of both)
-  return 1;                                        // peer[t] (CTA pairs): the other CTA's slot t is ready
+  return kEpilogueThreads / 32;                    // acc_empty: the four epilogue warps
 }
 
 // ------------------------------------------------------------------ host side

@@ -314,9 +314,10 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       mbar_init(bar0 + 8 * (kBarEmptyW + wp + 2 * lane), bar_count(kBarEmptyW + wp + 2 * lane));
     } else if (warp == 3 && kBarReady + lane - 8 < kNumBars) {
       const int i = kBarReady + lane - 8;
-      // a pair's accumulators are drained by both CTAs' epilogue warps
-      const uint32_t twice = PAIR && i >= kBarAccEmpty && i < kBarPeer ? 2u : 1u;
-      mbar_init(bar0 + 8 * i, twice * bar_count(i));
+      // The leader of a pair issues for both: its slots are ready with both CTAs' conversions, its accumulators
+      // empty with both CTAs' epilogue warps.
+      const uint32_t more = !PAIR ? 0u : i < kBarFree ? kTeamWarps : i >= kBarAccEmpty ? bar_count(i) : 0u;
+      mbar_init(bar0 + 8 * i, bar_count(i) + more);
     }
     if (lane == 0) {
       abort_flag = 0;
@@ -354,6 +355,11 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   pdl_launch_dependents();
 
   volatile int* abortp = &abort_flag;
+  // One lane's wait for MMAs (slots that are free again, accumulators that are complete): a pair's come from
+  // the leader.
+  auto wait_mma = [abortp](uint32_t bar, uint32_t parity) {
+    return PAIR ? mbar_wait_pair<false>(bar, parity, abortp) : mbar_wait(bar, parity, abortp);
+  };
 
   // Cluster mode: send this CTA's fp32 partial rows from accumulator `d_tmem` (already
   // offset to the calling warp's lane quadrant) to their owners' receive buffers.
@@ -483,7 +489,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       tc_fence_before();
       __syncwarp();
       if (lane == 0 && nwk == 1) {
-        if (PAIR) mbar_arrive_remote(bar0 + 8 * (kBarAccEmpty + b), 0);  // the leader issues for both
+        if (PAIR) mbar_arrive_pair(dsmem_addr(bar0 + 8 * (kBarAccEmpty + b), 0));  // the leader issues for both
         else mbar_arrive(bar0 + 8 * (kBarAccEmpty + b));
       }
       if (fused && !fused_finish()) return false;
@@ -645,13 +651,21 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
 #pragma unroll
         for (int t = 0; t < kAStages; ++t) {
           if (u < u_end && ok) {
-            ok = three ? mbar_wait(bar0 + 8 * (kBarFree + (t + 1) % kAStages), t < 3 ? ph : ph ^ 1u, abortp)
-                       : mbar_wait(bar0 + 8 * (kBarFree + t), ph, abortp);
+            ok = three ? wait_mma(bar0 + 8 * (kBarFree + (t + 1) % kAStages), t < 3 ? ph : ph ^ 1u)
+                       : wait_mma(bar0 + 8 * (kBarFree + t), ph);
             if (ok) {
               const uint32_t rb = bar0 + 8 * (kBarReady + t);
               if (!kMayBeThree) dst = x_ring + t * p.x_stage_bytes;
-              mbar_expect_tx(rb, x_bytes);
-              if (BITS == 4) {
+              // A pair: both CTAs' halves complete on the leader's barrier (this slot's free barrier is
+              // the commit of the MMAs before, so the leader's is in this unit's phase).
+              if (!PAIR) mbar_expect_tx(rb, x_bytes);
+              else if (crank == 0) mbar_expect_tx(rb, 2 * x_bytes);
+              if (PAIR && BITS == 4) {
+                tma_load_3d_pair(dst, &tm_x, dsmem_addr(rb, 0), ku * 64, row0, 0);
+              } else if (PAIR) {
+                tma_load_2d_pair(dst, &tm_x, dsmem_addr(rb, 0), ku * 128, row0);
+                tma_load_2d_pair(dst + (x_bytes >> 1), &tm_x, dsmem_addr(rb, 0), ku * 128 + 64, row0);
+              } else if (BITS == 4) {
                 tma_load_3d(dst, &tm_x, rb, ku * 64, row0, 0);
               } else {  // two k-blocks of 64, one per plane
                 tma_load_2d(dst, &tm_x, rb, ku * 128, row0);
@@ -685,29 +699,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     // warps that keep it about 80 % busy, so each of its instructions waits for a turn: as a
     // warp-uniform loop with a slot counter a unit's 8 products and its wait took 840 cycles beside
     // them, twice what the tensor pipe needs for 96 tokens; in this form they take 460.
-    if (PAIR && crank == 1) {
-      // The other CTA issues the MMAs: tell it about every unit that is ready here.
-      if (elect_one()) {
-        uint32_t ph = 0;
-        int left = u_end - u_begin;
-        bool ok = true;
-        while (left > 0 && ok) {
-#pragma unroll
-          for (int t = 0; t < kAStages; ++t) {
-            if (left > 0 && ok) {
-              ok = mbar_wait(bar0 + 8 * (kBarReady + t), ph, abortp);
-              if (ok) {
-                tc_fence_after();
-                tc_fence_before();
-                mbar_arrive_remote(bar0 + 8 * (kBarPeer + t), 0);
-                --left;
-              }
-            }
-          }
-          ph ^= 1u;
-        }
-      }
-    } else if (elect_one()) {
+    if ((!PAIR || crank == 0) && elect_one()) {
       const uint32_t idesc = idesc_bf16_f32(PAIR ? 2 * kTileN : kTileN, p.NU);
       const uint64_t xdesc0 = smem_desc_kmajor_sw128(x_ring);
       const uint32_t x_stage16 = static_cast<uint32_t>(p.x_stage_bytes) >> 4;
@@ -730,13 +722,15 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         if (PAIR) tc_commit_pair(bar);
         else tc_commit(bar);
       };
-      bool ok = seg > 0 && mbar_wait(bar0 + 8 * kBarAccEmpty, accph, abortp);  // there is more to do
+      auto wait = [abortp](uint32_t bar, uint32_t parity) {
+        return PAIR ? mbar_wait_pair<true>(bar, parity, abortp) : mbar_wait(bar, parity, abortp);
+      };
+      bool ok = seg > 0 && wait(bar0 + 8 * kBarAccEmpty, accph);  // there is more to do
       while (ok) {
 #pragma unroll
         for (int t = 0; t < kAStages; ++t) {
           if (ok) {
-            ok = mbar_wait(bar0 + 8 * (kBarReady + t), ph, abortp) &&
-                 (!PAIR || mbar_wait(bar0 + 8 * (kBarPeer + t), ph, abortp));
+            ok = wait(bar0 + 8 * (kBarReady + t), ph);
             if (ok) {
               tc_fence_after();
               if (BITS == 4 || MULTI) x_lo = x_lo0 + t * x_stage16;
@@ -762,7 +756,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                   left -= seg;
                   accumulate = 0;
                   d_tmem = tmem0 + b * p.NU;
-                  ok = mbar_wait(bar0 + 8 * (kBarAccEmpty + b), accph, abortp);
+                  ok = wait(bar0 + 8 * (kBarAccEmpty + b), accph);
                 }
               }
             }
@@ -784,7 +778,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       const int nun = left < (U - ku0) ? left : (U - ku0);
       float bias4[4];
       load_bias4(tile, bias4);
-      bool ok = mbar_wait_warp(bar0 + 8 * (kBarAccFull + b), accph, abortp);
+      bool ok = __all_sync(0xffffffffu, wait_mma(bar0 + 8 * (kBarAccFull + b), accph));  // see mbar_wait_warp
       // Sums over ranks and shared tiles synchronise the four epilogue warps: they go on together or not at all.
       if (MODE == kModeGeneral) ok = !named_bar_any(1, kEpilogueThreads, !ok);
       if (!ok) break;
@@ -821,7 +815,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     const int group_units = p.group / 64;   // quantisation group in planes of 64 k
     const int half_units = p.half_k / 64;    // int4: planes between the low and the high nibbles
     const uint32_t a_tmem = tmem0 + kACol0 + team * A_STAGE_COLS;
-    const uint32_t a_full_bar = bar0 + 8 * (kBarReady + team);
+    const uint32_t a_full_bar = PAIR ? dsmem_addr(bar0 + 8 * (kBarReady + team), 0) : bar0 + 8 * (kBarReady + team);
     const uint32_t a_empty_bar = bar0 + 8 * (kBarFree + team);
 
     // What a unit costs here beyond its conversion counts: the sixteen warps keep the schedulers
@@ -927,7 +921,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         }
         load_sz();
       }
-      ok = mbar_wait(a_empty_bar, aph ^ 1u, abortp) && ok;
+      ok = wait_mma(a_empty_bar, aph ^ 1u) && ok;
       if (!__all_sync(0xffffffffu, ok)) break;
       tc_fence_after();
       if (large) {
@@ -1038,7 +1032,10 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       tc_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(a_full_bar);
+      if (lane == 0) {
+        if (PAIR) mbar_arrive_pair(a_full_bar);
+        else mbar_arrive(a_full_bar);
+      }
       aph ^= 1u;
       s += kAStages;
       if (s >= SW) { s -= SW; ph ^= 1u; }

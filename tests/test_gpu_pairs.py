@@ -108,3 +108,20 @@ def test_a_wait_that_runs_out_leaves_the_counters_clean(m, k, n, bits, max_ctas,
     ws[:4] = 0
     got, status = call()
     assert status == 0 and torch.equal(got, want), why
+
+
+@pytest.mark.parametrize("m,k,n,bits,why", [
+    (256, 2048, 14336, 4, "blocks of 256: every unit of both CTAs goes through the leader's barriers"),
+    (300, 2048, 9216, 8, "blocks of 160, two loads per unit and CTA"),
+    (512, 14336, 3072, 8, "K split"),
+])
+def test_pairs_give_the_same_bits_every_time(m, k, n, bits, why, d):
+    torch.manual_seed(m)
+    xs = [torch.randn(m, k, device="cuda").to(torch.bfloat16) for _ in range(2)]
+    q = d.quantize((torch.randn(n, k, device="cuda") * 0.02).to(torch.bfloat16), bits=bits, symmetric=True)
+    fn = d.w4a16 if bits == 4 else d.w8a16
+    want = [fn(x, q.qweight, q.scales, None, None, 128) for x in xs]
+    # other activations in between: a slot read before its half has arrived shows the previous launch's
+    wrong = sum((fn(xs[i % 2], q.qweight, q.scales, None, None, 128) != want[i % 2]).any().int() for i in range(100))
+    assert int(wrong) == 0, why
+    assert d.ops.last_status() == 0
