@@ -58,6 +58,9 @@ SIGNATURES = {
     "dxb_w8a16": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                           c_int64, c_int, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
     "dxb_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
+    "dxb_scratch_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int]),
+    "dxb_workspace_init": (c_int, [c_void_p, c_size_t, c_void_p, c_void_p]),
+    "dxb_capture_id": (ctypes.c_ulonglong, [c_void_p]),
     "dxb_dequantize": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                c_void_p]),
     "dxb_quantize_scratch_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
@@ -115,8 +118,8 @@ def load_call():
             from . import _dxb_call
         except ImportError:
             return None
-        entries = (lib.dxb_wq_gemm_ex, lib.dxb_workspace_bytes_ex, lib.dxb_quantize, lib.dxb_quantize_scratch_bytes,
-                   lib.dxb_dequantize_ex)
+        entries = (lib.dxb_wq_gemm_ex, lib.dxb_scratch_bytes, lib.dxb_capture_id, lib.dxb_quantize,
+                   lib.dxb_quantize_scratch_bytes, lib.dxb_dequantize_ex)
         _dxb_call.bind(*(ctypes.cast(fn, c_void_p).value for fn in entries), _relaid)
         _call_module = _dxb_call
     return _call_module

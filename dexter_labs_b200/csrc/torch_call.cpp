@@ -8,9 +8,10 @@
 // types, contiguous, on the current device, weight already repacked, workspace already there -- and
 // returns None for everything else, errors included, which ops.py then handles as before.
 //
-//   bind(gemm_ex, workspace_bytes_ex, quantize, quantize_scratch_bytes, dequantize_ex, relaid)
+//   bind(gemm_ex, scratch_bytes, capture_id, quantize, quantize_scratch_bytes, dequantize_ex, relaid)
 //                                              addresses in the loaded library, the cache of repacked weights
-//   set_workspace(device, stream, ptr, bytes)  what ops.py holds for that stream (0 bytes: nothing)
+//   set_workspace(device, stream, ptr, bytes, scratch, scratch_bytes)
+//                                              what ops.py holds for that stream (0 bytes: nothing)
 //   call(bits, x, qweight, scales, zeros, bias, group_size, max_ctas, layout, epilogue, pinned) -> Tensor | None
 //   quantize(weight, bits, group_size, symmetric) -> (qweight, scales, zeros | None) | None
 //   dequantize(qweight, scales, zeros, group_size, bits, layout) -> Tensor | None
@@ -30,13 +31,15 @@
 namespace {
 
 using GemmEx = decltype(&dxb_wq_gemm_ex);
-using WorkspaceBytes = decltype(&dxb_workspace_bytes_ex);
+using GemmScratch = decltype(&dxb_scratch_bytes);
+using CaptureId = decltype(&dxb_capture_id);
 using Quantize = decltype(&dxb_quantize);
 using ScratchBytes = decltype(&dxb_quantize_scratch_bytes);
 using Dequantize = decltype(&dxb_dequantize_ex);
 
 GemmEx g_gemm = nullptr;
-WorkspaceBytes g_workspace_bytes = nullptr;
+GemmScratch g_gemm_scratch = nullptr;
+CaptureId g_capture_id = nullptr;
 Quantize g_quantize = nullptr;
 ScratchBytes g_scratch_bytes = nullptr;
 Dequantize g_dequantize = nullptr;
@@ -48,19 +51,27 @@ struct Mix {
   }
 };
 // All state below is only touched with the interpreter lock held.
-std::unordered_map<std::pair<uint64_t, uint64_t>, std::pair<void*, size_t>, Mix> g_workspaces;  // (device, stream)
-std::unordered_map<std::pair<uint64_t, uint64_t>, size_t, Mix> g_need;                          // (shape words)
+struct Workspace {
+  void* ptr;  // for calls that leave counters and partial sums alone
+  size_t bytes;
+  void* scratch;  // for the others, outside captures
+  size_t scratch_bytes;
+};
+std::unordered_map<std::pair<uint64_t, uint64_t>, Workspace, Mix> g_workspaces;  // (device, stream)
+std::unordered_map<std::pair<uint64_t, uint64_t>, size_t, Mix> g_need;           // (shape words) -> dxb_scratch_bytes
 
 template <class F>
 F at_address(unsigned long long v) { return reinterpret_cast<F>(static_cast<uintptr_t>(v)); }
 
 PyObject* bind(PyObject*, PyObject* args) {
-  unsigned long long gemm = 0, bytes = 0, quantize = 0, scratch = 0, dequantize = 0;
+  unsigned long long gemm = 0, gemm_scratch = 0, capture_id = 0, quantize = 0, scratch = 0, dequantize = 0;
   PyObject* relaid = nullptr;
-  if (!PyArg_ParseTuple(args, "KKKKKO!", &gemm, &bytes, &quantize, &scratch, &dequantize, &PyDict_Type, &relaid))
+  if (!PyArg_ParseTuple(args, "KKKKKKO!", &gemm, &gemm_scratch, &capture_id, &quantize, &scratch, &dequantize, &PyDict_Type,
+                        &relaid))
     return nullptr;
   g_gemm = at_address<GemmEx>(gemm);
-  g_workspace_bytes = at_address<WorkspaceBytes>(bytes);
+  g_gemm_scratch = at_address<GemmScratch>(gemm_scratch);
+  g_capture_id = at_address<CaptureId>(capture_id);
   g_quantize = at_address<Quantize>(quantize);
   g_scratch_bytes = at_address<ScratchBytes>(scratch);
   g_dequantize = at_address<Dequantize>(dequantize);
@@ -71,10 +82,10 @@ PyObject* bind(PyObject*, PyObject* args) {
 
 PyObject* set_workspace(PyObject*, PyObject* args) {
   int device = 0;
-  unsigned long long stream = 0, ptr = 0, bytes = 0;
-  if (!PyArg_ParseTuple(args, "iKKK", &device, &stream, &ptr, &bytes)) return nullptr;
-  g_workspaces[{static_cast<uint64_t>(device), stream}] = {reinterpret_cast<void*>(static_cast<uintptr_t>(ptr)),
-                                                           static_cast<size_t>(bytes)};
+  unsigned long long stream = 0, ptr = 0, bytes = 0, scratch = 0, scratch_bytes = 0;
+  if (!PyArg_ParseTuple(args, "iKKKKK", &device, &stream, &ptr, &bytes, &scratch, &scratch_bytes)) return nullptr;
+  g_workspaces[{static_cast<uint64_t>(device), stream}] = {at_address<void*>(ptr), static_cast<size_t>(bytes),
+                                                           at_address<void*>(scratch), static_cast<size_t>(scratch_bytes)};
   Py_RETURN_NONE;
 }
 
@@ -164,10 +175,16 @@ PyObject* call(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   auto need = g_need.find(shape);
   if (need == g_need.end()) {
     if (g_need.size() > 4096) g_need.clear();
-    need = g_need.emplace(shape, g_workspace_bytes(static_cast<int>(m), static_cast<int>(n), static_cast<int>(k),
-                                                   static_cast<int>(bits), static_cast<int>(max_ctas))).first;
+    need = g_need.emplace(shape, g_gemm_scratch(static_cast<int>(m), static_cast<int>(n), static_cast<int>(k),
+                                                static_cast<int>(bits), static_cast<int>(max_ctas))).first;
   }
-  if (ws->second.second < need->second) Py_RETURN_NONE;
+  void* space = ws->second.ptr;
+  size_t space_bytes = ws->second.bytes;
+  if (need->second > 0) {  // a captured call gets scratch of its graph's own, from ops.py
+    if (ws->second.scratch_bytes < need->second || g_capture_id(stream) != 0) Py_RETURN_NONE;
+    space = ws->second.scratch;
+    space_bytes = ws->second.scratch_bytes;
+  }
 
   try {
     at::Tensor out;
@@ -181,7 +198,7 @@ PyObject* call(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     const int rc = g_gemm(static_cast<int>(bits), xp, ldx, q->const_data_ptr(), s->const_data_ptr(),
                           z ? z->const_data_ptr() : nullptr, b ? b->const_data_ptr() : nullptr, out.mutable_data_ptr(), n,
                           static_cast<int>(m), static_cast<int>(n), static_cast<int>(k), static_cast<int>(group),
-                          ws->second.first, ws->second.second, &opts, stream);
+                          space, space_bytes, &opts, stream);
     if (rc != DXB_OK) Py_RETURN_NONE;  // the general path reports it
     return THPVariable_Wrap(std::move(out));
   } catch (const std::exception&) {

@@ -287,7 +287,10 @@ inline bool tc_supported(int M, int N, int K, int group, int bits) {
   return true;
 }
 
+// Head of a workspace: the status word, and at this many ints from it the address of another status word that
+// a kernel sets as well, or 0.
 constexpr size_t kStatusBytes = 256;
+constexpr int kStatusAlso = 2;
 
 // Polls (of about a quarter of a microsecond) a wait on a flag written by ANOTHER GPU makes
 // before it gives up; set through dxb_set_wait_limit_ms, about a second by default.

@@ -1259,7 +1259,22 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       if (t1 * U >= u_begin && u_end < (t1 + 1) * U && !(left_tiles & 2)) leave(t1);
     }
     atomicExch(p.status, DXB_ERR_KERNEL_TIMEOUT);
+    int* also = *reinterpret_cast<int**>(p.status + kStatusAlso);  // see dxb_workspace_init
+    if (also != nullptr) atomicExch(also, DXB_ERR_KERNEL_TIMEOUT);
   }
+}
+
+// A workspace ready for its first call (see dxb_workspace_init).
+__global__ void wq_workspace_init_kernel(uint4* ws, int vecs, int* also) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= vecs) return;
+  uint4 v = make_uint4(0u, 0u, 0u, 0u);
+  if (i == 0) {  // status word, its padding, the other status word's address
+    const unsigned long long a = reinterpret_cast<unsigned long long>(also);
+    v.z = static_cast<uint32_t>(a);
+    v.w = static_cast<uint32_t>(a >> 32);
+  }
+  ws[i] = v;
 }
 
 // ------------------------------------------------ load-time weight re-layout
@@ -1505,24 +1520,24 @@ static Plan make_pair_plan(int M, int N, int K, int bits, int pairs, int blocks)
   return pl;
 }
 
+struct PlanKey {
+  int M, N, K, bits, sms, max_ctas, split;
+  bool operator==(const PlanKey& o) const {
+    return M == o.M && N == o.N && K == o.K && bits == o.bits && sms == o.sms && max_ctas == o.max_ctas &&
+           split == o.split;
+  }
+};
+struct PlanKeyHash {
+  size_t operator()(const PlanKey& k) const {
+    size_t h = 1469598103934665603ull;
+    for (int v : {k.M, k.N, k.K, k.bits, k.sms, k.max_ctas, k.split}) h = (h ^ static_cast<size_t>(v)) * 1099511628211ull;
+    return h;
+  }
+};
 // Plans only depend on the shape, so they are computed once per shape and thread.
 static Plan make_plan(int M, int N, int K, int bits, int sms, int max_ctas, bool allow_split = true) {
-  struct Key {
-    int M, N, K, bits, sms, max_ctas, split;
-    bool operator==(const Key& o) const {
-      return M == o.M && N == o.N && K == o.K && bits == o.bits && sms == o.sms && max_ctas == o.max_ctas &&
-             split == o.split;
-    }
-  };
-  struct Hash {
-    size_t operator()(const Key& k) const {
-      size_t h = 1469598103934665603ull;
-      for (int v : {k.M, k.N, k.K, k.bits, k.sms, k.max_ctas, k.split}) h = (h ^ static_cast<size_t>(v)) * 1099511628211ull;
-      return h;
-    }
-  };
-  static thread_local std::unordered_map<Key, Plan, Hash> cache;
-  const Key key{M, N, K, bits, sms, max_ctas, allow_split ? 1 : 0};
+  static thread_local std::unordered_map<PlanKey, Plan, PlanKeyHash> cache;
+  const PlanKey key{M, N, K, bits, sms, max_ctas, allow_split ? 1 : 0};
   auto it = cache.find(key);
   if (it != cache.end()) return it->second;
   if (cache.size() > 4096) cache.clear();
@@ -1677,6 +1692,31 @@ static PairChoice choose_pairs(const Plan& pl, int M, int N, int K, int bits, in
   return choice;
 }
 
+// Workspace that one launch of this problem wants because it shares tiles between CTAs (counters and partial
+// sums); 0 where it leaves all but the status word alone.  (Tiles split over clusters add through distributed
+// shared memory; where no cluster is resident, launch_tc hands out whole tiles.)
+static size_t launch_scratch_bytes(int M, int N, int K, int bits, int max_ctas) {
+  static thread_local std::unordered_map<PlanKey, size_t, PlanKeyHash> cache;
+  const PlanKey key{M, N, K, bits, 0, max_ctas, 0};
+  auto it = cache.find(key);
+  if (it != cache.end()) return it->second;
+  const int sms = device_info().sms > 0 ? device_info().sms : 148;
+  const int budget = (max_ctas > 0 && max_ctas < sms) ? max_ctas : sms;
+  const Plan pl = make_plan(M, N, K, bits, sms, max_ctas);
+  PairChoice choice;
+  if (M > 128) choice = choose_pairs(pl, M, N, K, bits, budget / 2, budget, true);
+  size_t need = 0;
+  if (choice.blocks > 0) {
+    if (choice.split > 1)
+      need = kStatusBytes + counters_bytes(0) +
+             pair_split_bytes(make_pair_plan(M, N, K, bits, budget / 2, choice.blocks), choice.split);
+  } else if (pl.recv_bytes == 0 && pl.max_slots > 1) {
+    need = plan_workspace_bytes(M, N, K, bits, max_ctas);
+  }
+  if (cache.size() > 4096) cache.clear();
+  return cache.emplace(key, need).first->second;
+}
+
 template <int BITS, bool HAS_ZERO>
 static int launch_tc(const void* x, long long ldx, const void* qw, const void* scales,
                      const void* zeros, const void* bias, void* out, long long ldo, int M, int N,
@@ -1780,6 +1820,7 @@ static int launch_tc(const void* x, long long ldx, const void* qw, const void* s
       }
       cache[key] = cluster;
     }
+    if (cluster == 1) plan = make_plan(M, N, K, BITS, di.sms, max_ctas, false);
   }
   if (cluster == 1 && pair_blocks == 0) {
     const size_t need = kStatusBytes + counters_bytes(plp->tiles) +
@@ -2128,11 +2169,10 @@ static int gemm_dispatch(int bits, const void* x, int64_t ldx, const void* qweig
     const int rc = launch_small(bits, x, ldx, qweight, scales, zeros, bias, out, ldo, M, N, K, group_size, opts, stream);
     if (rc != DXB_ERR_UNSUPPORTED) return rc;
   }
-  // More than 128 tokens: one launch over all token blocks when the workspace holds the
-  // partial sums of that plan (dxb_workspace_bytes asks for it); a smaller workspace still
-  // works, block by block.
+  // More than 128 tokens: one launch over all token blocks when the workspace holds the partial sums that it
+  // parks, if any; a smaller workspace still works, block by block.
   if (M > 128 && aligned && gemm_tc_supported(M, N, K, group_size, bits) &&
-      workspace_bytes >= plan_workspace_bytes(M, N, K, bits, max_ctas))
+      workspace_bytes >= launch_scratch_bytes(M, N, K, bits, max_ctas))
     return launch(static_cast<const char*>(x), static_cast<char*>(out), M);
   // Token blocks of at most 128 rows per launch (the UMMA N of one accumulator); 96 when the
   // weight has so few tiles that the launch splits them over clusters, whose receive buffers
@@ -2295,6 +2335,38 @@ size_t dxb_workspace_bytes_ex(int M, int N, int K, int bits, int max_ctas) {
 }
 
 size_t dxb_workspace_bytes(int M, int N, int K, int bits) { return dxb_workspace_bytes_ex(M, N, K, bits, 0); }
+
+size_t dxb_scratch_bytes(int M, int N, int K, int bits, int max_ctas) {
+  using namespace dx;
+  if (M <= 0 || N <= 0 || K <= 0 || (bits != 4 && bits != 8)) return 0;
+  if ((bits == 4 ? K / 2 : K) < (bits == 4 ? 64 : 128)) return 0;
+  const long long tiles = static_cast<long long>((N + kTileN - 1) / kTileN) * ((M + 127) / 128);
+  if (tiles <= kMaxTiles) return launch_scratch_bytes(M, N, K, bits, max_ctas);
+  const size_t a = launch_scratch_bytes(128, N, K, bits, max_ctas), b = launch_scratch_bytes(96, N, K, bits, max_ctas);
+  return a > b ? a : b;  // block by block
+}
+
+int dxb_workspace_init(void* workspace, size_t workspace_bytes, void* status, void* cuda_stream) {
+  using namespace dx;
+  const size_t bytes = kStatusBytes + counters_bytes(0);
+  if (!workspace) return DXB_ERR_NULL;
+  if (workspace_bytes < bytes) return DXB_ERR_WORKSPACE;
+  if (reinterpret_cast<uintptr_t>(workspace) % 16 || reinterpret_cast<uintptr_t>(status) % 4) return DXB_ERR_UNSUPPORTED;
+  const int vecs = static_cast<int>(bytes / 16);
+  wq_workspace_init_kernel<<<(vecs + 255) / 256, 256, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
+      static_cast<uint4*>(workspace), vecs, static_cast<int*>(status));
+  return cudaGetLastError() == cudaSuccess ? DXB_OK : DXB_ERR_CUDA;
+}
+
+unsigned long long dxb_capture_id(void* cuda_stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(static_cast<cudaStream_t>(cuda_stream), &status, &id) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return status == cudaStreamCaptureStatusNone ? 0 : id + 1;
+}
 
 int dxb_relayout_w4(const void* qweight, void* out, int K, int N, int inverse, void* cuda_stream) {
   using namespace dx;

@@ -13,6 +13,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
 import weakref
 from typing import Dict, Optional, Tuple
 
@@ -30,22 +31,64 @@ KERNEL_NAMES = {"w4a16": "b200_w4a16_tcgen05", "w8a16": "b200_w8a16_tcgen05"}
 
 _LIB = _lib.load()
 
-# One workspace per (device, stream): status word, tile counters and split-K
-# partial sums.  Zero-filled when created; the kernel leaves it clean.
-_workspaces: Dict[Tuple[int, int], torch.Tensor] = {}
+# Workspaces.  Most launches only need a status word; those that share tiles between CTAs also need counters
+# and partial sums (dxb_scratch_bytes), which no two launches that may overlap can have in common.  Per
+# (device, stream), in whose order the eager launches of that stream run:
+#   _blocks    status word (and counters that nobody uses), kept for good, since captured graphs have its address
+#   _scratch   for eager launches, replaced when a larger one comes
+#   _captured  (capture, scratch) for the launches of the capture that is under way: a graph may be replayed on any
+#              stream, beside other graphs and eager launches, for as long as it lives, so its scratch comes out
+#              of its own memory pool and is made ready by the graph itself
+# Scratch passes errors on to the status word of its stream's block, which `last_status` reads.
+_Space = Tuple[torch.Tensor, int, int]  # tensor, address, bytes
+_blocks: Dict[Tuple[int, int], _Space] = {}
+_scratch: Dict[Tuple[int, int], _Space] = {}
+_captured: Dict[Tuple[int, int], Tuple[int, _Space]] = {}
+_lock = threading.Lock()
+_BLOCK_BYTES = 256 + 4 * 16384
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
 
-def _workspace(device: torch.device, stream: int, nbytes: int) -> torch.Tensor:
-    key = (device.index if device.index is not None else torch.cuda.current_device(), stream)
-    ws = _workspaces.get(key)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _workspaces[key] = ws
-    return ws
+def _ready(device: int, stream: int, nbytes: int, status: Optional[int]) -> _Space:
+    """Scratch of at least ``nbytes``, made ready on ``stream`` (the current one)."""
+    t = torch.empty(nbytes, dtype=torch.uint8, device=torch.device("cuda", device))
+    rc = _LIB.dxb_workspace_init(t.data_ptr(), nbytes, status, ctypes.c_void_p(stream))
+    if rc != _lib.OK:
+        _raise(rc)
+    return t, t.data_ptr(), nbytes
+
+
+def _workspace(device: int, stream: int, need: int) -> _Space:
+    """Workspace (tensor, address, bytes) for a launch on ``stream`` (the current one of ``device``, the
+    current device) that needs ``need`` bytes of scratch.  The caller holds on to it until it has launched."""
+    key = (device, stream)
+    block = _blocks.get(key)
+    if block is not None and need == 0:
+        return block
+    capture = _LIB.dxb_capture_id(ctypes.c_void_p(stream))
+    with _lock:
+        block = _blocks.get(key)
+        if capture:
+            held = _captured.get(key)
+            if held is None or held[0] != capture or held[1][2] < need:
+                held = (capture, _ready(device, stream, max(need, _BLOCK_BYTES), None if block is None else block[1]))
+                _captured[key] = held
+            return held[1]
+        if block is None:
+            t = torch.zeros(_BLOCK_BYTES, dtype=torch.uint8, device=torch.device("cuda", device))
+            block = _blocks[key] = (t, t.data_ptr(), _BLOCK_BYTES)
+        _captured.pop(key, None)  # that capture is over: its graph keeps the memory
+        scratch = _scratch.get(key)
+        if need > 0 and (scratch is None or scratch[2] < need):
+            scratch = _ready(device, stream, max(need, 1 << 20), block[1])
+        if _NATIVE is not None:  # before the old scratch is given back
+            _NATIVE.set_workspace(device, stream, *block[1:], *((0, 0) if scratch is None else scratch[1:]))
+        if scratch is not None:
+            _scratch[key] = scratch
+        return block if need == 0 else scratch
 
 
 def _raise(code: int) -> None:
@@ -57,10 +100,8 @@ def _raise(code: int) -> None:
 
 _LAYOUTS = {"dexter": _lib.LAYOUT_DEXTER, "b200": _lib.LAYOUT_B200}
 _EPILOGUES = {None: _lib.EPILOGUE_NONE, "gelu_tanh": _lib.EPILOGUE_GELU_TANH}
-_need_cache: Dict[Tuple[int, int, int, int, int], int] = {}  # workspace bytes per problem
+_need_cache: Dict[Tuple[int, int, int, int, int], int] = {}  # scratch bytes per problem
 _opts_cache: Dict[tuple, "_lib.GemmOpts"] = {}  # option structs of calls without a fused sum
-# (device, stream) -> (workspace tensor, its address, its size): see _workspace
-_ws_fast: Dict[Tuple[int, int], Tuple[torch.Tensor, int, int]] = {}
 _GEMM = _LIB.dxb_wq_gemm_ex
 _FAST = None if os.environ.get("DEXTER_B200_FASTCALL", "1") == "0" else _lib.load_fast()
 _raw_stream = torch._C._cuda_getCurrentRawStream
@@ -123,16 +164,13 @@ def _run(bits: int, x: torch.Tensor, qweight: torch.Tensor, scales: torch.Tensor
             copied = relaid[1]
             qweight, layout = relaid[0], "b200"
     stream = _raw_stream(dev)
-    ws = _ws_fast.get((dev, stream))
     key = (m, n, k_dim, bits, max_ctas)
     need = _need_cache.get(key)
     if need is None:
-        need = _need_cache[key] = _LIB.dxb_workspace_bytes_ex(m, n, k_dim, bits, max_ctas)
-    if ws is None or ws[2] < need:
-        t = _workspace(x.device, stream, need)
-        ws = _ws_fast[(dev, stream)] = (t, t.data_ptr(), t.numel())
-        if _NATIVE is not None:
-            _NATIVE.set_workspace(dev, stream, ws[1], ws[2])
+        if len(_need_cache) > 4096:
+            _need_cache.clear()
+        need = _need_cache[key] = _LIB.dxb_scratch_bytes(m, n, k_dim, bits, max_ctas)
+    ws = _workspace(dev, stream, need)
     if reduce is None and _FAST is not None:
         # compiled binding: same entry point, arguments as plain integers (0 = NULL)
         rc = _FAST(bits, x2.data_ptr(), x2.stride(0), qweight.data_ptr(), scales.data_ptr(),
@@ -142,10 +180,7 @@ def _run(bits: int, x: torch.Tensor, qweight: torch.Tensor, scales: torch.Tensor
         if rc != 0:
             _raise(rc)
         if _CHECK:
-            code = _LIB.dxb_read_status(ws[1], ctypes.c_void_p(stream))
-            if code != _lib.OK:
-                ws[0].zero_()
-                _raise(code)
+            _check(dev, stream)
         return out if x.dim() == 2 else out.view(*x.shape[:-1], n)
     if reduce is None:
         okey = (layout, epilogue, max_ctas, copied)
@@ -162,14 +197,23 @@ def _run(bits: int, x: torch.Tensor, qweight: torch.Tensor, scales: torch.Tensor
     if rc != 0:
         _raise(rc)
     if _CHECK:
-        code = _LIB.dxb_read_status(ws[1], ctypes.c_void_p(stream))
-        if code != _lib.OK:
-            ws[0].zero_()
-            _raise(code)
+        _check(dev, stream)
     return out if x.dim() == 2 else out.view(*x.shape[:-1], n)
 
 
 _CHECK = bool(os.environ.get("DEXTER_B200_CHECK"))
+
+
+def _check(device: int, stream: int) -> None:
+    """``DEXTER_B200_CHECK``: raise what the launches on ``stream`` have left in its status word."""
+    block = _blocks.get((device, stream))
+    if block is None or _LIB.dxb_capture_id(ctypes.c_void_p(stream)):
+        return  # a captured launch has not run
+    code = _LIB.dxb_read_status(block[1], ctypes.c_void_p(stream))
+    if code != _lib.OK:
+        block[0].zero_()
+        _raise(code)
+
 
 # ------------------------------------------------------------ load-time re-layout (int4)
 # id(qweight) -> (weak reference to it, its version counter, the repacked copy or None)
@@ -234,14 +278,15 @@ def prepared_w4(qweight: torch.Tensor, m: int, n: int, k_dim: int,
 
 
 def last_status(device: Optional[torch.device] = None) -> int:
-    """Synchronise and return the kernel status word of the current stream's workspace."""
+    """Synchronise and return the kernel status word of the current stream: what its eager launches and the
+    graphs captured on it have left there."""
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else device
     with torch.cuda.device(device):
         stream = torch.cuda.current_stream().cuda_stream
-        ws = _workspaces.get((device.index, stream))
-        if ws is None:
-            return _lib.OK
-        return _LIB.dxb_read_status(ws.data_ptr(), ctypes.c_void_p(stream))
+        key = (device.index if device.index is not None else torch.cuda.current_device(), stream)
+        # (a stream on which nothing but captures has happened has no block: the last capture's word)
+        ws = _blocks[key][1] if key in _blocks else _captured[key][1][1] if key in _captured else None
+        return _lib.OK if ws is None else _LIB.dxb_read_status(ws, ctypes.c_void_p(stream))
 
 
 def accepts(*args) -> bool:

@@ -51,8 +51,9 @@ enum {
  * (python/dexter/ops/gfx1151/gemm/quantized.py:47-183, 223-249).
  * `workspace` holds a status word, tile counters and split-K partial sums; it
  * must be at least dxb_workspace_bytes() and zero-filled once before its first
- * use (the kernel leaves it clean after every normal completion).  Two calls
- * that may overlap on the GPU need different workspaces.
+ * use (the kernel leaves the counters at zero, also when a wait ran out).  Two calls
+ * that may overlap on the GPU need different workspaces; so do two captured graphs that may, and a
+ * graph's workspace has to live as long as the graph (see dxb_scratch_bytes).
  * `max_ctas` <= 0 lets the library use every SM; a positive value caps the grid, so
  * that several independent GEMMs can run side by side on different streams.
  * Any M: up to 128 tokens are one accumulator block; more tokens are processed as blocks of
@@ -199,12 +200,26 @@ int dxb_peer_allreduce(const void* partial, void* out, int64_t elems, void* cons
 /* Bytes of workspace dxb_wq_gemm needs for this problem on the current device.  For more
  * than 128 tokens this is what the one-launch plan over all token blocks needs; dxb_wq_gemm
  * also accepts the smaller amount a 128-token (and 96-token) problem asks for and then
- * launches block by block. */
+ * launches block by block where the one launch needs more (dxb_scratch_bytes). */
 size_t dxb_workspace_bytes(int M, int N, int K, int bits);
 /* The same for a call that caps the grid (`max_ctas` of dxb_wq_gemm); a cap can change how
  * tiles are split and with it the scratch needed.  dxb_wq_gemm also accepts the uncapped
  * amount: it then hands out whole tiles, which need no partial sums. */
 size_t dxb_workspace_bytes_ex(int M, int N, int K, int bits, int max_ctas);
+
+/* What of that the launch really shares between its CTAs (tile counters and partial sums): the number of bytes to
+ * pass, or 0 where a call leaves everything but the status word alone.  Calls for which this is 0 may share one
+ * workspace of 65,792 bytes (status word and counters), even where they overlap; a caller whose calls are captured
+ * in graphs gives the others a workspace per graph that may overlap with anything else. */
+size_t dxb_scratch_bytes(int M, int N, int K, int bits, int max_ctas);
+/*
+ * Makes a workspace ready for its first call (one small kernel on `cuda_stream`; the same as zero-filling its first
+ * 65,792 bytes).  `status` (may be NULL): an int that is set as well whenever a kernel leaves an error code in
+ * this workspace's status word; it has to live as long as the workspace is used.
+ */
+int dxb_workspace_init(void* workspace, size_t workspace_bytes, void* status, void* cuda_stream);
+/* Nonzero while `cuda_stream` is being captured: a number of its own for every capture. */
+unsigned long long dxb_capture_id(void* cuda_stream);
 
 /*
  * Dense [K, N] bf16 weight, computed with the same bit-pattern arithmetic as the

@@ -337,3 +337,17 @@ int main() {
     subprocess.run(["g++", "-std=c++17", "-I", str(ROOT / "dexter_labs_b200" / "csrc"), str(source), "-o", str(exe)], check=True)
     out = subprocess.run([str(exe)], capture_output=True, text=True)
     assert out.returncode == 0 and int(out.stdout) > 1000, out.stdout
+
+
+def test_scratch_is_only_asked_for_where_tiles_are_shared(b200_lib):
+    need = b200_lib.dxb_scratch_bytes
+    for m, n, k, nbits, cap in ((1, 3072, 3072, 4, 0), (83, 14336, 3072, 4, 0), (83, 3072, 14336, 8, 0), (83, 3072, 3072, 4, 29),
+                                (256, 14336, 3072, 4, 0), (913, 13824, 5120, 4, 0)):
+        assert need(m, n, k, nbits, cap) == 0
+    # K split over CTA pairs; unit ranges that cut tiles
+    for m, n, k, nbits, cap in ((512, 3072, 14336, 8, 0), (83, 2688, 4096, 4, 20)):
+        assert 256 + 65536 < need(m, n, k, nbits, cap) <= b200_lib.dxb_workspace_bytes_ex(m, n, k, nbits, cap)
+    assert need(0, 16, 64, 4, 0) == 0 and need(8, 16, 64, 5, 0) == 0
+    assert b200_lib.dxb_workspace_init(None, 1 << 20, None, None) == -2
+    assert b200_lib.dxb_workspace_init(ctypes.c_void_p(256), 256, None, None) == -5
+    assert b200_lib.dxb_capture_id(None) == 0
