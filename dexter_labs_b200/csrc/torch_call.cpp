@@ -112,7 +112,7 @@ bool repacked(PyObject* obj, const at::Tensor& q, const at::Tensor** copy) {
   return true;
 }
 
-PyObject* call(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+PyObject* call(PyObject* const* a, Py_ssize_t n_args) {
   if (n_args != 11) {
     PyErr_SetString(PyExc_TypeError, "_dxb_call.call takes exactly 11 arguments");
     return nullptr;
@@ -186,27 +186,23 @@ PyObject* call(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     space_bytes = ws->second.scratch_bytes;
   }
 
-  try {
-    at::Tensor out;
-    if (dims == 2) {
-      out = at::empty({m, n}, x->options());
-    } else {
-      auto sizes = x->sizes().vec();
-      sizes.back() = n;
-      out = at::empty(sizes, x->options());
-    }
-    const int rc = g_gemm(static_cast<int>(bits), xp, ldx, q->const_data_ptr(), s->const_data_ptr(),
-                          z ? z->const_data_ptr() : nullptr, b ? b->const_data_ptr() : nullptr, out.mutable_data_ptr(), n,
-                          static_cast<int>(m), static_cast<int>(n), static_cast<int>(k), static_cast<int>(group),
-                          space, space_bytes, &opts, stream);
-    if (rc != DXB_OK) Py_RETURN_NONE;  // the general path reports it
-    return THPVariable_Wrap(std::move(out));
-  } catch (const std::exception&) {
-    Py_RETURN_NONE;  // out of memory and the like: the general path raises it
+  at::Tensor out;
+  if (dims == 2) {
+    out = at::empty({m, n}, x->options());
+  } else {
+    auto sizes = x->sizes().vec();
+    sizes.back() = n;
+    out = at::empty(sizes, x->options());
   }
+  const int rc = g_gemm(static_cast<int>(bits), xp, ldx, q->const_data_ptr(), s->const_data_ptr(),
+                        z ? z->const_data_ptr() : nullptr, b ? b->const_data_ptr() : nullptr, out.mutable_data_ptr(), n,
+                        static_cast<int>(m), static_cast<int>(n), static_cast<int>(k), static_cast<int>(group),
+                        space, space_bytes, &opts, stream);
+  if (rc != DXB_OK) Py_RETURN_NONE;  // the general path reports it
+  return THPVariable_Wrap(std::move(out));
 }
 
-PyObject* quantize(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+PyObject* quantize(PyObject* const* a, Py_ssize_t n_args) {
   if (n_args != 4) {
     PyErr_SetString(PyExc_TypeError, "_dxb_call.quantize takes exactly 4 arguments");
     return nullptr;
@@ -220,27 +216,23 @@ PyObject* quantize(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     Py_RETURN_NONE;
   const int64_t n = w->size(0), k = w->size(1);
   if (n <= 0 || k <= 0 || group <= 0 || k % group || n > INT32_MAX || k > INT32_MAX) Py_RETURN_NONE;
-  try {
-    const auto bytes = w->options().dtype(at::kByte);
-    at::Tensor q = at::empty({bits == 4 ? k / 2 : k, n}, bytes), s = at::empty({k / group, n}, w->options()), z, scratch;
-    if (!symmetric) z = at::empty({k / group, n}, w->options());
-    const size_t need = g_scratch_bytes(static_cast<int>(n), static_cast<int>(k), static_cast<int>(group), static_cast<int>(bits));
-    if (need) scratch = at::empty({static_cast<int64_t>(need)}, bytes);
-    const auto stream = c10::cuda::getCurrentCUDAStream(w->device().index()).stream();
-    const int rc = g_quantize(w->const_data_ptr(), q.mutable_data_ptr(), s.mutable_data_ptr(),
-                              symmetric ? nullptr : z.mutable_data_ptr(), need ? scratch.mutable_data_ptr() : nullptr,
-                              static_cast<int>(n), static_cast<int>(k), static_cast<int>(group), static_cast<int>(bits),
-                              symmetric ? 1 : 0, stream);
-    if (rc != DXB_OK) Py_RETURN_NONE;  // shapes the kernel does not take
-    PyObject* zeros = Py_NewRef(Py_None);
-    if (!symmetric) Py_SETREF(zeros, THPVariable_Wrap(std::move(z)));
-    return Py_BuildValue("(NNN)", THPVariable_Wrap(std::move(q)), THPVariable_Wrap(std::move(s)), zeros);
-  } catch (const std::exception&) {
-    Py_RETURN_NONE;
-  }
+  const auto bytes = w->options().dtype(at::kByte);
+  at::Tensor q = at::empty({bits == 4 ? k / 2 : k, n}, bytes), s = at::empty({k / group, n}, w->options()), z, scratch;
+  if (!symmetric) z = at::empty({k / group, n}, w->options());
+  const size_t need = g_scratch_bytes(static_cast<int>(n), static_cast<int>(k), static_cast<int>(group), static_cast<int>(bits));
+  if (need) scratch = at::empty({static_cast<int64_t>(need)}, bytes);
+  const auto stream = c10::cuda::getCurrentCUDAStream(w->device().index()).stream();
+  const int rc = g_quantize(w->const_data_ptr(), q.mutable_data_ptr(), s.mutable_data_ptr(),
+                            symmetric ? nullptr : z.mutable_data_ptr(), need ? scratch.mutable_data_ptr() : nullptr,
+                            static_cast<int>(n), static_cast<int>(k), static_cast<int>(group), static_cast<int>(bits),
+                            symmetric ? 1 : 0, stream);
+  if (rc != DXB_OK) Py_RETURN_NONE;  // shapes the kernel does not take
+  PyObject* zeros = Py_NewRef(Py_None);
+  if (!symmetric) Py_SETREF(zeros, THPVariable_Wrap(std::move(z)));
+  return Py_BuildValue("(NNN)", THPVariable_Wrap(std::move(q)), THPVariable_Wrap(std::move(s)), zeros);
 }
 
-PyObject* dequantize(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+PyObject* dequantize(PyObject* const* a, Py_ssize_t n_args) {
   if (n_args != 6) {
     PyErr_SetString(PyExc_TypeError, "_dxb_call.dequantize takes exactly 6 arguments");
     return nullptr;
@@ -257,28 +249,36 @@ PyObject* dequantize(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   if (dev.index() != c10::cuda::current_device() || s->device() != dev || (z && z->device() != dev)) Py_RETURN_NONE;
   const int64_t n = q->size(1), k = q->size(0) * (bits == 4 ? 2 : 1);
   if (n <= 0 || k <= 0 || n > INT32_MAX || k > INT32_MAX || group > INT32_MAX) Py_RETURN_NONE;
+  at::Tensor out = at::empty({k, n}, s->options());
+  const auto stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+  const int rc = g_dequantize(q->const_data_ptr(), s->const_data_ptr(), z ? z->const_data_ptr() : nullptr,
+                              out.mutable_data_ptr(), static_cast<int>(n), static_cast<int>(k), static_cast<int>(group),
+                              static_cast<int>(bits), static_cast<int>(layout), stream);
+  if (rc != DXB_OK) Py_RETURN_NONE;  // the general path reports it
+  return THPVariable_Wrap(std::move(out));
+}
+
+// Any C++ exception sends the call down the general path, which raises what there is to raise: tensors
+// without storage or strides (vmap, sparse) throw from the plainest accessors, allocations when memory is short.
+template <PyObject* (*F)(PyObject* const*, Py_ssize_t)>
+PyObject* guarded(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   try {
-    at::Tensor out = at::empty({k, n}, s->options());
-    const auto stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
-    const int rc = g_dequantize(q->const_data_ptr(), s->const_data_ptr(), z ? z->const_data_ptr() : nullptr,
-                                out.mutable_data_ptr(), static_cast<int>(n), static_cast<int>(k), static_cast<int>(group),
-                                static_cast<int>(bits), static_cast<int>(layout), stream);
-    if (rc != DXB_OK) Py_RETURN_NONE;  // the general path reports it
-    return THPVariable_Wrap(std::move(out));
-  } catch (const std::exception&) {
+    return F(a, n_args);
+  } catch (...) {
+    PyErr_Clear();
     Py_RETURN_NONE;
   }
 }
-
-PyCFunction fastcall(PyObject* (*f)(PyObject*, PyObject* const*, Py_ssize_t)) {
-  return reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f));
+template <PyObject* (*F)(PyObject* const*, Py_ssize_t)>
+PyCFunction fastcall() {
+  return reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&guarded<F>));
 }
 PyMethodDef methods[] = {
     {"bind", bind, METH_VARARGS, "bind(addresses in the library..., relaid)"},
     {"set_workspace", set_workspace, METH_VARARGS, "set_workspace(device, stream, ptr, bytes)"},
-    {"call", fastcall(call), METH_FASTCALL, "one eager GEMM, or None where the general path has to take it"},
-    {"quantize", fastcall(quantize), METH_FASTCALL, "a weight packed, or None where the general path has to do it"},
-    {"dequantize", fastcall(dequantize), METH_FASTCALL, "the dense weight, or None where the general path has to make it"},
+    {"call", fastcall<call>(), METH_FASTCALL, "one eager GEMM, or None where the general path has to take it"},
+    {"quantize", fastcall<quantize>(), METH_FASTCALL, "a weight packed, or None where the general path has to do it"},
+    {"dequantize", fastcall<dequantize>(), METH_FASTCALL, "the dense weight, or None where the general path has to make it"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_dxb_call", "native eager call", -1, methods,
                           nullptr, nullptr, nullptr, nullptr};

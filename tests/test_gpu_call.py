@@ -79,3 +79,28 @@ def test_pin_and_platform_still_rule_the_call(d, monkeypatch):
         platform.override_platform(None)
     linear()
     assert registry.leading("gemm/w4a16") is d.ops._SPECS[4]
+
+
+def test_tensors_that_throw_reach_the_general_path(d):
+    # their accessors throw C++ exceptions, which must not leave the native entries
+    q = weight(d)
+    x = torch.randn(3, 6, 256, device="cuda").to(torch.bfloat16)
+    d.w4a16(x[0], q.qweight, q.scales, q.zeros, q.bias, 128)
+
+    def plain(t):
+        return d.w4a16(t, q.qweight, q.scales, q.zeros, q.bias, 128)
+
+    for bad in (lambda: torch.vmap(plain)(x), lambda: plain(x[0].to_sparse()),
+                lambda: torch.vmap(lambda s: d.dequantize(q.qweight, s, q.zeros, 128, 4))(q.scales.expand(2, -1, -1).contiguous()),
+                lambda: d.dequantize(q.qweight.to_sparse(), q.scales, q.zeros, 128, 4)):
+        with pytest.raises((RuntimeError, NotImplementedError)):
+            bad()
+    # quantize goes on with tensor expressions, which vmap can follow
+    w = (torch.randn(2, 48, 256, device="cuda") * 0.02).to(torch.bfloat16)
+    try:
+        codes = torch.vmap(lambda t: d.quantize(t, bits=8).qweight)(w)
+    except RuntimeError:
+        pass
+    else:
+        assert torch.equal(codes[1], d.quantize(w[1], bits=8).qweight)
+    assert torch.isfinite(plain(x[0]).float()).all()
