@@ -43,7 +43,8 @@ CaptureId g_capture_id = nullptr;
 Quantize g_quantize = nullptr;
 ScratchBytes g_scratch_bytes = nullptr;
 Dequantize g_dequantize = nullptr;
-PyObject* g_relaid = nullptr;  // id(qweight) -> (weak reference, version, repacked copy or None), owned by ops.py
+// id(qweight) -> (weak reference, version, repacked copy or None, address, streams that may read it, ...), owned by ops.py
+PyObject* g_relaid = nullptr;
 
 struct Mix {
   size_t operator()(const std::pair<uint64_t, uint64_t>& k) const {
@@ -94,19 +95,29 @@ const at::Tensor* plain_tensor(PyObject* o) {
   return THPVariable_CheckExact(o) ? &THPVariable_Unpack(o) : nullptr;
 }
 
-// Looks an int4 weight up in the cache of repacked copies: false when ops.py has not seen it yet (or
-// it has changed since); else `copy` is its repacked copy, or nullptr where its shape takes none.
-bool repacked(PyObject* obj, const at::Tensor& q, const at::Tensor** copy) {
+// Looks an int4 weight up in the cache of repacked copies: false when ops.py has not seen it yet, it has changed
+// since, or this stream has not waited for the copy; else `copy` is its repacked copy, or nullptr where its
+// shape takes none.
+bool repacked(PyObject* obj, const at::Tensor& q, cudaStream_t stream, const at::Tensor** copy) {
   *copy = nullptr;
   PyObject* key = PyLong_FromVoidPtr(obj);
   if (!key) { PyErr_Clear(); return false; }
   PyObject* hit = PyDict_GetItemWithError(g_relaid, key);  // borrowed
   Py_DECREF(key);
-  if (!hit || !PyTuple_CheckExact(hit) || PyTuple_GET_SIZE(hit) < 3) { PyErr_Clear(); return false; }
+  if (!hit || !PyTuple_CheckExact(hit) || PyTuple_GET_SIZE(hit) < 5) { PyErr_Clear(); return false; }
   if (PyWeakref_GetObject(PyTuple_GET_ITEM(hit, 0)) != obj) return false;
-  if (q.is_inference() || PyLong_AsUnsignedLong(PyTuple_GET_ITEM(hit, 1)) != q._version()) { PyErr_Clear(); return false; }
+  if (q.is_inference() || PyLong_AsUnsignedLong(PyTuple_GET_ITEM(hit, 1)) != q._version() ||
+      PyLong_AsVoidPtr(PyTuple_GET_ITEM(hit, 3)) != q.const_data_ptr()) {
+    PyErr_Clear();
+    return false;
+  }
   PyObject* item = PyTuple_GET_ITEM(hit, 2);
   if (item == Py_None) return true;
+  PyObject* raw = PyLong_FromVoidPtr(stream);
+  if (!raw) { PyErr_Clear(); return false; }
+  const int known = PySet_Contains(PyTuple_GET_ITEM(hit, 4), raw);
+  Py_DECREF(raw);
+  if (known != 1) { PyErr_Clear(); return false; }
   if (!THPVariable_CheckExact(item)) return false;
   *copy = &THPVariable_Unpack(item);
   return true;
@@ -157,16 +168,16 @@ PyObject* call(PyObject* const* a, Py_ssize_t n_args) {
   opts.weight_layout = static_cast<int>(layout);
   opts.epilogue = static_cast<int>(epilogue);
   opts.max_ctas = static_cast<int>(max_ctas);
+  const auto stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
   if (layout == DXB_LAYOUT_DEXTER && bits == 4) {
     const at::Tensor* copy;
-    if (!repacked(a[2], *q, &copy)) Py_RETURN_NONE;
+    if (!repacked(a[2], *q, stream, &copy)) Py_RETURN_NONE;
     if (copy) {
       q = copy;
       opts.weight_layout = DXB_LAYOUT_B200;
     }
   }
 
-  const auto stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
   const auto ws = g_workspaces.find({static_cast<uint64_t>(dev.index()), reinterpret_cast<uint64_t>(stream)});
   if (ws == g_workspaces.end()) Py_RETURN_NONE;
   const std::pair<uint64_t, uint64_t> shape{(static_cast<uint64_t>(m) << 32) | static_cast<uint64_t>(n),

@@ -2358,6 +2358,16 @@ int dxb_workspace_init(void* workspace, size_t workspace_bytes, void* status, vo
   return cudaGetLastError() == cudaSuccess ? DXB_OK : DXB_ERR_CUDA;
 }
 
+int dxb_event_done(void* cuda_event) {
+  // A query is refused while any stream is captured in the usual mode, unless its thread is in this one.
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) { cudaGetLastError(); return 0; }
+  const cudaError_t rc = cudaEventQuery(static_cast<cudaEvent_t>(cuda_event));
+  if (rc != cudaSuccess) cudaGetLastError();
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  return rc == cudaSuccess ? 1 : 0;
+}
+
 unsigned long long dxb_capture_id(void* cuda_stream) {
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   unsigned long long id = 0;

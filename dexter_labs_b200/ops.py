@@ -216,8 +216,10 @@ def _check(device: int, stream: int) -> None:
 
 
 # ------------------------------------------------------------ load-time re-layout (int4)
-# id(qweight) -> (weak reference to it, its version counter, the repacked copy or None)
-_relaid: Dict[int, Tuple[object, int, Optional[torch.Tensor]]] = _lib._relaid
+# id(qweight) -> (weak reference to it, its version counter, the repacked copy or None, its address, the raw streams
+# that may read the copy, an event after it was written: the stream's, recorded again after each of its repacks)
+_relaid: Dict[int, Tuple[object, int, Optional[torch.Tensor], int, set, Optional[torch.cuda.Event]]] = _lib._relaid
+_repacked: Dict[Tuple[int, int], Tuple[torch.cuda.Event, torch.cuda.Stream]] = {}  # (device, stream) -> that event
 _AUTO_RELAYOUT = os.environ.get("DEXTER_B200_RELAYOUT", "1") != "0"
 
 # The plain eager call in native code (csrc/torch_call.cpp).  It answers None whenever anything about
@@ -258,23 +260,52 @@ def prepared_w4(qweight: torch.Tensor, m: int, n: int, k_dim: int,
                 group_size: int) -> Optional[Tuple[torch.Tensor, bool]]:
     """The cached repacked copy of ``qweight`` for calls that come in with the reference
     layout (the registered kernels), as ``(copy, made_just_now)``, or None where the repack
-    does not apply: shapes the plain CUDA-core kernel serves, a stream that is being captured
-    before the copy exists, ``DEXTER_B200_RELAYOUT=0``.  The copy is made on the first call
-    with a given tensor object and dropped when that tensor is freed or modified in place."""
-    if not _AUTO_RELAYOUT:
+    does not apply: shapes the tcgen05 kernel does not take, a stream that is being captured
+    before the copy exists, a tensor without a version counter (made under inference mode),
+    ``DEXTER_B200_RELAYOUT=0``.  The copy is made on the first call with a given tensor object and
+    dropped when that tensor is freed; a tensor modified in place has it written again, at the same address (which
+    captured graphs may hold).  Writes that go around the version counter (through ``.data``, raw
+    pointers) are not seen."""
+    if not _AUTO_RELAYOUT or qweight.is_inference():
         return None
+    stream = _raw_stream(qweight.device.index)
     key = id(qweight)
     hit = _relaid.get(key)
-    if hit is not None and hit[0]() is qweight and hit[1] == qweight._version:
-        return None if hit[2] is None else (hit[2], False)
+    if hit is not None and hit[0]() is not qweight:
+        hit = None
+    if hit is not None and hit[1] == qweight._version and hit[3] == qweight.data_ptr():
+        copy = hit[2]
+        if copy is None:
+            return None
+        if stream not in hit[4]:
+            # written on another stream: this one waits for that, once, and holds the memory from now on
+            if not _LIB.dxb_capture_id(ctypes.c_void_p(stream)):
+                torch.cuda.current_stream().wait_event(hit[5])
+            elif not _LIB.dxb_event_done(ctypes.c_void_p(hit[5].cuda_event)):
+                return None  # a capture cannot wait for work outside of it
+            copy.record_stream(torch.cuda.current_stream())
+            hit[4].add(stream)
+        return copy, False
     takes_none = (qweight.shape[0] % 2 or n % 4 or qweight.data_ptr() % 16
                   or not _LIB.dxb_uses_tensor_cores(m, n, k_dim, group_size, 4))
     if not takes_none and torch.cuda.is_current_stream_capturing():
         return None
-    relaid = None if takes_none else relayout_w4(qweight)
+    copy = event = None
+    if not takes_none:
+        old = None if hit is None else hit[2]
+        if old is not None and (old.shape != qweight.shape or old.device != qweight.device):
+            old = None
+        if old is not None:
+            torch.cuda.current_stream().wait_event(hit[5])
+        copy = relayout_w4(qweight, out=old)
+        pair = _repacked.get((qweight.device.index, stream))
+        if pair is None:
+            pair = _repacked[(qweight.device.index, stream)] = (torch.cuda.Event(), torch.cuda.current_stream())
+        event = pair[0]
+        event.record(pair[1])
     _relaid[key] = (weakref.ref(qweight, lambda _r, key=key, table=_relaid: table.pop(key, None)),
-                    qweight._version, relaid)
-    return None if relaid is None else (relaid, True)
+                    qweight._version, copy, qweight.data_ptr(), {stream}, event)
+    return None if copy is None else (copy, True)
 
 
 def last_status(device: Optional[torch.device] = None) -> int:

@@ -220,6 +220,8 @@ size_t dxb_scratch_bytes(int M, int N, int K, int bits, int max_ctas);
 int dxb_workspace_init(void* workspace, size_t workspace_bytes, void* status, void* cuda_stream);
 /* Nonzero while `cuda_stream` is being captured: a number of its own for every capture. */
 unsigned long long dxb_capture_id(void* cuda_stream);
+/* 1 when a recorded cudaEvent_t has completed, 0 when not; may be called while a stream is being captured. */
+int dxb_event_done(void* cuda_event);
 
 /*
  * Dense [K, N] bf16 weight, computed with the same bit-pattern arithmetic as the

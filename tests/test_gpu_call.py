@@ -104,3 +104,70 @@ def test_tensors_that_throw_reach_the_general_path(d):
     else:
         assert torch.equal(codes[1], d.quantize(w[1], bits=8).qweight)
     assert torch.isfinite(plain(x[0]).float()).all()
+
+
+def expected(oracle, x, q):
+    return oracle.torch_wq_gemm(x, q.qweight, q.scales, q.zeros, q.bias, q.group_size, q.bits).float()
+
+
+def close(got, want):
+    return ((got.float() - want).abs().max() / want.abs().max()).item() < 1e-2
+
+
+def test_a_repacked_weight_is_waited_for_on_other_streams(d, oracle):
+    q = weight(d, n=2048, k=2048)
+    x = torch.randn(83, 2048, device="cuda").to(torch.bfloat16)
+    want = expected(oracle, x, q)
+    first, second, third = (torch.cuda.Stream() for _ in range(3))
+    torch.cuda.synchronize()
+    with torch.cuda.stream(second):
+        d.linear(x, weight(d, n=2048, k=2048).qweight, scales=q.scales, zeros=q.zeros)  # allocations, code
+    torch.cuda.synchronize()
+    junk = torch.full((1 << 21,), 0xFF, dtype=torch.uint8, device="cuda")  # what the copy's memory held
+    del junk
+
+    def linear():
+        return d.linear(x, q.qweight, q.bias, scales=q.scales, zeros=q.zeros, group_size=128, bits=4)
+
+    with torch.cuda.stream(first):
+        torch.cuda._sleep(40_000_000)  # about 20 ms: the repack is queued behind it
+        y1 = linear()
+    with torch.cuda.stream(second):
+        ys = [linear() for _ in range(2)]
+    torch.cuda.synchronize()
+    assert all(close(y, want) for y in (y1, *ys))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=third):  # a capture cannot wait for the copy, but sees that it is there
+        y3 = linear()
+    assert third.cuda_stream in d.ops._relaid[id(q.qweight)][4]
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y3, y1)
+    # written anew at the same address: the graph follows the weight
+    q.qweight.bitwise_xor_(0x11)
+    with torch.cuda.stream(first):
+        first.wait_stream(torch.cuda.current_stream())
+        y1 = linear()
+    torch.cuda.synchronize()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert close(y1, expected(oracle, x, q)) and torch.equal(y3, y1)
+
+
+def test_weights_made_under_inference_mode(d, oracle):
+    with torch.inference_mode():
+        q = weight(d)
+        x = torch.randn(83, 256, device="cuda").to(torch.bfloat16)
+        for _ in range(2):
+            y = d.linear(x, q.qweight, q.bias, scales=q.scales, zeros=q.zeros, group_size=128, bits=4)
+            assert close(y, expected(oracle, x, q))
+            q.qweight.bitwise_xor_(0x11)  # no version counter tells of this
+
+
+def test_a_weight_whose_storage_is_exchanged(d, oracle):
+    q, other = weight(d, n=160), weight(d, n=160, k=256)
+    x = torch.randn(83, 256, device="cuda").to(torch.bfloat16)
+    d.w4a16(x, q.qweight, q.scales, q.zeros, q.bias, 128)
+    q.qweight.data = other.qweight.bitwise_xor(0x11)
+    for _ in range(2):
+        assert close(d.w4a16(x, q.qweight, q.scales, q.zeros, q.bias, 128), expected(oracle, x, q))
