@@ -159,8 +159,11 @@ __device__ __forceinline__ uint32_t fetch_q4(const uint8_t* __restrict__ qw, int
 // between the FFN linears (torch gelu(approximate="tanh") on the bf16 output of the up
 // projection, python/dexter/models/dreamzero/model.py:279-285): evaluated in fp32, rounded once.
 // 0.5 (1 + tanh u) is the logistic function of 2u, which needs one exponential and one division and does
-// not cancel for negative u; the fast forms are good to a few 1e-7 relative, bf16 to 4e-3.  (tanhf with
-// its branches made the epilogue of 83 x 14336 outputs 7 us longer and its code evicted the main loop's.)
+// not cancel for negative u.  The fast forms' documented errors are 2 + 1.2 |2u| units of fp32 for the
+// exponential and 2 for the division: 5e-6 relative where the result reaches 2^-100, against 2e-3 for half a step
+// of bf16.  Over all bf16 inputs, 5 results (from -10.06 to -10.31, below 2^-122) are not the exact value's
+// rounding; 155 are with tanhf, which cancels below -3.5.  (tanhf with its branches also made the
+// epilogue of 83 x 14336 outputs 7 us longer and its code evicted the main loop's.)
 __device__ __forceinline__ float gelu_tanh(float v) {
   const float u2 = -1.5957691216057308f * (v + 0.044715f * v * v * v);
   return __fdividef(v, 1.0f + __expf(u2));

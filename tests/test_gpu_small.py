@@ -96,3 +96,24 @@ def test_symmetric_int4_over_the_whole_range_of_scales(m, k, n, relaid, d, oracl
     x = torch.zeros(m, k, device="cuda", dtype=torch.bfloat16)
     x[torch.arange(m, device="cuda"), rows] = 1
     assert torch.equal(d.w4a16(x, q, s, None, None, 64), want[rows])
+
+
+@pytest.mark.parametrize("m", [1, 200])  # few-token kernel, CTA pairs
+def test_gelu_of_every_bf16_value(m, d):
+    """A weight of zeros leaves the bias: the epilogue sees all bf16 values.  Bound: half a step of rounding plus the
+    fast exponential's error, 5e-6 relative where the result is 2^-100 or more, i.e. 0.0013 steps."""
+    n, k = 65536, 128
+    bias = torch.arange(n, dtype=torch.int32).to(torch.int16).view(torch.bfloat16).cuda()
+    q = torch.full((k, n), 128, dtype=torch.uint8, device="cuda")
+    s = torch.full((1, n), 0.01, device="cuda").to(torch.bfloat16)
+    y = d.ops.w8a16_gelu(torch.zeros(m, k, device="cuda", dtype=torch.bfloat16), q, s, None, bias, k)
+    v = bias.double()
+    exact = v * torch.sigmoid(2 * (2 / torch.pi) ** 0.5 * (v + 0.044715 * v ** 3))
+    usual = torch.isfinite(v) & (exact.abs() >= 2.0 ** -100)
+    step = torch.exp2(torch.floor(torch.log2(exact.abs())) - 7)
+    for row in (y[0], y[-1]):
+        assert ((row.double() - exact).abs() / step)[usual].max().item() < 0.502
+        tiny = torch.isfinite(v) & (exact.abs() < 2.0 ** -100)
+        assert (row.double()[tiny].abs() <= 2.0 ** -100).all()
+        # (the exact value at -inf is 0; the formula gives NaN in fp32 whatever its form)
+        assert torch.isnan(row[torch.isnan(v)]).all() and (row[v == float("inf")] == float("inf")).all()
