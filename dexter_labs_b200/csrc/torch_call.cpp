@@ -149,6 +149,8 @@ PyObject* call(PyObject* const* a, Py_ssize_t n_args) {
   if (!q->is_contiguous() || !s->is_contiguous() || (z && !z->is_contiguous()) || (b && !b->is_contiguous()))
     Py_RETURN_NONE;
   const int64_t n = q->size(1), k = bits == 4 ? 2 * q->size(0) : q->size(0);
+  const int64_t cells = group > 0 ? k / group * n : 0;
+  if (s->numel() < cells || (z && z->numel() < cells) || (b && b->numel() < n)) Py_RETURN_NONE;
   const int64_t dims = x->dim();
   if (dims < 1 || x->size(dims - 1) != k || k <= 0) Py_RETURN_NONE;
   int64_t m, ldx;
@@ -260,6 +262,8 @@ PyObject* dequantize(PyObject* const* a, Py_ssize_t n_args) {
   if (dev.index() != c10::cuda::current_device() || s->device() != dev || (z && z->device() != dev)) Py_RETURN_NONE;
   const int64_t n = q->size(1), k = q->size(0) * (bits == 4 ? 2 : 1);
   if (n <= 0 || k <= 0 || n > INT32_MAX || k > INT32_MAX || group > INT32_MAX) Py_RETURN_NONE;
+  const int64_t cells = group > 0 ? k / group * n : 0;
+  if (s->numel() < cells || (z && z->numel() < cells)) Py_RETURN_NONE;
   at::Tensor out = at::empty({k, n}, s->options());
   const auto stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
   const int rc = g_dequantize(q->const_data_ptr(), s->const_data_ptr(), z ? z->const_data_ptr() : nullptr,

@@ -108,6 +108,22 @@ _raw_stream = torch._C._cuda_getCurrentRawStream
 _current_device = torch.cuda.current_device
 
 
+def _check_operands(device: torch.device, k_dim: int, n: int, group_size: int, qweight: torch.Tensor, scales: torch.Tensor,
+                    zeros: Optional[torch.Tensor], bias: Optional[torch.Tensor] = None) -> None:
+    """What the kernels read without a look at its size: on this device, and as much of it as they read."""
+    groups = k_dim // group_size if group_size > 0 else 0  # (bad group sizes are the library's to report)
+    for name, t, need in (("qweight", qweight, 0), ("scales", scales, groups * n), ("zeros", zeros, groups * n),
+                          ("bias", bias, n)):
+        if t is None:
+            continue
+        if t.device != device:
+            raise RuntimeError(f"{name} is on {t.device}, expected {device}")
+        if need and t.dtype != torch.bfloat16:
+            raise RuntimeError(f"the B200 backend takes bf16 {name} only, got {t.dtype}")
+        if t.numel() < need:
+            raise ValueError(f"{name} has {t.numel()} values but K={k_dim}, N={n}, group size {group_size} take {need}")
+
+
 def _run(bits: int, x: torch.Tensor, qweight: torch.Tensor, scales: torch.Tensor,
          zeros: Optional[torch.Tensor], bias: Optional[torch.Tensor], group_size: int,
          max_ctas: int = 0, *, layout: str = "dexter", epilogue: Optional[str] = None,
@@ -128,6 +144,7 @@ def _run(bits: int, x: torch.Tensor, qweight: torch.Tensor, scales: torch.Tensor
     k_in = x.shape[-1]
     if k_in != k_dim:
         raise ValueError(f"x has K={k_in} but the packed weight has K={k_dim}")
+    _check_operands(x.device, k_dim, n, group_size, qweight, scales, zeros, bias)
     # A weight tensor that has to be copied here is written by the kernel right before the
     # GEMM on this stream, which the GEMM must then not overtake (it normally starts early
     # and reads its weights at once): such a call is launched in plain stream order.
@@ -487,6 +504,7 @@ def dequantize(qweight: torch.Tensor, scales: torch.Tensor, zeros: Optional[torc
         raise RuntimeError("the B200 backend needs CUDA tensors; there is no CPU path")
     k_dim = qweight.shape[0] * (2 if bits == 4 else 1)
     n = qweight.shape[1]
+    _check_operands(qweight.device, k_dim, n, group_size, qweight, scales, zeros)
     out = torch.empty((k_dim, n), device=qweight.device, dtype=torch.bfloat16)
     with torch.cuda.device(qweight.device):
         stream = torch.cuda.current_stream().cuda_stream

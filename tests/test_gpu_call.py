@@ -171,3 +171,32 @@ def test_a_weight_whose_storage_is_exchanged(d, oracle):
     q.qweight.data = other.qweight.bitwise_xor(0x11)
     for _ in range(2):
         assert close(d.w4a16(x, q.qweight, q.scales, q.zeros, q.bias, 128), expected(oracle, x, q))
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+def test_operands_that_are_elsewhere_or_too_small_raise(bits, d):
+    q = weight(d, bits=bits)
+    x = torch.randn(6, 256, device="cuda").to(torch.bfloat16)
+    fn = d.w4a16 if bits == 4 else d.w8a16
+    fn(x, q.qweight, q.scales, q.zeros, q.bias, 128)
+    for at in range(4):
+        ops = [q.qweight, q.scales, q.zeros, q.bias]
+        ops[at] = ops[at].cpu()
+        with pytest.raises(RuntimeError):
+            fn(x, *ops, 128)
+        if at < 3:
+            with pytest.raises(RuntimeError):
+                d.dequantize(*ops[:3], 128, bits)
+        if at == 0:
+            continue
+        ops = [q.qweight, q.scales, q.zeros, q.bias]
+        ops[at] = ops[at][..., :-1].contiguous()
+        with pytest.raises(ValueError):
+            fn(x, *ops, 128)
+        if at < 3:
+            with pytest.raises(ValueError):
+                d.dequantize(*ops[:3], 128, bits)
+    with pytest.raises(ValueError):
+        fn(x, q.qweight, q.scales, q.zeros, q.bias, 64)  # twice the groups that are there
+    with pytest.raises(RuntimeError):
+        fn(x, q.qweight, q.scales, q.zeros.float(), q.bias, 128)
