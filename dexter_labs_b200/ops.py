@@ -508,10 +508,10 @@ def dequantize(qweight: torch.Tensor, scales: torch.Tensor, zeros: Optional[torc
     out = torch.empty((k_dim, n), device=qweight.device, dtype=torch.bfloat16)
     with torch.cuda.device(qweight.device):
         stream = torch.cuda.current_stream().cuda_stream
-        rc = _LIB.dxb_dequantize_ex(qweight.contiguous().data_ptr(), scales.contiguous().data_ptr(),
-                                    None if zeros is None else zeros.contiguous().data_ptr(),
-                                    out.data_ptr(), n, k_dim, group_size, bits, _LAYOUTS[layout],
-                                    ctypes.c_void_p(stream))
+        # copies, where these are any, live until the launch
+        qweight, scales, zeros = (None if t is None else t.contiguous() for t in (qweight, scales, zeros))
+        rc = _LIB.dxb_dequantize_ex(qweight.data_ptr(), scales.data_ptr(), _ptr(zeros), out.data_ptr(), n, k_dim,
+                                    group_size, bits, _LAYOUTS[layout], ctypes.c_void_p(stream))
     if rc != _lib.OK:
         _raise(rc)
     return out

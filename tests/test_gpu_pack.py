@@ -74,3 +74,12 @@ def test_quantize_of_values_on_rounding_boundaries(bits, symmetric, d):
     got = d.quantize(w, bits=bits, symmetric=symmetric)
     want = d.quantize(w.clone().requires_grad_(), bits=bits, symmetric=symmetric)
     assert torch.equal(got.qweight, want.qweight) and torch.equal(got.scales, want.scales.detach())
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+def test_dequantize_of_strided_tensors(bits, d, oracle):
+    w = (torch.randn(96, 512, device="cuda") * 0.02).to(torch.bfloat16)
+    q = d.quantize(w, bits=bits)
+    turned = [t.t().contiguous().t() for t in (q.qweight, q.scales, q.zeros)]
+    want = oracle.torch_dequantize(q.qweight, q.scales, q.zeros, 128, bits)
+    assert torch.equal(d.dequantize(*turned, 128, bits), want)
