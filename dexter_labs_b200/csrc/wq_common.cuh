@@ -53,9 +53,9 @@ __device__ __forceinline__ uint32_t cvt_bf16x2(float hi, float lo) {
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
   return d;
 }
-// (w & mask) | bits in ONE instruction.  Written as a C expression, its two constants become immediates of two instructions (a three-input LOP3 takes one immediate only), which makes the
-// conversion, bound by the integer pipe, 20 % slower: 405 against 325 cycles per 128 x 128 int4 weights
-// with sixteen warps at it.
+// (w & mask) | bits in ONE instruction.  Written as a C expression, its two constants become immediates of two
+// instructions (a three-input LOP3 takes one immediate only), which makes the conversion, bound by the integer
+// pipe, 20 % slower: 405 against 325 cycles per 128 x 128 int4 weights with sixteen warps at it.
 __device__ __forceinline__ uint32_t and_or(uint32_t w, uint32_t mask, uint32_t bits) {
   uint32_t d;
   asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(w), "r"(mask), "r"(bits));
@@ -263,7 +263,6 @@ inline bool make_map(CUtensorMap* m, const void* base, CUtensorMapDataType dt, i
 
 struct DeviceInfo {
   int sms = 0;
-  bool attr_set = false;
 };
 inline DeviceInfo& device_info() {
   static std::mutex mu;
@@ -276,7 +275,8 @@ inline DeviceInfo& device_info() {
   return d;
 }
 
-// Shapes the tensor-core kernel takes.  Everything else goes to wq_gemm_simt.
+// Shapes whose tiles the tcgen05 kernel takes (int8 also wants whole units, see gemm_tc_supported).  The others go
+// to wq_gemm_small, or to wq_gemm_simt where that cannot take them either.
 inline bool tc_supported(int M, int N, int K, int group, int bits) {
   if (M < 1) return false;
   if (N % 16 || N < 16) return false;

@@ -195,8 +195,8 @@ __device__ __forceinline__ uint2 finish_row4(float f0, float f1, float f2, float
 // pair.  The single-block kernel carries none of that bookkeeping.
 // RELAID (int4 only): the packed bytes were rewritten by wq_relayout_w4_kernel so that one
 // 32-bit word holds the k-pairs the TMEM store wants (see there); saves the byte permutes.
-// MODE: the same pipeline compiled three times.  The two lean instances carry only what the
-// common launches execute, which keeps their code a third of the general instance's: these
+// MODE: the same pipeline compiled five times.  All but the general instance carry only what their
+// launches execute, which keeps their code a third of the general instance's: these
 // launches last 8-15 us, and a kernel whose code is larger than the instruction cache pays for
 // fetching it again in every launch (measured: 12.6 against 13.5 us on the headline shape).
 //   kModeGeneral  the sum over ranks, tiles shared between CTAs through global partial sums, clusters
@@ -1311,10 +1311,9 @@ __global__ void wq_relayout_w4_kernel(const uint32_t* __restrict__ in, uint32_t*
 }
 
 // ------------------------------------------------------ any-shape CUDA path
-// Plain CUDA-core kernel for shapes the tensor-core kernel does not take (N not
-// a multiple of 16, groups that are not a multiple of 64 rows, K/2 not a multiple
-// of 64).  One thread per output column, 8 tokens per block row; slow but exact
-// in the same sense (bit-identical W, fp32 accumulation).
+// Plain CUDA-core kernel for what neither wq_gemm_tc nor wq_gemm_small takes: groups or packed rows that are
+// no multiple of 32, weights and activations off the alignment of their loads.  One thread per output
+// column, 8 tokens per block row; slow but exact in the same sense (bit-identical W, fp32 accumulation).
 template <int BITS>
 __global__ void wq_gemm_simt(const __nv_bfloat16* __restrict__ x, long long ldx, const uint8_t* __restrict__ qw,
                              const __nv_bfloat16* __restrict__ scales, const __nv_bfloat16* __restrict__ zeros,
@@ -1391,13 +1390,10 @@ struct Plan {
 // Cost, in units, of finishing a tile that equal unit ranges cut between CTAs: the finisher
 // reads the other CTAs' fp32 partial tiles from L2 and adds them to its accumulator.
 static int fixup_units(int NU) {
-  static const int forced = [] {
-    const char* e = getenv("DEXTER_B200_FIXUP_UNITS");
-    return e ? atoi(e) : -1;
-  }();
-  if (forced >= 0) return forced;
-  // measured: 83 x 3072 x 14336 takes 19 us with 148 equal ranges against 14 us with one tile
-  // on each of 112 CTAs, i.e. finishing shared tiles costs about as much as 20 units
+  // Measured, us equal ranges / whole tiles, int4 with 83 tokens: 3072 x 14336 (112 tiles) 17.8 / 10.2, i.e. finishing
+  // shared tiles costs about as much as 20 units; 157 tiles, a second round for nine of them: 3072 x 20096 18.9 /
+  // 16.5 (the line lies a little early here), 8192 x 20096 32.2 / 40.5, 14336 x 20096 51.3 / 72.7; 128 tokens 3072 x
+  // 20096 21.9 / 19.7, 8192 x 20096 39.1 / 46.0.
   return NU > 96 ? 32 : 20;
 }
 
@@ -1650,20 +1646,9 @@ struct PairChoice {
 // tokens (0.36 us int4, 0.42 int8); few tiles are split over clusters instead, at 7.5 us for the
 // exchange.  Which wins turns mostly on how full the last round of tiles is.
 static PairChoice choose_pairs(const Plan& pl, int M, int N, int K, int bits, int pairs, int budget, bool may_split) {
-  static const int forced = [] { const char* e = getenv("DEXTER_B200_PAIR"); return e ? atoi(e) : -1; }();
   const int least = (M + 255) / 256;  // a block has at most 256 tokens
   PairChoice choice;
   if (pairs < 1) return choice;
-  if (forced >= 0) {  // blocks + 1000 * split
-    choice.blocks = forced % 1000;
-    if (choice.blocks > 0 && choice.blocks < least) choice.blocks = least;
-    choice.split = may_split && forced >= 1000 ? forced / 1000 : 1;
-    if (choice.blocks > 0) {
-      const Plan pp = make_pair_plan(M, N, K, bits, pairs, choice.blocks);
-      if (choice.split > pp.units_per_tile || pp.tiles * choice.split > pairs) choice.split = 1;
-    }
-    return choice;
-  }
   const double U = pl.units_per_tile, unit = bits == 4 ? 0.36 : 0.42;
   double best;
   if (pl.recv_bytes > 0 && pl.tiles * 2 <= budget && pl.units_per_tile >= 2) {
@@ -2129,13 +2114,17 @@ static int read_opts(const dxb_gemm_opts* o, int bits, int M, int N, int K, Opts
 
 // Few tokens and a weight that is read in little more than the fixed cost of a launch: there the kernel
 // without set-up is ahead; with more to convert (once per 16 tokens, there) the tcgen05 pipeline is.
-// The lines lie where the two crossed, us small / tcgen05: int4 1 token 3072 x 9216 6.9 / 7.8, 8 tokens 7.9 /
-// 7.9, 16 tokens 3072 x 3072 5.4 / 5.9, 32 tokens 2048 x 2048 4.5 / 4.9, 64 tokens 1024 x 1024 3.4 / 4.7; int8
-// 8 tokens 3072 x 3072 6.5 / 6.7, 16 tokens 2048 x 2048 5.1 / 5.1, 64 tokens 1024 x 1024 4.0 / 4.9, 128 tokens 5.6 /
-// 7.0 (from 97 tokens on the pipeline's split launches cost two more us).
+// The lines lie where the two crossed over 14 weights of 0.5 to 44 x 2^20 values and 18 token counts from 1 to 256 (both
+// kernels on all of them: profiles/few_token_line.md).  Near the lines, us small / tcgen05: int4 1 token 3072 x
+// 9216 6.4 / 7.2 and 3072 x 11264 8.3 / 8.3, 8 tokens 4096 x 4096 5.4 / 6.1 and 3072 x 6144 6.4 / 6.1, 16 tokens 3072 x
+// 3072 4.9 / 5.3 and 4096 x 4096 6.3 / 6.1, 32 tokens 2048 x 2048 4.2 / 4.6 and 2048 x 3072 5.7 / 5.1, 96 tokens
+// 1024 x 1024 3.9 / 5.1 and 1024 x 2048 6.0 / 5.4, 128 tokens 1024 x 2048 6.1 / 7.0 and 2048 x 2048 8.9 / 7.5 (from 97
+// tokens on the pipeline's clusters have their receive buffers over the rings, two more us), 160 tokens 512 x 1024
+// 4.6 / 4.5; int8 8 tokens 3072 x 3072 6.1 / 6.4 and 4096 x 4096 7.9 / 7.8, 16 tokens 2048 x 2048 4.9 / 5.0 and 3072 x
+// 3072 6.9 / 6.4, 80 tokens 1024 x 1024 5.0 / 4.9, 128 tokens 5.4 / 6.8 and 1024 x 2048 8.1 / 7.4.  The choice is
+// within 4 % of the better kernel at 733 of the 756 points and 14 % off at worst (up to 4 tokens 5120 x 5120: 160
+// tiles, so CTAs of eight warps, of which a second one fits an SM but most SMs get one).
 static bool small_is_faster(int M, int N, int K, int bits) {
-  static const int forced = [] { const char* e = getenv("DEXTER_B200_SMALL_TOKENS"); return e ? atoi(e) : -1; }();
-  if (forced >= 0) return M <= forced;
   const long long weights = static_cast<long long>(N) * K, mega = 1 << 20;
   if (M <= 8) return weights <= (bits == 8 ? 10 : M <= 4 ? 30 : 16) * mega;
   const long long converted = weights * ((M + 15) / 16);

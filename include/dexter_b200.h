@@ -56,8 +56,8 @@ enum {
  * graph's workspace has to live as long as the graph (see dxb_scratch_bytes).
  * `max_ctas` <= 0 lets the library use every SM; a positive value caps the grid, so
  * that several independent GEMMs can run side by side on different streams.
- * Any M: up to 128 tokens are one accumulator block; more tokens are processed as blocks of
- * 128 inside ONE launch (every (token block, 128-column tile) pair is a tile of the grid).
+ * Any M: up to 128 tokens are one accumulator block; more tokens are processed as blocks of up to
+ * 256 inside ONE launch (every (token block, column tile) pair is a tile of the grid).
  * Launch order: the kernel is launched with programmatic stream serialisation, so it may
  * begin while the kernel before it on `cuda_stream` is still running.  It waits for that
  * kernel before it reads `x` or writes `out` / `workspace`, but it reads `qweight`, `scales`,
@@ -247,9 +247,10 @@ size_t dxb_quantize_scratch_bytes(int N, int K, int group_size, int bits);
 int dxb_quantize(const void* weight, void* qweight, void* scales, void* zeros, void* scratch, int N, int K,
                  int group_size, int bits, int symmetric, void* cuda_stream);
 
-/* 1 when dxb_wq_gemm runs this shape on the tcgen05 kernel, 0 when it takes the
- * plain CUDA-core kernel (the counterpart of the reference's `accepts` shape
- * predicate, python/dexter/registry.py:58-60). */
+/* 1 when the tcgen05 kernel takes this shape (with few tokens on a small weight the few-token kernel may still be
+ * chosen, being faster there), 0 when the few-token kernel or, off its steps and alignments too, the plain
+ * CUDA-core kernel serves it (the counterpart of the reference's `accepts` shape predicate,
+ * python/dexter/registry.py:58-60). */
 int dxb_uses_tensor_cores(int M, int N, int K, int group_size, int bits);
 
 /* Synchronises `cuda_stream` and returns the status word of `workspace`:

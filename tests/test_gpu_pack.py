@@ -13,7 +13,7 @@ def d(b200_lib):
     return dexter_labs_b200
 
 
-# (K, N, bits, group): whole spans, spans cut at the end, output widths around the tile of 128 and
+# (K, N, bits, group): whole spans, spans cut at the end, output widths around the tile of 64 and
 # off every alignment, one scale per channel, groups that no span covers
 SHAPES = [(256, 128, 4, 128), (512, 131, 4, 128), (384, 40, 4, 64), (192, 9, 4, 32), (640, 1, 4, 160),
           (3072, 260, 4, 3072), (256, 1000, 8, 128), (384, 127, 8, 64), (96, 33, 8, 32), (1040, 200, 8, 1040),
