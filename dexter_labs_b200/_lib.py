@@ -60,6 +60,7 @@ SIGNATURES = {
     "dxb_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
     "dxb_scratch_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int]),
     "dxb_workspace_init": (c_int, [c_void_p, c_size_t, c_void_p, c_void_p]),
+    "dxb_shared_workspace": (c_int, [ctypes.POINTER(c_void_p)]),
     "dxb_event_done": (c_int, [c_void_p]),
     "dxb_capture_id": (ctypes.c_ulonglong, [c_void_p]),
     "dxb_dequantize": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,

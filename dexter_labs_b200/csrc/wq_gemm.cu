@@ -2229,25 +2229,34 @@ int dxb_wq_gemm(int bits, const void* x, int64_t ldx, const void* qweight, const
 constexpr size_t kStaticScratchBytes = static_cast<size_t>(24) << 20;
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
 
+// A status word (and counters that nobody uses) for launches that have no scratch, see dxb_shared_workspace.
+static __device__ __align__(256) unsigned char g_shared_workspace[dx::kStatusBytes + dx::kMaxTiles * 4];
+
 namespace dx {
 constexpr int kMaxDevices = 64;
-// Device address of g_static_scratch on the CURRENT device, looked up once per device.
-static int static_scratch_address(void** out) {
-  static std::mutex mu;
-  static void* addr[kMaxDevices] = {};
+struct SymbolAddress {
+  std::mutex mu;
+  void* addr[kMaxDevices] = {};
+};
+// Device address of a symbol of this library on the CURRENT device, looked up once per device.
+static int symbol_address(SymbolAddress& known, const void* symbol, void** out) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return DXB_ERR_CUDA;
-  std::lock_guard<std::mutex> lock(mu);
-  if (addr[dev] == nullptr) {
+  std::lock_guard<std::mutex> lock(known.mu);
+  if (known.addr[dev] == nullptr) {
     void* p = nullptr;
-    if (cudaGetSymbolAddress(&p, g_static_scratch) != cudaSuccess || p == nullptr) {
+    if (cudaGetSymbolAddress(&p, symbol) != cudaSuccess || p == nullptr) {
       cudaGetLastError();  // clear the sticky-less error so later calls start clean
       return DXB_ERR_CUDA;
     }
-    addr[dev] = p;
+    known.addr[dev] = p;
   }
-  *out = addr[dev];
+  *out = known.addr[dev];
   return DXB_OK;
+}
+static int static_scratch_address(void** out) {
+  static SymbolAddress known;
+  return symbol_address(known, g_static_scratch, out);
 }
 }  // namespace dx
 
@@ -2345,6 +2354,18 @@ int dxb_workspace_init(void* workspace, size_t workspace_bytes, void* status, vo
   wq_workspace_init_kernel<<<(vecs + 255) / 256, 256, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
       static_cast<uint4*>(workspace), vecs, static_cast<int*>(status));
   return cudaGetLastError() == cudaSuccess ? DXB_OK : DXB_ERR_CUDA;
+}
+
+int dxb_shared_workspace(void** workspace) {
+  if (!workspace) return DXB_ERR_NULL;
+  static dx::SymbolAddress known;
+  // The first look-up on a device may load code there, which is refused while a stream is captured in the
+  // usual mode, unless the thread is in this one.
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) { cudaGetLastError(); return DXB_ERR_CUDA; }
+  const int rc = dx::symbol_address(known, g_shared_workspace, workspace);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  return rc;
 }
 
 int dxb_event_done(void* cuda_event) {

@@ -39,8 +39,9 @@ _LIB = _lib.load()
 #   _captured  (capture, scratch) for the launches of the capture that is under way: a graph may be replayed on any
 #              stream, beside other graphs and eager launches, for as long as it lives, so its scratch comes out
 #              of its own memory pool and is made ready by the graph itself
-# Scratch passes errors on to the status word of its stream's block, which `last_status` reads.
-_Space = Tuple[torch.Tensor, int, int]  # tensor, address, bytes
+# A stream on which nothing but captures has happened yet has no block; the library's own stands in for it
+# (_shared).  Scratch passes errors on to the status word of its stream's block, which `last_status` reads.
+_Space = Tuple[Optional[torch.Tensor], int, int]  # tensor, address, bytes
 _blocks: Dict[Tuple[int, int], _Space] = {}
 _scratch: Dict[Tuple[int, int], _Space] = {}
 _captured: Dict[Tuple[int, int], Tuple[int, _Space]] = {}
@@ -52,7 +53,16 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
 
-def _ready(device: int, stream: int, nbytes: int, status: Optional[int]) -> _Space:
+def _shared() -> _Space:
+    """The library's own block on the current device."""
+    address = ctypes.c_void_p()
+    rc = _LIB.dxb_shared_workspace(ctypes.byref(address))
+    if rc != _lib.OK:
+        _raise(rc)
+    return None, address.value, _BLOCK_BYTES
+
+
+def _ready(device: int, stream: int, nbytes: int, status: int) -> _Space:
     """Scratch of at least ``nbytes``, made ready on ``stream`` (the current one)."""
     t = torch.empty(nbytes, dtype=torch.uint8, device=torch.device("cuda", device))
     rc = _LIB.dxb_workspace_init(t.data_ptr(), nbytes, status, ctypes.c_void_p(stream))
@@ -72,10 +82,12 @@ def _workspace(device: int, stream: int, need: int) -> _Space:
     with _lock:
         block = _blocks.get(key)
         if capture:
+            block = _shared() if block is None else block
+            if need == 0:
+                return block
             held = _captured.get(key)
             if held is None or held[0] != capture or held[1][2] < need:
-                held = (capture, _ready(device, stream, max(need, _BLOCK_BYTES), None if block is None else block[1]))
-                _captured[key] = held
+                held = _captured[key] = (capture, _ready(device, stream, need, block[1]))
             return held[1]
         if block is None:
             t = torch.zeros(_BLOCK_BYTES, dtype=torch.uint8, device=torch.device("cuda", device))
@@ -332,9 +344,7 @@ def last_status(device: Optional[torch.device] = None) -> int:
     with torch.cuda.device(device):
         stream = torch.cuda.current_stream().cuda_stream
         key = (device.index if device.index is not None else torch.cuda.current_device(), stream)
-        # (a stream on which nothing but captures has happened has no block: the last capture's word)
-        ws = _blocks[key][1] if key in _blocks else _captured[key][1][1] if key in _captured else None
-        return _lib.OK if ws is None else _LIB.dxb_read_status(ws, ctypes.c_void_p(stream))
+        return _LIB.dxb_read_status((_blocks.get(key) or _shared())[1], ctypes.c_void_p(stream))
 
 
 def accepts(*args) -> bool:

@@ -212,6 +212,10 @@ size_t dxb_workspace_bytes_ex(int M, int N, int K, int bits, int max_ctas);
  * workspace of 65,792 bytes (status word and counters), even where they overlap; a caller whose calls are captured
  * in graphs gives the others a workspace per graph that may overlap with anything else. */
 size_t dxb_scratch_bytes(int M, int N, int K, int bits, int max_ctas);
+/* Address of a workspace of 65,792 bytes inside the library, one per device, ready from the start: for calls whose
+ * dxb_scratch_bytes is 0 and which have no workspace yet where none can be set up (under capture).  They share
+ * its status word. */
+int dxb_shared_workspace(void** workspace);
 /*
  * Makes a workspace ready for its first call (one small kernel on `cuda_stream`; the same as zero-filling its first
  * 65,792 bytes).  `status` (may be NULL): an int that is set as well whenever a kernel leaves an error code in

@@ -93,6 +93,24 @@ def test_eager_calls_after_a_capture_that_never_ran(d):
         assert d.ops.last_status() == 0
 
 
+def test_a_capture_on_a_fresh_stream_adds_nothing_to_a_small_graph(d):
+    # no scratch, no block yet: the library's own block serves, without a node that makes one ready
+    x, q = problem(d, 83, 1024, 1024, 8)
+    want = call(d, x, q)
+    stream = torch.cuda.ExternalStream(torch.cuda.Stream().cuda_stream)
+    key = (torch.cuda.current_device(), stream.cuda_stream)
+    block, _ = d.ops._blocks.pop(key, None), d.ops._captured.pop(key, None)
+    try:
+        graph, y = capture(d, x, q, stream)
+        assert key not in d.ops._captured and key not in d.ops._blocks
+        with torch.cuda.stream(stream):
+            graph.replay()
+            assert torch.equal(y, want) and d.ops.last_status() == 0
+    finally:
+        if block is not None:  # (streams come from a pool: an earlier test may have used this one)
+            d.ops._blocks[key] = block
+
+
 def test_status_of_scratch_reaches_the_streams_status_word(d):
     x, q = problem(d, *SPLIT)
     stream = torch.cuda.Stream()
