@@ -852,9 +852,9 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     };
     if (left > 0) { seek_sz(); load_sz(); }
     while (left > 0) {
-      // (Lanes that gave up carry on to the second wait, where the warp decides (see mbar_wait_warp).  One
-      // decision per unit instead of two: FFN of 913 tokens, 5120 x
-      // 13824, 238.5 us against 246.9; int8 FFN of 83 tokens 36.0 against 36.7.)
+      // (Lanes that gave up carry on to the end of the unit, where the warp decides, see mbar_wait_warp: once per unit
+      // and off its critical path.  A decision after each wait: FFN of 913 tokens 5120 x 13824 246.9 us, 236.4 so;
+      // one after the second wait: int8 with zero points 160 tokens 14336 x 3072 31.4 against 30.2.)
       ok = mbar_wait(bar0 + 8 * (kBarFullW + s), ph, abortp);
       const uint32_t wsrc = w_ring + s * W_STAGE;
       uint32_t w0[8], w1[8];
@@ -922,7 +922,6 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         load_sz();
       }
       ok = wait_mma(a_empty_bar, aph ^ 1u) && ok;
-      if (!__all_sync(0xffffffffu, ok)) break;
       tc_fence_after();
       if (large) {
         // The same with scales of 2 and more, see sym4_any; a body of its own, so that the usual one is
@@ -1031,7 +1030,9 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       }
       tc_wait_st();
       tc_fence_before();
+      ok = __all_sync(0xffffffffu, ok);
       __syncwarp();
+      if (!ok) break;
       if (lane == 0) {
         if (PAIR) mbar_arrive_pair(a_full_bar);
         else mbar_arrive(a_full_bar);
