@@ -45,7 +45,7 @@ _Space = Tuple[Optional[torch.Tensor], int, int]  # tensor, address, bytes
 _blocks: Dict[Tuple[int, int], _Space] = {}
 _scratch: Dict[Tuple[int, int], _Space] = {}
 _captured: Dict[Tuple[int, int], Tuple[int, _Space]] = {}
-_lock = threading.Lock()
+_lock = threading.RLock()  # (an allocation may run finalisers, which may come back here)
 _BLOCK_BYTES = 256 + 4 * 16384
 
 
