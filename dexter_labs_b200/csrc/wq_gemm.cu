@@ -2115,8 +2115,8 @@ static int read_opts(const dxb_gemm_opts* o, int bits, int M, int N, int K, Opts
 
 // Few tokens and a weight that is read in little more than the fixed cost of a launch: there the kernel
 // without set-up is ahead; with more to convert (once per 16 tokens, there) the tcgen05 pipeline is.
-// The lines lie where the two crossed over 14 weights of 0.5 to 44 x 2^20 values and 18 token counts from 1 to 256 (both
-// kernels on all of them: profiles/few_token_line.md).  Near the lines, us small / tcgen05: int4 1 token 3072 x
+// The lines lie where the two crossed over 14 weights of 0.5 to 44 x 2^20 values and 18 token counts from 1 to 256, with
+// both kernels on all of them.  Near the lines, us small / tcgen05: int4 1 token 3072 x
 // 9216 6.4 / 7.2 and 3072 x 11264 8.3 / 8.3, 8 tokens 4096 x 4096 5.4 / 6.1 and 3072 x 6144 6.4 / 6.1, 16 tokens 3072 x
 // 3072 4.9 / 5.3 and 4096 x 4096 6.3 / 6.1, 32 tokens 2048 x 2048 4.2 / 4.6 and 2048 x 3072 5.7 / 5.1, 96 tokens
 // 1024 x 1024 3.9 / 5.1 and 1024 x 2048 6.0 / 5.4, 128 tokens 1024 x 2048 6.1 / 7.0 and 2048 x 2048 8.9 / 7.5 (from 97

@@ -119,7 +119,11 @@ def test_status_of_scratch_reaches_the_streams_status_word(d):
         want = call(d, x, q)
         key = (torch.cuda.current_device(), stream.cuda_stream)
         d.ops._scratch[key][0][256:260].view(torch.int32).fill_(0x8000)  # the finisher's wait runs out
-        call(d, x, q)
-        assert d.ops.last_status() == -8
-        d.ops._blocks[key][0].zero_()
+        if d.ops._CHECK:  # every call reads the word and clears it
+            with pytest.raises(RuntimeError, match="TIMEOUT"):
+                call(d, x, q)
+        else:
+            call(d, x, q)
+            assert d.ops.last_status() == -8
+            d.ops._blocks[key][0].zero_()
         assert torch.equal(call(d, x, q), want) and d.ops.last_status() == 0
