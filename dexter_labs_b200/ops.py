@@ -405,25 +405,33 @@ def w8a16_gelu(x, qweight, scales, zeros, bias, group_size):
 
 def gemm_group(bits: int, problems, group_size: int, *, layout: str = "dexter"):
     """Independent linears ``(x, qweight, scales, zeros, bias)`` over the same number of tokens and the same K as
-    ONE launch; the list of their results, or None where they cannot go together (more than 128 tokens, shapes
-    off the tensor-core kernel's tiles, some with zero points and some without): call them one by one then."""
-    x0 = problems[0][0]
-    if not x0.is_cuda or x0.device.index != _current_device() or not 1 <= len(problems) <= 8:
+    ONE launch; the list of their results, or None where they cannot go together (no tokens or more than 128, shapes
+    off the tensor-core kernel's tiles, some with zero points and some without): call them one by one then.
+    Leading dimensions of an ``x`` are flattened, and are those of its result, as in one call."""
+    if not 1 <= len(problems) <= 8 or any(x.dim() == 0 for x, *_ in problems):
         return None
-    m, k_dim = x0.shape
+    x0 = problems[0][0]
+    if not x0.is_cuda or x0.device.index != _current_device() or x0.numel() == 0:
+        return None
+    k_dim = x0.shape[-1]
+    m = x0.numel() // k_dim
     items = (_lib.GroupItem * len(problems))()
-    outs = []
+    outs, flat = [], []  # (flattened activations may be copies, which live until the launch)
     for item, (x, qweight, scales, zeros, bias) in zip(items, problems):
         rows, n = qweight.shape
-        if (x.shape != x0.shape or x.dtype != torch.bfloat16 or x.stride(1) != 1 or x.device != x0.device
+        if (x.shape[-1] != k_dim or x.numel() != m * k_dim or x.dtype != torch.bfloat16 or x.device != x0.device
                 or qweight.dtype != torch.uint8 or rows * (2 if bits == 4 else 1) != k_dim):
             return None
         if not all(t is None or t.is_contiguous() for t in (qweight, scales, zeros, bias)):
             return None
         _check_operands(x.device, k_dim, n, group_size, qweight, scales, zeros, bias)
+        x2 = x if x.dim() == 2 else x.reshape(-1, k_dim)
+        if x2.stride(1) != 1:
+            return None
         out = torch.empty((m, n), device=x.device, dtype=torch.bfloat16)
-        outs.append(out)
-        item.x, item.ldx, item.qweight, item.scales = x.data_ptr(), x.stride(0), qweight.data_ptr(), scales.data_ptr()
+        flat.append(x2)
+        outs.append(out if x.dim() == 2 else out.view(*x.shape[:-1], n))
+        item.x, item.ldx, item.qweight, item.scales = x2.data_ptr(), x2.stride(0), qweight.data_ptr(), scales.data_ptr()
         item.zeros, item.bias, item.out, item.ldo, item.n = _ptr(zeros), _ptr(bias), out.data_ptr(), n, n
     stream = _raw_stream(x0.device.index)
     ws = _workspace(x0.device.index, stream, 0)

@@ -121,7 +121,7 @@ int dxb_wq_gemm_ex(int bits, const void* x, int64_t ldx, const void* qweight, co
                    int group_size, void* workspace, size_t workspace_bytes,
                    const dxb_gemm_opts* opts, void* cuda_stream);
 
-/* Several problems of the same M, K, bit width, group size and options in one launch (M at most 128, 1 to 8 items,
+/* Several problems of the same M, K, bit width, group size and options in one launch (M 1 to 128, 1 to 8 items,
  * all with zero points or all without, max_ctas 0, no sum over ranks, shapes and pointers as the tensor-core kernel
  * takes them; DXB_ERR_UNSUPPORTED otherwise: issue them one by one).  The results are those of
  * dxb_wq_gemm_ex up to the order of the fp32 sums.  Inputs must not depend on outputs of the same launch.  Of the

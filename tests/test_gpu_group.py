@@ -71,3 +71,20 @@ def test_group_in_a_graph_follows_its_inputs(d, oracle):
     for y, ((x, _, s, z, b), plain) in zip(outs, made):
         want = oracle.torch_wq_gemm(x, plain, s, z, b, 128, 4).double()
         assert (y.double() - want).abs().max() <= 1e-2 * want.abs().max()
+
+
+def test_leading_dimensions_are_flattened_and_no_tokens_are_declined(d):
+    made = [p for p, _ in problems(d, 40, 256, (128, 256), 4, 128, True, "dexter")]
+    want = d.ops.gemm_group(4, made, 128)
+    flat = [p[0].contiguous() for p in made]
+    strided = torch.stack((flat[0], flat[0]), 1)[:, 0].view(5, 8, 256)  # rows 512 apart, in two dimensions
+    shapes = [(flat[0].view(2, 20, 256), (2, 20)), (strided, (5, 8)), (flat[0].view(1, 40, 256), (1, 40))]
+    for x, lead in shapes:
+        got = d.ops.gemm_group(4, [(x, *made[0][1:]), (flat[1], *made[1][1:])], 128)
+        assert [y.shape for y in got] == [(*lead, 128), (40, 256)]
+        assert torch.equal(got[0].view(40, 128), want[0]) and torch.equal(got[1], want[1])
+    empty = flat[0][:0]
+    for x in (empty, empty.view(3, 0, 256)):
+        assert d.ops.gemm_group(4, [(x, *p[1:]) for p in made], 128) is None
+    assert d.ops.gemm_group(4, [], 128) is None
+    assert d.ops.gemm_group(4, [(flat[0][0], *made[0][1:])], 128)[0].shape == (128,)
