@@ -181,7 +181,7 @@ class LayerSet:
     _peer: Optional[object] = None  # ops.PeerAllReduce, see enable_peer_reduce
     _fused: Optional[object] = None  # ops.FusedReduce, see enable_fused_reduce
     _plain: Dict[int, QuantizedWeight] = field(default_factory=dict)  # see _g
-    _grouped: bool = False  # the last concurrent pass ran each block's independent linears as one launch
+    _saved: int = 0  # launches that the last pass saved by running independent linears as one
 
     def enable_peer_reduce(self, tokens: int, device) -> bool:
         """Set up the peer-memory all-reduce for outputs of up to ``tokens x dim`` bf16.
@@ -316,8 +316,8 @@ class LayerSet:
 
     @property
     def launches(self) -> int:
-        """Kernel launches of the last pass: one per GEMM, or one for a block's five independent ones."""
-        return self.num_gemms - 4 * self.blocks * self._grouped
+        """Kernel launches of the last :meth:`forward`: one per GEMM, or one for a block's five independent ones."""
+        return self.num_gemms - self._saved
 
     @property
     def num_linears(self) -> int:
@@ -426,8 +426,8 @@ class LayerSet:
         if self.world > 1:
             return self._block_forward_overlapped(L, x, ctx)
         first = self._group((x, L["self_q"]), (x, L["self_k"]), (x, L["self_v"]), (ctx, L["cross_k"]), (ctx, L["cross_v"]))
-        self._grouped = first is not None
         if first is not None:
+            self._saved += len(first) - 1
             x = self._row(first[2], L["self_o"])
             g(x, L["cross_q"])
             x = self._row(first[4], L["cross_o"])
@@ -593,6 +593,7 @@ class LayerSet:
 
     def forward(self, x: torch.Tensor, ctx: Optional[torch.Tensor] = None) -> torch.Tensor:
         ctx = x if ctx is None else ctx
+        self._saved = 0
         for blk in range(self.blocks):
             x = self.block_forward(blk, x, ctx)
         return x

@@ -51,17 +51,17 @@ def recorded(monkeypatch, ls):
     return seen
 
 
-@pytest.mark.parametrize("lead,ctx_lead,bits,group,symmetric,relayout,together", [
-    ((1,), (1,), 4, 128, True, True, True),
-    ((83,), (83,), 4, 64, False, True, True),
-    ((128,), (128,), 8, 128, False, True, True),
-    ((2, 20), (40,), 8, 0, True, True, True),     # leading dimensions are flattened
-    ((129,), (129,), 4, 128, True, True, False),  # more than one token block
-    ((40,), (17,), 4, 128, True, True, False),    # a context of another length
-    ((40,), (200,), 8, 128, True, True, False),
-    ((3, 7), (3, 7), 4, 128, True, False, False),  # int4 in the reference layout
-    ((0,), (0,), 4, 128, True, True, False),      # no tokens
-    ((2, 0), (2, 0), 8, 128, True, True, False),
+@pytest.mark.parametrize("lead,ctx_lead,bits,group,symmetric,relayout,together", [  # together: blocks with one launch for five
+    ((1,), (1,), 4, 128, True, True, 2),
+    ((83,), (83,), 4, 64, False, True, 2),
+    ((128,), (128,), 8, 128, False, True, 2),
+    ((2, 20), (40,), 8, 0, True, True, 2),      # leading dimensions are flattened
+    ((129,), (129,), 4, 128, True, True, 0),    # more than one token block
+    ((40,), (17,), 4, 128, True, True, 1),      # a context of another length (a block's result has the context's)
+    ((40,), (200,), 8, 128, True, True, 0),
+    ((3, 7), (3, 7), 4, 128, True, False, 0),   # int4 in the reference layout
+    ((0,), (0,), 4, 128, True, True, 0),        # no tokens
+    ((2, 0), (2, 0), 8, 128, True, True, 0),
 ])
 def test_concurrent_pass(lead, ctx_lead, bits, group, symmetric, relayout, together, d, oracle, monkeypatch):
     ls = layer_set(bits, group, symmetric, relayout)
@@ -73,6 +73,7 @@ def test_concurrent_pass(lead, ctx_lead, bits, group, symmetric, relayout, toget
     seen = recorded(monkeypatch, ls)
     y = ls.forward(x, ctx)
     assert len(seen) == ls.num_gemms
+    assert ls.launches == ls.num_gemms - 4 * together
     assert y.shape == (*ctx_lead, DIM)
     assert torch.equal(y, seen["ffn_down", BLOCKS - 1][1])
     for b, row in enumerate(ls.layers):
@@ -87,3 +88,14 @@ def test_concurrent_pass(lead, ctx_lead, bits, group, symmetric, relayout, toget
             assert got.shape == want.shape
             if want.numel():
                 assert (got.double() - want).abs().max() <= 1e-2 * want.abs().max(), (l.name, b)
+
+
+def test_launches_are_those_of_the_last_pass(d):
+    ls = layer_set(4, 128, True, True)
+    x = torch.randn(24, DIM, device="cuda").to(torch.bfloat16)
+    counts = []
+    for concurrent in (True, True, False, True):
+        ls.concurrent = concurrent
+        ls.forward(x)
+        counts.append(ls.launches)
+    assert counts == [12, 12, 20, 12]
