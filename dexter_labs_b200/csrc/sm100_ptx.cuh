@@ -106,8 +106,10 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tmap, uint
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(x), "r"(y)
       : "memory");
 }
-// The same with an L2 eviction priority, one of the words that createpolicy.fractional yields on this architecture
-// (kept on the host: the instruction wants its policy in a uniform register, where a kernel parameter already is).
+// The same with an L2 eviction priority: one of the words that createpolicy.fractional yields on this architecture, which
+// tests/test_gpu_l2_policy.py compares with what it gives on the device.  They are kept here and travel as a kernel
+// parameter because the load wants its policy in a uniform register, where a parameter already is; made
+// by createpolicy in the kernel, 8 tokens 3072 x 9216 take 7.37 us instead of 7.24.
 constexpr uint64_t kL2EvictFirst = 0x12F0000000000000ull;      // L2::evict_first, all lines
 constexpr uint64_t kL2EvictFirstHalf = 0x1270000000000000ull;  // L2::evict_first, half of them
 constexpr uint64_t kL2EvictNormal = 0x16F0000000000000ull;     // L2::evict_normal
