@@ -162,8 +162,8 @@ def workload_config(n_gpus: int, collective: str = "fused") -> dict:
     return {"workload": f"{PRESET.upper()} backbone linear set: {blocks} blocks x (self q,k,v,o; cross q,k,v,o; "
                         f"ffn up,down), int4 group 128 symmetric + bias, M={M_TOKENS}, seeded random weights",
             "gemms_per_step": (10 if n_gpus == 1 else 7) * blocks,
-            "schedule": ("per block: self q,k,v and cross k,v on parallel streams, then o, cross q, cross o, "
-                         "up, down; one CUDA graph per pass") if n_gpus == 1 else
+            "schedule": (f"per block: self q,k,v and cross k,v {'as one launch' if M_TOKENS <= 128 else 'on parallel streams'}, "
+                         "then o, cross q, cross o, up, down; one CUDA graph per pass") if n_gpus == 1 else
                         ("per block: self q,k,v as one launch, o with its sum over ranks beside cross k,v as one "
                          "launch on a side stream, cross q, cross o, up, down; one CUDA graph per pass"),
             "tokens": M_TOKENS, "dim": dim, "ffn_dim": ffn,
@@ -554,8 +554,8 @@ def run_ours(args) -> int:
     t_mma_ms = set_flops / world / (tensor_peak * 1e9)
     roofline_ms = max(t_mem_ms, t_mma_ms)
     # dominant kernel: wq_gemm_tc (int4, symmetric, repacked weights); averages over the pass, per
-    # rank: the pass time divided by its launches, which overlap -- not the
-    # duration of one launch (the "gemm" key times one shape's launches back to back)
+    # rank: the pass time divided by its launches, which overlap (each starts under the end of the one before, some run
+    # on parallel streams) -- not the duration of one launch (the "gemm" key times one shape's launches back to back)
     pass_us_per_launch = ms_per_step * 1e3 / launches_per_step
     flops_per_launch = set_flops / world / launches_per_step
     bytes_per_launch = set_bytes / world / launches_per_step
