@@ -117,12 +117,13 @@ __device__ __forceinline__ uint32_t sym4_mid(uint32_t w, uint32_t scale, uint32_
 __device__ __forceinline__ uint32_t sym4_scale_low(uint32_t s2) { return mul_bf16x2(s2, 0x7F007F00u); }  // 2^(133-6)
 __device__ __forceinline__ uint32_t sym4_scale_mid(uint32_t s2) { return mul_bf16x2(s2, 0x7D007D00u); }  // 2^(129-6)
 __device__ __forceinline__ uint32_t sym4_offset(uint32_t s2) { return mul_bf16x2(s2, 0xBE00BE00u); }     // -8 * 2^-6
-// One byte -> fp32 by bit pattern: 0x4B0000qq = 8388608 + q.  `cz` = 8388608 +
-// zero point; subtract and multiply are both exact in fp32 (8-bit x 8-bit
-// significands), so the later cvt.rn to bf16 is the only rounding.
-__device__ __forceinline__ float deq8(uint32_t word, uint32_t byte_sel, float cz, float scale) {
+// One byte -> fp32 by bit pattern: 0x4B0000qq = 8388608 + q.  8388608 and the zero point are taken off in turn: added up
+// first, zero points that are no whole numbers would be rounded to one.  The difference is exact as far as fp32's 24
+// bits go (zero points whose last bit is 2^-8 or more have 16 of them), its product with an 8-bit
+// scale then too, and the later cvt.rn to bf16 is the only rounding.
+__device__ __forceinline__ float deq8(uint32_t word, uint32_t byte_sel, float zero, float scale) {
   const float f = __uint_as_float(prmt(word, 0x4B000000u, 0x7650u + byte_sel));
-  return (f - cz) * scale;
+  return ((f - 8388608.0f) - zero) * scale;
 }
 // Bytes in GEMMs.  As bf16 the pattern 0x00qq is q * 2^-133 for all 256 bytes (the first normal binade has the
 // subnormals' step), so two byte permutes per four bytes pair them up, and
@@ -132,7 +133,7 @@ __device__ __forceinline__ float deq8(uint32_t word, uint32_t byte_sel, float cz
 //     that range and the multiply by 2^127 * scale is the only rounding.
 // Weights and sums are divided by kSymAcc as on int4's symmetric grid.  2.5 and 3.5 instructions per two
 // weights, of which 1.5 are on the integer pipe.  Scales of 2 and more and other zero points take
-// deq8_any, in a body of its own: 5 instructions per two weights.  Measured, us with deq8_any / so: 83 tokens 3072 x
+// deq8_any, in a body of its own: 9 instructions per two weights.  Measured, us with deq8_any / so: 83 tokens 3072 x
 // 14336 13.9 / 13.2, 14336 x 3072 15.2 / 14.2, with zero points 13.7 / 12.9; 16 tokens 3072 x 9216 10.4 / 9.5; one
 // token 3072 x 3072 6.1 / 5.4.  (125 tokens 3072 x 8192 on clusters of two: 12.7 either way.)
 __device__ __forceinline__ uint32_t byte_pairs(uint32_t w0, uint32_t w1, bool high) {  // columns 0, 1 or 2, 3 of two rows
@@ -157,21 +158,10 @@ __device__ __forceinline__ uint32_t deq8_zeros(uint32_t z2, uint32_t& odd) {
   odd |= (r & 0xFF00FF00u) | (mul_bf16x2(r, 0x7F007F00u) ^ mul_bf16x2(z2, 0x3C803C80u));
   return r;
 }
-// Any scale and zero point: 0x4300qq00 = 128 + q / 256 in fp32, so that one fused multiply-add with 256 * scale and
-// -(128 + zero / 256) * 256 * scale (both divided by kSymAcc) gives the weight: the constant has 16 + 8 significant
-// bits and the result 17, all of it exact in fp32, and the conversion to bf16 is the only rounding.
-__device__ __forceinline__ void deq8_constants(float scale, float zero, uint32_t& scale256, uint32_t& offset) {
-  const float s = scale * (256.0f / kSymAcc);
-  scale256 = __float_as_uint(s);
-  offset = __float_as_uint(-__fmaf_rn(zero, 1.0f / 256.0f, 128.0f) * s);
-}
-// Byte `b` of two words (consecutive k of one column) -> a bf16 pair.
-__device__ __forceinline__ uint32_t deq8_any(uint32_t w0, uint32_t w1, uint32_t b, uint32_t scale256, uint32_t offset) {
-  auto one = [&](uint32_t w) {
-    return __fmaf_rn(__uint_as_float(prmt(w, 0x43000000u, 0x7504u + (b << 4))), __uint_as_float(scale256),
-                     __uint_as_float(offset));
-  };
-  return cvt_bf16x2(one(w1), one(w0));
+// Any scale and zero point.  Byte `b` of two words (consecutive k of one column) -> a bf16 pair; `scale` is divided by
+// kSymAcc.
+__device__ __forceinline__ uint32_t deq8_any(uint32_t w0, uint32_t w1, uint32_t b, float zero, float scale) {
+  return cvt_bf16x2(deq8(w1, b, zero, scale), deq8(w0, b, zero, scale));
 }
 
 __device__ __forceinline__ uint32_t dup_lo(uint32_t w) { return prmt(w, w, 0x1010u); }

@@ -951,7 +951,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         if (lane == 0) mbar_arrive(bar0 + 8 * (kBarEmptyW + s));
       }
       // This unit's scales and zero points as the conversion wants them (int4: in both halves of a
-      // word; int8: the same, or the constants of deq8_any); then the next unit's rows.
+      // word; int8: the same, or in fp32 for deq8_any); then the next unit's rows.
       uint32_t s2[PLANES][4], z2[PLANES][4];
       // Constants outside the short conversions' range (never a model's): bodies of their own, so that the usual one is
       // scheduled as if they did not exist (a branch in front of each store made launches 6 % longer).
@@ -995,8 +995,10 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
             const uint32_t zx[2] = {HAS_ZERO ? zr[pl].x : 0x43004300u, HAS_ZERO ? zr[pl].y : 0x43004300u};  // 128
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-              deq8_constants(bf16lo_f32(sx[i]), bf16lo_f32(zx[i]), s2[pl][2 * i], z2[pl][2 * i]);
-              deq8_constants(bf16hi_f32(sx[i]), bf16hi_f32(zx[i]), s2[pl][2 * i + 1], z2[pl][2 * i + 1]);
+              s2[pl][2 * i] = __float_as_uint(bf16lo_f32(sx[i]) / kSymAcc);
+              s2[pl][2 * i + 1] = __float_as_uint(bf16hi_f32(sx[i]) / kSymAcc);
+              z2[pl][2 * i] = zx[i] << 16;
+              z2[pl][2 * i + 1] = zx[i] & 0xFFFF0000u;
             }
           } else {
 #pragma unroll
@@ -1123,7 +1125,7 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
 #pragma unroll
                   for (int o = 0; o < 2; ++o) {
                     const int i = 2 * h + o;
-                    r[h][2 * sl + o] = ANY ? deq8_any(x0, x1, i, s2[pl][i], z2[pl][i])
+                    r[h][2 * sl + o] = ANY ? deq8_any(x0, x1, i, __uint_as_float(z2[pl][i]), __uint_as_float(s2[pl][i]))
                                        : HAS_ZERO ? deq8_zero(byte_pair(pairs, o), s2[pl][i], z2[pl][i])
                                                   : deq8_sym(byte_pair(pairs, o), s2[pl][i], z2[pl][i]);
                   }
@@ -1446,8 +1448,8 @@ __global__ void wq_gemm_simt(const __nv_bfloat16* __restrict__ x, long long ldx,
       const uint32_t z = zeros ? __bfloat16_as_ushort(zeros[static_cast<long long>(gi) * N + n]) : 0x4308u;
       w = __uint_as_float(deq4(byte, z | (z << 16), sbits | (sbits << 16)) << 16);
     } else {
-      const float cz = 8388608.0f + (zeros ? __bfloat162float(zeros[static_cast<long long>(gi) * N + n]) : 128.0f);
-      const float v = deq8(qw[static_cast<long long>(k) * N + n], 0, cz, __uint_as_float(sbits << 16));
+      const float zero = zeros ? __bfloat162float(zeros[static_cast<long long>(gi) * N + n]) : 128.0f;
+      const float v = deq8(qw[static_cast<long long>(k) * N + n], 0, zero, __uint_as_float(sbits << 16));
       w = __uint_as_float((cvt_bf16x2(0.0f, v) & 0xFFFFu) << 16);
     }
 #pragma unroll

@@ -14,6 +14,20 @@ namespace dx {
 // 16-byte stores, consecutive lanes on consecutive columns (256 B read and 512 B written per row
 // and warp).  Eight rows because every group and plane boundary is a multiple of 8 (the rule
 // below) and so scales never change inside a thread.
+//
+// int8: deq8 of two weights at a time, both differences and the product one instruction for the two.  (3072 x 14336 with
+// zero points: 21.0 us; 21.7 with deq8.)
+__device__ __forceinline__ uint32_t deq8_pair(uint32_t word, uint32_t high, uint32_t zero2, uint32_t scale2) {
+  const uint32_t q0 = prmt(word, 0x4B000000u, 0x7650u + 2 * high), q1 = prmt(word, 0x4B000000u, 0x7651u + 2 * high);
+  float lo, hi;
+  asm("{\n\t.reg .b64 v, b, z, s;\n\tmov.b64 v, {%2, %3};\n\tmov.b64 b, {%4, %4};\n\tmov.b64 z, {%5, %6};\n\t"
+      "mov.b64 s, {%7, %8};\n\tadd.rn.f32x2 v, v, b;\n\tadd.rn.f32x2 v, v, z;\n\tmul.rn.f32x2 v, v, s;\n\t"
+      "mov.b64 {%0, %1}, v;\n\t}\n"
+      : "=f"(lo), "=f"(hi)
+      : "r"(q0), "r"(q1), "f"(-8388608.0f), "f"(-bf16lo_f32(zero2)), "f"(-bf16hi_f32(zero2)), "f"(bf16lo_f32(scale2)),
+        "f"(bf16hi_f32(scale2)));
+  return cvt_bf16x2(hi, lo);
+}
 template <int BITS, bool RELAID>
 __global__ void __launch_bounds__(128)
 wq_dequant_kernel(const uint8_t* __restrict__ qw, const __nv_bfloat16* __restrict__ scales,
@@ -62,9 +76,7 @@ wq_dequant_kernel(const uint8_t* __restrict__ qw, const __nv_bfloat16* __restric
           v[h] = deq4(pair, z[h], s[h]);
         } else {
           const uint32_t word = h < 2 ? w[i].x : w[i].y;
-          const float lo = deq8(word, 2 * (h & 1), 8388608.0f + bf16lo_f32(z[h]), bf16lo_f32(s[h]));
-          const float hi = deq8(word, 2 * (h & 1) + 1, 8388608.0f + bf16hi_f32(z[h]), bf16hi_f32(s[h]));
-          v[h] = cvt_bf16x2(hi, lo);
+          v[h] = deq8_pair(word, h & 1, z[h], s[h]);
         }
       }
       __stcs(reinterpret_cast<uint4*>(out + static_cast<long long>(k0 + i) * N + n),
@@ -90,7 +102,7 @@ wq_dequant_cols_kernel(const uint8_t* __restrict__ qw, const __nv_bfloat16* __re
   const int n = blockIdx.x * 128 + (threadIdx.x & 31);
   if (r0 >= rows) return;
   uint32_t s[PLANES][4], z[PLANES][4];
-  float cz[4];
+  float z8[4];
   int left[PLANES];  // rows until the plane's next group
   auto load = [&](int pl, int gi) {
 #pragma unroll
@@ -99,7 +111,7 @@ wq_dequant_cols_kernel(const uint8_t* __restrict__ qw, const __nv_bfloat16* __re
       const long long so = static_cast<long long>(gi) * N + n + 32 * j;
       s[pl][j] = __bfloat16_as_ushort(scales[so]);
       if (BITS == 4) z[pl][j] = zeros ? __bfloat16_as_ushort(zeros[so]) : 0x4308u;
-      else cz[j] = 8388608.0f + (zeros ? __bfloat162float(zeros[so]) : 128.0f);
+      else z8[j] = zeros ? __bfloat162float(zeros[so]) : 128.0f;
     }
   };
 #pragma unroll
@@ -129,7 +141,7 @@ wq_dequant_cols_kernel(const uint8_t* __restrict__ qw, const __nv_bfloat16* __re
       for (int j = 0; j < 4; ++j) {
         if (n + 32 * j >= N) continue;
         const uint32_t v = BITS == 4 ? deq4(q[j] >> (4 * pl), z[pl][j], s[pl][j])
-                                     : cvt_bf16x2(0.0f, deq8(q[j], 0, cz[j], __uint_as_float(s[pl][j] << 16)));
+                                     : cvt_bf16x2(0.0f, deq8(q[j], 0, z8[j], __uint_as_float(s[pl][j] << 16)));
         dst[32 * j] = __ushort_as_bfloat16(static_cast<unsigned short>(v & 0xFFFFu));
       }
     }

@@ -358,8 +358,10 @@ __global__ void __launch_bounds__(CPW == 1 ? 512 : 256, CPW == 1 ? 1 : 2) wq_gem
                 s0 = dup_lo(sv8); s1 = dup_hi(sv8);
                 z0 = dup_lo(zv8); z1 = dup_hi(zv8);
               } else {
-                deq8_constants(bf16lo_f32(sp), has_zero ? bf16lo_f32(zp) : 128.0f, s0, z0);
-                deq8_constants(bf16hi_f32(sp), has_zero ? bf16hi_f32(zp) : 128.0f, s1, z1);
+                s0 = __float_as_uint(bf16lo_f32(sp) / kSymAcc);
+                s1 = __float_as_uint(bf16hi_f32(sp) / kSymAcc);
+                z0 = has_zero ? zp << 16 : __float_as_uint(128.0f);
+                z1 = has_zero ? zp & 0xFFFF0000u : __float_as_uint(128.0f);
               }
 #pragma unroll
               for (int h = 0; h < 2; ++h) {
@@ -385,8 +387,8 @@ __global__ void __launch_bounds__(CPW == 1 ? 512 : 256, CPW == 1 ? 1 : 2) wq_gem
                     a[2 * j] = deq8_zero(byte_pair(pairs, 0), s0, z0);
                     a[2 * j + 1] = deq8_zero(byte_pair(pairs, 1), s1, z1);
                   } else {
-                    a[2 * j] = deq8_any(we, wo, 2 * th, s0, z0);
-                    a[2 * j + 1] = deq8_any(we, wo, 2 * th + 1, s1, z1);
+                    a[2 * j] = deq8_any(we, wo, 2 * th, __uint_as_float(z0), __uint_as_float(s0));
+                    a[2 * j + 1] = deq8_any(we, wo, 2 * th + 1, __uint_as_float(z1), __uint_as_float(s1));
                   }
                 }
 #pragma unroll

@@ -41,3 +41,27 @@ def test_one_nonzero_activation_reads_back_the_exact_weight(m, n, why, zeros, d)
         y = d.w8a16(x, q, s, z, None, group)
         assert torch.equal(y[:have], want[k0:k0 + have]), why
         assert not y[have:].any()
+
+
+@pytest.mark.parametrize("k,n,group,m,why", [
+    (256, 2048, 128, 8, "eight by eight weights a thread; few-token kernel"),
+    (256, 33, 64, 8, "columns one by one; few-token kernel off the tiles"),
+    (144, 24, 48, 8, "CUDA cores"),
+    (1024, 6144, 1024, 96, "tcgen05 kernel"),
+])
+def test_zero_points_that_are_no_whole_numbers(k, n, group, m, why, d):
+    pool = torch.tensor((127.5, 16.25, -0.375, 0.01171875, 300.0, 128.0, float("inf")), device="cuda")
+    gen = torch.Generator(device="cuda").manual_seed(k)
+    q = torch.randint(0, 256, (k, n), dtype=torch.uint8, device="cuda", generator=gen)
+    rows = torch.arange(k // group, device="cuda")[:, None] + torch.arange(n, device="cuda")[None]
+    z = pool[rows % len(pool)].bfloat16()
+    s = (torch.rand(k // group, n, device="cuda", generator=gen) * 0.01 - 0.005).bfloat16()
+    full = lambda t: t.double().repeat_interleave(group, 0)
+    want = ((q.double() - full(z)) * full(s)).bfloat16()  # exact up to the rounding to bf16, as above
+    # (as bytes: a zero has its sign)
+    assert torch.equal(d.dequantize(q, s, z, group, 8).view(torch.int16), want.view(torch.int16)), why
+    x = torch.zeros(m, k, device="cuda", dtype=torch.bfloat16)
+    x[torch.arange(m), torch.arange(m) * (k // m)] = 1
+    y, row = d.w8a16(x, q, s, z, None, group), want[::k // m][:m]
+    finite = torch.isfinite(z).all(0)  # (an infinite weight times an activation of zero is no number)
+    assert torch.equal(y[:, finite], row[:, finite]), why
