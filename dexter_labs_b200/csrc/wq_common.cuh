@@ -94,7 +94,8 @@ __device__ __forceinline__ uint32_t mid_zero(uint32_t zero2) {  // from 128 + ze
 // q times 2^-133), q * scale - 8 * scale is exact up to the final rounding -- 8 * scale is a bf16, which
 // zero * scale in general is not -- so (q - 8) * scale needs no subtraction of its own.  2^133 * scale would
 // overflow, so the weights come out divided by 64, and so do the products and their fp32 sums, bit for
-// bit; whoever reads an accumulator multiplies by kSymAcc (exact down to 2^-120).  2^127 * scale still
+// bit; whoever reads an accumulator multiplies by kSymAcc.  (Weights below 2^-120 lose bits: divided, they are bf16
+// subnormals.  The quantiser's scales are 1e-8 and more.)  2^127 * scale still
 // overflows for |scale| >= 2, where sym4_any converts the long way (never with a model's weights, so the
 // check is one OR of exponents per unit: sym4_large).  Measured against deq4 / deq4_mid: 83 tokens 3072 x 14336
 // 10.9 -> 10.65 us, 14336 x 3072 12.4 -> 11.85, 16 tokens 9.25 -> 9.0; the check costs 0.25 us of it.
@@ -131,7 +132,9 @@ __device__ __forceinline__ float deq8(uint32_t word, uint32_t byte_sel, float ze
 //     rounding of the result is the only one, as in sym4_low;
 //   with zero points that are whole numbers from 0 to 255, which a quantiser's are: the difference is exact in
 //     that range and the multiply by 2^127 * scale is the only rounding.
-// Weights and sums are divided by kSymAcc as on int4's symmetric grid.  2.5 and 3.5 instructions per two
+// Weights and sums are divided by kSymAcc as on int4's symmetric grid, in deq8_any as well, with the same limit: weights
+// below 2^-120 lose bits (of all bytes and significands without zero points, none at a scale of 2^-120, 128 of
+// 32768 at 2^-121, 7128 at 2^-126).  2.5 and 3.5 instructions per two
 // weights, of which 1.5 are on the integer pipe.  Scales of 2 and more and other zero points take
 // deq8_any, in a body of its own: 9 instructions per two weights.  Measured, us with deq8_any / so: 83 tokens 3072 x
 // 14336 13.9 / 13.2, 14336 x 3072 15.2 / 14.2, with zero points 13.7 / 12.9; 16 tokens 3072 x 9216 10.4 / 9.5; one

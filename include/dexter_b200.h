@@ -21,6 +21,12 @@
  *            4-bit zero points are stored with +128 added (quant.py:118-122)
  *   bias     [N] bf16 or NULL
  *   out      [M, N]    bf16, row stride `ldo` elements (>= N)
+ *
+ * Arithmetic: a weight is (q - zero) * scale with one rounding, to bf16: the reference's bits wherever q - zero is a
+ * bf16, as with whole zero points from 0 to 255, which are the quantiser's.  Inside the GEMMs that holds for int4
+ * without zero points and for int8 where the weight is 0 or at least 2^-120 in magnitude; smaller ones keep
+ * fewer bits there (the quantiser's scales are 1e-8 and more).  Products are added up in fp32, the sum
+ * is rounded to bf16, and the bias, if any, is added to that and rounded again.
  */
 #ifndef DEXTER_B200_H_
 #define DEXTER_B200_H_

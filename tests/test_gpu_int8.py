@@ -43,6 +43,25 @@ def test_one_nonzero_activation_reads_back_the_exact_weight(m, n, why, zeros, d)
         assert not y[have:].any()
 
 
+@pytest.mark.parametrize("m,n,why", [(8, 2048, "few tokens"), (96, 6144, "whole tiles or clusters"), (160, 8192, "CTA pairs")])
+@pytest.mark.parametrize("zero", [None, 3.0, 16.25])
+def test_weights_are_exact_from_2_to_the_minus_120_on(m, n, why, zero, d):
+    # every byte and every significand of the scale, two binades higher where the difference can be a quarter
+    k, group = 256, 256
+    low = -120 if zero is None or zero % 1 == 0 else -118
+    q = torch.arange(256, dtype=torch.uint8, device="cuda")[:, None].repeat(1, n)
+    s = ((1 + torch.arange(n, device="cuda") % 128 / 128).double() * 2.0 ** low).bfloat16()[None]
+    z = None if zero is None else torch.full_like(s, zero)
+    want = ((q.double() - (128.0 if zero is None else zero)) * s.double()).bfloat16()
+    for k0 in range(0, k, m):
+        have = min(m, k - k0)
+        x = torch.zeros(m, k, device="cuda", dtype=torch.bfloat16)
+        x[torch.arange(have), k0 + torch.arange(have)] = 1
+        y = d.w8a16(x, q, s, z, None, group)
+        assert torch.equal(y[:have], want[k0:k0 + have]), why
+        assert not y[have:].any()
+
+
 @pytest.mark.parametrize("k,n,group,m,why", [
     (256, 2048, 128, 8, "eight by eight weights a thread; few-token kernel"),
     (256, 33, 64, 8, "columns one by one; few-token kernel off the tiles"),
