@@ -1755,13 +1755,17 @@ constexpr int kMaxPairSplit = 8;
 struct PairChoice {
   int blocks = 0, split = 1;
 };
-// The shortest of the
-// times below, all fitted to measurements on shapes between 160 x 3072 x 3072 and 913 x 13824 x 5120.
+// The shortest of the times below, all fitted to measurements on shapes between 160 x 3072 x 3072 and 913 x 13824 x
+// 5120, before int8's conversion became shorter and before the activation function went beside the next tile's products.
 // What they trade: a pair's unit takes as long as the MMA of its tokens (0.56 us at 256, 0.31 at
 // 128), converted once for all of them, but its accumulator of more than 128 tokens is not
 // double-buffered, so every further tile shows its epilogue; single CTAs convert a unit per 128
 // tokens (0.36 us int4, 0.42 int8); few tiles are split over clusters instead, at 7.5 us for the
 // exchange.  Which wins turns mostly on how full the last round of tiles is.
+// How good the choice is: with pairs wherever they can be, without, and as chosen, over 15 weights of 2 to 157 x 2^20
+// values, 10 token counts from 129 to 913 and both grids, it is within 4 % of the better at 269 of 300 points for int4
+// and 267 of 300 for int8.  Furthest off, us as chosen / the other way: int8 256 tokens 1024 x 2048 8.5 / 6.6, 129
+// 14336 x 3072 32.3 / 26.2, 768 1024 x 14336 29.5 / 24.1; int4 200 8192 x 20096 80.6 / 68.4, 160 14336 x 3072 24.5 / 22.0.
 static PairChoice choose_pairs(const Plan& pl, int M, int N, int K, int bits, int pairs, int budget, bool may_split) {
   const int least = (M + 255) / 256;  // a block has at most 256 tokens
   PairChoice choice;
@@ -1845,12 +1849,15 @@ static const CUtensorMap* activation_map(int bits, const void* x, long long ldx,
 }
 
 // Streaming past, weights push activations, scales and results out of L2 before their next use, unless they are
-// told to go first.  That costs where a weight would have been there again at its next use, so it
-// depends on its size: from a quarter of the L2 on all of its lines go first, from an eighth on half of
-// them.  Measured, us with normal priority / half / all, three sets of weights in turn: FFN of 83 tokens 3072 x
-// 14336 int8 (44 MB a weight) 35.0 / 33.9 / 32.4, int4 (22 MB) 26.3 / 25.2 / 25.3; 125 tokens int8 3072 x 8192
-// (25 MB, three of them fit) 12.3 / 12.4 / 12.9; 8 tokens int4 3072 x 9216 (14 MB) 7.19 / 7.30 / -; eight of 83
-// tokens 3072 x 3072 int4 (4.7 MB) 6.45 / - / 6.6.  (Activations told to stay instead: half the gain, and they
+// told to go first.  That costs where a weight would have been there again at its next use.  Whether it would depends on
+// all that a program reads in between; the launch only knows one weight's size, so it goes by that: from a
+// quarter of the L2 on all of its lines go first, from an eighth on half of them, below that none.  The lines are set for
+// programs of few weights, which are those that lose: three sets in turn, us with normal priority / half / all: FFN of
+// 83 tokens 3072 x 14336 int8 (44 MB a weight) 35.0 / 33.9 / 32.4, int4 (22 MB) 26.3 / 25.2 / 25.3; 125 tokens int8 3072 x
+// 8192 (25 MB, three of them fit) 12.3 / 12.4 / 12.9; 8 tokens int4 3072 x 9216 (14 MB) 7.19 / 7.30 / -; eight of 83
+// tokens 3072 x 3072 int4 (4.7 MB) 6.45 / - / 6.6.  Where a model's weights exceed the L2 by far, none of them is ever there
+// again, and all lines first would be the better: two int4 blocks of width 3072, 125.7 us with
+// this rule, 123.3 so.  Nobody tells the launch.  (Activations told to stay instead: half the gain, and they
 // would stay after their use.  A prefetch of the activations into L2: a tenth of it.)
 static uint64_t weight_policy(long long bytes, bool read_once) {
   const long long l2 = device_info().l2_bytes;
@@ -2330,15 +2337,17 @@ static int read_opts(const dxb_gemm_opts* o, int bits, int M, int N, int K, Opts
 // Few tokens and a weight that is read in little more than the fixed cost of a launch: there the kernel
 // without set-up is ahead; with more to convert (once per 16 tokens, there) the tcgen05 pipeline is.
 // The lines lie where the two crossed over 14 weights of 0.5 to 44 x 2^20 values and 18 token counts from 1 to 256, with
-// both kernels on all of them.  Near the lines, us small / tcgen05: int4 1 token 3072 x
-// 9216 6.4 / 7.2 and 3072 x 11264 8.3 / 8.3, 8 tokens 4096 x 4096 5.4 / 6.1 and 3072 x 6144 6.4 / 6.1, 16 tokens 3072 x
-// 3072 4.9 / 5.3 and 4096 x 4096 6.3 / 6.1, 32 tokens 2048 x 2048 4.2 / 4.6 and 2048 x 3072 5.7 / 5.1, 96 tokens
-// 1024 x 1024 3.9 / 5.1 and 1024 x 2048 6.0 / 5.4, 128 tokens 1024 x 2048 6.1 / 7.0 and 2048 x 2048 8.9 / 7.5 (from 97
-// tokens on the pipeline's clusters have their receive buffers over the rings, two more us), 160 tokens 512 x 1024
-// 4.6 / 4.5; int8 8 tokens 3072 x 3072 6.1 / 6.4 and 4096 x 4096 7.9 / 7.8, 16 tokens 2048 x 2048 4.9 / 5.0 and 3072 x
-// 3072 6.9 / 6.4, 80 tokens 1024 x 1024 5.0 / 4.9, 128 tokens 5.4 / 6.8 and 1024 x 2048 8.1 / 7.4.  The choice is
-// within 4 % of the better kernel at 733 of the 756 points and 14 % off at worst (up to 4 tokens 5120 x 5120: 160
-// tiles, so CTAs of eight warps, of which a second one fits an SM but most SMs get one).
+// both kernels on all of them (int8's before its conversion became shorter).  Near the lines, us small / tcgen05 on the
+// symmetric grids: int4 1 token 3072 x 9216 6.6 / 7.2 and 3072 x 11264 8.7 / 8.6, 8 tokens 4096 x 4096 5.5 / 6.2 and 3072 x
+// 6144 6.4 / 6.3, 16 tokens 3072 x 3072 5.1 / 5.4 and 4096 x 4096 6.6 / 6.2, 32 tokens 2048 x 2048 4.3 / 4.7 and 2048 x 3072
+// 5.9 / 5.1, 96 tokens 1024 x 1024 4.1 / 5.1 and 1024 x 2048 6.2 / 5.5, 128 tokens 1024 x 2048 6.3 / 7.0 and 2048 x 2048 9.1 /
+// 7.6 (from 97 tokens on the pipeline's clusters have their receive buffers over the rings, two more us), 160 tokens
+// 512 x 1024 4.8 / 4.8; int8 8 tokens 3072 x 3072 5.6 / 5.9 and 4096 x 4096 7.2 / 7.1, 16 tokens 2048 x 2048 4.7 / 4.7 and
+// 3072 x 3072 6.2 / 6.0, 80 tokens 1024 x 1024 4.6 / 4.8, 128 tokens 5.0 / 6.7 and 1024 x 2048 7.4 / 7.3.  With zero points
+// as well, the choice is within 4 % of the better kernel at 981 of the 1008 points (int4 493 of 504, int8 488) and
+// 14 % off at worst: up to 4 tokens 5120 x 5120 int4 (160 tiles, so CTAs of eight warps, of which a second one
+// fits an SM but most SMs get one); int8 5 to 10 % at 12 and 16 tokens 2048 x 3072 and up to 8 tokens 3072 x 4096, 13 % at
+// 96 tokens 1024 x 1024, where the line is a little low.
 static bool small_is_faster(int M, int N, int K, int bits) {
   const long long weights = static_cast<long long>(N) * K, mega = 1 << 20;
   if (M <= 8) return weights <= (bits == 8 ? 10 : M <= 4 ? 30 : 16) * mega;
