@@ -135,10 +135,11 @@ __device__ __forceinline__ float deq8(uint32_t word, uint32_t byte_sel, float ze
 // Weights and sums are divided by kSymAcc as on int4's symmetric grid, in deq8_any as well, with the same limit: weights
 // below 2^-120 lose bits (of all bytes and significands without zero points, none at a scale of 2^-120, 128 of
 // 32768 at 2^-121, 7128 at 2^-126).  2.5 and 3.5 instructions per two
-// weights, of which 1.5 are on the integer pipe.  Scales of 2 and more and other zero points take
-// deq8_any, in a body of its own: 9 instructions per two weights.  Measured, us with deq8_any / so: 83 tokens 3072 x
-// 14336 13.9 / 13.2, 14336 x 3072 15.2 / 14.2, with zero points 13.7 / 12.9; 16 tokens 3072 x 9216 10.4 / 9.5; one
-// token 3072 x 3072 6.1 / 5.4.  (125 tokens 3072 x 8192 on clusters of two: 12.7 either way.)
+// weights, of which 1.5 are on the integer pipe.  Scales of 2 and more take deq8_sym_any, or with zero points, as do other
+// zero points, deq8_any, in bodies of their own: 3.5 and 9 instructions per two weights.  Measured, us with a
+// conversion of 5 instructions through fp32 / so: 83 tokens 3072 x 14336 13.9 / 13.2, 14336 x 3072 15.2 / 14.2, with zero
+// points 13.7 / 12.9; 16 tokens 3072 x 9216 10.4 / 9.5; one token 3072 x 3072 6.1 / 5.4.  (125 tokens 3072 x 8192 on
+// clusters of two: 12.7 either way.)
 __device__ __forceinline__ uint32_t byte_pairs(uint32_t w0, uint32_t w1, bool high) {  // columns 0, 1 or 2, 3 of two rows
   return prmt(w0, w1, high ? 0x7632u : 0x5410u);
 }
@@ -160,6 +161,12 @@ __device__ __forceinline__ uint32_t deq8_zeros(uint32_t z2, uint32_t& odd) {
   const uint32_t r = mul_bf16x2(z2, 0x00010001u);  // times 2^-133: exact for those, and back below
   odd |= (r & 0xFF00FF00u) | (mul_bf16x2(r, 0x7F007F00u) ^ mul_bf16x2(z2, 0x3C803C80u));
   return r;
+}
+// Without zero points, any scale: the difference is a bf16, so it goes to bf16 (divided by kSymAcc) and is multiplied there.
+__device__ __forceinline__ uint32_t deq8_sym_any(uint32_t pair, uint32_t scale) {
+  uint32_t d;
+  asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(pair), "r"(0x7F007F00u), "r"(0xC000C000u));  // q / 64 - 2
+  return mul_bf16x2(d, scale);
 }
 // Any scale and zero point.  Byte `b` of two words (consecutive k of one column) -> a bf16 pair; `scale` is divided by
 // kSymAcc.

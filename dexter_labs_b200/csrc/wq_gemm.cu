@@ -950,8 +950,8 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         __syncwarp();  // every lane has its words in registers
         if (lane == 0) mbar_arrive(bar0 + 8 * (kBarEmptyW + s));
       }
-      // This unit's scales and zero points as the conversion wants them (int4: in both halves of a
-      // word; int8: the same, or in fp32 for deq8_any); then the next unit's rows.
+      // This unit's scales and zero points as the conversion wants them (in both halves of a word; in
+      // fp32 for deq8_any); then the next unit's rows.
       uint32_t s2[PLANES][4], z2[PLANES][4];
       // Constants outside the short conversions' range (never a model's): bodies of their own, so that the usual one is
       // scheduled as if they did not exist (a branch in front of each store made launches 6 % longer).
@@ -991,14 +991,20 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
           }
         } else {
           const uint32_t sx[2] = {sc[pl].x, sc[pl].y};
-          if (large) {
-            const uint32_t zx[2] = {HAS_ZERO ? zr[pl].x : 0x43004300u, HAS_ZERO ? zr[pl].y : 0x43004300u};  // 128
+          if (large && HAS_ZERO) {
+            const uint32_t zx[2] = {zr[pl].x, zr[pl].y};
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
               s2[pl][2 * i] = __float_as_uint(bf16lo_f32(sx[i]) / kSymAcc);
               s2[pl][2 * i + 1] = __float_as_uint(bf16hi_f32(sx[i]) / kSymAcc);
               z2[pl][2 * i] = zx[i] << 16;
               z2[pl][2 * i + 1] = zx[i] & 0xFFFF0000u;
+            }
+          } else if (large) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              s2[pl][2 * i] = dup_lo(sx[i]); s2[pl][2 * i + 1] = dup_hi(sx[i]);
+              z2[pl][2 * i] = z2[pl][2 * i + 1] = 0u;
             }
           } else {
 #pragma unroll
@@ -1125,7 +1131,8 @@ wq_gemm_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
 #pragma unroll
                   for (int o = 0; o < 2; ++o) {
                     const int i = 2 * h + o;
-                    r[h][2 * sl + o] = ANY ? deq8_any(x0, x1, i, __uint_as_float(z2[pl][i]), __uint_as_float(s2[pl][i]))
+                    r[h][2 * sl + o] = ANY && HAS_ZERO ? deq8_any(x0, x1, i, __uint_as_float(z2[pl][i]), __uint_as_float(s2[pl][i]))
+                                       : ANY ? deq8_sym_any(byte_pair(pairs, o), s2[pl][i])
                                        : HAS_ZERO ? deq8_zero(byte_pair(pairs, o), s2[pl][i], z2[pl][i])
                                                   : deq8_sym(byte_pair(pairs, o), s2[pl][i], z2[pl][i]);
                   }
